@@ -339,7 +339,7 @@ static int with_condition(hx_ccsd *h, int ph, F body)
 // that phase's mask (every launch skips the molecules that are not its own).
 static int run_group(hx_ccsd *h, Group &g)
 {
-    if (g.tiles == 0) return HX_OK;
+    if (g.tiles.count == 0) return HX_OK;
     if (h->tce) {
         int n[PH_COUNT] = {};
         for (int mi = 0; mi < h->nmol; ++mi)

@@ -2,9 +2,8 @@
 #pragma once
 #include "hx_plan.h"
 
-long long hx_tgemm_f64_prepare(TgemmDesc *descs, int n);
-cudaError_t hx_tgemm_f64_launch(const TgemmDesc *d_descs, int n, long long total_tiles,
-                                const int *d_active, cudaStream_t s);
+F64Tiles hx_tgemm_f64_prepare(TgemmDesc *descs, int n);
+cudaError_t hx_tgemm_f64_launch(const TgemmDesc *d_descs, int n, F64Tiles tiles, const int *d_active, cudaStream_t s);
 
 cudaError_t hx_scf_launch(const ScfMol *d_mols, int nmol, int nmax, const ScfParams &p, double *d_gpart,
                           cudaStream_t s);

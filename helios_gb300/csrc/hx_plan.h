@@ -69,11 +69,17 @@ struct DiisMol {
     long long L;
 };
 
+// Launch shape of a group on the FP64 CUDA-core GEMM: tiles over all its problems, size x size outputs each.
+struct F64Tiles {
+    long long count = 0;
+    int size = 16;
+};
+
 // One grouped tensor-GEMM launch of the plan (descriptors on host and device).
 struct Group {
     std::vector<TgemmDesc> h;
     TgemmDesc *d = nullptr;
-    long long tiles = 0;
+    F64Tiles tiles;
 };
 
 // ---------------------------------------------------------------- schedules

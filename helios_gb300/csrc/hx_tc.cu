@@ -1304,7 +1304,7 @@ static int build_sub(Engine *e, int mode, int var, const Group &g, SubGroup &sg)
 static cudaError_t run_sub(Engine *e, SubGroup &sg, int mode, const int *d_active, cudaStream_t s)
 {
     const Variant &V = variant_of(mode, sg.var);
-    if (sg.fp64.tiles > 0) {
+    if (sg.fp64.tiles.count > 0) {
         cudaError_t r = hx_tgemm_f64_launch(sg.fp64.d, (int)sg.fp64.h.size(), sg.fp64.tiles, d_active, s);
         if (r != cudaSuccess) return r;
     }
