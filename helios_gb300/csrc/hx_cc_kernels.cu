@@ -624,6 +624,54 @@ __global__ void __launch_bounds__(NT) k_energy_finish(const CCMol *__restrict__ 
     m.res[5] = x[1];
 }
 
+// ---------------------------------------------------------------- amplitude layouts
+// Between the reference's t1(o, v), t2(o, o, v, v) (column-major; a staging
+// copy on the device) and the engine's t1 [i][a], t2 [i][a][j][b]: for fixed
+// (j, a) an o x v transpose between i (contiguous in the column-major array)
+// and b (contiguous in the pair layout), in 32 x 32 tiles through shared
+// memory, so that both sides are read and written along their contiguous
+// dimension. HBM bound: 32 bytes per element moved, 0.05 ms for 56^4 elements
+// where the host's transpose took 20 ms. Block 0 also transposes t1.
+constexpr int LT = 32;
+template <bool TO_ENGINE>
+__global__ void __launch_bounds__(256) k_layout(double *__restrict__ t1, double *__restrict__ t2,
+                                                double *__restrict__ f1, double *__restrict__ f2, int o, int v)
+{
+    __shared__ double s[LT][LT + 1];
+    const int ti = (o + LT - 1) / LT, tb = (v + LT - 1) / LT;
+    unsigned x = blockIdx.x;
+    const int b0 = (int)(x % tb) * LT;
+    x /= tb;
+    const int i0 = (int)(x % ti) * LT;
+    x /= ti;
+    const int j = (int)(x % o), a = (int)(x / o);
+    const long long ov = (long long)o * v, vov = v * ov, oo = (long long)o * o, oov = oo * v;
+    double *__restrict__ e = t2 + a * ov + (long long)j * v;                 // [i][.][.][b]
+    double *__restrict__ f = f2 + (long long)j * o + a * oo;                 // (i, ., ., b)
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r = ty; r < LT; r += 8) {
+        if (TO_ENGINE) {
+            if (b0 + r < v && i0 + tx < o) s[tx][r] = f[i0 + tx + (b0 + r) * oov];
+        } else {
+            if (i0 + r < o && b0 + tx < v) s[r][tx] = e[(i0 + r) * vov + b0 + tx];
+        }
+    }
+    __syncthreads();
+    for (int r = ty; r < LT; r += 8) {
+        if (TO_ENGINE) {
+            if (i0 + r < o && b0 + tx < v) e[(i0 + r) * vov + b0 + tx] = s[r][tx];
+        } else {
+            if (b0 + r < v && i0 + tx < o) f[i0 + tx + (b0 + r) * oov] = s[tx][r];
+        }
+    }
+    if (blockIdx.x == 0)
+        for (int k = threadIdx.x; k < o * v; k += 256) {
+            const int p = k / v + o * (k % v);
+            if (TO_ENGINE) t1[k] = f1[p];
+            else f1[p] = t1[k];
+        }
+}
+
 // ---------------------------------------------------------------- set-up
 // Constants after SCF: denominators, ZDO vectors of the undressed ov space,
 // and the reference guess (guessCC r-ccsd, mod_cc.f90:634-650) when asked.
@@ -707,6 +755,15 @@ cudaError_t hx_ew_setup(const CCMol *m, const int *act, const HxSched &S, cudaSt
 { LAUNCH_EW(k_setup, SK_SETUP); return cudaSuccess; }
 cudaError_t hx_ew_setup2(const CCMol *m, const int *act, const HxSched &S, int guess, cudaStream_t s)
 { LAUNCH_EW(k_setup2, SK_PAIR, guess); return cudaSuccess; }
+
+cudaError_t hx_layout(double *t1, double *t2, double *f1, double *f2, int o, int v, bool to_engine, cudaStream_t s)
+{
+    const unsigned g = (unsigned)o * v * ((o + LT - 1) / LT) * ((v + LT - 1) / LT);
+    if (to_engine) k_layout<true><<<g, 256, 0, s>>>(t1, t2, f1, f2, o, v);
+    else k_layout<false><<<g, 256, 0, s>>>(t1, t2, f1, f2, o, v);
+    hx_count_launches(1);
+    return cudaGetLastError();
+}
 
 // dynamic shared memory of the pair-unit kernels (bytes): the largest over the batch
 size_t hx_unit_smem(const int *o, const int *v, int nmol, int kernel)

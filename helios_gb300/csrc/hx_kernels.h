@@ -26,6 +26,10 @@ cudaError_t hx_tail(const CCMol *m, const DiisMol *h, const int *act, const HxSc
 cudaError_t hx_energy(const CCMol *m, const DiisMol *h, const int *act, const HxSched &S, size_t smem, double *part,
                       cudaStream_t s);
 
+// amplitudes between the engine's layout (t1, t2) and the reference's column-major
+// arrays on the device (f1: o*v, f2: (o*v)^2 doubles)
+cudaError_t hx_layout(double *t1, double *t2, double *f1, double *f2, int o, int v, bool to_engine, cudaStream_t s);
+
 // (T) triples (hx_triples.cu): ZDO pair products of the occupied and virtual
 // orbitals; the energy partials of a slab of triples (i, j, k) for one i, the
 // pairs (j, k) listed in `pairs`, and their ordered sum (out[0] = E[4],

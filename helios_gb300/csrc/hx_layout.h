@@ -1,5 +1,6 @@
-// Host-side conversions between the reference's amplitude arrays and the
-// engine's. The reference (and its Fortran caller) holds t1(o, v) and
+// The amplitude layouts on the host: conversions between the reference's arrays
+// and the engine's, the plain statement of what k_layout (hx_cc_kernels.cu)
+// does on the device for the C ABI's transfers. The reference (and its Fortran caller) holds t1(o, v) and
 // t2(o, o, v, v) column-major (mod_cc.f90:2727 allocates t1(Nocc, Nocc+1:N)
 // and t2(Nocc, Nocc, Nocc+1:N, Nocc+1:N)); the engine keeps t1 row-major [i][a]
 // and t2 in pair order [i][a][j][b]. For each (a, j) the t2 conversion is an
