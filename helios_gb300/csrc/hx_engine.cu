@@ -609,7 +609,7 @@ static int allocate(hx_ccsd *h)
         HX_CU(hx_unit_kernels_init(mx));
     }
     HX_CU(cudaMalloc(&h->d_part, sizeof(double) * std::max<size_t>((size_t)h->sched.blocks[SK_UP] * HX_PART_STRIDE,
-                                                                   2 * HX_SCF_GRID_MAX)));
+                                                                   (size_t)HX_SCF_PART * h->nmol)));
     HX_CU(cudaMalloc(&h->d_act_ph[0], sizeof(int) * PH_COUNT * h->nmol));
     for (int ph = 1; ph < PH_COUNT; ++ph) h->d_act_ph[ph] = h->d_act_ph[0] + (size_t)ph * h->nmol;
     HX_CU(cudaMalloc(&h->d_ctl, sizeof(CtlMol) * h->nmol));

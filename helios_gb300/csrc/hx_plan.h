@@ -3,7 +3,8 @@
 #include <vector>
 #include "hx_common.cuh"
 
-#define HX_SCF_GRID_MAX 152    // CTAs of the cooperative SCF (global partials are sized for it)
+#define HX_SCF_GRID_MAX 152    // CTAs of an SCF launch whose clusters all run at once, one CTA per SM
+#define HX_SCF_PART 64         // doubles of global partials per molecule (4 x cluster size)
 #define HX_MAX_DIIS 50         // largest coupled-cluster:diis-steps (definebd.f90: range 2..50)
 
 struct ScfParams {

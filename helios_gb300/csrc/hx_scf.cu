@@ -15,10 +15,26 @@
 // accumulates the rotations into V. Eigenpairs are then sorted ascending, as
 // the reference's tred4 returns them (src/modules/mod_math.f90:31-230).
 //
-// The SCF body is written once over an execution context: a batch runs one
-// CTA per molecule (BlockCtx, barriers are __syncthreads); a single large
-// molecule runs on a cooperative grid (GridCtx, barriers are grid syncs) so
-// that every Jacobi round and every N^3 product is spread over many SMs.
+// What bounds it: GB300's FP64 pipe (two multiply-adds per clock and SM) and
+// the barrier of every Jacobi round. So
+//  * a molecule is shared by a cluster of CTAs (16 or 8 SMs' FP64 pipes, the
+//    cluster barrier instead of a grid-wide one); at most kBlockN sites run in
+//    one CTA with every matrix in shared memory;
+//  * a round is one pass: the rotated matrix is written to a second buffer, as
+//    2 x 2 blocks J_k^T A J_l of its upper triangle, so a round has one barrier
+//    and every CTA derives the next round's rotations from the finished matrix;
+//  * the rotation angle is taken in FP32 (a tangent within 1e-6 of the exact
+//    one leaves an off-diagonal 1e-6 of its size, which the quadratic
+//    convergence absorbs); its cosine is brought to FP64 by one third-order
+//    Newton step on 1/sqrt(1 + t^2), so the rotation is orthogonal to FP64;
+//  * pairs far below the convergence threshold are not rotated.
+// Measured on whole calls, one CTA (a cooperative grid for one molecule above
+// 64 sites) with three barriers a round before: a 38-site energy 88 -> 75 ms,
+// 63 sites 182 -> 143 ms, 160 sites 1672 -> 1591 ms, a batch of 128 molecules
+// of 8-64 sites 1077 -> 984 ms.
+//
+// The SCF body is written once over an execution context (BlockCtx, one CTA;
+// ClusterCtx, a thread-block cluster).
 #include <algorithm>
 #include <cooperative_groups.h>
 #include "hx_common.cuh"
@@ -26,59 +42,66 @@
 
 namespace {
 namespace cg = cooperative_groups;
-constexpr int NT = 512;
+constexpr int NT = 256;
+constexpr int kBlockN = 24;      // largest molecule of the one-CTA, shared-memory form
 
 // ---- execution contexts -------------------------------------------------
-struct BlockCtx {
-    int tid, nt;
-    double *sh;          // >= 33 doubles of shared scratch
-    __device__ BlockCtx(double *s) : tid(threadIdx.x), nt(blockDim.x), sh(s) {}
-    __device__ void sync() { __syncthreads(); }
-    __device__ double reduce(double v, bool mx)
-    {
-        for (int o = 16; o > 0; o >>= 1) {
-            double w = __shfl_xor_sync(0xffffffffu, v, o);
-            v = mx ? fmax(v, w) : v + w;
-        }
-        int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        __syncthreads();
-        if (lane == 0) sh[wid] = v;
-        __syncthreads();
-        if (wid == 0) {
-            v = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) {
-                double w = __shfl_xor_sync(0xffffffffu, v, o);
-                v = mx ? fmax(v, w) : v + w;
-            }
-            if (lane == 0) sh[32] = v;
-        }
-        __syncthreads();
-        double r = sh[32];
-        __syncthreads();
-        return r;
+// two sums (or one maximum in a) over the CTA, valid in every thread
+__device__ __forceinline__ void block_reduce(double &a, double &b, bool mx, double *sh)
+{
+    for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_xor_sync(0xffffffffu, a, o), y = __shfl_xor_sync(0xffffffffu, b, o);
+        a = mx ? fmax(a, x) : a + x;
+        b += y;
     }
+    const int wid = threadIdx.x >> 5;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) { sh[wid] = a; sh[NT / 32 + wid] = b; }
+    __syncthreads();
+    a = sh[0];
+    b = sh[NT / 32];
+    for (int w = 1; w < NT / 32; ++w) { a = mx ? fmax(a, sh[w]) : a + sh[w]; b += sh[NT / 32 + w]; }
+    __syncthreads();
+}
+
+struct BlockCtx {
+    int tid, nt, rank = 0, size = 1;
+    double *sh;          // 2 NT / 32 doubles of shared scratch
+    __device__ explicit BlockCtx(double *s) : tid(threadIdx.x), nt(NT), sh(s) {}
+    __device__ void sync() { __syncthreads(); }
+    __device__ void reduce2(double &a, double &b, bool mx) { block_reduce(a, b, mx, sh); }
+    __device__ static double ld(const double *p) { return *p; }
 };
 
-struct GridCtx {
-    int tid, nt;
+struct ClusterCtx {
+    int tid, nt, rank, size;
     double *sh;          // shared scratch of this CTA
-    double *gpart;       // 2 x gridDim.x global partials
-    int parity;
-    __device__ GridCtx(double *s, double *gp)
-        : tid(blockIdx.x * blockDim.x + threadIdx.x), nt(gridDim.x * blockDim.x), sh(s), gpart(gp), parity(0) {}
-    __device__ void sync() { cg::this_grid().sync(); }
-    __device__ double reduce(double v, bool mx)
+    double *gpart;       // 4 x cluster size global partials of this cluster
+    int parity = 0;
+    __device__ ClusterCtx(double *s, double *gp)
+        : rank((int)cg::this_cluster().block_rank()), size((int)cg::this_cluster().num_blocks()), sh(s), gpart(gp)
     {
-        BlockCtx b(sh);
-        v = b.reduce(v, mx);
-        double *p = gpart + parity * gridDim.x;
-        parity ^= 1;
-        if (threadIdx.x == 0) p[blockIdx.x] = v;
-        sync();
-        double r = mx ? 0.0 : 0.0;
-        for (unsigned k = 0; k < gridDim.x; ++k) r = mx ? fmax(r, p[k]) : r + p[k];
-        return r;   // the same ordered sum in every thread
+        tid = rank * NT + threadIdx.x;
+        nt = size * NT;
     }
+    __device__ void sync() { cg::this_cluster().sync(); }
+    __device__ void reduce2(double &a, double &b, bool mx)
+    {
+        block_reduce(a, b, mx, sh);
+        double *p = gpart + parity * 2 * size;          // two sets: the next reduction writes the other one
+        parity ^= 1;
+        if (threadIdx.x == 0) { __stcg(p + 2 * rank, a); __stcg(p + 2 * rank + 1, b); }
+        sync();
+        a = __ldcg(p);
+        b = __ldcg(p + 1);
+        for (int k = 1; k < size; ++k) {                // the same ordered sums in every thread
+            const double x = __ldcg(p + 2 * k), y = __ldcg(p + 2 * k + 1);
+            a = mx ? fmax(a, x) : a + x;
+            b += y;
+        }
+    }
+    // matrices another CTA of the cluster wrote are read from L2
+    __device__ static double ld(const double *p) { return __ldcg(p); }
 };
 
 // C = op(A) op(B) for N x N row-major matrices (ta/tb: use the transpose).
@@ -128,96 +151,142 @@ __device__ void density(Ctx &c, double *D, const double *V, int n, int nocc)
     c.sync();
 }
 
-// Jacobi eigen-decomposition of symmetric A (n x n, destroyed: its diagonal
-// ends as the eigenvalues); rotations accumulate into V. W is n x n scratch.
-// pp/pq/pc/ps are shared arrays of the CTA: every CTA derives the rotations
-// of a round itself from the same matrix entries, so a round needs only the
-// two barriers between its column and row passes.
-template <class Ctx>
-__device__ int jacobi(Ctx &c, double *A, double *V, double *E, double *W, int n, int *pp, int *pq, double *pc,
-                      double *ps)
+// Pair k of round r in the circle ordering of np = n + (n & 1) players: p < q;
+// q == n is the bye of an odd n.
+__device__ __forceinline__ void circle_pair(int k, int r, int np, int &p, int &q)
 {
-    const int np = n + (n & 1);
-    int sweeps = 0;
-    for (; sweeps < 40; ++sweeps) {
+    int x = k - 1 + r, y = np - 2 - k + r;
+    if (x >= np - 1) x -= np - 1;
+    if (y >= np - 1) y -= np - 1;
+    p = k == 0 ? 0 : 1 + x;
+    q = 1 + y;
+    if (p > q) { const int t = p; p = q; q = t; }
+}
+
+// Rotation (c, s) that annihilates apq to within FP32's precision of the
+// tangent; the identity when |apq| <= thr.
+__device__ __forceinline__ void rotation(double app, double aqq, double apq, double thr, double &c, double &s)
+{
+    c = 1.0;
+    s = 0.0;
+    if (!(fabs(apq) > thr)) return;
+    const float den = (float)(apq + apq);
+    if (den == 0.0f) return;
+    const float theta = (float)(aqq - app) / den;
+    const float m = fabsf(theta);
+    const float tf = m > 1e9f ? 0.5f / theta : copysignf(1.0f / (m + sqrtf(m * m + 1.0f)), theta);
+    const double t = (double)tf, x = fma(t, t, 1.0);
+    const double y = (double)rsqrtf((float)x);          // within 1e-6 of 1 / sqrt(x)
+    const double e = fma(-x * y, y, 1.0);               // 1 - x y^2
+    c = fma(y * e, fma(0.375, e, 0.5), y);              // y (1 + e / 2 + 3 e^2 / 8): the error is of order e^3
+    s = t * c;
+}
+
+// Jacobi eigen-decomposition of the symmetric n x n matrix in A (upper
+// triangle read; A and A2 are both overwritten); rotations accumulate into V.
+// W is n x n scratch. pc, ps, pd and rank_s are shared arrays of the CTA.
+template <class Ctx>
+__device__ void jacobi(Ctx &c, double *A, double *A2, double *V, double *E, double *W, int n, double *pc, double *ps,
+                       double *pd, int *rank_s)
+{
+    const int np = n + (n & 1), h = np / 2;
+    // items of a round: 2 x 2 blocks (k, l), k <= l, of the upper triangle (row
+    // k and row h - 1 - k folded into h + 1 items), and row pieces of V
+    const int nblk = ((h + 1) / 2) * (h + 1);
+    const int rows = (n + c.size - 1) / c.size, row0 = c.rank * rows, nrow = max(0, min(rows, n - row0));
+    double *cur = A, *nxt = A2;
+    for (int sweep = 0; sweep < 40; ++sweep) {
         double off = 0.0, tot = 0.0;
         for (int e = c.tid; e < n * n; e += c.nt) {
-            double a = A[e] * A[e];
-            tot += a;
-            if (e / n != e % n) off += a;
+            const int i = e / n, j = e - i * n;
+            if (i > j) continue;
+            const double x = c.ld(cur + e), a = x * x;
+            if (i == j) tot += a; else off += a;
         }
-        off = c.reduce(off, false);
-        tot = c.reduce(tot, false);
+        c.reduce2(off, tot, false);
+        off += off;
+        tot += off;
         if (off <= 1e-30 * tot || off < 1e-300) break;
+        // all pairs at thr would leave off at a quarter of its bound
+        const double thr = 0.5e-15 * sqrt(tot) / n;
         for (int r = 0; r < np - 1; ++r) {
-            for (int k = threadIdx.x; k < np / 2; k += blockDim.x) {
-                int x = k, y = np - 1 - k;
-                int p = (x == 0) ? 0 : 1 + (x - 1 + r) % (np - 1);
-                int q = 1 + (y - 1 + r) % (np - 1);
-                if (p > q) { int t = p; p = q; q = t; }
+            for (int k = threadIdx.x; k < h; k += NT) {
+                int p, q;
                 double cc = 1.0, s = 0.0;
-                if (q < n) {
-                    double apq = A[p * n + q];
-                    if (fabs(apq) > 1e-300) {
-                        double theta = (A[q * n + q] - A[p * n + p]) / (2.0 * apq);
-                        double t;
-                        if (fabs(theta) > 1e150) t = 0.5 / theta;
-                        else t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                        cc = 1.0 / sqrt(t * t + 1.0);
-                        s = t * cc;
-                    }
-                } else {
-                    p = -1;   // bye for odd n
+                circle_pair(k, r, np, p, q);
+                if (q < n) rotation(c.ld(cur + p * n + p), c.ld(cur + q * n + q), c.ld(cur + p * n + q), thr, cc, s);
+                pc[k] = cc;
+                ps[k] = s;
+            }
+            __syncthreads();
+            for (int e = c.tid; e < nblk; e += c.nt) {
+                const int k0 = e / (h + 1), d = e - k0 * (h + 1);
+                int k, l;
+                if (d < h - k0) { k = k0; l = k0 + d; }
+                else { k = h - 1 - k0; l = k + d - (h - k0); if (k == k0) continue; }
+                int p, q, u, v;
+                circle_pair(k, r, np, p, q);
+                circle_pair(l, r, np, u, v);
+                const bool hq = q < n, hv = v < n;                     // (both p and u exist)
+                const int i00 = p < u ? p * n + u : u * n + p, i01 = p < v ? p * n + v : v * n + p;
+                const int i10 = q < u ? q * n + u : u * n + q, i11 = q < v ? q * n + v : v * n + q;
+                const double a00 = c.ld(cur + i00), a01 = hv ? c.ld(cur + i01) : 0.0;
+                const double a10 = hq ? c.ld(cur + i10) : 0.0, a11 = hq && hv ? c.ld(cur + i11) : 0.0;
+                const double ck = pc[k], sk = ps[k], cl = pc[l], sl = ps[l];
+                double x00 = a00, x01 = a01, x10 = a10, x11 = a11;
+                if (sl != 0.0) {
+                    x00 = cl * a00 - sl * a01; x01 = sl * a00 + cl * a01;
+                    x10 = cl * a10 - sl * a11; x11 = sl * a10 + cl * a11;
                 }
-                pp[k] = p; pq[k] = q; pc[k] = cc; ps[k] = s;
+                if (sk != 0.0) {
+                    const double y00 = x00, y01 = x01;
+                    x00 = ck * y00 - sk * x10; x01 = ck * y01 - sk * x11;
+                    x10 = sk * y00 + ck * x10; x11 = sk * y01 + ck * x11;
+                }
+                nxt[i00] = x00;
+                if (hv) nxt[i01] = x01;
+                if (hq && k != l) nxt[i10] = x10;
+                if (hq && hv) nxt[i11] = x11;
             }
-            // every CTA has read the pair entries before any column is rotated
-            c.sync();
-            // columns of A and V: X <- X J
-            for (int e = c.tid; e < (np / 2) * n; e += c.nt) {
-                int k = e / n, row = e % n, p = pp[k], q = pq[k];
-                if (p < 0 || ps[k] == 0.0) continue;
-                double cs = pc[k], s = ps[k];
-                double akp = A[row * n + p], akq = A[row * n + q];
-                A[row * n + p] = cs * akp - s * akq;
-                A[row * n + q] = s * akp + cs * akq;
-                double vkp = V[row * n + p], vkq = V[row * n + q];
-                V[row * n + p] = cs * vkp - s * vkq;
-                V[row * n + q] = s * vkp + cs * vkq;
-            }
-            c.sync();
-            // rows of A: A <- J^T A
-            for (int e = c.tid; e < (np / 2) * n; e += c.nt) {
-                int k = e / n, col = e % n, p = pp[k], q = pq[k];
-                if (p < 0 || ps[k] == 0.0) continue;
-                double cs = pc[k], s = ps[k];
-                double apk = A[p * n + col], aqk = A[q * n + col];
-                A[p * n + col] = cs * apk - s * aqk;
-                A[q * n + col] = s * apk + cs * aqk;
+            // this CTA's rows of V: V <- V J
+            for (int e = threadIdx.x; e < nrow * h; e += NT) {
+                const int i = e / h, k = e - i * h;
+                const double s = ps[k];
+                if (s == 0.0) continue;                                // (a bye has s = 0)
+                const double cs = pc[k];
+                int p, q;
+                circle_pair(k, r, np, p, q);
+                double *row = V + (row0 + i) * n;
+                const double x = row[p], y = row[q];
+                row[p] = cs * x - s * y;
+                row[q] = s * x + cs * y;
             }
             c.sync();
+            double *t = cur; cur = nxt; nxt = t;
         }
     }
     // sort ascending: rank each eigenvalue, permute V's columns through W
-    for (int e = c.tid; e < n * n; e += c.nt) {
-        int row = e / n, p = e % n;
-        double ep = A[p * n + p];
+    for (int p = threadIdx.x; p < n; p += NT) pd[p] = c.ld(cur + p * n + p);
+    __syncthreads();
+    for (int p = threadIdx.x; p < n; p += NT) {
+        const double ep = pd[p];
         int rank = 0;
-        for (int q = 0; q < n; ++q) {
-            double eq = A[q * n + q];
-            rank += (eq < ep) || (eq == ep && q < p);
-        }
-        W[row * n + rank] = V[row * n + p];
-        if (row == 0) E[rank] = ep;
+        for (int q = 0; q < n; ++q) rank += (pd[q] < ep) || (pd[q] == ep && q < p);
+        rank_s[p] = rank;
+        if (c.rank == 0) E[rank] = ep;
     }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nrow * n; e += NT) {
+        const int row = row0 + e / n, p = e % n;
+        W[row * n + rank_s[p]] = V[row * n + p];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nrow * n; e += NT) V[row0 * n + e] = W[row0 * n + e];
     c.sync();
-    for (int e = c.tid; e < n * n; e += c.nt) V[e] = W[e];
-    c.sync();
-    return sweeps;
 }
 
 template <class Ctx>
-__device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, int *pp, int *pq, double *pc, double *ps)
+__device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, double *pc, double *ps, double *pd, int *rank_s)
 {
     const int n = m.N, no = m.nocc, nn = n * n;
     double *F = m.F, *D = m.D, *V = m.V, *A = m.A, *W1 = m.W1, *W2 = m.W2;
@@ -233,7 +302,7 @@ __device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, int *pp,
             V[e] = (e / n == e % n) ? 1.0 : 0.0;
         }
         c.sync();
-        jacobi(c, A, V, m.E, W1, n, pp, pq, pc, ps);
+        jacobi(c, A, W2, V, m.E, W1, n, pc, ps, pd, rank_s);
         density(c, D, V, n, no);
     }
     fock(c, F, m.core, m.G, D, n);
@@ -250,16 +319,16 @@ __device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, int *pp,
         for (int e = c.tid; e < nn; e += c.nt) A[e] = W1[e] - W1[(e % n) * n + e / n];
         c.sync();
         mm(c, W1, A, W2, n, false, false, n);           // Fmin
-        double acc = 0.0;
+        double acc = 0.0, unused = 0.0;
         for (int e = c.tid; e < nn; e += c.nt) acc = fmax(acc, fabs(W1[e]));
-        acc = c.reduce(acc, true);
+        c.reduce2(acc, unused, true);
         for (int e = c.tid; e < nn; e += c.nt) D[e] -= prm.step * W1[e];
         c.sync();
         fock(c, F, m.core, m.G, D, n);
         // diagonalise F in the current basis: A = V^T F V
         mm(c, W1, F, V, n, false, false, n);
         mm(c, A, V, W1, n, true, false, n);
-        jacobi(c, A, V, m.E, W1, n, pp, pq, pc, ps);
+        jacobi(c, A, W2, V, m.E, W1, n, pc, ps, pd, rank_s);
         density(c, D, V, n, no);
         fock(c, F, m.core, m.G, D, n);
 
@@ -279,8 +348,7 @@ __device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, int *pp,
         eel += D[e] * (m.core[e] + F[e]);
         if (e / n < e % n) enuc += m.G[e];
     }
-    eel = c.reduce(eel, false);
-    enuc = c.reduce(enuc, false);
+    c.reduce2(eel, enuc, false);
     if (c.tid == 0) {
         m.out[0] = eel + enuc;
         m.out[1] = eel;
@@ -294,50 +362,59 @@ __device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, int *pp,
     mm(c, m.Fmo, V, W1, n, true, false, n);
 }
 
-__global__ void __launch_bounds__(NT) scf_kernel(const ScfMol *__restrict__ mols, ScfParams prm)
+// One cluster per molecule; at most kBlockN sites: its first CTA alone, in
+// shared memory.
+__global__ void __launch_bounds__(NT) scf_kernel(const ScfMol *__restrict__ mols, ScfParams prm, double *gpart)
 {
-    __shared__ double sh[40];
-    __shared__ int pp[HX_MAX_MOL_N / 2], pq[HX_MAX_MOL_N / 2];
-    __shared__ double pc[HX_MAX_MOL_N / 2], ps[HX_MAX_MOL_N / 2];
-    const ScfMol m = mols[blockIdx.x];
+    __shared__ double sh[2 * NT / 32];
+    __shared__ double pc[HX_MAX_MOL_N / 2], ps[HX_MAX_MOL_N / 2], pd[HX_MAX_MOL_N];
+    __shared__ int rank_s[HX_MAX_MOL_N];
+    __shared__ double mat[6][kBlockN * kBlockN];
+    const int cs = (int)cg::this_cluster().num_blocks(), mol = (int)blockIdx.x / cs;
+    ScfMol m = mols[mol];
+    if (m.N > kBlockN) {
+        ClusterCtx c(sh, gpart + (long long)mol * 4 * cs);
+        scf_body(c, m, prm, pc, ps, pd, rank_s);
+        return;
+    }
+    if (cg::this_cluster().block_rank() != 0) return;
     BlockCtx c(sh);
-    scf_body(c, m, prm, pp, pq, pc, ps);
-}
-
-__global__ void __launch_bounds__(256) scf_grid_kernel(const ScfMol *__restrict__ mols, ScfParams prm, double *gpart)
-{
-    __shared__ double sh[40];
-    __shared__ int pp[HX_MAX_MOL_N / 2], pq[HX_MAX_MOL_N / 2];
-    __shared__ double pc[HX_MAX_MOL_N / 2], ps[HX_MAX_MOL_N / 2];
-    const ScfMol m = mols[0];
-    GridCtx c(sh, gpart);
-    scf_body(c, m, prm, pp, pq, pc, ps);
+    const ScfMol g = m;
+    m.F = mat[0]; m.D = mat[1]; m.V = mat[2]; m.A = mat[3]; m.W1 = mat[4]; m.W2 = mat[5];
+    scf_body(c, m, prm, pc, ps, pd, rank_s);
+    __syncthreads();
+    for (int e = threadIdx.x; e < m.N * m.N; e += NT) { g.F[e] = m.F[e]; g.D[e] = m.D[e]; g.V[e] = m.V[e]; }
 }
 }  // namespace
 
-// One molecule of more than 64 sites runs on a cooperative grid (one CTA per
-// Jacobi pair, at most one per SM); batches run one CTA per molecule.
+// Cluster size: 16 CTAs (the non-portable size, where the device takes it)
+// while every molecule's cluster has its SMs to itself, else 8. Molecules of
+// at most kBlockN sites use one CTA of their cluster, so a launch of only
+// such molecules takes clusters of one.
 cudaError_t hx_scf_launch(const ScfMol *d_mols, int nmol, int nmax, const ScfParams &p, double *d_gpart,
                           cudaStream_t s)
 {
-    if (nmol == 1 && nmax > 64 && d_gpart) {
-        int dev = 0, nsm = 0, per_sm = 0, coop = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scf_grid_kernel, 256, 0);
-        int grid = std::min(nmax / 2, nsm * std::max(per_sm, 1));
-        grid = std::min(grid, HX_SCF_GRID_MAX);
-        if (coop && per_sm > 0 && grid >= 2) {
-            ScfParams pc = p;
-            const ScfMol *pm = d_mols;
-            double *gp = d_gpart;
-            void *args[] = {(void *)&pm, (void *)&pc, (void *)&gp};
-            hx_count_launches(1);
-            return cudaLaunchCooperativeKernel((void *)scf_grid_kernel, dim3(grid), dim3(256), args, 0, s);
+    int cs = nmax <= kBlockN ? 1 : (nmol * 16 <= HX_SCF_GRID_MAX ? 16 : 8);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.blockDim = dim3(NT);
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cs > 8) {
+        int n = 0;
+        at[0].val.clusterDim.x = cs;
+        cfg.gridDim = dim3((unsigned)cs);
+        if (cudaFuncSetAttribute(scf_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, scf_kernel, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            cs = 8;
         }
     }
-    scf_kernel<<<nmol, NT, 0, s>>>(d_mols, p);
+    at[0].val.clusterDim.x = cs;
+    cfg.gridDim = dim3((unsigned)nmol * cs);
     hx_count_launches(1);
-    return cudaGetLastError();
+    return cudaLaunchKernelEx(&cfg, scf_kernel, d_mols, p, d_gpart);
 }
