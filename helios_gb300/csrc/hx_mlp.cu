@@ -459,28 +459,26 @@ __global__ void __launch_bounds__(BG_THREADS, 1) bgemm(const __grid_constant__ C
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(H));
 }
 
-// bf16 copies of an FP32 [rows x cols] matrix (cols a multiple of 32): row-major
-// (dst) and transposed (dstT, [cols x rows]), through 32 x 32 shared tiles so
-// that both are written coalesced.
-__global__ void k_bf16_copies(const float *src, int rows, int cols, __nv_bfloat16 *dst, __nv_bfloat16 *dstT)
+// bf16 copies, row-major (dst) and transposed (dstT), of the two hidden weight
+// matrices W2 and W3 of the blob, through 32 x 32 shared tiles so that both
+// are written coalesced; block = one tile.
+__global__ void __launch_bounds__(256) k_weight_copies(const float *P, __nv_bfloat16 *W2, __nv_bfloat16 *W2T,
+                                                       __nv_bfloat16 *W3, __nv_bfloat16 *W3T)
 {
     __shared__ float t[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;          // 32 x 8 threads
-    const int ct = cols / 32, tiles = ((rows + 31) / 32) * ct;
-    for (int u = blockIdx.x; u < tiles; u += gridDim.x) {
-        const int r0 = (u / ct) * 32, c0 = (u % ct) * 32;
-        for (int y = ty; y < 32; y += 8) {
-            const int r = r0 + y;
-            const float v = r < rows ? src[(long long)r * cols + c0 + tx] : 0.f;
-            t[y][tx] = v;
-            if (dst && r < rows) dst[(long long)r * cols + c0 + tx] = __float2bfloat16_rn(v);
-        }
-        __syncthreads();
-        if (dstT)
-            for (int y = ty; y < 32; y += 8)
-                if (r0 + tx < rows) dstT[(long long)(c0 + y) * rows + r0 + tx] = __float2bfloat16_rn(t[tx][y]);
-        __syncthreads();
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, ct = H / 32;
+    const bool second = blockIdx.x >= ct * ct;
+    const int u = second ? blockIdx.x - ct * ct : blockIdx.x;
+    const float *src = P + (second ? O_W3 : O_W2);
+    __nv_bfloat16 *dst = second ? W3 : W2, *dstT = second ? W3T : W2T;
+    const int r0 = (u / ct) * 32, c0 = (u % ct) * 32;
+    for (int y = ty; y < 32; y += 8) {
+        const float v = src[(r0 + y) * H + c0 + tx];
+        t[y][tx] = v;
+        dst[(r0 + y) * H + c0 + tx] = __float2bfloat16_rn(v);
     }
+    __syncthreads();
+    for (int y = ty; y < 32; y += 8) dstT[(c0 + y) * H + r0 + tx] = __float2bfloat16_rn(t[tx][y]);
 }
 
 __global__ void k_to_bf16(const float *src, __nv_bfloat16 *dst, int n)
@@ -489,57 +487,6 @@ __global__ void k_to_bf16(const float *src, __nv_bfloat16 *dst, int n)
 }
 
 // ------------------------------------------------------------------ SIMT training kernels
-// C[M x N] = alpha * sum_k A(m,k) B(k,n) (+ bias[n]) + beta C, with
-// A(m,k) = A[m*ar + k*ac], B(k,n) = B[k*br + n*bc] (a stride of 0 broadcasts),
-// C row-major with leading dimension ldc; optional bf16 rounding of B.
-__global__ void __launch_bounds__(256) sgemm(int M, int N, int K, float alpha, const float *A, long long ar,
-                                              long long ac, const float *B, long long br, long long bc, float beta,
-                                              float *C, int ldc, const float *bias, int round_b)
-{
-    __shared__ float As[16][65], Bs[16][65];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int e = threadIdx.x; e < 64 * 16; e += 256) {
-            const int kk = e % 16, mm = e / 16;
-            const int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < K) ? A[m * ar + k * ac] : 0.f;
-            const int nn = e % 64, kb = e / 64;
-            const int n = n0 + nn, k2 = k0 + kb;
-            const float vb = (n < N && k2 < K) ? B[k2 * br + n * bc] : 0.f;
-            Bs[kb][nn] = round_b ? bf16r(vb) : vb;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[kk][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty + 16 * i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx + 16 * j;
-            if (n >= N) continue;
-            float r = alpha * acc[i][j] + (bias ? bias[n] : 0.f);
-            if (beta != 0.f) r += beta * C[(long long)m * ldc + n];
-            C[(long long)m * ldc + n] = r;
-        }
-    }
-}
-
 // x = (X[idx] - shift) * scale and t = T[idx] for the rows of one batch (idx NULL = identity)
 __global__ void k_gather_norm(const float *X, const float *T, const long long *idx, const float *P, float *x,
                               float *t, int n)
@@ -551,42 +498,160 @@ __global__ void k_gather_norm(const float *X, const float *T, const long long *i
         if (f == 0) t[r] = T[src];
     }
 }
-// h = silu(z), rounded to bf16 when it feeds a bf16 layer
-__global__ void k_silu(const float *z, float *h, long long n, int round)
+// The element-wise kernels between the products: a block takes TR rows of the
+// batch x all H columns, in TR x 32 column tiles (thread = (column, every
+// eighth row)), writes the bf16 operand of the next product in both orders
+// and adds its column sums (bias and output-weight gradients) to G, so every
+// activation is read once and no product is spent on a sum. The sums over
+// the batch as one-column products on the 64 x 64 SIMT tile took 0.2 ms each,
+// a step of 4096 rows 3.0 ms.
+constexpr int TR = 32;
+struct Tile {
+    float t[TR][33];
+    float red[8][32];
+};
+
+// bf16 copies of the staged tile (rows r0.., columns c0..): dst [rows x H], dstT [H x rows]
+__device__ __forceinline__ void store_tile(const Tile &s, int r0, int c0, int rows, __nv_bfloat16 *dst, __nv_bfloat16 *dstT)
 {
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const float s = silu(z[e]);
-        h[e] = round ? bf16r(s) : s;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int y = ty; y < TR; y += 8) dst[(long long)(r0 + y) * H + c0 + tx] = __float2bfloat16_rn(s.t[y][tx]);
+    for (int y = ty; y < 32; y += 8) dstT[(long long)(c0 + y) * rows + r0 + tx] = __float2bfloat16_rn(s.t[tx][y]);
+}
+// adds the block's sums of a column tile to out[c0 ..] (v: this thread's share of column tx)
+__device__ __forceinline__ void add_columns(Tile &s, float v, float *out)
+{
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    __syncthreads();
+    s.red[ty][tx] = v;
+    __syncthreads();
+    if (ty == 0) {
+        float a = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a += s.red[k][tx];
+        atomicAdd(out + tx, a);
     }
 }
-// residual in network units r = y + b4 - T / y_scale; dy = 2 r / M; loss += mean r^2
-__global__ void k_loss(const float *y, const float *T, const float *P, float *dy, float *loss, int n)
+
+// layer 1: z1 = x W1^T + b1, h1 = bf16(silu(z1))
+__global__ void __launch_bounds__(256) k_layer1(const float *x, const float *P, float *z1, __nv_bfloat16 *h, __nv_bfloat16 *hT, int rows)
 {
-    __shared__ float sh[256];
-    float acc = 0.f;
-    const float s = P[O_YS], b4 = P[O_B4];
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const float r = y[e] + b4 - T[e] / s;
-        dy[e] = 2.f * r / n;
-        acc += r * r;
+    __shared__ Tile s;
+    __shared__ float xs[TR][F];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * TR;
+    for (int e = threadIdx.x; e < TR * F; e += 256) xs[e / F][e % F] = x[(long long)r0 * F + e];
+    for (int c0 = 0; c0 < H; c0 += 32) {
+        const int c = c0 + tx;
+        float w[F];
+#pragma unroll
+        for (int f = 0; f < F; ++f) w[f] = P[O_W1 + c * F + f];
+        const float b = P[O_B1 + c];
+        __syncthreads();
+        for (int y = ty; y < TR; y += 8) {
+            float a = 0.f;
+#pragma unroll
+            for (int f = 0; f < F; ++f) a = fmaf(xs[y][f], w[f], a);
+            const float z = a + b;
+            z1[(long long)(r0 + y) * H + c] = z;
+            s.t[y][tx] = silu(z);
+        }
+        __syncthreads();
+        store_tile(s, r0, c0, rows, h, hT);
     }
-    sh[threadIdx.x] = acc;
+}
+// h = bf16(silu(z))
+__global__ void __launch_bounds__(256) k_act(const float *z, __nv_bfloat16 *h, __nv_bfloat16 *hT, int rows)
+{
+    __shared__ Tile s;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * TR;
+    for (int c0 = 0; c0 < H; c0 += 32) {
+        __syncthreads();
+        for (int y = ty; y < TR; y += 8) s.t[y][tx] = silu(z[(long long)(r0 + y) * H + c0 + tx]);
+        __syncthreads();
+        store_tile(s, r0, c0, rows, h, hT);
+    }
+}
+// output unit, loss and the gradient of z3: h3 = silu(z3), residual in network
+// units r = h3 w4 + b4 - T / y_scale, dy = 2 r / n (0 for the padded rows
+// >= n), loss += mean r^2, dz3 = dy w4 silu'(z3); dw4, db4, db3 added to G
+__global__ void __launch_bounds__(256) k_out(const float *z3, const float *T, const float *P, float *G, float *loss,
+                                             __nv_bfloat16 *dz, __nv_bfloat16 *dzT, int n, int rows)
+{
+    __shared__ Tile s;
+    __shared__ float dy[TR], rr[TR];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * TR;
+    const float *W4 = P + O_W4;
+    for (int y = ty; y < TR; y += 8) {
+        float a = 0.f;
+#pragma unroll
+        for (int c = 0; c < H; c += 32) a = fmaf(silu(z3[(long long)(r0 + y) * H + c + tx]), W4[c + tx], a);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (tx == 0) {
+            const bool live = r0 + y < n;
+            const float r = live ? a + P[O_B4] - T[r0 + y] / P[O_YS] : 0.f;
+            dy[y] = 2.f * r / n;
+            rr[y] = r * r;
+        }
+    }
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    if (ty == 0) {
+        float d = dy[tx], q = rr[tx];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) { d += __shfl_xor_sync(0xffffffffu, d, o); q += __shfl_xor_sync(0xffffffffu, q, o); }
+        if (tx == 0) { atomicAdd(G + O_B4, d); atomicAdd(loss, q / n); }
+    }
+    for (int c0 = 0; c0 < H; c0 += 32) {
+        float gw = 0.f, gb = 0.f;
+        for (int y = ty; y < TR; y += 8) {
+            const float z = z3[(long long)(r0 + y) * H + c0 + tx], g = dy[y] * W4[c0 + tx] * dsilu(z);
+            gw = fmaf(dy[y], silu(z), gw);
+            gb += g;
+            s.t[y][tx] = g;
+        }
+        add_columns(s, gw, G + O_W4 + c0);
+        add_columns(s, gb, G + O_B3 + c0);
+        store_tile(s, r0, c0, rows, dz, dzT);
         __syncthreads();
     }
-    if (threadIdx.x == 0) atomicAdd(loss, sh[0] / n);
 }
-// dz = dh * silu'(z), with dh[m][j] = dy[m] * w4[j] when w4 is given
-__global__ void k_dsilu(const float *dh, const float *dy, const float *w4, const float *z, float *dz, int M)
+// dz = dh silu'(z), its column sums added to db
+__global__ void __launch_bounds__(256) k_dact(const float *dh, const float *z, float *db, __nv_bfloat16 *dz, __nv_bfloat16 *dzT, int rows)
 {
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < (long long)M * H;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int m = (int)(e / H), j = (int)(e % H);
-        const float g = w4 ? dy[m] * w4[j] : dh[e];
-        dz[e] = g * dsilu(z[e]);
+    __shared__ Tile s;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * TR;
+    for (int c0 = 0; c0 < H; c0 += 32) {
+        float gb = 0.f;
+        for (int y = ty; y < TR; y += 8) {
+            const long long e = (long long)(r0 + y) * H + c0 + tx;
+            const float g = dh[e] * dsilu(z[e]);
+            gb += g;
+            s.t[y][tx] = g;
+        }
+        add_columns(s, gb, db + c0);
+        store_tile(s, r0, c0, rows, dz, dzT);
+        __syncthreads();
     }
+}
+// layer 1's gradients: dz1 = dh silu'(z1), db1 and dW1 = dz1^T x added to G; thread = column
+__global__ void __launch_bounds__(H) k_dlayer1(const float *dh, const float *z1, const float *x, float *G)
+{
+    __shared__ float xs[TR][F];
+    const int c = threadIdx.x, r0 = blockIdx.x * TR;
+    for (int e = threadIdx.x; e < TR * F; e += H) xs[e / F][e % F] = x[(long long)r0 * F + e];
+    __syncthreads();
+    float gb = 0.f, gw[F] = {};
+#pragma unroll 4
+    for (int y = 0; y < TR; ++y) {
+        const long long e = (long long)(r0 + y) * H + c;
+        const float g = dh[e] * dsilu(z1[e]);
+        gb += g;
+#pragma unroll
+        for (int f = 0; f < F; ++f) gw[f] = fmaf(g, xs[y][f], gw[f]);
+    }
+    atomicAdd(G + O_B1 + c, gb);
+#pragma unroll
+    for (int f = 0; f < F; ++f) atomicAdd(G + O_W1 + c * F + f, gw[f]);
 }
 // Adam on the trainable prefix of the blob
 __global__ void k_adam(float *P, const float *G, float *m1, float *m2, int n, float lr, float b1, float b2, float eps,
@@ -605,13 +670,6 @@ static inline unsigned nblocks(long long n, int t = 256)
 {
     long long b = (n + t - 1) / t;
     return (unsigned)std::max(1LL, std::min(b, 65535LL));
-}
-
-static void gemm(cudaStream_t s, int M, int N, int K, const float *A, long long ar, long long ac, const float *B,
-                 long long br, long long bc, float *C, int ldc, const float *bias = nullptr, int round_b = 0)
-{
-    dim3 g((N + 63) / 64, (M + 63) / 64);
-    sgemm<<<g, 256, 0, s>>>(M, N, K, 1.f, A, ar, ac, B, br, bc, 0.f, C, ldc, bias, round_b);
 }
 
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
@@ -647,9 +705,8 @@ static int map_bf16(CUtensorMap *map, const void *base, long long rows, int cols
 // the 128-row tile: the padded rows have zero inputs and zero loss gradient)
 struct Work {
     int M = 0, Mp = 0;
-    float *x = nullptr, *t = nullptr, *z1 = nullptr, *h1 = nullptr, *z2 = nullptr, *h2 = nullptr, *z3 = nullptr,
-          *h3 = nullptr, *y = nullptr, *dy = nullptr, *dz = nullptr, *dh = nullptr, *G = nullptr, *loss = nullptr,
-          *ones = nullptr;
+    float *x = nullptr, *t = nullptr, *z1 = nullptr, *z2 = nullptr, *z3 = nullptr, *dh = nullptr, *G = nullptr,
+          *loss = nullptr;
     // bf16 operands of the tensor-core GEMMs: activations and gradients (and
     // their transposes, [H x Mp]) and the two hidden weight matrices
     __nv_bfloat16 *h1b = nullptr, *h2b = nullptr, *h1T = nullptr, *h2T = nullptr, *dzb = nullptr, *dzT = nullptr,
@@ -661,7 +718,7 @@ struct Work {
         M = m;
         Mp = (m + TILE - 1) / TILE * TILE;
         const size_t act = (size_t)Mp * H * 4, actb = (size_t)Mp * H * 2, wb = (size_t)H * H * 2;
-        float **big[] = {&z1, &h1, &z2, &h2, &z3, &h3, &dz, &dh};
+        float **big[] = {&z1, &z2, &z3, &dh};
         for (float **b : big)
             if (cudaMalloc(b, act) != cudaSuccess) return HX_ERR_NOMEM;
         __nv_bfloat16 **bb[] = {&h1b, &h2b, &h1T, &h2T, &dzb, &dzT};
@@ -671,13 +728,12 @@ struct Work {
         for (__nv_bfloat16 **b : wbs)
             if (cudaMalloc(b, wb) != cudaSuccess) return HX_ERR_NOMEM;
         if (cudaMalloc(&x, (size_t)Mp * F * 4) != cudaSuccess || cudaMalloc(&t, (size_t)Mp * 4) != cudaSuccess ||
-            cudaMalloc(&y, (size_t)Mp * 4) != cudaSuccess || cudaMalloc(&dy, (size_t)Mp * 4) != cudaSuccess ||
             cudaMalloc(&G, (size_t)NPARAM * 4) != cudaSuccess || cudaMalloc(&loss, 4) != cudaSuccess ||
-            cudaMalloc(&ones, (size_t)Mp * 4) != cudaSuccess || cudaMalloc(&err, 4) != cudaSuccess)
+            cudaMalloc(&err, 4) != cudaSuccess)
             return HX_ERR_NOMEM;
-        // padded rows: zero inputs and targets, and a zero loss gradient (k_loss writes the first M only)
+        // padded rows: zero inputs and targets (and a zero loss gradient, k_out)
         if (cudaMemset(x, 0, (size_t)Mp * F * 4) != cudaSuccess || cudaMemset(t, 0, (size_t)Mp * 4) != cudaSuccess ||
-            cudaMemset(dy, 0, (size_t)Mp * 4) != cudaSuccess || cudaMemset(err, 0, 4) != cudaSuccess)
+            cudaMemset(err, 0, 4) != cudaSuccess)
             return HX_ERR_CUDA;
         int rc = HX_OK;
         if (rc == HX_OK) rc = map_bf16(&mH1b, h1b, Mp, H, TILE);
@@ -695,8 +751,7 @@ struct Work {
             hx_set_error("cannot reserve shared memory for the training GEMM");
             return HX_ERR_CUDA;
         }
-        std::vector<float> one(Mp, 1.f);
-        return cudaMemcpy(ones, one.data(), (size_t)Mp * 4, cudaMemcpyHostToDevice) == cudaSuccess ? HX_OK : HX_ERR_CUDA;
+        return HX_OK;
     }
     int error_word() const
     {
@@ -706,7 +761,7 @@ struct Work {
     }
     ~Work()
     {
-        float *all[] = {x, t, z1, h1, z2, h2, z3, h3, y, dy, dz, dh, G, loss, ones};
+        float *all[] = {x, t, z1, z2, z3, dh, G, loss};
         for (float *b : all) cudaFree(b);
         __nv_bfloat16 *allb[] = {h1b, h2b, h1T, h2T, dzb, dzT, W2b, W3b, W2T, W3T};
         for (__nv_bfloat16 *b : allb) cudaFree(b);
@@ -714,19 +769,13 @@ struct Work {
     }
 };
 
-// bf16 copies (row-major and transposed) of an FP32 [rows x H] matrix
-static void copies(cudaStream_t s, const float *src, int rows, __nv_bfloat16 *dst, __nv_bfloat16 *dstT)
-{
-    k_bf16_copies<<<nblocks((long long)((rows + 31) / 32) * (H / 32), 1), 256, 0, s>>>(src, rows, H, dst, dstT);
-}
 // tensor-core GEMM C[rows x H] = A B^T (+ bias) over nkb 64-deep K-blocks; splits > 1
-// add into C (cleared first) from that many K ranges
+// add into C (zero before) from that many K ranges
 static void bf16_gemm(cudaStream_t s, const CUtensorMap &a, const CUtensorMap &b, int rows, int nkb, int splits,
                     float *C, const float *bias, int *err)
 {
     const int kb_per = (nkb + splits - 1) / splits;
     const dim3 grid(rows / TILE, (nkb + kb_per - 1) / kb_per);
-    if (grid.y > 1) cudaMemsetAsync(C, 0, (size_t)rows * H * 4, s);
     bgemm<<<grid, BG_THREADS, BG_SMEM, s>>>(a, b, C, H, bias, nkb, kb_per, err);
 }
 
@@ -735,44 +784,30 @@ static void bf16_gemm(cudaStream_t s, const CUtensorMap &a, const CUtensorMap &b
 // six 256-wide products (layers 2 and 3 forward, their weight gradients and
 // the gradients of their inputs) run on the tensor cores in BF16 with FP32
 // accumulation (bgemm); the 8-wide first layer, the 1-wide output and the
-// bias sums stay on the CUDA cores. The loss gradient dz entering a bf16
-// product is rounded to bf16 (oracle/mlp.py applies the same roundings).
+// bias sums are part of the element-wise kernels between them. The loss
+// gradient dz entering a bf16 product is rounded to bf16 (oracle/mlp.py
+// applies the same roundings).
 static void fwd_bwd(cudaStream_t s, Work &w, const float *P, int M)
 {
     const int Mp = w.Mp, nk = H / 64, nkm = Mp / 64;
-    const long long MH = (long long)Mp * H;
-    k_bf16_copies<<<64, 256, 0, s>>>(P + O_W2, H, H, w.W2b, w.W2T);
-    k_bf16_copies<<<64, 256, 0, s>>>(P + O_W3, H, H, w.W3b, w.W3T);
-    gemm(s, Mp, H, F, w.x, F, 1, P + O_W1, 1, F, w.z1, H, P + O_B1);
-    k_silu<<<nblocks(MH), 256, 0, s>>>(w.z1, w.h1, MH, 1);
-    copies(s, w.h1, Mp, w.h1b, w.h1T);
+    const unsigned g = (unsigned)(Mp / TR);
+    cudaMemsetAsync(w.G, 0, (size_t)O_XS * 4, s);
+    k_weight_copies<<<2 * (H / 32) * (H / 32), 256, 0, s>>>(P, w.W2b, w.W2T, w.W3b, w.W3T);
+    k_layer1<<<g, 256, 0, s>>>(w.x, P, w.z1, w.h1b, w.h1T, Mp);
     bf16_gemm(s, w.mH1b, w.mW2b, Mp, nk, 1, w.z2, P + O_B2, w.err);
-    k_silu<<<nblocks(MH), 256, 0, s>>>(w.z2, w.h2, MH, 1);
-    copies(s, w.h2, Mp, w.h2b, w.h2T);
+    k_act<<<g, 256, 0, s>>>(w.z2, w.h2b, w.h2T, Mp);
     bf16_gemm(s, w.mH2b, w.mW3b, Mp, nk, 1, w.z3, P + O_B3, w.err);
-    k_silu<<<nblocks(MH), 256, 0, s>>>(w.z3, w.h3, MH, 0);
-    gemm(s, Mp, 1, H, w.h3, H, 1, P + O_W4, 1, 0, w.y, 1);
-    k_loss<<<nblocks(M), 256, 0, s>>>(w.y, w.t, P, w.dy, w.loss, M);
-    // output layer
-    gemm(s, 1, H, Mp, w.dy, 0, 1, w.h3, H, 1, w.G + O_W4, H);             // dw4 = h3^T dy
-    gemm(s, 1, 1, Mp, w.dy, 0, 1, w.ones, 1, 0, w.G + O_B4, 1);            // db4 = sum dy
-    k_dsilu<<<nblocks(MH), 256, 0, s>>>(nullptr, w.dy, P + O_W4, w.z3, w.dz, Mp);
-    copies(s, w.dz, Mp, w.dzb, w.dzT);
+    k_out<<<g, 256, 0, s>>>(w.z3, w.t, P, w.G, w.loss, w.dzb, w.dzT, M, Mp);
     // layer 3
     bf16_gemm(s, w.mDzT, w.mH2T, H, nkm, std::max(1, nkm / 4), w.G + O_W3, nullptr, w.err);   // dW3 = bf16(dz3)^T h2
-    gemm(s, 1, H, Mp, w.ones, 0, 1, w.dz, H, 1, w.G + O_B3, H);            // db3
     bf16_gemm(s, w.mDzb, w.mW3T, Mp, nk, 1, w.dh, nullptr, w.err);          // dh2 = bf16(dz3) bf16(W3)
-    k_dsilu<<<nblocks(MH), 256, 0, s>>>(w.dh, nullptr, nullptr, w.z2, w.dz, Mp);
-    copies(s, w.dz, Mp, w.dzb, w.dzT);
+    k_dact<<<g, 256, 0, s>>>(w.dh, w.z2, w.G + O_B2, w.dzb, w.dzT, Mp);
     // layer 2
     bf16_gemm(s, w.mDzT, w.mH1T, H, nkm, std::max(1, nkm / 4), w.G + O_W2, nullptr, w.err);
-    gemm(s, 1, H, Mp, w.ones, 0, 1, w.dz, H, 1, w.G + O_B2, H);
     bf16_gemm(s, w.mDzb, w.mW2T, Mp, nk, 1, w.dh, nullptr, w.err);
-    k_dsilu<<<nblocks(MH), 256, 0, s>>>(w.dh, nullptr, nullptr, w.z1, w.dz, Mp);
     // layer 1
-    gemm(s, H, F, Mp, w.dz, 1, H, w.x, F, 1, w.G + O_W1, F);
-    gemm(s, 1, H, Mp, w.ones, 0, 1, w.dz, H, 1, w.G + O_B1, H);
-    hx_count_launches(30);
+    k_dlayer1<<<g, H, 0, s>>>(w.dh, w.z1, w.x, w.G);
+    hx_count_launches(12);
 }
 
 
