@@ -243,6 +243,44 @@ __device__ __forceinline__ void block_sum_n(double (&x)[K])
     }
 }
 
+// Eight sums over the block; thread q < 8 returns sum q. Each exchange of the
+// warp stage halves the values a lane carries (9 FP64 adds per lane instead
+// of 40: on GB300's FP64 pipe the full butterflies of 20 DIIS dots cost more
+// than the dots of a 1024-element unit).
+__device__ __forceinline__ double block_sum8(double (&x)[8])
+{
+    __shared__ double sh[8][NT / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int n = 4, o = 16; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int q = 0; q < n; ++q) {
+            const double send = up ? x[q] : x[q + n], keep = up ? x[q + n] : x[q];
+            x[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+    __syncthreads();
+    if ((lane & 3) == 0) sh[lane >> 2][w] = x[0];      // bits 4, 3, 2 of the lane: values 4, 2, 1
+    __syncthreads();
+    double r = 0.0;
+    if (threadIdx.x < 8)
+#pragma unroll
+        for (int k = 0; k < NT / 32; ++k) r += sh[threadIdx.x][k];
+    return r;
+}
+
+// max of two magnitudes by their bit patterns (NaN ignored, as fmax does;
+// integer compares instead of the FP64 pipe)
+__device__ __forceinline__ double max_abs(double mx, double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+    const unsigned long long m = (unsigned long long)__double_as_longlong(mx);
+    return b > m && b <= 0x7FF0000000000000ull ? __longlong_as_double((long long)b) : mx;
+}
+
 // u[i][a][j][b] = 2 t[i][a][j][b] - t[i][b][j][a]  (SK_FULL units)
 __global__ void __launch_bounds__(NT) k_make_u(const CCMol *__restrict__ mols, const int *__restrict__ active,
                                                const int *__restrict__ start, int nmol)
@@ -277,9 +315,10 @@ __global__ void __launch_bounds__(NT) k_make_u(const CCMol *__restrict__ mols, c
 //   doubles of a block (i, j), i <= j: w = Omega2(ia, jb) assembled as
 //     r2 + X2 + X2 pair-transposed (the E and C/D terms), d2 = 2 w(ab) - w(ba)
 //     (= w on a diagonal block, whose canonical element is the same for both);
-//     g = 3 w ("2-1") or d2 ("1"); t2 += s2 g / D2 with D2 = (F_ii + F_jj) -
-//     (F_aa + F_bb) (the grouping the set-up uses, so (ia,jb) and (jb,ia)
-//     round alike).
+//     g = 3 w ("2-1") or d2 ("1"); t2 += s2 g / D2, the quotient as
+//     q = s2 g R2 and one correction q + (s2 g - q D2) R2 with the stored
+//     reciprocal R2 = 1/D2 (Markstein's division: three FP64 operations
+//     instead of a division's dozen).
 // push = 1: (t, g) go into the ring slot count % nd and part gets the dots of
 // g with every stored error vector. The error vector keeps the pair (ia, ib)
 // of a diagonal block once (a <= b; the mirror element is stored as 0), so a
@@ -297,11 +336,10 @@ __global__ void __launch_bounds__(NT) k_step_push(const CCMol *__restrict__ mols
     if (active && !active[w.mol]) return;
     const CCMol &m = mols[w.mol];
     const DiisMol &h = diis[w.mol];
-    const int o = m.o, v = m.v, n = m.N, ov = o * v;
+    const int o = m.o, v = m.v, ov = o * v;
     double *P = part + (long long)blockIdx.x * HX_PART_STRIDE;
     const int cnt = push ? h.count[0] : 0;
     const int slot = push ? cnt % h.nd : 0, nvec = push ? min(cnt + 1, h.nd) : 0;
-    const double *__restrict__ Fmo = m.Fmo;
     double *__restrict__ t2 = m.t2;
     const double *__restrict__ X2 = m.X2;
     double *S = sm;                              // the assembled residual of the unit's blocks
@@ -346,19 +384,19 @@ __global__ void __launch_bounds__(NT) k_step_push(const CCMol *__restrict__ mols
         __syncthreads();
         ROW_LOOP(nrows) {
             const int lb = row_ / v, a = row_ - lb * v, i = bi[lb], j = bj[lb];
-            const double fij = Fmo[i * n + i] + Fmo[j * n + j], faa = Fmo[(o + a) * n + o + a];
             const double *srow = S + (lb * v + a) * (v + 1);
-            double *trow = t2 + pair_off(i, a, j, 0, o, v);
+            const long long f0 = pair_off(i, a, j, 0, o, v);
+            double *trow = t2 + f0;
+            const double *Drow = m.D2 + f0, *Rrow = m.R2 + f0;
             const long long hrow = hoff + (long long)(lb * v + a) * v;
             COL_LOOP(b, v) {
                 const double sab = srow[b], sba = S[(lb * v + b) * (v + 1) + a];
                 double wv, d2;
                 if (i < j) { wv = sab; d2 = 2.0 * sab - sba; }
                 else { wv = a <= b ? sab : sba; d2 = wv; }
-                mx = fmax(mx, fabs(d2));
-                const double g = proj == 1 ? d2 : 3.0 * wv;
-                const double D = fij - (faa + Fmo[(o + b) * n + o + b]);
-                const double t = trow[b] + s2 * g / D;
+                mx = max_abs(mx, d2);
+                const double g = proj == 1 ? d2 : 3.0 * wv, sg = s2 * g, R = Rrow[b];
+                const double q = sg * R, t = trow[b] + fma(fma(-q, Drow[b], sg), R, q);
                 if (push) {
                     h.Ht[(long long)slot * h.L + hrow + b] = t;
                     // a diagonal block holds (ia, ib) and (ib, ia), the same pair: the
@@ -399,9 +437,8 @@ __global__ void __launch_bounds__(NT) k_step_push(const CCMol *__restrict__ mols
 #pragma unroll
             for (int q = 0; q < 8; ++q) acc[q] += g * Ek[q][e];
         }
-        block_sum_n<8>(acc);
-        if (threadIdx.x == 0)
-            for (int q = 0; q < 8 && k0 + q < nvec; ++q) P[2 + k0 + q] = acc[q];
+        const double sum = block_sum8(acc);
+        if (threadIdx.x < 8 && k0 + (int)threadIdx.x < nvec) P[2 + k0 + threadIdx.x] = sum;
     }
 }
 
@@ -445,73 +482,92 @@ __global__ void __launch_bounds__(NT) k_diis_solve(const CCMol *__restrict__ mol
         return;
     }
     __shared__ double g[HX_MAX_DIIS];
-    for (int k = 0; k < n; ++k) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int k = warp; k < n; k += NT / 32) {          // a warp per dot, no block barriers
         double s = 0.0;
-        for (int u = u0 + threadIdx.x; u < u1; u += NT) s += part[(long long)u * HX_PART_STRIDE + 2 + k];
-        s = block_red(s, false);
-        if (threadIdx.x == 0) g[k] = s;
+        for (int u = u0 + lane; u < u1; u += 32) s += part[(long long)u * HX_PART_STRIDE + 2 + k];
+        s = warp_sum(s);
+        if (lane == 0) g[k] = s;
     }
     __syncthreads();
+    for (int k = threadIdx.x; k < n; k += NT) {
+        h.gram[slot * h.nd + k] = g[k];
+        h.gram[k * h.nd + slot] = g[k];
+    }
     if (threadIdx.x == 0) {
-        for (int k = 0; k < n; ++k) {
-            h.gram[slot * h.nd + k] = g[k];
-            h.gram[k * h.nd + slot] = g[k];
-        }
         h.count[0] = cnt + 1;
         h.coef[HX_MAX_DIIS + 1] = slot;
         h.coef[HX_MAX_DIIS] = 1.0;
     }
     if (n == 1) return;                                // newCCVectors(1) returns early
     // the bordered system [B 1; 1 0] c = e by Gaussian elimination with partial
-    // pivoting in shared memory: pivot search and back substitution in one
-    // thread, the row updates in parallel (each row's operations in the same
-    // order as a serial elimination)
-    constexpr int MB = HX_MAX_DIIS + 1;
-    __shared__ double A[MB * MB], x[MB];
+    // pivoting in shared memory, the right-hand side as one more column: warp 0
+    // searches the pivot and divides the column by it, all threads update the
+    // rows (a serial elimination of 21 x 21 in one thread took 40 us of a
+    // 12-site iteration)
+    constexpr int MB = HX_MAX_DIIS + 1, LD = MB + 1;
+    __shared__ double A[MB * LD], f[MB];
     __shared__ int piv_s;
     const int nb = n + 1;
     __syncthreads();
-    for (int e = threadIdx.x; e < nb * nb; e += NT) {
-        const int p = e / nb, q = e % nb;
+    for (int e = threadIdx.x; e < nb * (nb + 1); e += NT) {
+        const int p = e / (nb + 1), q = e % (nb + 1);
         double val;
-        if (p == n && q == n) val = 0.0;
+        if (q == nb) val = p == n ? 1.0 : 0.0;
+        else if (p == n && q == n) val = 0.0;
         else if (p == n || q == n) val = 1.0;
-        else val = h.gram[p * h.nd + q];
-        A[p * nb + q] = val;
+        else val = (p == slot || q == slot) ? g[p == slot ? q : p] : h.gram[p * h.nd + q];
+        A[p * LD + q] = val;
     }
-    for (int p = threadIdx.x; p < nb; p += NT) x[p] = (p == n) ? 1.0 : 0.0;
     __syncthreads();
     for (int k = 0; k < nb; ++k) {
-        if (threadIdx.x == 0) {
+        if (warp == 0) {
+            double best = -1.0;
             int piv = k;
-            for (int r = k + 1; r < nb; ++r)
-                if (fabs(A[r * nb + k]) > fabs(A[piv * nb + k])) piv = r;
-            piv_s = piv;
+            for (int r = k + lane; r < nb; r += 32)
+                if (fabs(A[r * LD + k]) > best) { best = fabs(A[r * LD + k]); piv = r; }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {         // the first row of the largest magnitude
+                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int op = __shfl_xor_sync(0xffffffffu, piv, o);
+                if (ob > best || (ob == best && op < piv)) { best = ob; piv = op; }
+            }
+            const double d = A[piv * LD + k];
+            for (int r = k + lane; r < nb; r += 32)    // row factors, in the order after the swap
+                if (r != k) f[r] = A[(r == piv ? k : r) * LD + k] / d;
+            if (lane == 0) piv_s = piv;
         }
         __syncthreads();
         const int piv = piv_s;
         if (piv != k) {
-            for (int c = threadIdx.x; c < nb; c += NT) { double t = A[k * nb + c]; A[k * nb + c] = A[piv * nb + c]; A[piv * nb + c] = t; }
-            if (threadIdx.x == 0) { double t = x[k]; x[k] = x[piv]; x[piv] = t; }
+            for (int c = k + threadIdx.x; c <= nb; c += NT) {
+                const double t = A[k * LD + c];
+                A[k * LD + c] = A[piv * LD + c];
+                A[piv * LD + c] = t;
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        for (int r = k + 1 + threadIdx.x; r < nb; r += NT) {
-            const double f = A[r * nb + k] / A[k * nb + k];
-            for (int c = k; c < nb; ++c) A[r * nb + c] -= f * A[k * nb + c];
-            x[r] -= f * x[k];
+        const int w = nb - k;                          // columns k + 1 .. nb
+        for (int e = threadIdx.x; e < (nb - 1 - k) * w; e += NT) {
+            const int r = k + 1 + e / w, c = k + 1 + e % w;
+            A[r * LD + c] -= f[r] * A[k * LD + c];
         }
         __syncthreads();
     }
-    if (threadIdx.x != 0) return;
+    if (warp != 0) return;
+    // back substitution by columns: once x_k is known every row above takes its share
     for (int k = nb - 1; k >= 0; --k) {
-        double s = x[k];
-        for (int c = k + 1; c < nb; ++c) s -= A[k * nb + c] * x[c];
-        x[k] = s / A[k * nb + k];
+        const double xk = A[k * LD + nb] / A[k * LD + k];
+        __syncwarp();
+        for (int r = lane; r < k; r += 32) A[r * LD + nb] -= A[r * LD + k] * xk;
+        if (lane == 0) A[k * LD + nb] = xk;
+        __syncwarp();
     }
-    for (int k = 0; k < n; ++k)
-        if (!isfinite(x[k])) return;                   // singular subspace: no mixing
-    for (int k = 0; k < n; ++k) h.coef[k] = x[k];
-    h.coef[HX_MAX_DIIS] = (double)n;
+    bool ok = true;
+    for (int k = lane; k < n; k += 32) ok = ok && isfinite(A[k * LD + nb]);
+    if (!__all_sync(0xffffffffu, ok)) return;          // singular subspace: no mixing
+    for (int k = lane; k < n; k += 32) h.coef[k] = A[k * LD + nb];
+    if (lane == 0) h.coef[HX_MAX_DIIS] = (double)n;
 }
 
 // ---------------------------------------------------------------- amplitudes and energy
@@ -692,7 +748,9 @@ __global__ void k_setup(EW_ARGS)
             int a = (int)(r % v);
             int i = (int)(r / v);
             // grouped so that (ia),(jb) and (jb),(ia) round identically
-            m.D2[f] = (m.Fmo[i * n + i] + m.Fmo[j * n + j]) - (m.Fmo[(o + a) * n + o + a] + m.Fmo[(o + b) * n + o + b]);
+            const double d = (m.Fmo[i * n + i] + m.Fmo[j * n + j]) - (m.Fmo[(o + a) * n + o + a] + m.Fmo[(o + b) * n + o + b]);
+            m.D2[f] = d;
+            m.R2[f] = 1.0 / d;
         } else {
             long long f = e - ov - ov * ov;
             int mu = (int)(f / ov), r = (int)(f % ov), k = r / v, c = r % v;

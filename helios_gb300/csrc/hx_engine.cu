@@ -529,7 +529,7 @@ static int allocate(hx_ccsd *h)
             m.Cmo = s.V; m.G = s.G; m.h = s.core; m.Fmo = s.Fmo;
             m.Bov0 = A.take<double>(N * ov); m.GBov0 = A.take<double>(N * ov);
             m.gov = A.take<double>(pr); m.Lov = A.take<double>(pr);
-            m.D1 = A.take<double>(ov); m.D2 = A.take<double>(pr);
+            m.D1 = A.take<double>(ov); m.D2 = A.take<double>(pr); m.R2 = A.take<double>(pr);
             m.t1 = A.take<double>(ov); m.t2 = A.take<double>(pr);
             m.r1 = A.take<double>(ov); m.r2 = A.take<double>(pr); m.u = A.take<double>(pr);
             m.X = A.take<double>(nn); m.Y = A.take<double>(nn); m.Pm = A.take<double>(nn);

@@ -33,7 +33,7 @@ struct CCMol {
     const double *Cmo, *G, *h, *Fmo;      // N x N
     double *Bov0, *GBov0;                 // [N][o*v]  C_mu,k C_mu,c and G . it
     double *gov, *Lov;                    // pair: (kc|ld), 2(kc|ld)-(kd|lc)
-    double *D1, *D2;                      // denominators F_ii-F_aa, F_ii+F_jj-F_aa-F_bb
+    double *D1, *D2, *R2;                 // denominators F_ii-F_aa, F_ii+F_jj-F_aa-F_bb, and 1/D2
     // amplitudes and residuals
     double *t1, *t2, *r1, *r2, *u;
     // T1-dressed factors
