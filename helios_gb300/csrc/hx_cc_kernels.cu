@@ -153,17 +153,19 @@ __global__ void k_fock_blocks(EW_ARGS)
     }
 }
 
-// X2[i][a][j][b] = 0.5 Cp[i][a][j][b] + Cp[j][a][i][b]  (consecutive b read consecutively)
+// X2[i][a][j][b] += Cint[i][a][j][b] + 0.5 Cp[i][a][j][b] + Cp[j][a][i][b]  (consecutive b read
+// consecutively; X2 and Cint hold the two E products)
 __global__ void k_c_combine(EW_ARGS)
 {
     EW_PROLOGUE
     const unsigned o = (unsigned)m.o, v = (unsigned)m.v;
     const double *__restrict__ Cp = m.Cp;
+    const double *__restrict__ E2 = m.Cint;
     double *__restrict__ X2 = m.X2;
     EW_LOOP(e, (long long)o * v * o * v) {
         const unsigned x = (unsigned)e;                  // o^2 v^2 < 2^32
         const unsigned b = x % v, r = x / v, j = r % o, r2 = r / o, a = r2 % v, i = r2 / v;
-        X2[e] = 0.5 * Cp[e] + Cp[((j * v + a) * o + i) * v + b];
+        X2[e] = (X2[e] + E2[e]) + (0.5 * Cp[e] + Cp[((j * v + a) * o + i) * v + b]);
     }
 }
 

@@ -26,6 +26,7 @@ struct TgemmDesc {
     int mol;            // molecule index (skipped when that molecule is inactive)
     int ksplit;         // K is cut into ksplit slices accumulated atomically (needs beta == 1)
     int a_const, b_const;   // operand unchanged between hx_ccsd_init calls (prepared once)
+    int a_keep, b_keep;     // operand unchanged from its first use in an iteration to its last (prepared once per iteration)
     int tiles_m, tiles_n;
     long long tile_start;   // prefix sum of batch*tiles_m*tiles_n over the group
 };

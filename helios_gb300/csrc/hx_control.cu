@@ -66,11 +66,13 @@ __global__ void k_control(const CCMol *__restrict__ mols, const DiisMol *__restr
     }
     if (P.mixed) {
         // vectors of a finished cheaper phase leave the extrapolation once the
-        // residual is below purge x the level at which that phase ended: their
-        // Gram row and column are cleared and the diagonal made huge
+        // residual is below purge x the level at which that phase ended, or above
+        // twice that level (the phase had converged below its own error, and its
+        // vectors would draw the iteration back to that point): their Gram row and
+        // column are cleared and the diagonal made huge
         const int valid = (int)(c.dcount < nd ? c.dcount : nd);
         for (int p2 = PH_HIGH; p2 < PH_COUNT; ++p2) {
-            if (!(c.ph_end[p2] > 0.0) || !(a < P.purge * c.ph_end[p2])) continue;
+            if (!(c.ph_end[p2] > 0.0) || !(a < P.purge * c.ph_end[p2] || a > 2.0 * c.ph_end[p2])) continue;
             for (int k = 0; k < valid; ++k) {
                 if (c.slot_phase[k] != p2) continue;
                 for (int q = 0; q < nd; ++q) h.gram[k * nd + q] = h.gram[q * nd + k] = 0.0;
@@ -83,7 +85,10 @@ __global__ void k_control(const CCMol *__restrict__ mols, const DiisMol *__restr
     if (ph >= PH_HIGH && !cancel) {
         // tensor-core phases never claim convergence: they hand over
         if (a < c.best) { c.best = a; c.stall = 0; } else ++c.stall;
-        const double fin = P.high_margin * c.fin_scale * P.eps;
+        // a target below what HIGH's contractions resolve: hand over at their
+        // error and let the check phase iterate on
+        const bool deep = P.high_margin * P.eps < 0.1 * P.high_floor;
+        const double fin = deep ? P.high_floor : P.high_margin * c.fin_scale * P.eps;
         const double below = ph == PH_LOW ? P.mixed_switch : ph == PH_MID ? P.mid_span * P.mixed_switch : 0.0;
         const bool stalled = c.stall >= P.patience;
         int next = ph;
@@ -99,7 +104,7 @@ __global__ void k_control(const CCMol *__restrict__ mols, const DiisMol *__restr
             c.best = 1e300;
             c.ph_end[ph] = a;
             // HIGH stalled above its hand-over target: the check phase iterates on
-            if (ph == PH_HIGH && a >= fin) c.fp_returns = P.max_returns;
+            if ((ph == PH_HIGH && a >= fin) || (deep && next == P.check_ph)) c.fp_returns = P.max_returns;
             if (stalled && a >= fin && ph != PH_HIGH) {              // LOW or MID: restart DIIS
                 h.count[0] = 0;
                 c.dcount = 0;

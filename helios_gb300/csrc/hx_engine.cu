@@ -234,13 +234,13 @@ struct hx_ccsd {
                                          // still running, [2..6] per phase next), [8] the stop request
                                          // (read by the device)
     bool device_ctl = false;             // solve_all: the device decides phases and masks
-    bool capturing = false;              // iteration_body is being captured: phases become conditional nodes
+    bool capturing = false;              // an iteration is being captured: phases become conditional nodes
     bool profiling = false;              // per-launch GEMM timing: iterations are launched one by one
     cudaStream_t st2 = nullptr;          // captures the bodies of the conditional nodes
-    // conditional handles of a captured iteration, one per conditional node
-    // (a plan group's launches of one phase), made as the nodes are captured
+    // conditional handles of a captured iteration, one per phase, made as the
+    // nodes are captured
     std::vector<PhaseCondition> cond;
-    PhaseCondition *d_cond = nullptr;    // room for one per (plan group, phase)
+    PhaseCondition *d_cond = nullptr;
     std::vector<std::vector<std::array<double, 5>>> trace;
     // device time of the last hx_ccsd_init and solve (events on st)
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -265,24 +265,40 @@ static TgemmDesc tg(const double *A, const double *B, double *C, int batch, int 
 }
 
 // Operands that stay fixed between hx_ccsd_init calls: the tensor-core
-// backend slices them once per initialisation.
+// backend slices them once per initialisation. Those that an iteration writes
+// before their first use as an operand and not again (keep) are sliced once
+// per iteration for all their uses.
 static void mark_constants(hx_ccsd *h)
 {
     for (auto &g : h->plan)
         for (auto &d : g.h) {
             const CCMol &m = h->cc[d.mol];
-            auto fixed = [&](const double *p) {
-                const double *lo[] = {m.Cmo, m.G, m.gov, m.Lov, m.Bov0, m.GBov0};
-                const size_t n[] = {(size_t)m.N * m.N, (size_t)m.N * m.N, (size_t)m.o * m.v * m.o * m.v,
-                                    (size_t)m.o * m.v * m.o * m.v, (size_t)m.N * m.o * m.v, (size_t)m.N * m.o * m.v};
-                for (int k = 0; k < 6; ++k)
-                    if (p >= lo[k] && p < lo[k] + n[k]) return 1;
+            const size_t N = m.N, o = m.o, v = m.v, ov = o * v;
+            struct Range { const double *p; size_t n; };
+            auto in = [](const double *p, std::initializer_list<Range> list) {
+                for (const Range &r : list)
+                    if (r.p && p >= r.p && p < r.p + r.n) return 1;
                 return 0;
+            };
+            auto fixed = [&](const double *p) {
+                return in(p, {{m.Cmo, N * N}, {m.G, N * N}, {m.gov, ov * ov}, {m.Lov, ov * ov}, {m.Bov0, N * ov}, {m.GBov0, N * ov}});
+            };
+            auto keep = [&](const double *p) {
+                return in(p, {{m.t1, ov}, {m.t2, ov * ov}, {m.u, ov * ov}, {m.Bia, N * ov}, {m.GBia, N * ov}, {m.Boo, N * o * o},
+                              {m.GBoo, N * o * o}, {m.Bvv, N * v * v}, {m.GBvv, N * v * v}, {m.UG, ov * N}});
             };
             d.a_const = fixed(d.A);
             d.b_const = fixed(d.B);
+            d.a_keep = keep(d.A);
+            d.b_keep = keep(d.B);
         }
 }
+
+// A level's smallest contractions stay on the FP64 kernel in the LOW, MID and
+// HIGH phases while they take at most this many multiply-adds together: 2e6
+// are 3.3 us of the GPU's FP64 rate, less than the slicing and the tensor-core
+// launch they would need of their own.
+static const double kFp64Work = 2e6;
 
 static int upload_group(Group &g)
 {
@@ -293,8 +309,8 @@ static int upload_group(Group &g)
     return HX_OK;
 }
 
-// While an iteration is captured: a conditional (if) node on phase ph's
-// condition is added to the capture, and body(s2) is captured into its graph.
+// While a solve is captured: a conditional (if) node on phase ph's condition
+// is added to the capture, and body(s2) is captured into its graph.
 template <class F>
 static int with_condition(hx_ccsd *h, int ph, F body)
 {
@@ -311,7 +327,7 @@ static int with_condition(hx_ccsd *h, int ph, F body)
     memset(&pc, 0, sizeof(pc));
     pc.phase = ph;
     HX_CU(cudaGraphConditionalHandleCreate(&pc.handle, g, 0, 0));
-    if (h->cond.size() >= h->plan.size() * PH_COUNT) { hx_set_error("too many conditional nodes"); return HX_ERR_STATE; }
+    if (h->cond.size() >= PH_COUNT) { hx_set_error("too many conditional nodes"); return HX_ERR_STATE; }
     h->cond.push_back(pc);
     np.conditional.handle = pc.handle;
     np.conditional.type = cudaGraphCondTypeIf;
@@ -322,46 +338,26 @@ static int with_condition(hx_ccsd *h, int ph, F body)
     HX_CU(cudaStreamBeginCaptureToGraph(h->st2, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal));
     const long long before = g_launches.load();
-    const cudaError_t e = body(h->st2);
+    const int rc = body(h->st2);
     h->phase_nodes[ph] += g_launches.load() - before;
     cudaGraph_t out = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(h->st2, &out);
-    HX_CU(e);
+    if (rc < 0) return rc;
     HX_CU(e2);
     return HX_OK;
 }
 
-// Each molecule runs the group in its current phase: the tensor-core modes
-// on tcgen05, FP64 on the CUDA-core kernel; one launch per phase in use, with
-// that phase's mask (every launch skips the molecules that are not its own).
-static int run_group(hx_ccsd *h, Group &g)
+// One contraction level for the molecules of phase ph (launch mask act): the
+// tensor-core modes on tcgen05, FP64 on the CUDA-core kernel.
+static int run_group(hx_ccsd *h, Group &g, int ph, const int *act, cudaStream_t s)
 {
     if (g.tiles.count == 0) return HX_OK;
-    if (h->tce) {
-        int n[PH_COUNT] = {};
-        for (int mi = 0; mi < h->nmol; ++mi)
-            if (h->active[mi]) ++n[h->phase[mi]];
-        if (h->device_ctl && h->capturing) {
-            // each phase's launches become the body of a conditional node that
-            // runs only when some molecule is in that phase this iteration
-            for (int ph = 0; ph < PH_COUNT; ++ph)
-                HX_TRY(with_condition(h, ph, [&](cudaStream_t s2) {
-                    if (ph == PH_FP64) return hx_tgemm_f64_launch(g.d, (int)g.h.size(), g.tiles, h->d_act_ph[PH_FP64], s2);
-                    return tc::run_group(h->tce, g.h.data(), (int)g.h.size(), h->d_act_ph[ph], s2, tc_mode(ph));
-                }));
-            return HX_OK;
-        }
-        if (h->device_ctl)                       // the phases the device counted for this iteration
-            for (int ph = 0; ph < PH_COUNT; ++ph) n[ph] = h->h_pinned[2 + ph];
-        for (int ph = PH_LOW; ph >= PH_EXACT; --ph) {
-            if (!n[ph]) continue;
-            cudaError_t e = tc::run_group(h->tce, g.h.data(), (int)g.h.size(), h->d_act_ph[ph], h->st, tc_mode(ph));
-            if (e != cudaSuccess) { hx_set_error("tensor-core group: %s", cudaGetErrorString(e)); return HX_ERR_CUDA; }
-        }
-        if (n[PH_FP64]) HX_CU(hx_tgemm_f64_launch(g.d, (int)g.h.size(), g.tiles, h->d_act_ph[PH_FP64], h->st));
+    if (ph == PH_FP64) {
+        HX_CU(hx_tgemm_f64_launch(g.d, (int)g.h.size(), g.tiles, act, s));
         return HX_OK;
     }
-    HX_CU(hx_tgemm_f64_launch(g.d, (int)g.h.size(), g.tiles, h->d_active, h->st));
+    const cudaError_t e = tc::run_group(h->tce, g.h.data(), (int)g.h.size(), act, s, tc_mode(ph));
+    if (e != cudaSuccess) { hx_set_error("tensor-core group: %s", cudaGetErrorString(e)); return HX_ERR_CUDA; }
     return HX_OK;
 }
 
@@ -418,14 +414,25 @@ static bool mo_ladder(const hx_ccsd *h, int mi)
     return h->p.precision != HX_PRECISION_FP64 && h->v[mi] <= kMoLadderMaxV;
 }
 
-// Descriptors of every contraction of one iteration, for every molecule.
+// Descriptors of every contraction of one iteration, for every molecule, in
+// dependency levels: the contractions of a level read only what earlier levels
+// (and the element-wise kernels between them, iteration_body) wrote, and no
+// two of them write the same tensor, so a level is one launch. An iteration
+// of a small molecule is a chain of launches, so its length is what counts:
+// seven levels instead of one launch per contraction (35), and what several
+// contractions of a level read is sliced once.
 // Index conventions are spelled out in hx_plan.h; each block cites the term
 // of the T1-dressed closed-shell CCSD equations it evaluates.
 static void build_plan(hx_ccsd *h)
 {
-    enum { G_DRESS_XY, G_DRESS_P, G_FD1, G_FD2, G_GB, G_LEAD, G_LAD_A, G_LAD_B, G_LAD_D, G_LAD_E, G_W_D,
-           G_W_E, G_W_INT, G_HH, G_CINT1, G_CINT2, G_CTERM, G_DINT1, G_DINT2, G_DINT3, G_DTERM, G_FVOO,
-           G_E1, G_E2, G_S1, G_S_UG, G_S_V, G_S_R1, G_COUNT };
+    // level of each contraction (L_x + the element-wise kernels of iteration_body)
+    enum { G_DRESS_XY = 0, G_LAD_A = 0, G_S_U = 0, G_W_MO = 0,
+           G_DRESS_P = 1, G_GB = 1, G_LAD_B = 1, G_S_UG = 1,
+           G_FD1 = 2, G_LEAD = 2, G_CINT1 = 2, G_DINT1 = 2, G_V_MO = 2, G_LAD_D = 2, G_S_V = 2,
+           G_FD2 = 3, G_CINT2 = 3, G_DINT2 = 3, G_LAD_E = 3, G_W_E = 3, G_W_INT_MO = 3,
+           G_FVOO = 4, G_S1 = 4, G_DINT3 = 4, G_CTERM = 4, G_W_INT = 4, G_HH_MO = 4,
+           G_E1 = 5, G_E2 = 5, G_HH = 5, G_S_R1 = 5,
+           G_DTERM = 6, G_S_R1B = 6, G_COUNT = 7 };
     h->plan.assign(G_COUNT, Group());
     auto &P = h->plan;
     for (int mi = 0; mi < h->nmol; ++mi) {
@@ -451,10 +458,10 @@ static void build_plan(hx_ccsd *h)
         const long long vv = (long long)v * v, vov = (long long)v * ov;
         if (mo_ladder(h, mi)) {
             // (ac|bd)~ = sum_mu Bvv[mu][ac] GBvv[mu][bd]; r2_ij^ab += sum_cd (ac|bd)~ t_ij^cd
-            P[G_LAD_A].h.push_back(tg(m.Bvv, m.GBvv, m.Vvv, 1, (int)vv, (int)vv, N, (int)vv, (int)vv, N, {0, 1, 0, vv, 0}, {0, 1, 0, vv, 0}, {0, vv, 0, 1, 0}, 1.0, 0.0, mi));
+            P[G_V_MO].h.push_back(tg(m.Bvv, m.GBvv, m.Vvv, 1, (int)vv, (int)vv, N, (int)vv, (int)vv, N, {0, 1, 0, vv, 0}, {0, 1, 0, vv, 0}, {0, vv, 0, 1, 0}, 1.0, 0.0, mi));
             P[G_LAD_E].h.push_back(tg(m.t2, m.Vvv, m.r2, 1, o * o, (int)vv, (int)vv, o, v, v, {vov, v, ov, 1, 0}, {vv * v, v, vv, 1, 0}, {vov, v, ov, 1, 0}, 1.0, 1.0, mi));
             // W_klij = sum_cd (kc|ld) t_ij^cd into Woo[i][k][j][l] ((ki|lj)~ is added below)
-            P[G_W_E].h.push_back(tg(m.gov, m.t2, m.Woo, 1, o * o, o * o, (int)vv, o, o, v, {(long long)v * ov, v, ov, 1, 0}, {vov, v, ov, 1, 0}, {(long long)o * o, 1, (long long)o * o * o, o, 0}, 1.0, 0.0, mi));
+            P[G_W_MO].h.push_back(tg(m.gov, m.t2, m.Woo, 1, o * o, o * o, (int)vv, o, o, v, {(long long)v * ov, v, ov, 1, 0}, {vov, v, ov, 1, 0}, {(long long)o * o, 1, (long long)o * o * o, o, 0}, 1.0, 0.0, mi));
         } else {
             P[G_LAD_A].h.push_back(tg(m.t2, Cmo + o, m.T1s, 1, o * v * o, N, v, o * v * o, N, v, {0, v, 0, 1, 0}, {0, N, 0, 1, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
             P[G_LAD_B].h.push_back(tg(Cmo + o, m.T1s, m.Ts, o, N, o * N, v, N, o * N, v, {0, N, 0, 1, 0}, {0, 1, 0, (long long)o * N, (long long)v * o * N}, {0, (long long)o * N, 0, 1, (long long)N * o * N}, 1.0, 0.0, mi));
@@ -464,11 +471,10 @@ static void build_plan(hx_ccsd *h)
             P[G_LAD_D].h.push_back(tg(m.Ts, m.X, m.Z, 1, o * N * o, N, N, o * N * o, N, N, {0, N, 0, 1, 0}, {0, 1, 0, N, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
             P[G_LAD_E].h.push_back(tg(m.X + o, m.Z + o, m.r2, o, v, ov, N, v, v, N, {0, 1, 0, N, 0}, {N, 1, 0, (long long)o * N, (long long)N * o * N}, {0, ov, v, 1, (long long)v * ov}, 1.0, 1.0, mi));
             // hole-hole ladder: W_klij = (ki|lj)~ + sum_cd t_ij^cd (kc|ld), the latter through the site basis
-            //   (G_W_D stays empty: Z's occupied columns are the former Zo = Ts Co)
             P[G_W_E].h.push_back(tg(Cmo, m.Z, m.Woo, o, o, o * o, N, o, o, N, {0, 1, 0, N, 0}, {N, 1, 0, (long long)o * N, (long long)N * o * N}, {0, o * o, o, 1, (long long)o * o * o}, 1.0, 0.0, mi));
         }
-        P[G_W_INT].h.push_back(tg(m.Boo, m.GBoo, m.Woo, 1, o * o, o * o, N, o, o, N, {o, 1, 0, o * o, 0}, {o, 1, 0, o * o, 0}, {(long long)o * o, (long long)o * o * o, 1, o, 0}, 1.0, 1.0, mi));
-        P[G_HH].h.push_back(tg(m.Woo, m.t2, m.r2, 1, o * o, v * v, o * o, o, v, o, {(long long)o * o * o, o, (long long)o * o, 1, 0}, {ov, 1, (long long)v * ov, v, 0}, {(long long)v * ov, v, ov, 1, 0}, 1.0, 1.0, mi));
+        P[mo_ladder(h, mi) ? G_W_INT_MO : G_W_INT].h.push_back(tg(m.Boo, m.GBoo, m.Woo, 1, o * o, o * o, N, o, o, N, {o, 1, 0, o * o, 0}, {o, 1, 0, o * o, 0}, {(long long)o * o, (long long)o * o * o, 1, o, 0}, 1.0, 1.0, mi));
+        P[mo_ladder(h, mi) ? G_HH_MO : G_HH].h.push_back(tg(m.Woo, m.t2, m.r2, 1, o * o, v * v, o * o, o, v, o, {(long long)o * o * o, o, (long long)o * o, 1, 0}, {ov, 1, (long long)v * ov, v, 0}, {(long long)v * ov, v, ov, 1, 0}, 1.0, 1.0, mi));
         // C: Cint_kiac = (ki|ac)~ - 1/2 sum_ld t_li^ad (kd|lc);  C_ij^ab = -sum_kc t_kj^bc Cint_kiac
         P[G_CINT1].h.push_back(tg(m.Boo, m.GBvv, m.Cint, 1, o * o, v * v, N, o * o, v * v, N, {0, 1, 0, o * o, 0}, {0, 1, 0, v * v, 0}, {0, v * v, 0, 1, 0}, 1.0, 0.0, mi));
         P[G_CINT2].h.push_back(tg(m.t2, m.gov, m.Cint, 1, ov, ov, ov, v, v, v, {v, ov, (long long)v * ov, 1, 0}, {(long long)v * ov, 1, v, ov, 0}, {(long long)v * v, v, (long long)ov * v, 1, 0}, -0.5, 1.0, mi));
@@ -482,26 +488,22 @@ static void build_plan(hx_ccsd *h)
         P[G_FVOO].h.push_back(tg(m.u, m.gov, m.Fvv2, 1, v, v, o * ov, v, v, ov, {0, ov, (long long)v * ov, 1, 0}, {0, ov, (long long)v * ov, 1, 0}, {0, v, 0, 1, 0}, -1.0, 1.0, mi));
         P[G_FVOO].h.push_back(tg(m.gov, m.u, m.Foo2, 1, o, o, v * ov, o, o, ov, {0, (long long)v * ov, ov, 1, 0}, {0, (long long)v * ov, ov, 1, 0}, {0, o, 0, 1, 0}, 1.0, 1.0, mi));
         //    E_ij^ab = sum_c t_ij^ac F'_bc - sum_k t_ik^ab F'_kj
-        P[G_E1].h.push_back(tg(m.t2, m.Fvv2, m.X2, 1, o * v * o, v, v, o * v * o, v, v, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, 1.0, 1.0, mi));
-        //    (one GEMM per molecule: N runs over (ia, b), so C rows are contiguous in b)
-        P[G_E2].h.push_back(tg(m.Foo2, m.t2, m.X2, 1, o, ov * v, o, o, v, o, {0, 1, 0, o, 0}, {ov, 1, 0, v, 0}, {0, v, ov, 1, 0}, -1.0, 1.0, mi));
+        P[G_E1].h.push_back(tg(m.t2, m.Fvv2, m.X2, 1, o * v * o, v, v, o * v * o, v, v, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, 1.0, 0.0, mi));
+        //    (one GEMM per molecule: N runs over (ia, b), so C rows are contiguous in b; into Cint,
+        //    which CTERM was the last to read, so that both E products share a level: c_combine adds it)
+        P[G_E2].h.push_back(tg(m.Foo2, m.t2, m.Cint, 1, o, ov * v, o, o, v, o, {0, 1, 0, o, 0}, {ov, 1, 0, v, 0}, {0, v, ov, 1, 0}, -1.0, 0.0, mi));
         // singles: r1 = F~_ai + sum_kc u_ik^ac F~_kc + sum_kcd u_ki^cd (ad|kc)~ - sum_klc u_kl^ac (ki|lc)~
         P[G_S1].h.push_back(tg(m.u, m.Fd + o, m.r1, 1, ov, 1, ov, ov, 1, v, {0, ov, v, 1, 0}, {0, 0, N, 1, 0}, {0, 1, 0, 0, 0}, 1.0, 1.0, mi));
-        P[G_S1].h.push_back(tg(m.u, m.Bov0, m.U, 1, ov, N, ov, ov, N, ov, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
+        P[G_S_U].h.push_back(tg(m.u, m.Bov0, m.U, 1, ov, N, ov, ov, N, ov, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
         P[G_S_UG].h.push_back(tg(m.U, G, m.UG, 1, ov, N, N, ov, N, N, {0, N, 0, 1, 0}, {0, N, 0, 1, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
         P[G_S_V].h.push_back(tg(m.UG, m.Y + o, m.Vs, N, o, 1, v, o, 1, v, {0, (long long)v * N, 0, N, 1}, {0, 0, 0, 1, N}, {0, N, 0, 0, 1}, 1.0, 0.0, mi));
         P[G_S_R1].h.push_back(tg(m.Vs, m.X + o, m.r1, 1, o, v, N, o, v, N, {0, N, 0, 1, 0}, {0, 1, 0, N, 0}, {0, v, 0, 1, 0}, 1.0, 1.0, mi));
-        P[G_S_R1].h.push_back(tg(m.Boo, m.UG, m.r1, 1, o, v, o * N, o, v, N, {0, 1, o, (long long)o * o, 0}, {0, N, (long long)v * N, 1, 0}, {0, v, 0, 1, 0}, -1.0, 1.0, mi));
+        P[G_S_R1B].h.push_back(tg(m.Boo, m.UG, m.r1, 1, o, v, o * N, o, v, N, {0, 1, o, (long long)o * o, 0}, {0, N, (long long)v * N, 1, 0}, {0, v, 0, 1, 0}, -1.0, 1.0, mi));
     }
-    // Note G_S_R1 holds two GEMMs into r1: they run in one launch on disjoint
-    // tiles of the same output, so they must not overlap -> keep separate groups.
-    Group extra;
-    extra.h.assign(P[G_S_R1].h.begin() + 0, P[G_S_R1].h.end());
-    P[G_S_R1].h.clear();
-    Group g1, g2;
-    for (size_t k = 0; k < extra.h.size(); ++k) (k % 2 == 0 ? g1 : g2).h.push_back(extra.h[k]);
-    P[G_S_R1] = g1;
-    P.push_back(g2);
+    // longest products first: the tiles of a launch are dealt out in order, so
+    // the short ones fill its last wave
+    for (auto &g : P)
+        std::stable_sort(g.h.begin(), g.h.end(), [](const TgemmDesc &a, const TgemmDesc &b) { return a.K > b.K; });
 }
 
 // ---------------------------------------------------------------- allocation
@@ -537,8 +539,11 @@ static int allocate(hx_ccsd *h)
             m.Bia = A.take<double>(N * ov); m.GBia = A.take<double>(N * ov);
             m.Boo = A.take<double>((size_t)N * o * o); m.GBoo = A.take<double>((size_t)N * o * o);
             m.Bvv = A.take<double>((size_t)N * v * v); m.GBvv = A.take<double>((size_t)N * v * v);
-            m.T1s = A.take<double>((size_t)o * v * o * N); m.Ts = A.take<double>((size_t)o * N * o * N);
-            m.Z = A.take<double>((size_t)o * N * o * N);
+            if (!mo_ladder(h, mi)) {
+                m.T1s = A.take<double>((size_t)o * v * o * N);
+                m.Ts = A.take<double>((size_t)o * N * o * N);
+                m.Z = A.take<double>((size_t)o * N * o * N);
+            }
             m.Woo = A.take<double>((size_t)o * o * o * o);
             m.Vvv = mo_ladder(h, mi) ? A.take<double>((size_t)v * v * v * v) : nullptr;
             m.Cint = A.take<double>(pr); m.Cp = A.take<double>(pr); m.Dint = A.take<double>(pr); m.X2 = A.take<double>(pr);
@@ -586,7 +591,7 @@ static int allocate(hx_ccsd *h)
                 case SK_NN: work = N * N; break;
                 case SK_ZDO: work = N * (ov + o * o + v * v); break;
                 case SK_PAIR: work = ov * ov; break;
-                case SK_ONON: work = o * N * o * N; break;
+                case SK_ONON: work = mo_ladder(h, mi) ? 0 : o * N * o * N; break;
                 case SK_FOCK: work = ov + v * v + o * o; break;
                 case SK_SETUP: work = ov + ov * ov + N * ov; break;
                 }
@@ -734,7 +739,7 @@ int hx_ccsd_create_batch(const hx_ppp_model *ms, int32_t n, const hx_cc_params *
         if (rc < 0) { hx_ccsd_destroy(h); return rc; }
     }
     if (p->precision != HX_PRECISION_FP64) {
-        rc = tc::create(&h->tce, h->plan, h->st, p->tile_tuning, p->tile_force);
+        rc = tc::create(&h->tce, h->plan, h->st, p->tile_tuning, p->tile_force, -1, kFp64Work);
         if (rc < 0) { hx_ccsd_destroy(h); return rc; }
     }
     if (cudaStreamSynchronize(h->st) != cudaSuccess) { hx_set_error("set-up failed"); hx_ccsd_destroy(h); return HX_ERR_CUDA; }
@@ -851,52 +856,52 @@ int hx_ccsd_init(hx_ccsd *h)
     return HX_OK;
 }
 
-// One iterationCC for every active molecule (no host synchronisation).
-static int iteration_body(hx_ccsd *h, double eps)
+// One iterationCC of the molecules in phase ph, whose launch mask is act, on
+// stream s (no host synchronisation).
+static int iteration_body(hx_ccsd *h, int ph, const int *act, cudaStream_t s)
 {
-    if (!h->device_ctl && eps != h->gate_eps) { h->gate_eps = eps; HX_TRY(upload_masks(h)); }
     auto &P = h->plan;
-    int k = 0;
-    HX_CU(hx_ew_dress_init(h->d_cc, h->d_active, h->sched, h->st));
-    HX_TRY(run_group(h, P[k++]));                                    // dress X, Y
-    HX_TRY(run_group(h, P[k++]));                                    // Pm
-    HX_CU(hx_ew_dress_fock(h->d_cc, h->d_active, h->sched, h->st));
-    HX_TRY(run_group(h, P[k++]));                                    // W1 = H2 Y
-    HX_TRY(run_group(h, P[k++]));                                    // Fd = X^T W1
-    HX_CU(hx_ew_zdo_products(h->d_cc, h->d_active, h->sched, h->st));
-    HX_TRY(run_group(h, P[k++]));                                    // G B
-    HX_CU(hx_ew_make_u(h->d_cc, h->d_active, h->sched, h->unit_smem[0], h->st));
-    HX_CU(hx_ew_fock_blocks(h->d_cc, h->d_active, h->sched, h->st));
-    HX_TRY(run_group(h, P[k++]));                                    // lead
-    HX_TRY(run_group(h, P[k++]));                                    // lad_a
-    HX_TRY(run_group(h, P[k++]));                                    // lad_b
-    HX_CU(hx_ew_gamma_scale(h->d_cc, h->d_active, h->sched, h->st));
-    HX_TRY(run_group(h, P[k++]));                                    // lad_d
-    HX_TRY(run_group(h, P[k++]));                                    // lad_e
-    HX_TRY(run_group(h, P[k++]));                                    // w_d
-    HX_TRY(run_group(h, P[k++]));                                    // w_e
-    HX_TRY(run_group(h, P[k++]));                                    // w_int
-    HX_TRY(run_group(h, P[k++]));                                    // hh
-    HX_TRY(run_group(h, P[k++]));                                    // cint1
-    HX_TRY(run_group(h, P[k++]));                                    // cint2
-    HX_TRY(run_group(h, P[k++]));                                    // cterm
-    HX_CU(hx_ew_c_combine(h->d_cc, h->d_active, h->sched, h->st));
-    HX_TRY(run_group(h, P[k++]));                                    // dint1
-    HX_TRY(run_group(h, P[k++]));                                    // dint2
-    HX_TRY(run_group(h, P[k++]));                                    // dint3
-    HX_TRY(run_group(h, P[k++]));                                    // dterm
-    HX_TRY(run_group(h, P[k++]));                                    // F'vv, F'oo
-    HX_TRY(run_group(h, P[k++]));                                    // e1
-    HX_TRY(run_group(h, P[k++]));                                    // e2
+    HX_CU(hx_ew_dress_init(h->d_cc, act, h->sched, s));
+    HX_CU(hx_ew_make_u(h->d_cc, act, h->sched, h->unit_smem[0], s));
+    HX_TRY(run_group(h, P[0], ph, act, s));               // X, Y; T1s = t2 Cv; U = u Bov0; (kc|ld) t2
+    HX_CU(hx_ew_zdo_products(h->d_cc, act, h->sched, s));
+    HX_TRY(run_group(h, P[1], ph, act, s));               // Pm; G B; Ts = Cv T1s; UG
+    HX_CU(hx_ew_dress_fock(h->d_cc, act, h->sched, s));
+    HX_CU(hx_ew_gamma_scale(h->d_cc, act, h->sched, s));
+    HX_TRY(run_group(h, P[2], ph, act, s));               // H2 Y; leading term; Cint, Dint, (ac|bd)~; Z; Vs
+    HX_TRY(run_group(h, P[3], ph, act, s));               // Fd; Cint; Dint; ladder; W_klij
+    HX_CU(hx_ew_fock_blocks(h->d_cc, act, h->sched, s));
+    HX_TRY(run_group(h, P[4], ph, act, s));               // F'vv, F'oo; u F; Dint; C ring; W_klij or hole-hole ladder
+    HX_TRY(run_group(h, P[5], ph, act, s));               // E terms; hole-hole ladder; r1 += Vs Xv
+    HX_CU(hx_ew_c_combine(h->d_cc, act, h->sched, s));
+    HX_TRY(run_group(h, P[6], ph, act, s));               // D ring; r1 -= Boo UG
     // (r2 += X2 + X2 pair-transposed is part of the step below)
-    HX_TRY(run_group(h, P[k++]));                                    // singles: u F, U
-    HX_TRY(run_group(h, P[k++]));                                    // UG
-    HX_TRY(run_group(h, P[k++]));                                    // Vs
-    HX_TRY(run_group(h, P[k++]));                                    // r1 += Vs Xv
-    HX_TRY(run_group(h, P[k++]));                                    // r1 -= Boo UG
     const int use_diis = h->p.diis_enabled ? 1 : 0;
-    HX_CU(hx_tail(h->d_cc, h->d_diis, h->d_active, h->sched, h->unit_smem + 1, h->p.t1_step, h->p.t2_step,
-                  h->p.projection_type, use_diis, h->d_gate, h->d_part, h->st));
+    HX_CU(hx_tail(h->d_cc, h->d_diis, act, h->sched, h->unit_smem + 1, h->p.t1_step, h->p.t2_step,
+                  h->p.projection_type, use_diis, h->d_gate, h->d_part, s));
+    return HX_OK;
+}
+
+// One iterationCC for every active molecule. A molecule's iteration depends on
+// no other's, so each phase in use runs its molecules' whole iteration: in a
+// captured solve as the body of one conditional node, else launched here.
+static int iterate_phases(hx_ccsd *h)
+{
+    if (!h->tce) return iteration_body(h, PH_FP64, h->d_active, h->st);
+    if (h->capturing) {
+        for (int ph = 0; ph < PH_COUNT; ++ph)
+            HX_TRY(with_condition(h, ph, [&](cudaStream_t s2) { return iteration_body(h, ph, h->d_act_ph[ph], s2); }));
+        return HX_OK;
+    }
+    int n[PH_COUNT] = {};
+    if (h->device_ctl) {                             // the phases the device counted for this iteration
+        for (int ph = 0; ph < PH_COUNT; ++ph) n[ph] = h->h_pinned[2 + ph];
+    } else {
+        for (int mi = 0; mi < h->nmol; ++mi)
+            if (h->active[mi]) ++n[h->phase[mi]];
+    }
+    for (int ph = PH_LOW; ph >= PH_FP64; --ph)
+        if (n[ph]) HX_TRY(iteration_body(h, ph, h->d_act_ph[ph], h->st));
     return HX_OK;
 }
 
@@ -911,7 +916,8 @@ int hx_ccsd_iterate(hx_ccsd *h, int32_t iteration, double eps, double acc[5])
 {
     if (!h || !h->initialized) { hx_set_error("hx_ccsd_iterate before hx_ccsd_init"); return HX_ERR_STATE; }
     (void)iteration;
-    HX_TRY(iteration_body(h, eps));
+    if (eps != h->gate_eps) { h->gate_eps = eps; HX_TRY(upload_masks(h)); }
+    HX_TRY(iterate_phases(h));
     HX_TRY(fetch_results(h));
     if (acc) {
         acc[0] = h->res[0]; acc[1] = h->res[1];
@@ -942,7 +948,8 @@ static void diis_mirror_reset(hx_ccsd *h, int mi)
 // to kPurge of the level at which that phase ended, its vectors are taken out
 // of the extrapolation: their Gram row and column are cleared and the
 // diagonal made huge, so their DIIS coefficients vanish; the slots are
-// reused by later pushes as usual.
+// reused by later pushes as usual. The same happens when the residual of the
+// next phase turns out more than twice that level.
 static const double kPurge = 0.1;
 
 
@@ -969,15 +976,22 @@ static const double kPurge = 0.1;
 // and the DIIS history restarts (its error vectors are then too noisy to mix
 // with more accurate ones).
 static const double kMidSpan = 1e-3;
+// HIGH's contractions err by about 3e-11 of their largest outputs (a few eV).
+// For targets that would take HIGH to a tenth of kHighFloor or below, it hands
+// over at kHighFloor: iterated further it converges to its own perturbed
+// solution (residual 2e-12 where the 7-slice residual is 4e-11), and the DIIS
+// vectors of that stretch held the 7-slice iterations at 4e-11 for twenty
+// iterations (63 sites, eps 1e-12).
+static const double kHighFloor = 1e-10;
 static const int kMaxFp64Returns = 3;
 
 // The iterator runs on the device (k_control, after every iteration). The
 // host uploads each molecule's iterator state and builds one CUDA graph for
 // the whole solve: a conditional while node whose body is one captured
 // iteration -- a node that sets each phase's condition from the number of
-// molecules in that phase, every contraction group with one conditional node
-// per phase (its launches masked per molecule), the element-wise kernels, the
-// tail, k_control, and a node that continues the loop while a molecule is
+// molecules in that phase, one conditional node per phase whose body is the
+// whole iteration of that phase's molecules (launches masked per molecule),
+// k_control, and a node that continues the loop while a molecule is
 // still running (at most maxiter + 8 times, so the loop always ends). The
 // host launches it once and waits. A stop request (hx_ccsd_cancel) is a word
 // of mapped host memory that k_control reads every iteration. With per-launch
@@ -1028,7 +1042,7 @@ static int solve_all(hx_ccsd *h, int maxiter, double eps)
     P.patience = h->p.mixed_patience; P.max_returns = kMaxFp64Returns; P.diis_enabled = h->p.diis_enabled;
     P.check_div = h->p.check_divergence; P.check_stag = h->p.check_stagnation; P.stag_after = h->p.stagnation_after;
     P.trace_cap = h->trace_cap; P.eps = eps; P.mixed_switch = h->p.mixed_switch; P.mid_span = kMidSpan;
-    P.high_margin = kHighMargin; P.purge = kPurge; P.div_thr = h->p.divergence_threshold;
+    P.high_margin = kHighMargin; P.high_floor = kHighFloor; P.purge = kPurge; P.div_thr = h->p.divergence_threshold;
     P.stag_thr = h->p.stagnation_threshold;
     HX_CU(cudaMemcpyAsync(h->d_ctl, c.data(), sizeof(CtlMol) * n, cudaMemcpyHostToDevice, h->st));
     h->h_pinned[0] = remaining;
@@ -1055,12 +1069,12 @@ static int solve_all(hx_ccsd *h, int maxiter, double eps)
     if (graph) {
         const long long before = g_launches.load();
         // one graph for the whole solve: a while node whose body is one
-        // iteration (the phase-condition node, every group with one conditional
-        // node per phase, the tail, k_control, then the loop condition)
+        // iteration (the phase-condition node, one conditional node per phase,
+        // k_control, then the loop condition)
         cudaGraph_t gr = nullptr;
         const char *step = "cudaGraphCreate";
         cudaError_t ce = cudaGraphCreate(&gr, 0);
-        const int ncond = (int)(h->plan.size() * PH_COUNT);
+        const int ncond = PH_COUNT;
         h->cond.clear();
         for (int ph = 0; ph < PH_COUNT; ++ph) h->phase_nodes[ph] = 0;
         if (ce == cudaSuccess && mixed && !h->d_cond) {
@@ -1094,7 +1108,7 @@ static int solve_all(hx_ccsd *h, int maxiter, double eps)
                     ce = hx_phase_conditions(h->d_occ, h->d_cond, ncond, h->d_runs, h->st);
                 }
                 h->capturing = true;
-                if (ce == cudaSuccess) rc = iteration_body(h, eps);
+                if (ce == cudaSuccess) rc = iterate_phases(h);
                 h->capturing = false;
                 if (ce == cudaSuccess && rc == HX_OK) { step = "the control kernel"; ce = control(); }
                 if (ce == cudaSuccess && rc == HX_OK) {
@@ -1158,7 +1172,7 @@ static int solve_all(hx_ccsd *h, int maxiter, double eps)
             hx_set_error("solve: cudaMemsetAsync failed");
             rc = HX_ERR_CUDA;
         }
-        if (rc == HX_OK) rc = iteration_body(h, eps);
+        if (rc == HX_OK) rc = iterate_phases(h);
         if (rc == HX_OK && control() != cudaSuccess) { hx_set_error("iterator kernel launch failed"); rc = HX_ERR_CUDA; }
         ++launched;
         if (rc != HX_OK) break;

@@ -137,5 +137,5 @@ struct CtlMol {
 struct CtlParams {
     int nmol, maxiter, mixed, check_ph, patience, max_returns, diis_enabled;
     int check_div, check_stag, stag_after, trace_cap;
-    double eps, mixed_switch, mid_span, high_margin, purge, div_thr, stag_thr;
+    double eps, mixed_switch, mid_span, high_margin, high_floor, purge, div_thr, stag_thr;
 };

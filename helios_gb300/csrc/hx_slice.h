@@ -36,6 +36,8 @@ __host__ __device__ __forceinline__ int exp_of_bits(unsigned long long mb)
 #endif
 }
 
+__host__ __device__ __forceinline__ unsigned shr_clamped(unsigned m, unsigned s);
+
 // Signed base-256 digits of a = x 2^(7-e), |a| < 128 (e from exp_of_bits of
 // the row): a = s_0 + 2^-8 s_1 + ... + 2^-8(S-1) s_(S-1) + r with |s_p| <= 128
 // and |r| <= 2^-8(S-1)-1. Integer arithmetic on the bit pattern: a rounded to
@@ -76,8 +78,31 @@ __host__ __device__ __forceinline__ void slice_digits_fast(double x, int e, int 
     constexpr int F = 8 * (S - 1);
     const unsigned long long bits = dbits(x);
     const int ex = (int)((bits >> 52) & 0x7FF);
-    const long long mant = (long long)(bits & 0xFFFFFFFFFFFFFull) | (ex ? (1LL << 52) : 0LL);
     const int sh = (ex ? ex : 1) - 1075 + 7 - e + F;       // A = mant 2^sh = a 2^F
+    if constexpr (S <= 4) {
+        // |A| <= 2^31 and, for a normal x, -sh >= 22: the top 32 bits of the significand
+        // are enough, (mant + 2^(n-1)) >> n = ((mant >> (n-1)) + 1) >> 1 with n = -sh
+        const unsigned m = 0x80000000u | (unsigned)(bits >> 21);
+        const unsigned w = shr_clamped(m, (unsigned)(-sh - 22));
+        unsigned A = (w >> 1) + (w & 1u);
+        if (ex == 0) {                                                 // zero or subnormal
+            const unsigned long long mant = bits & 0xFFFFFFFFFFFFFull;
+            A = mant == 0 || sh < -62 ? 0u : (unsigned)(sh >= 0 ? mant << sh : (mant + (1ull << (-sh - 1))) >> (-sh));
+        }
+        const bool neg = (bits >> 63) != 0;
+        if (neg) A = 0u - A;
+        int Lprev = 0;
+#pragma unroll
+        for (int k = 0; k < S - 1; ++k) {
+            const int L = (int)(A << (24 - 8 * k)) >> (24 - 8 * k);    // centered residue modulo 2^8(k+1)
+            s[S - 1 - k] = (L - Lprev) >> (8 * k);
+            Lprev = L;
+        }
+        const int top = (int)(A - (unsigned)Lprev) >> F;
+        s[0] = (S == 4 && !neg && top == -128) ? 128 : top;            // (A = 2^31 wraps)
+        return;
+    }
+    const long long mant = (long long)(bits & 0xFFFFFFFFFFFFFull) | (ex ? (1LL << 52) : 0LL);
     long long A;
     if (mant == 0 || sh < -62) A = 0;
     else if (sh >= 0) A = mant << sh;
@@ -88,12 +113,15 @@ __host__ __device__ __forceinline__ void slice_digits_fast(double x, int e, int 
 #pragma unroll
     for (int k = 0; k < S - 1; ++k) {
         const int w = 8 * (k + 1);                             // residue modulo 2^w
-        long long L;
-        if (w < 32) L = (long long)(int)((lo + (1u << (w - 1))) & ((1u << w) - 1u)) - (1LL << (w - 1));
-        else if (w == 32) L = (long long)(int)lo;
-        else L = ((A + (1LL << (w - 1))) & ((1LL << w) - 1)) - (1LL << (w - 1));
-        s[S - 1 - k] = w < 32 ? (int)((int)(L - Lprev) >> (8 * k)) : (int)((L - Lprev) >> (8 * k));
-        Lprev = L;
+        if (w < 32) {
+            const int L = (int)(lo << (32 - w)) >> (32 - w);
+            s[S - 1 - k] = (L - (int)Lprev) >> (8 * k);
+            Lprev = L;
+        } else {
+            const long long L = w == 32 ? (long long)(int)lo : ((A + (1LL << (w - 1))) & ((1LL << w) - 1)) - (1LL << (w - 1));
+            s[S - 1 - k] = (int)((L - Lprev) >> (8 * k));
+            Lprev = L;
+        }
     }
     s[0] = (int)((A - Lprev) >> F);
 }

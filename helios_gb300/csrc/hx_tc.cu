@@ -27,9 +27,14 @@
 //   1. row_scale: per row of A and B (through the descriptor's strides) the
 //      binary exponent of the largest |entry|, over 32 x 64 tiles staged in
 //      shared memory (coalesced along the source's contiguous dimension).
-//   2. split_gather: the slices, K-major, zero-padded, from the same tiles:
-//      [slice][batch][rows][Kp] (rows to 128 for A, to the tile width for B;
-//      Kp to 64). Integer arithmetic only.
+//   2. split_gather: the slices, K-major, from the same tiles:
+//      [slice][batch][rows][Kp], Kp = K to the next 8 (a TMA row pitch). No
+//      padding to tiles: TMA fills k >= K with zeros, and a tile that runs past
+//      the last row reads the next rows of the buffer (finite values), whose
+//      products only reach outputs that are not stored. So an operand's slices
+//      do not depend on the tile or on the side it is used on, and one that
+//      several products read is sliced once (per iteration, where it is marked
+//      so). Integer arithmetic only.
 //   3. tc_gemm: one CTA per 128 x BN output tile (or per K slice of it).
 //      A producer warp streams 64-deep k-blocks of all slices with TMA
 //      (cp.async.bulk.tensor, 128-byte swizzle) through a ring of stages; one
@@ -142,11 +147,11 @@ using Mid = Cfg<4, 3, 2, 64, 2, 6, 16, 64>;
 using High = Cfg<5, 4, 3, 48, 3, 8, 12, 32>;
 using Exact = Cfg<7, 6, 5, 32, 3, 6, 16, 32>;
 constexpr int TMEM_COLS = 512;
-constexpr int BM = 128, KPAD = 64;   // K is padded to KPAD (the slicing tile depth)
+constexpr int BM = 128;
 constexpr unsigned long long WAIT_NS = 4000000000ull; // a wait longer than 4 s is declared failed
 
 struct TcDesc {
-    int batch, M, N, K, Mp, Np, Kp;
+    int batch, M, N, K;
     int Mi, Ni;
     long long c[5];
     double alpha, beta;
@@ -158,8 +163,8 @@ struct TcDesc {
     int mol;
     int ksplit;                      // K slices accumulated with FP64 atomics (beta == 1 only)
     int kb_per;                      // k-blocks per slice
-    const int *expA, *expB;          // per-row binary exponents ([batch][Mp], [batch][Np])
-    CUtensorMap mapA, mapB;          // 2D maps over this desc's scratch
+    const int *expA, *expB;          // per-row binary exponents ([batch][M], [batch][N])
+    CUtensorMap mapA, mapB;          // 2D maps over the operands' slices
 };
 
 // ------------------------------------------------------------------ PTX helpers
@@ -301,13 +306,13 @@ constexpr int PT_R = 32, PT_K = 64, PT_THREADS = 256;
 
 struct PrepDesc {
     const double *src;
-    __nv_bfloat16 *dst;              // [S][batch][Rp][Kp]
-    int *rexp;                       // [batch][Rp] binary exponent of each row's largest entry
-    int batch, R, K, Rp, Kp, Ri, Ki;
+    __nv_bfloat16 *dst;              // [S][batch][R][Kp]
+    int *rexp;                       // [batch][R] binary exponent of each row's largest entry
+    int batch, R, K, Kp, Ri, Ki;     // Kp: K to the next 8
     long long s[5];                  // r0, r1, k0, k1, batch strides of the FP64 source
-    long long work_start;            // prefix of tiles (batch * ceil(Rp/PT_R) * Kp/PT_K) over the launch
-    long long row_start;             // prefix of batch*Rp over the launch
-    long long band_start;            // prefix of bands (batch * ceil(Rp/rb)) over the launch
+    long long work_start;            // prefix of tiles (batch * ceil(R/PT_R) * ceil(Kp/PT_K)) over the launch
+    long long row_start;             // prefix of batch*R over the launch
+    long long band_start;            // prefix of bands (batch * ceil(R/rb)) over the launch
     int mol;
     int rfast;                       // rows (1) or k (0) are the contiguous dimension of the source
     int rb;                          // rows per band (slice_band), 0: sliced by row_scale + split_gather
@@ -340,16 +345,15 @@ struct PrepTile {
 // Stage tile `u` of the launch in shared memory (zero outside R x K); returns
 // false (uniformly) when its molecule is inactive.
 __device__ __forceinline__ bool load_tile(const PrepDesc *__restrict__ pd, int n, long long u, const int *active,
-                                          PrepTile &t, int &b, int &r0, int &k0, bool skip_single = false)
+                                          PrepTile &t, int &b, int &r0, int &k0)
 {
     if (threadIdx.x == 0) t.desc = find_desc(pd, n, u);
     __syncthreads();
     const PrepDesc &d = pd[t.desc];
     if (active && !active[d.mol]) return false;
     if (d.rb) return false;                              // sliced by slice_band (holds no tiles)
-    if (skip_single && d.Kp == PT_K) return false;      // split_gather scales these rows itself
     long long local = u - d.work_start;
-    const int tk = d.Kp / PT_K, tr = (d.Rp + PT_R - 1) / PT_R;
+    const int tk = (d.Kp + PT_K - 1) / PT_K, tr = (d.R + PT_R - 1) / PT_R;
     k0 = (int)(local % tk) * PT_K;
     local /= tk;
     r0 = (int)(local % tr) * PT_R;
@@ -396,8 +400,7 @@ __global__ void rexp_init(const PrepDesc *__restrict__ pd, int n, long long rows
 
 // Row exponents: e with max|row| < 2^e (frexp), combined over the k tiles of a row by
 // atomicMax (the list's exponents start at INT_MIN; a row that stays there is
-// all zero and is treated as e = 0). Operands with one k tile per row are left
-// to split_gather, which scales them from the tile it slices.
+// all zero and is treated as e = 0).
 __global__ void __launch_bounds__(PT_THREADS) row_scale(const PrepDesc *__restrict__ pd, int n, long long units,
                                                         const int *__restrict__ active)
 {
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(PT_THREADS) row_scale(const PrepDesc *__restri
     const int rr = threadIdx.x >> 3, part = threadIdx.x & 7;
     for (long long u = blockIdx.x; u < units; u += gridDim.x) {
         int b, r0, k0;
-        if (load_tile(pd, n, u, active, t, b, r0, k0, true)) {
+        if (load_tile(pd, n, u, active, t, b, r0, k0)) {
             const PrepDesc &d = pd[t.desc];
             // magnitudes compare as their bit patterns with the sign cleared
             unsigned long long mb = 0;
@@ -420,7 +423,7 @@ __global__ void __launch_bounds__(PT_THREADS) row_scale(const PrepDesc *__restri
                 mb = v > mb ? v : mb;
             }
             if (part == 0 && mb != 0 && r0 + rr < d.R)
-                atomicMax(&d.rexp[(long long)b * d.Rp + r0 + rr], exp_of_bits(mb));
+                atomicMax(&d.rexp[(long long)b * d.R + r0 + rr], exp_of_bits(mb));
         }
         __syncthreads();
     }
@@ -439,42 +442,16 @@ __global__ void __launch_bounds__(PT_THREADS) split_gather(const PrepDesc *__res
         int b, r0, k0;
         if (load_tile(pd, n, u, active, t, b, r0, k0)) {
             const PrepDesc &d = pd[t.desc];
-            const bool in_rows = r0 + rr < d.Rp;  // a partial last row tile has rows beyond Rp: they write nothing
-            int e;
-            if (d.Kp == PT_K) {
-                // one k tile per row (K <= 64): the row's scale from this tile,
-                // so these operands skip row_scale (all lanes join the shuffle)
-                unsigned long long mb = 0;
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const unsigned long long v = dbits(t.x[rr][c8 + q]) & 0x7FFFFFFFFFFFFFFFull;
-                    mb = v > mb ? v : mb;
-                }
-#pragma unroll
-                for (int o = 1; o < 8; o <<= 1) {
-                    const unsigned long long v = __shfl_xor_sync(0xffffffffu, mb, o);
-                    mb = v > mb ? v : mb;
-                }
-                if ((threadIdx.x & 7) == 0 && mb != 0 && r0 + rr < d.R)
-                    d.rexp[(long long)b * d.Rp + r0 + rr] = exp_of_bits(mb);
-                e = mb != 0 ? exp_of_bits(mb) : 0;
-            } else {
-                e = in_rows ? d.rexp[(long long)b * d.Rp + r0 + rr] : 0;
+            if (r0 + rr < d.R && k0 + c8 < d.Kp) {
+                int e = d.rexp[(long long)b * d.R + r0 + rr];
                 if (e == INT_MIN) e = 0;
-            }
-            if (in_rows) {
                 uint4 out[S];
-                if (r0 + rr < d.R && k0 + c8 < d.K) {
-                    double v[8];
+                double v[8];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) v[q] = t.x[rr][c8 + q];
-                    slice8<S>(v, e, out);
-                } else {                                         // zero padding: no digits to compute
-#pragma unroll
-                    for (int p = 0; p < S; ++p) out[p] = make_uint4(0u, 0u, 0u, 0u);
-                }
-                const long long plane = (long long)d.batch * d.Rp * d.Kp;
-                const long long off = ((long long)b * d.Rp + r0 + rr) * d.Kp + k0 + c8;
+                for (int q = 0; q < 8; ++q) v[q] = t.x[rr][c8 + q];      // (zero past K)
+                slice8<S>(v, e, out);
+                const long long plane = (long long)d.batch * d.R * d.Kp;
+                const long long off = ((long long)b * d.R + r0 + rr) * d.Kp + k0 + c8;
 #pragma unroll
                 for (int p = 0; p < S; ++p) *reinterpret_cast<uint4 *>(d.dst + p * plane + off) = out[p];
             }
@@ -516,7 +493,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
         const PrepDesc &d = pd[*sdesc];
         if (d.rb == 0 || (active && !active[d.mol])) { __syncthreads(); continue; }
         const int rb = d.rb, Kp = d.Kp, ld = Kp + 2;
-        const int nb = (d.Rp + rb - 1) / rb;
+        const int nb = (d.R + rb - 1) / rb;
         const long long local = u - d.band_start;
         const int b = (int)(local / nb), r0 = (int)(local % nb) * rb;
         for (int k = threadIdx.x; k < Kp; k += PT_THREADS) koff[k] = k < d.K ? split_off(k, d.Ki, d.s[2], d.s[3]) : 0;
@@ -564,33 +541,27 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
             }
             if (lane == 0) {
                 rexp_s[r] = mb ? exp_of_bits(mb) : 0;
-                if (r < rlim) d.rexp[(long long)b * d.Rp + r0 + r] = mb ? exp_of_bits(mb) : INT_MIN;
+                if (r < rlim) d.rexp[(long long)b * d.R + r0 + r] = mb ? exp_of_bits(mb) : INT_MIN;
             }
         }
         __syncthreads();
         // (row, 8-k chunk) c of the band, walked without divisions: c advances by
         // the block size, its row and k by the block size's quotient and rest
-        const int cpr = Kp / 8, rows_band = min(rb, d.Rp - r0);
+        const int cpr = Kp / 8;
         const int dr = PT_THREADS / cpr, dk = (PT_THREADS % cpr) * 8;
-        const long long plane = (long long)d.batch * d.Rp * Kp;
-        __nv_bfloat16 *__restrict__ dst = d.dst + ((long long)b * d.Rp + r0) * Kp;
+        const long long plane = (long long)d.batch * d.R * Kp;
+        __nv_bfloat16 *__restrict__ dst = d.dst + ((long long)b * d.R + r0) * Kp;
         int r = threadIdx.x / cpr, k8 = (threadIdx.x % cpr) * 8;
-        const int rlive = min(rows_band, rlim);                 // rows past R and k past K are zero padding
-        while (r < rows_band) {
+        while (r < rlim) {
             uint4 out[S];
-            if (r < rlive && k8 < K) {
-                double v[8];
+            double v[8];
 #pragma unroll
-                for (int q = 0; q < 8; q += 2) {
-                    const double2 w2 = *reinterpret_cast<const double2 *>(x + r * ld + k8 + q);
-                    v[q] = w2.x;
-                    v[q + 1] = w2.y;
-                }
-                slice8<S>(v, rexp_s[r], out);
-            } else {
-#pragma unroll
-                for (int p = 0; p < S; ++p) out[p] = make_uint4(0u, 0u, 0u, 0u);
+            for (int q = 0; q < 8; q += 2) {
+                const double2 w2 = *reinterpret_cast<const double2 *>(x + r * ld + k8 + q);
+                v[q] = w2.x;
+                v[q + 1] = w2.y;
             }
+            slice8<S>(v, rexp_s[r], out);
 #pragma unroll
             for (int p = 0; p < S; ++p) *reinterpret_cast<uint4 *>(dst + p * plane + (long long)r * Kp + k8) = out[p];
             r += dr;
@@ -635,7 +606,7 @@ __device__ __forceinline__ TileWork tile_work(const TcDesc *__restrict__ descs, 
     w.tm = first_m + in_g % gsz;
     w.tn = in_g / gsz;
     w.kb0 = ks * d.kb_per;
-    w.nkb = min(d.Kp / C::BK - w.kb0, d.kb_per);  // >= 1 by construction
+    w.nkb = min((d.K + C::BK - 1) / C::BK - w.kb0, d.kb_per);  // >= 1 by construction
     w.nchunk = (w.nkb + C::KC - 1) / C::KC;
     return w;
 }
@@ -699,8 +670,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                 const TileWork w = tile_work<C>(descs, ndesc, tile);
                 const TcDesc &d = descs[w.di];
                 if (active && !active[d.mol]) continue;
-                const int arow0 = w.bt * d.Mp + w.tm * BM, brow0 = w.bt * d.Np + w.tn * C::BN;
-                const int aplane = d.batch * d.Mp, bplane = d.batch * d.Np;
+                const int arow0 = w.bt * d.M + w.tm * BM, brow0 = w.bt * d.N + w.tn * C::BN;
+                const int aplane = d.batch * d.M, bplane = d.batch * d.N;
                 for (int kb = 0; kb < w.nkb && ok; ++kb, ++g) {
                     const int st = (int)(g % C::STAGES);
                     const uint32_t ph = (uint32_t)((g / C::STAGES) & 1);
@@ -874,13 +845,13 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
             if (threadIdx.x < mv) {
                 const int m = w.tm * BM + threadIdx.x;
                 srow[threadIdx.x] = split_off(m, d.Mi, d.c[0], d.c[1]);
-                sexp[threadIdx.x] = d.expA[(long long)w.bt * d.Mp + m];
+                sexp[threadIdx.x] = d.expA[(long long)w.bt * d.M + m];
             }
             int eb = INT_MIN;
             double *Cn = nullptr;
             if (rr < RSTEP && nn < nv) {
                 const int n = w.tn * C::BN + nn;
-                eb = d.expB[(long long)w.bt * d.Np + n];
+                eb = d.expB[(long long)w.bt * d.N + n];
                 Cn = d.C + (long long)w.bt * d.c[4] + split_off(n, d.Ni, d.c[2], d.c[3]);
             }
             const bool load_c = d.ksplit == 1 && d.beta != 0.0;
@@ -997,22 +968,52 @@ struct PrepList {                    // operands sliced by one set of launches
     std::vector<PrepDesc> h;
     PrepDesc *d = nullptr;
     long long work = 0, rows = 0, bands = 0;
+    void add(PrepDesc p)
+    {
+        p.work_start = work;
+        p.row_start = rows;
+        p.band_start = bands;
+        if (p.rb) bands += (long long)p.batch * ((p.R + p.rb - 1) / p.rb);
+        else work += (long long)p.batch * ((p.R + PT_R - 1) / PT_R) * ((p.Kp + PT_K - 1) / PT_K);
+        rows += (long long)p.batch * p.R;
+        h.push_back(p);
+    }
 };
+
+// One operand as the products see it: a 2D view (rows x k) of an FP64 tensor
+// through split strides. Products that read the same view share its slices:
+// within a group always, across groups where the operand is constant (const)
+// or kept over an iteration (keep).
+struct Operand {
+    PrepDesc p;
+    int first, last;                 // groups of its first and last use
+    bool fixed;                      // constant between initialisations
+    size_t elems, rows;              // slice elements (S planes) and row exponents
+    size_t off = 0, roff = 0;
+};
+using OperandKey = std::array<long long, 12>;
 
 struct SubGroup {                    // one plan group in one precision mode and tile variant
     int var = 0;
     std::vector<TcDesc> tcd;         // tensor-core problems
     TcDesc *d_tcd = nullptr;
-    PrepList var_ops, fixed;         // operands sliced every run / once per initialisation
-    __nv_bfloat16 *fixed_buf = nullptr;   // slices of the constant operands (persistent)
-    int *fixed_rexp = nullptr;
-    int fixed_gen = -1;              // generation the fixed slices were made for
+    PrepList var_ops;                // operands sliced every run, before this group
     long long tiles = 0;
     Group fp64;                      // problems too small for the tensor cores
 };
 
 struct Mode {                        // one precision: one SubGroup per plan group, same order
     std::vector<SubGroup> groups;
+    std::vector<Operand> ops;
+    std::map<OperandKey, int> index;
+    std::vector<std::vector<std::array<int, 2>>> use;   // operands (A, B) of each group's tensor-core problems
+    std::vector<std::vector<char>> on_tc;               // which problems of each group run on the tensor cores
+    size_t fixed_elems = 0, fixed_rows = 0, var_elems = 0, var_rows = 0;
+    PrepList fixed;                  // operands sliced once per initialisation
+    __nv_bfloat16 *fixed_buf = nullptr;   // their slices (persistent)
+    int *fixed_rexp = nullptr;
+    int fixed_gen = -1;              // generation the fixed slices were made for
+    unsigned char *blob = nullptr;   // every descriptor array of the mode, one allocation
 };
 
 struct Engine {
@@ -1072,13 +1073,14 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
     return fn;
 }
 
-// 2D map over slices [rows][kp] bf16: boxes of bk x box_rows, swizzled to the
-// k-block's row length (128 bytes for bk = 64, 64 bytes for bk = 32).
-static int make_map(CUtensorMap *map, void *base, long long rows, int kp, int box_rows, int bk)
+// 2D map over slices [rows][kp] bf16 of which k < K are read (zeros beyond):
+// boxes of bk x box_rows, swizzled to the k-block's row length (128 bytes for
+// bk = 64, 64 bytes for bk = 32).
+static int make_map(CUtensorMap *map, void *base, long long rows, int K, int kp, int box_rows, int bk)
 {
     auto fn = encode_fn();
     if (!fn) { hx_set_error("cuTensorMapEncodeTiled is unavailable"); return HX_ERR_CUDA; }
-    cuuint64_t dims[2] = {(cuuint64_t)kp, (cuuint64_t)rows};
+    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)kp * 2};
     cuuint32_t box[2] = {(cuuint32_t)bk, (cuuint32_t)box_rows};
     cuuint32_t es[2] = {1, 1};
@@ -1164,160 +1166,215 @@ static cudaError_t prep_launch(const PrepDesc *d, int n, long long tiles, long l
 // are faster on the tensor cores; only the tiniest stay on FP64.
 static const double kMinTcWork = 1.0e4;
 
-static bool on_tc(const TgemmDesc &t) { return (double)t.batch * t.M * t.N * t.K >= kMinTcWork; }
-
-
-static void free_sub(SubGroup &sg)
+// Which problems of a group run on the tensor cores: those of at least
+// kMinTcWork multiply-adds, less the smallest ones while all that stay on the
+// FP64 kernel together take at most fp64_work.
+static std::vector<char> choose_tc(const Group &g, double fp64_work)
 {
-    cudaFree(sg.d_tcd);
-    cudaFree(sg.var_ops.d);
-    cudaFree(sg.fixed.d);
-    cudaFree(sg.fp64.d);
-    cudaFree(sg.fixed_buf);
-    cudaFree(sg.fixed_rexp);
-    sg = SubGroup();
+    const size_t n = g.h.size();
+    std::vector<char> on(n);
+    std::vector<std::pair<double, size_t>> w(n);
+    for (size_t k = 0; k < n; ++k) {
+        const TgemmDesc &t = g.h[k];
+        w[k] = {(double)t.batch * t.M * t.N * t.K, k};
+    }
+    std::sort(w.begin(), w.end());
+    double sum = 0.0;
+    for (const auto &x : w) {
+        sum += x.first;
+        on[x.second] = x.first >= kMinTcWork && sum > fp64_work;
+    }
+    return on;
 }
 
-// Slice elements (and padded rows) of a group's variable operands in one variant.
-static void var_need(const Group &g, const Variant &V, size_t &elems, size_t &rows)
+// (outer, inner) strides of a dimension of n elements split at ni: one stride
+// where the split makes no difference
+static void plain_stride(int n, int &ni, long long &s0, long long &s1)
 {
-    elems = rows = 0;
-    for (const TgemmDesc &t : g.h) {
-        if (!on_tc(t)) continue;
-        const size_t Kp = rup(t.K, KPAD), Ma = rup(t.M, BM), Nb = rup(t.N, V.BN);
-        if (!t.a_const) { elems += (size_t)V.S * t.batch * Ma * Kp; rows += (size_t)t.batch * Ma; }
-        if (!t.b_const) { elems += (size_t)V.S * t.batch * Nb * Kp; rows += (size_t)t.batch * Nb; }
+    if (ni >= n || s0 == ni * s1) { ni = n; s0 = 0; }
+    else if (ni == 1) { ni = n; s1 = s0; s0 = 0; }
+}
+
+static int add_operand(Mode &M, int S, int gi, int mol, const double *src, int batch, int R, int K, int Ri, int Ki, const long long *st,
+                       bool fixed, bool keep)
+{
+    PrepDesc p;
+    memset(&p, 0, sizeof(p));
+    p.src = src;
+    p.mol = mol;
+    p.batch = batch; p.R = R; p.K = K; p.Kp = (int)rup(K, 8); p.Ri = Ri; p.Ki = Ki;
+    for (int k = 0; k < 5; ++k) p.s[k] = st[k];
+    plain_stride(R, p.Ri, p.s[0], p.s[1]);
+    plain_stride(K, p.Ki, p.s[2], p.s[3]);
+    if (batch == 1) p.s[4] = 0;
+    p.rfast = prep_rfast(p);
+    p.rb = band_rows(p.Kp);
+    const OperandKey key{(long long)(size_t)src, batch, R, K, p.Ri, p.Ki, p.s[0], p.s[1], p.s[2], p.s[3], p.s[4],
+                         fixed || keep ? -1 : gi};
+    auto it = M.index.find(key);
+    if (it != M.index.end()) {
+        M.ops[it->second].last = gi;
+        return it->second;
+    }
+    Operand x;
+    x.p = p;
+    x.first = x.last = gi;
+    x.fixed = fixed;
+    x.rows = (size_t)batch * R;
+    x.elems = (size_t)S * x.rows * p.Kp;
+    M.ops.push_back(x);
+    M.index[key] = (int)M.ops.size() - 1;
+    return (int)M.ops.size() - 1;
+}
+
+// The operands of a plan in one precision mode and where their slices live:
+// constant ones in a buffer of the mode; the others in the scratch every mode
+// and group shares, those used by several groups in its front part, the rest
+// behind it, over again for each group.
+static void lay_out(Mode &M, int mode, const std::vector<const Group *> &plan, double fp64_work)
+{
+    const int S = variant_of(mode, 0).S;
+    M.use.resize(plan.size());
+    for (size_t gi = 0; gi < plan.size(); ++gi) {
+        // EXACT emulates FP64 with the smaller error of the two: it keeps what it has always run
+        M.on_tc.push_back(choose_tc(*plan[gi], mode == 3 ? 0.0 : fp64_work));
+        for (size_t k = 0; k < plan[gi]->h.size(); ++k) {
+            if (!M.on_tc[gi][k]) continue;
+            const TgemmDesc &t = plan[gi]->h[k];
+            M.use[gi].push_back({add_operand(M, S, (int)gi, t.mol, t.A, t.batch, t.M, t.K, t.Mi, t.Ki, t.a, t.a_const, t.a_keep),
+                                 add_operand(M, S, (int)gi, t.mol, t.B, t.batch, t.N, t.K, t.Ni, t.Ki, t.b, t.b_const, t.b_keep)});
+        }
+    }
+    size_t keep = 0, krows = 0;
+    for (Operand &x : M.ops) {
+        size_t &e = x.fixed ? M.fixed_elems : keep, &r = x.fixed ? M.fixed_rows : krows;
+        if (!x.fixed && x.first == x.last) continue;
+        x.off = e; x.roff = r;
+        e += rup(x.elems, 8); r += x.rows;
+    }
+    M.var_elems = keep; M.var_rows = krows;
+    for (size_t gi = 0; gi < plan.size(); ++gi) {
+        size_t e = keep, r = krows;
+        for (Operand &x : M.ops) {
+            if (x.fixed || x.first != (int)gi || x.last != (int)gi) continue;
+            x.off = e; x.roff = r;
+            e += rup(x.elems, 8); r += x.rows;
+        }
+        M.var_elems = std::max(M.var_elems, e);
+        M.var_rows = std::max(M.var_rows, r);
     }
 }
 
-// Descriptors, tensor maps and constant-slice storage of one plan group in
-// one precision mode and tile variant.
-static int build_sub(Engine *e, int mode, int var, const Group &g, SubGroup &sg)
+static void free_mode(Mode &M)
 {
-    const Variant &V = variant_of(mode, var);
-    const int S = V.S, BN = V.BN;
-    sg = SubGroup();
-    sg.var = var;
-    size_t fneed = 0, frows = 0;
-    for (const TgemmDesc &t : g.h) {
-        if (!on_tc(t)) continue;
-        const size_t Kp = rup(t.K, KPAD), Ma = rup(t.M, BM), Nb = rup(t.N, BN);
-        if (t.a_const) { fneed += (size_t)S * t.batch * Ma * Kp; frows += (size_t)t.batch * Ma; }
-        if (t.b_const) { fneed += (size_t)S * t.batch * Nb * Kp; frows += (size_t)t.batch * Nb; }
-    }
-    if ((fneed && cudaMalloc(&sg.fixed_buf, fneed * sizeof(__nv_bfloat16)) != cudaSuccess) ||
-        (frows && cudaMalloc(&sg.fixed_rexp, frows * sizeof(int)) != cudaSuccess)) {
-        hx_set_error("cudaMalloc of %zu bytes of constant slices failed", fneed * 2 + frows * 4);
+    cudaFree(M.blob);
+    cudaFree(M.fixed_buf);
+    cudaFree(M.fixed_rexp);
+    M = Mode();
+}
+
+// Descriptors and tensor maps of a laid-out mode (tile variant var[gi] for
+// group gi), and the storage of its constant slices.
+static int finish_mode(Engine *e, Mode &M, int mode, const std::vector<const Group *> &plan, const std::vector<int> &var)
+{
+    if ((M.fixed_elems && cudaMalloc(&M.fixed_buf, M.fixed_elems * sizeof(__nv_bfloat16)) != cudaSuccess) ||
+        (M.fixed_rows && cudaMalloc(&M.fixed_rexp, M.fixed_rows * sizeof(int)) != cudaSuccess)) {
+        hx_set_error("cudaMalloc of %zu bytes of constant slices failed", M.fixed_elems * 2 + M.fixed_rows * 4);
         return HX_ERR_NOMEM;
     }
-    size_t off = 0, roff = 0, foff = 0, froff = 0;
-    long long tiles = 0;
-    for (const TgemmDesc &t : g.h) {
-        if (!on_tc(t)) { sg.fp64.h.push_back(t); continue; }
-        TcDesc d;
-        memset(&d, 0, sizeof(d));
-        d.batch = t.batch; d.M = t.M; d.N = t.N; d.K = t.K;
-        d.Mp = (int)rup(t.M, BM); d.Np = (int)rup(t.N, BN); d.Kp = (int)rup(t.K, KPAD);
-        d.Mi = t.Mi; d.Ni = t.Ni;
-        for (int k = 0; k < 5; ++k) d.c[k] = t.c[k];
-        set_scalars(d, t.alpha, t.beta);
-        d.C = t.C; d.mol = t.mol;
-        d.tiles_m = d.Mp / BM; d.tiles_n = d.Np / BN;
-        // long K over few output tiles: cut K into slices that fill the GPU
-        const int nkb = d.Kp / V.BK, n64 = d.Kp / KPAD;
-        const long long out_tiles = (long long)d.batch * d.tiles_m * d.tiles_n;
-        int ks = 1;
-        if (t.beta == 1.0 && out_tiles < e->nsm && n64 >= 16)
-            ks = (int)std::min<long long>((e->nsm + out_tiles - 1) / out_tiles, n64 / 8);
-        d.kb_per = (nkb + ks - 1) / ks;
-        d.ksplit = (nkb + d.kb_per - 1) / d.kb_per;
-        d.tile_start = tiles;
-        tiles += out_tiles * d.ksplit;
-        const size_t asz = (size_t)S * d.batch * d.Mp * d.Kp;
-        const size_t bsz = (size_t)S * d.batch * d.Np * d.Kp;
-        __nv_bfloat16 *abuf, *bbuf;
-        int *aexp, *bexp;
-        if (t.a_const) { abuf = sg.fixed_buf + foff; foff += asz; aexp = sg.fixed_rexp + froff; froff += (size_t)t.batch * d.Mp; }
-        else { abuf = e->scratch + off; off += asz; aexp = e->rexp + roff; roff += (size_t)t.batch * d.Mp; }
-        if (t.b_const) { bbuf = sg.fixed_buf + foff; foff += bsz; bexp = sg.fixed_rexp + froff; froff += (size_t)t.batch * d.Np; }
-        else { bbuf = e->scratch + off; off += bsz; bexp = e->rexp + roff; roff += (size_t)t.batch * d.Np; }
-        if (off > e->scratch_elems) { hx_set_error("tensor-core scratch overflow"); return HX_ERR_STATE; }
-        int rc = make_map(&d.mapA, abuf, (long long)S * d.batch * d.Mp, d.Kp, BM, V.BK);
-        if (rc == HX_OK) rc = make_map(&d.mapB, bbuf, (long long)S * d.batch * d.Np, d.Kp, BN, V.BK);
-        if (rc < 0) return rc;
-        PrepDesc pa, pb;
-        memset(&pa, 0, sizeof(pa));
-        pa.src = t.A; pa.dst = abuf; pa.batch = t.batch; pa.R = t.M; pa.K = t.K;
-        pa.Rp = d.Mp; pa.Kp = d.Kp; pa.Ri = t.Mi; pa.Ki = t.Ki; pa.mol = t.mol;
-        pa.s[0] = t.a[0]; pa.s[1] = t.a[1]; pa.s[2] = t.a[2]; pa.s[3] = t.a[3]; pa.s[4] = t.a[4];
-        pa.rexp = aexp;
-        d.expA = aexp;
-        pb = pa;
-        pb.src = t.B; pb.dst = bbuf; pb.R = t.N; pb.Rp = d.Np; pb.Ri = t.Ni;
-        pb.s[0] = t.b[0]; pb.s[1] = t.b[1]; pb.s[2] = t.b[2]; pb.s[3] = t.b[3]; pb.s[4] = t.b[4];
-        pb.rexp = bexp;
-        d.expB = bexp;
-        auto add = [&](PrepList &L, PrepDesc p) {
-            p.work_start = L.work;
-            p.row_start = L.rows;
-            p.band_start = L.bands;
-            p.rfast = prep_rfast(p);
-            p.rb = band_rows(p.Kp);
-            if (p.rb) L.bands += (long long)p.batch * ((p.Rp + p.rb - 1) / p.rb);
-            else L.work += (long long)p.batch * ((p.Rp + PT_R - 1) / PT_R) * (p.Kp / PT_K);
-            L.rows += (long long)p.batch * p.Rp;
-            L.h.push_back(p);
-        };
-        add(t.a_const ? sg.fixed : sg.var_ops, pa);
-        add(t.b_const ? sg.fixed : sg.var_ops, pb);
-        sg.tcd.push_back(d);
+    if (M.var_elems > e->scratch_elems) { hx_set_error("tensor-core scratch overflow"); return HX_ERR_STATE; }
+    M.groups.resize(plan.size());
+    for (Operand &x : M.ops) {
+        x.p.dst = (x.fixed ? M.fixed_buf : e->scratch) + x.off;
+        x.p.rexp = (x.fixed ? M.fixed_rexp : e->rexp) + x.roff;
+        (x.fixed ? M.fixed : M.groups[x.first].var_ops).add(x.p);
     }
-    sg.tiles = tiles;
-    if (!sg.tcd.empty()) {
-        if (cudaMalloc(&sg.d_tcd, sizeof(TcDesc) * sg.tcd.size()) != cudaSuccess) {
-            hx_set_error("descriptor allocation failed");
-            return HX_ERR_NOMEM;
+    for (size_t gi = 0; gi < plan.size(); ++gi) {
+        SubGroup &sg = M.groups[gi];
+        sg.var = var[gi];
+        const Variant &V = variant_of(mode, sg.var);
+        size_t u = 0;
+        for (size_t k = 0; k < plan[gi]->h.size(); ++k) {
+            const TgemmDesc &t = plan[gi]->h[k];
+            if (!M.on_tc[gi][k]) { sg.fp64.h.push_back(t); continue; }
+            const Operand &a = M.ops[M.use[gi][u][0]], &b = M.ops[M.use[gi][u][1]];
+            ++u;
+            TcDesc d;
+            memset(&d, 0, sizeof(d));
+            d.batch = t.batch; d.M = t.M; d.N = t.N; d.K = t.K;
+            d.Mi = t.Mi; d.Ni = t.Ni;
+            for (int c = 0; c < 5; ++c) d.c[c] = t.c[c];
+            set_scalars(d, t.alpha, t.beta);
+            d.C = t.C; d.mol = t.mol;
+            d.tiles_m = (t.M + BM - 1) / BM; d.tiles_n = (t.N + V.BN - 1) / V.BN;
+            // long K over few output tiles: cut K into slices that fill the GPU
+            const int nkb = (t.K + V.BK - 1) / V.BK, n64 = (t.K + 63) / 64;
+            const long long out_tiles = (long long)d.batch * d.tiles_m * d.tiles_n;
+            int ks = 1;
+            if (t.beta == 1.0 && out_tiles < e->nsm && n64 >= 16)
+                ks = (int)std::min<long long>((e->nsm + out_tiles - 1) / out_tiles, n64 / 8);
+            d.kb_per = (nkb + ks - 1) / ks;
+            d.ksplit = (nkb + d.kb_per - 1) / d.kb_per;
+            d.tile_start = sg.tiles;
+            sg.tiles += out_tiles * d.ksplit;
+            d.expA = a.p.rexp;
+            d.expB = b.p.rexp;
+            int rc = make_map(&d.mapA, a.p.dst, (long long)V.S * t.batch * t.M, t.K, a.p.Kp, BM, V.BK);
+            if (rc == HX_OK) rc = make_map(&d.mapB, b.p.dst, (long long)V.S * t.batch * t.N, t.K, b.p.Kp, V.BN, V.BK);
+            if (rc < 0) return rc;
+            sg.tcd.push_back(d);
         }
-        cudaMemcpy(sg.d_tcd, sg.tcd.data(), sizeof(TcDesc) * sg.tcd.size(), cudaMemcpyHostToDevice);
-        for (PrepList *L : {&sg.var_ops, &sg.fixed}) {
-            if (L->h.empty()) continue;
-            if (cudaMalloc(&L->d, sizeof(PrepDesc) * L->h.size()) != cudaSuccess) {
-                hx_set_error("descriptor allocation failed");
-                return HX_ERR_NOMEM;
-            }
-            cudaMemcpy(L->d, L->h.data(), sizeof(PrepDesc) * L->h.size(), cudaMemcpyHostToDevice);
-        }
-    }
-    if (!sg.fp64.h.empty()) {
         sg.fp64.tiles = hx_tgemm_f64_prepare(sg.fp64.h.data(), (int)sg.fp64.h.size());
-        if (cudaMalloc(&sg.fp64.d, sizeof(TgemmDesc) * sg.fp64.h.size()) != cudaSuccess) {
-            hx_set_error("descriptor allocation failed");
-            return HX_ERR_NOMEM;
-        }
-        cudaMemcpy(sg.fp64.d, sg.fp64.h.data(), sizeof(TgemmDesc) * sg.fp64.h.size(), cudaMemcpyHostToDevice);
     }
+    // every descriptor array of the mode in one allocation and one copy
+    std::vector<unsigned char> host;
+    auto put = [&](const void *p, size_t bytes) {
+        const size_t at = rup(host.size(), 256);
+        host.resize(at + bytes);
+        if (bytes) memcpy(host.data() + at, p, bytes);
+        return at;
+    };
+    std::vector<std::array<size_t, 3>> at(plan.size());
+    for (size_t gi = 0; gi < plan.size(); ++gi) {
+        SubGroup &sg = M.groups[gi];
+        at[gi] = {put(sg.tcd.data(), sizeof(TcDesc) * sg.tcd.size()), put(sg.var_ops.h.data(), sizeof(PrepDesc) * sg.var_ops.h.size()),
+                  put(sg.fp64.h.data(), sizeof(TgemmDesc) * sg.fp64.h.size())};
+    }
+    const size_t at_fixed = put(M.fixed.h.data(), sizeof(PrepDesc) * M.fixed.h.size());
+    if (host.empty()) return HX_OK;
+    if (cudaMalloc(&M.blob, host.size()) != cudaSuccess ||
+        cudaMemcpy(M.blob, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        hx_set_error("descriptor allocation failed");
+        return HX_ERR_NOMEM;
+    }
+    for (size_t gi = 0; gi < plan.size(); ++gi) {
+        SubGroup &sg = M.groups[gi];
+        sg.d_tcd = (TcDesc *)(M.blob + at[gi][0]);
+        sg.var_ops.d = (PrepDesc *)(M.blob + at[gi][1]);
+        sg.fp64.d = (TgemmDesc *)(M.blob + at[gi][2]);
+    }
+    M.fixed.d = (PrepDesc *)(M.blob + at_fixed);
     return HX_OK;
 }
 
-// One plan group in its mode and variant: slice the operands (the constant
-// ones once per initialisation), then the persistent tcgen05 GEMM.
-static cudaError_t run_sub(Engine *e, SubGroup &sg, int mode, const int *d_active, cudaStream_t s)
+// The constant slices of a mode, once per initialisation and for every
+// molecule (molecules enter a mode at different iterations).
+static cudaError_t slice_fixed(Engine *e, Mode &M, int mode, cudaStream_t s)
+{
+    if (M.fixed_gen == e->generation) return cudaSuccess;
+    M.fixed_gen = e->generation;
+    return prep_launch(M.fixed.d, (int)M.fixed.h.size(), M.fixed.work, M.fixed.rows, M.fixed.bands, variant_of(mode, 0).S, nullptr,
+                       s, e->nsm);
+}
+
+// One plan group in its mode and variant: slice the operands first used here
+// (the constant ones once per initialisation), then the persistent tcgen05 GEMM.
+static cudaError_t run_sub(Engine *e, Mode &M, SubGroup &sg, int mode, const int *d_active, cudaStream_t s)
 {
     const Variant &V = variant_of(mode, sg.var);
-    if (sg.fp64.tiles.count > 0) {
-        cudaError_t r = hx_tgemm_f64_launch(sg.fp64.d, (int)sg.fp64.h.size(), sg.fp64.tiles, d_active, s);
-        if (r != cudaSuccess) return r;
-    }
-    if (sg.tiles == 0) return cudaSuccess;
-    cudaError_t r = cudaSuccess;
-    // constant slices are made once per initialisation, for every molecule
-    // (molecules enter a mode at different iterations)
-    if (sg.fixed_gen != e->generation) {
-        if ((r = prep_launch(sg.fixed.d, (int)sg.fixed.h.size(), sg.fixed.work, sg.fixed.rows, sg.fixed.bands, V.S,
-                             nullptr, s, e->nsm)) != cudaSuccess)
-            return r;
-        sg.fixed_gen = e->generation;
-    }
+    cudaError_t r = hx_tgemm_f64_launch(sg.fp64.d, (int)sg.fp64.h.size(), sg.fp64.tiles, d_active, s);
+    if (r != cudaSuccess || sg.tiles == 0) return r;
+    if ((r = slice_fixed(e, M, mode, s)) != cudaSuccess) return r;
     if ((r = prep_launch(sg.var_ops.d, (int)sg.var_ops.h.size(), sg.var_ops.work, sg.var_ops.rows, sg.var_ops.bands,
                          V.S, d_active, s, e->nsm)) != cudaSuccess)
         return r;
@@ -1328,7 +1385,7 @@ static cudaError_t run_sub(Engine *e, SubGroup &sg, int mode, const int *d_activ
         pend.b = take_event(e);
         for (const TcDesc &d : sg.tcd) {
             pend.flops += 2.0 * d.batch * (double)d.M * d.N * d.K;
-            pend.hwflops += 2.0 * d.batch * (double)d.Mp * d.Np * d.Kp * V.products;
+            pend.hwflops += 2.0 * d.batch * (double)d.tiles_m * BM * d.tiles_n * V.BN * rup(d.K, V.BK) * V.products;
         }
         cudaEventRecord(pend.a, s);
     }
@@ -1353,12 +1410,13 @@ using TileKey = std::array<int, 4>;
 static std::mutex g_tile_mu;
 static std::map<TileKey, int> g_tile_table;
 
-static TileKey tile_key(int mode, int gi, const Group &g)
+static TileKey tile_key(int mode, int gi, const Group &g, const std::vector<char> &on_tc)
 {
     long long maxn = 0;
     double work = 0.0;
-    for (const TgemmDesc &t : g.h) {
-        if (!on_tc(t)) continue;
+    for (size_t k = 0; k < g.h.size(); ++k) {
+        const TgemmDesc &t = g.h[k];
+        if (!on_tc[k]) continue;
         maxn = std::max<long long>(maxn, t.N);
         work += (double)t.batch * t.M * t.N * t.K;
     }
@@ -1370,7 +1428,7 @@ static TileKey tile_key(int mode, int gi, const Group &g)
 // Time every candidate of one group (one warm-up run that also slices the
 // constant operands, then the mean of three runs, CUDA events on s) and
 // return the fastest; *ms gets the time spent.
-static int tune_group(Engine *e, int mode, const Group &g, cudaStream_t s, int *best, double *spent)
+static int tune_group(Engine *e, int mode, const Group &g, double fp64_work, cudaStream_t s, int *best, double *spent)
 {
     *best = 0;
     float best_ms = 1e30f;
@@ -1382,18 +1440,22 @@ static int tune_group(Engine *e, int mode, const Group &g, cudaStream_t s, int *
     const auto t0 = std::chrono::steady_clock::now();
     int rc = HX_OK;
     for (int v = 0; v < kNumVariants[mode] && rc == HX_OK; ++v) {
-        SubGroup sg;
-        rc = build_sub(e, mode, v, g, sg);
-        if (rc == HX_OK && sg.tiles == 0) { free_sub(sg); break; }
+        Mode M;
+        const std::vector<const Group *> one{&g};
+        lay_out(M, mode, one, fp64_work);
+        rc = finish_mode(e, M, mode, one, {v});
+        if (rc == HX_OK && M.groups[0].tiles == 0) { free_mode(M); break; }
         cudaError_t ce = cudaSuccess;
-        if (rc == HX_OK) ce = run_sub(e, sg, mode, nullptr, s);
+        auto go = [&]() { return run_sub(e, M, M.groups[0], mode, nullptr, s); };
+        if (rc == HX_OK) ce = go();
         if (rc == HX_OK && ce == cudaSuccess) ce = cudaEventRecord(a, s);
-        for (int r = 0; r < 3 && rc == HX_OK && ce == cudaSuccess; ++r) ce = run_sub(e, sg, mode, nullptr, s);
+        for (int r = 0; r < 3 && rc == HX_OK && ce == cudaSuccess; ++r) ce = go();
         if (rc == HX_OK && ce == cudaSuccess) ce = cudaEventRecord(b, s);
         if (rc == HX_OK && ce == cudaSuccess) ce = cudaEventSynchronize(b);
         float ms = 0.f;
         if (rc == HX_OK && ce == cudaSuccess) ce = cudaEventElapsedTime(&ms, a, b);
-        free_sub(sg);
+        cudaStreamSynchronize(s);
+        free_mode(M);
         if (rc == HX_OK && ce != cudaSuccess) { hx_set_error("autotuner: %s", cudaGetErrorString(ce)); rc = HX_ERR_CUDA; }
         if (rc == HX_OK && error_word(e) != 0) { hx_set_error("autotuner: a tensor-core wait timed out"); rc = HX_ERR_KERNEL; }
         if (rc == HX_OK && ms < best_ms) { best_ms = ms; *best = v; }
@@ -1404,10 +1466,10 @@ static int tune_group(Engine *e, int mode, const Group &g, cudaStream_t s, int *
     return rc;
 }
 
-static int choose_variant(Engine *e, int mode, int gi, const Group &g, cudaStream_t s, int tuning, int force)
+static int choose_variant(Engine *e, int mode, int gi, const Group &g, double fp64_work, cudaStream_t s, int tuning, int force)
 {
     if (force >= 0) return std::min(force, kNumVariants[mode] - 1);
-    const TileKey key = tile_key(mode, gi, g);
+    const TileKey key = tile_key(mode, gi, g, e->mode[mode].on_tc[gi]);
     if (tuning != 2) {
         std::lock_guard<std::mutex> lock(g_tile_mu);
         auto it = g_tile_table.find(key);
@@ -1415,14 +1477,14 @@ static int choose_variant(Engine *e, int mode, int gi, const Group &g, cudaStrea
     }
     if (tuning != 1) return 0;
     int best = 0;
-    const int rc = tune_group(e, mode, g, s, &best, &e->tune_ms);
+    const int rc = tune_group(e, mode, g, fp64_work, s, &best, &e->tune_ms);
     if (rc < 0) return rc;
     std::lock_guard<std::mutex> lock(g_tile_mu);
     g_tile_table[key] = best;
     return best;
 }
 
-int create(Engine **out, const std::vector<Group> &plan, cudaStream_t s, int tuning, int force, int only_mode)
+int create(Engine **out, const std::vector<Group> &plan, cudaStream_t s, int tuning, int force, int only_mode, double fp64_work)
 {
     *out = nullptr;
     Engine *e = new Engine();
@@ -1433,16 +1495,16 @@ int create(Engine **out, const std::vector<Group> &plan, cudaStream_t s, int tun
         hx_set_error("cannot query the device's multiprocessor count");
         return HX_ERR_CUDA;
     }
-    // variable operands share one scratch: the largest group of any mode and variant
+    // variable operands share one scratch, the largest any mode needs
     size_t need = 0, need_rows = 0;
-    for (int md = 0; md < 4; ++md)
-        for (int v = 0; v < kNumVariants[md] && (only_mode < 0 || md == only_mode); ++v)
-            for (const Group &g : plan) {
-                size_t ge, gr;
-                var_need(g, variant_of(md, v), ge, gr);
-                need = std::max(need, ge);
-                need_rows = std::max(need_rows, gr);
-            }
+    std::vector<const Group *> groups;
+    for (const Group &g : plan) groups.push_back(&g);
+    for (int md = 0; md < 4; ++md) {
+        if (only_mode >= 0 && md != only_mode) continue;
+        lay_out(e->mode[md], md, groups, fp64_work);
+        need = std::max(need, e->mode[md].var_elems);
+        need_rows = std::max(need_rows, e->mode[md].var_rows);
+    }
     if ((need && cudaMalloc(&e->scratch, need * sizeof(__nv_bfloat16)) != cudaSuccess) ||
         (need_rows && cudaMalloc(&e->rexp, need_rows * sizeof(int)) != cudaSuccess) ||
         cudaMalloc(&e->d_err, sizeof(int)) != cudaSuccess) {
@@ -1464,16 +1526,16 @@ int create(Engine **out, const std::vector<Group> &plan, cudaStream_t s, int tun
         hx_set_error("cannot reserve shared memory for slice_band");
         return HX_ERR_CUDA;
     }
-    for (int md = 0; md < 4; ++md)
+    for (int md = 0; md < 4; ++md) {
+        if (only_mode >= 0 && md != only_mode) continue;
+        std::vector<int> var(plan.size());
         for (size_t gi = 0; gi < plan.size(); ++gi) {
-            if (only_mode >= 0 && md != only_mode) { e->mode[md].groups.emplace_back(); continue; }
-            int var = choose_variant(e, md, (int)gi, plan[gi], s, tuning, force);
-            if (var < 0) { destroy(e); return var; }
-            SubGroup sg;
-            int rc = build_sub(e, md, var, plan[gi], sg);
-            e->mode[md].groups.push_back(std::move(sg));
-            if (rc < 0) { destroy(e); return rc; }
+            var[gi] = choose_variant(e, md, (int)gi, plan[gi], fp64_work, s, tuning, force);
+            if (var[gi] < 0) { destroy(e); return var[gi]; }
         }
+        const int rc = finish_mode(e, e->mode[md], md, groups, var);
+        if (rc < 0) { destroy(e); return rc; }
+    }
     for (const Group &g : plan) e->keys.push_back(&g);
     ++e->generation;                  // tuning runs made constant slices of zeros: make them again
     *out = e;
@@ -1485,22 +1547,19 @@ cudaError_t run_group(Engine *e, const TgemmDesc *descs, int n, const int *d_act
     int gi = -1;
     for (size_t k = 0; k < e->keys.size(); ++k)
         if (e->keys[k]->h.data() == descs) { gi = (int)k; break; }
-    if (gi < 0 || mode < 0 || mode > 3) return cudaErrorInvalidValue;
+    if (gi < 0 || mode < 0 || mode > 3 || e->mode[mode].groups.empty()) return cudaErrorInvalidValue;
     (void)n;
-    return run_sub(e, e->mode[mode].groups[gi], mode, d_active, s);
+    return run_sub(e, e->mode[mode], e->mode[mode].groups[gi], mode, d_active, s);
 }
 
 cudaError_t prepare_fixed(Engine *e, cudaStream_t s)
 {
     if (!e) return cudaSuccess;
-    for (int md = 0; md < 4; ++md)
-        for (SubGroup &sg : e->mode[md].groups) {
-            if (sg.tiles == 0 || sg.fixed_gen == e->generation) continue;
-            const cudaError_t r = prep_launch(sg.fixed.d, (int)sg.fixed.h.size(), sg.fixed.work, sg.fixed.rows,
-                                              sg.fixed.bands, variant_of(md, sg.var).S, nullptr, s, e->nsm);
-            if (r != cudaSuccess) return r;
-            sg.fixed_gen = e->generation;
-        }
+    for (int md = 0; md < 4; ++md) {
+        if (e->mode[md].groups.empty()) continue;
+        const cudaError_t r = slice_fixed(e, e->mode[md], md, s);
+        if (r != cudaSuccess) return r;
+    }
     return cudaSuccess;
 }
 
@@ -1525,8 +1584,7 @@ double tune_ms(Engine *e) { return e ? e->tune_ms : 0.0; }
 void destroy(Engine *e)
 {
     if (!e) return;
-    for (Mode &md : e->mode)
-        for (auto &g : md.groups) free_sub(g);
+    for (Mode &md : e->mode) free_mode(md);
     for (auto &p : e->pending) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (auto x : e->pool) cudaEventDestroy(x);
     cudaFree(e->scratch);
@@ -1584,13 +1642,11 @@ namespace {
 constexpr size_t na_rup(size_t x, size_t m) { return (x + m - 1) / m * m; }
 constexpr int NA_DIM = HX_NOALLOC_MAX_DIM;
 constexpr int na_max(int a, int b) { return a > b ? a : b; }
-// padded rows of A (to 128) and of B (to either mode's tile width), padded K
-constexpr int NA_AROWS = (int)na_rup(NA_DIM, BM);
-constexpr int NA_BROWS = na_max((int)na_rup(NA_DIM, Low::BN), (int)na_rup(NA_DIM, High::BN));
-constexpr int NA_KP = (int)na_rup(NA_DIM, KPAD);
+constexpr int NA_AROWS = NA_DIM;
+constexpr int NA_BROWS = NA_DIM;
+constexpr int NA_KP = (int)na_rup(NA_DIM, 8);
 constexpr size_t NA_A_BYTES = (size_t)na_max(Low::S, High::S) * NA_AROWS * NA_KP * sizeof(__nv_bfloat16);
-constexpr size_t NA_B_BYTES = (size_t)na_max(Low::S * (int)na_rup(NA_DIM, Low::BN), High::S * (int)na_rup(NA_DIM, High::BN)) *
-                              NA_KP * sizeof(__nv_bfloat16);
+constexpr size_t NA_B_BYTES = (size_t)na_max(Low::S, High::S) * NA_BROWS * NA_KP * sizeof(__nv_bfloat16);
 constexpr size_t NA_OFF_A = 0;
 constexpr size_t NA_OFF_B = na_rup(NA_OFF_A + NA_A_BYTES, 1024);
 constexpr size_t NA_OFF_REXP = na_rup(NA_OFF_B + NA_B_BYTES, 256);          // int[NA_AROWS + NA_BROWS]
@@ -1678,34 +1734,34 @@ extern "C" int hx_gemm_noalloc(const double *dA, const double *dB, double *dC, i
     memset(&d, 0, sizeof(d));
     d.batch = 1; d.M = M; d.N = N; d.K = K;
     const int BK = high ? High::BK : Low::BK;
-    d.Mp = (int)rup(M, BM); d.Np = (int)rup(N, BN); d.Kp = (int)rup(K, KPAD);
+    const int Kp = (int)rup(K, 8);
     d.Mi = M; d.Ni = N;
     d.c[0] = 0; d.c[1] = N; d.c[2] = 0; d.c[3] = 1; d.c[4] = 0;
     set_scalars(d, 1.0, 1.0);
     d.C = dC; d.mol = 0;
-    d.tiles_m = d.Mp / BM; d.tiles_n = d.Np / BN;
-    d.kb_per = d.Kp / BK;            // K <= 512: at most 16 k-blocks, never split
+    d.tiles_m = (M + BM - 1) / BM; d.tiles_n = (N + BN - 1) / BN;
+    d.kb_per = (K + BK - 1) / BK;    // K <= 512: at most 16 k-blocks, never split
     d.ksplit = 1;
     d.tile_start = 0;
     d.expA = aexp; d.expB = bexp;
-    if ((rc = make_map(&d.mapA, abuf, (long long)S * d.Mp, d.Kp, BM, BK)) != HX_OK) return rc;
-    if ((rc = make_map(&d.mapB, bbuf, (long long)S * d.Np, d.Kp, BN, BK)) != HX_OK) return rc;
+    if ((rc = make_map(&d.mapA, abuf, (long long)S * M, K, Kp, BM, BK)) != HX_OK) return rc;
+    if ((rc = make_map(&d.mapB, bbuf, (long long)S * N, K, Kp, BN, BK)) != HX_OK) return rc;
     PrepDesc p[2];
     memset(p, 0, sizeof(p));
     p[0].src = dA; p[0].dst = abuf; p[0].rexp = aexp; p[0].batch = 1; p[0].R = M; p[0].K = K;
-    p[0].Rp = d.Mp; p[0].Kp = d.Kp; p[0].Ri = M; p[0].Ki = K;
+    p[0].Kp = Kp; p[0].Ri = M; p[0].Ki = K;
     p[0].s[0] = 0; p[0].s[1] = K; p[0].s[2] = 0; p[0].s[3] = 1; p[0].s[4] = 0;
     p[1] = p[0];
-    p[1].src = dB; p[1].dst = bbuf; p[1].rexp = bexp; p[1].R = N; p[1].Rp = d.Np; p[1].Ri = N;
+    p[1].src = dB; p[1].dst = bbuf; p[1].rexp = bexp; p[1].R = N; p[1].Ri = N;
     p[0].rfast = prep_rfast(p[0]);
     p[1].rfast = prep_rfast(p[1]);
     // K <= 512: both operands are sliced in one pass, in bands of rb rows
-    const int rb = band_rows(d.Kp);
+    const int rb = band_rows(Kp);
     p[0].rb = p[1].rb = rb;
-    p[1].band_start = (d.Mp + rb - 1) / rb;
-    p[1].row_start = d.Mp;
-    const long long rows = (long long)d.Mp + d.Np;
-    const long long bands = p[1].band_start + (d.Np + rb - 1) / rb;
+    p[1].band_start = (M + rb - 1) / rb;
+    p[1].row_start = M;
+    const long long rows = (long long)M + N;
+    const long long bands = p[1].band_start + (N + rb - 1) / rb;
     const long long tiles = (long long)d.tiles_m * d.tiles_n;
 
     // what must start at zero: the error word and C (accumulated with beta = 1)
