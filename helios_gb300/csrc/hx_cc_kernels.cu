@@ -20,6 +20,8 @@
 //                 energy partials of the result.
 // Only the canonical blocks i <= j are stepped and stored, as the reference
 // stores only the pairs (ia) <= (jb).
+#include <mutex>
+
 #include "hx_common.cuh"
 #include "hx_plan.h"
 #include "hx_kernels.h"
@@ -839,14 +841,22 @@ size_t hx_unit_smem(const int *o, const int *v, int nmol, int kernel)
     return (size_t)mx * sizeof(double);
 }
 
+// The attribute belongs to the kernel, not to a handle: it is only ever
+// raised, so that a handle of small molecules does not take it from under one
+// of large molecules made before.
 cudaError_t hx_unit_kernels_init(size_t smem_max)
 {
-    cudaError_t e = cudaSuccess;
-    const int b = (int)smem_max;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_make_u, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_push, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_amplitudes_energy, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    return e;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    const void *kernels[] = {(const void *)k_make_u, (const void *)k_step_push, (const void *)k_amplitudes_energy};
+    for (const void *k : kernels) {
+        cudaFuncAttributes a;
+        cudaError_t e = cudaFuncGetAttributes(&a, k);
+        if (e == cudaSuccess && (size_t)a.maxDynamicSharedSizeBytes < smem_max)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t hx_ew_make_u(const CCMol *m, const int *act, const HxSched &S, size_t smem, cudaStream_t s)
