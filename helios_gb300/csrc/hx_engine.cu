@@ -1418,8 +1418,8 @@ void hx_ccsd_destroy(hx_ccsd *h)
 // formulas), over the occupied triples i <= j <= k. The integrals come from
 // the site basis: I1[i][a][b][d] = (ai|bd) = (G C_ai)^T C_bd and J[k][c][j][l]
 // = (ck|jl) = C_ck^T G C_jl, FP64 GEMMs once per call. The triples are taken
-// in slabs (one i, a range of j, every k >= j), each within a byte budget
-// (a few GB whatever the molecule): for a slab W_ijk^abc is formed directly as
+// in slabs (whole (i, j) rows, every k >= j; one slab up to about 64 sites),
+// each within a byte budget: for a slab W_ijk^abc is formed directly as
 // the six pair permutations of X, twelve GEMMs of (v^2 x v x v) and
 // (v^2 x v x o) per (i, j), batched over k, on the 7-slice tensor-core GEMM
 // (an emulated FP64 product, as accurate as the FP64 one), then the energy
@@ -1473,10 +1473,11 @@ int hx_ccsd_triples(hx_ccsd *h, int32_t mol, double e[4])
     // slab budget: W (v^3 doubles per triple) plus the 7-slice bf16 copies of the
     // operands a k-batched term (P4, P6) slices per triple (14 B per element of a
     // v^2 x K tile, K padded to 64)
-    const double per_pair = 8.0 * vvv + 14.0 * ((v * v + 127) / 128 * 128) * (double)((v + 63) / 64 * 64);
+    // (its own operands are sliced once per slab: 14 B per element of (bd|ai), (ck|jl) and t2)
+    const double per_pair = 8.0 * vvv + 14.0 * (double)(v * v) * ((v + 7) / 8 * 8);
     size_t fre = 0, tot = 0;
     HX_CU(cudaMemGetInfo(&fre, &tot));
-    const double fixed_bytes = 8.0 * (nI1 + nJ + nBvv + 2 * nBoo);
+    const double fixed_bytes = 8.0 * (nI1 + nJ + nBvv + 2 * nBoo) + 28.0 * (2.0 * nI1 + 4.0 * nJ + 6.0 * (double)ov * ov);
     const double budget = std::min(24e9, 0.5 * ((double)fre - fixed_bytes));
     const long long max_pairs = (long long)(budget / per_pair);
     if (max_pairs < o) {
@@ -1484,26 +1485,31 @@ int hx_ccsd_triples(hx_ccsd *h, int32_t mol, double e[4])
                      "%.1f GB are free", N, (fixed_bytes + o * per_pair) / 1e9, fre / 1e9);
         return HX_ERR_NOMEM;
     }
-    // slabs: (i, j0, j1) with sum_{j0 <= j < j1} (o - j) <= max_pairs
-    struct Slab { int i, j0, j1; long long pairs; };
-    std::vector<Slab> slabs;
+    // slabs of rows (i, j) with sum (o - j) <= max_pairs triples
+    struct Slab { std::vector<std::array<int, 2>> rows; long long pairs = 0; };
+    std::vector<Slab> slabs(1);
     long long maxp = 0;
     for (int i = 0; i < o; ++i)
-        for (int j0 = i; j0 < o;) {
-            int j1 = j0;
-            long long p = 0;
-            while (j1 < o && p + (o - j1) <= max_pairs) { p += o - j1; ++j1; }
-            slabs.push_back({i, j0, j1, p});
-            maxp = std::max(maxp, p);
-            j0 = j1;
+        for (int j = i; j < o; ++j) {
+            if (slabs.back().pairs + (o - j) > max_pairs) slabs.emplace_back();
+            slabs.back().rows.push_back({i, j});
+            slabs.back().pairs += o - j;
+            maxp = std::max(maxp, slabs.back().pairs);
         }
+    std::vector<unsigned> abc;
+    for (int a = 0; a < v; ++a)
+        for (int b = 0; b <= a; ++b)
+            for (int c = 0; c <= b; ++c) abc.push_back((unsigned)a << 16 | (unsigned)b << 8 | (unsigned)c);
     const size_t nW = (size_t)maxp * vvv;
     const size_t elems = nI1 + nJ + nBvv + 2 * nBoo + nW + 2 * (size_t)maxp + 2 * slabs.size();
     double *buf = nullptr;
-    int2 *d_pairs = nullptr;
+    int3 *d_triples = nullptr;
+    unsigned *d_abc = nullptr;
     HX_CU(cudaMalloc(&buf, elems * sizeof(double)));
-    if (cudaMalloc(&d_pairs, sizeof(int2) * (size_t)maxp) != cudaSuccess) {
+    if (cudaMalloc(&d_triples, sizeof(int3) * (size_t)maxp) != cudaSuccess ||
+        cudaMalloc(&d_abc, sizeof(unsigned) * abc.size()) != cudaSuccess) {
         cudaFree(buf);
+        cudaFree(d_triples);
         hx_set_error("hx_ccsd_triples: allocation failed");
         return HX_ERR_NOMEM;
     }
@@ -1521,26 +1527,33 @@ int hx_ccsd_triples(hx_ccsd *h, int32_t mol, double e[4])
         rc = upload_group(g);
         if (rc == HX_OK) ce = hx_tgemm_f64_launch(g.d, (int)g.h.size(), g.tiles, nullptr, h->st);
     }
-    std::vector<int2> pairs;
+    if (ce == cudaSuccess && rc == HX_OK)
+        ce = cudaMemcpyAsync(d_abc, abc.data(), sizeof(unsigned) * abc.size(), cudaMemcpyHostToDevice, h->st);
+    std::vector<int3> triples;
     for (size_t si = 0; si < slabs.size() && rc == HX_OK && ce == cudaSuccess; ++si) {
         const Slab &sl = slabs[si];
         std::vector<Group> plan(12);
-        pairs.clear();
-        for (int j = sl.j0; j < sl.j1; ++j) {
-            double *Wj = W + (long long)pairs.size() * vvv;
-            for (int t = 0; t < 12; ++t) plan[t].h.push_back(triples_term(t, m, I1, J, Wj, sl.i, j));
-            for (int k = j; k < o; ++k) pairs.push_back(make_int2(j, k));
+        triples.clear();
+        for (const auto &row : sl.rows) {
+            const int i = row[0], j = row[1];
+            double *Wj = W + (long long)triples.size() * vvv;
+            for (int t = 0; t < 12; ++t) {
+                TgemmDesc d = triples_term(t, m, I1, J, Wj, i, j);
+                d.a_keep = d.b_keep = 1;                 // t2 and the integrals stay: sliced once for all terms
+                plan[t].h.push_back(d);
+            }
+            for (int k = j; k < o; ++k) triples.push_back(make_int3(i, j, k));
         }
         tc::Engine *te = nullptr;
         rc = tc::create(&te, plan, h->st, 2, 0, 3);      // the 7-slice (emulated FP64) mode only
         for (int t = 0; t < 12 && rc == HX_OK && ce == cudaSuccess; ++t)
             ce = tc::run_group(te, plan[t].h.data(), (int)plan[t].h.size(), nullptr, h->st, 3);
         if (rc == HX_OK && ce == cudaSuccess)
-            ce = cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice, h->st);
+            ce = cudaMemcpyAsync(d_triples, triples.data(), sizeof(int3) * triples.size(), cudaMemcpyHostToDevice, h->st);
         if (rc == HX_OK && ce == cudaSuccess)
-            ce = hx_triples_energy(W, d_pairs, (int)pairs.size(), sl.i, m.t1, m.gov, m.Fmo, N, o, part, out + 2 * si,
-                                   h->st);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->st);   // the pair list is pageable host memory
+            ce = hx_triples_energy(W, d_triples, (int)triples.size(), d_abc, (int)abc.size(), m.t1, m.gov, m.Fmo, N, o, part,
+                                   out + 2 * si, h->st);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->st);   // the lists are pageable host memory
         if (rc == HX_OK && ce == cudaSuccess && te && tc::error_word(te)) {
             hx_set_error("hx_ccsd_triples: a tensor-core wait timed out");
             rc = HX_ERR_KERNEL;
@@ -1553,7 +1566,8 @@ int hx_ccsd_triples(hx_ccsd *h, int32_t mol, double e[4])
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->st);
     for (auto &g : gs) if (g.d) cudaFree(g.d);
     cudaFree(buf);
-    cudaFree(d_pairs);
+    cudaFree(d_triples);
+    cudaFree(d_abc);
     if (rc != HX_OK) return rc;
     if (ce != cudaSuccess) { hx_set_error("hx_ccsd_triples: %s", cudaGetErrorString(ce)); return HX_ERR_CUDA; }
     double e4 = 0.0, e5 = 0.0;

@@ -31,13 +31,13 @@ cudaError_t hx_energy(const CCMol *m, const DiisMol *h, const int *act, const Hx
 cudaError_t hx_layout(double *t1, double *t2, double *f1, double *f2, int o, int v, bool to_engine, cudaStream_t s);
 
 // (T) triples (hx_triples.cu): ZDO pair products of the occupied and virtual
-// orbitals; the energy partials of a slab of triples (i, j, k) for one i, the
-// pairs (j, k) listed in `pairs`, and their ordered sum (out[0] = E[4],
-// out[1] = E[5] of the slab, each triple weighted by its permutations).
+// orbitals; the energy partials of a slab of triples i <= j <= k, and their
+// ordered sum (out[0] = E[4], out[1] = E[5] of the slab, each triple weighted
+// by its permutations). abc: the virtual triples a >= b >= c, 8 bits each.
 cudaError_t hx_triples_pairs(const double *C, int N, int o, double *Bvv0, double *Boo0, cudaStream_t s);
-cudaError_t hx_triples_energy(const double *W, const int2 *pairs, int npairs, int i, const double *t1,
-                              const double *gov, const double *Fmo, int N, int o, double *part, double *out,
-                              cudaStream_t s);
+cudaError_t hx_triples_energy(const double *W, const int3 *triples, int ntriples, const unsigned *abc, int nabc,
+                              const double *t1, const double *gov, const double *Fmo, int N, int o, double *part,
+                              double *out, cudaStream_t s);
 
 // Device-side iterator (hx_control.cu): record the solve's start time; after an
 // iteration apply the stop rules and the phase ladder, write the next

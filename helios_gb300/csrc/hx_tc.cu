@@ -61,6 +61,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <unordered_map>
 #include <vector>
 
 #include "hx_common.cuh"
@@ -990,8 +991,18 @@ struct Operand {
     bool fixed;                      // constant between initialisations
     size_t elems, rows;              // slice elements (S planes) and row exponents
     size_t off = 0, roff = 0;
+    CUtensorMap map[2];              // as A and as B, made at the first use on that side
+    int box[2] = {0, 0}, bk[2] = {0, 0};
 };
 using OperandKey = std::array<long long, 12>;
+struct OperandHash {
+    size_t operator()(const OperandKey &k) const
+    {
+        unsigned long long x = 1469598103934665603ull;
+        for (long long v : k) x = (x ^ (unsigned long long)v) * 1099511628211ull;
+        return (size_t)(x ^ (x >> 29));
+    }
+};
 
 struct SubGroup {                    // one plan group in one precision mode and tile variant
     int var = 0;
@@ -1005,7 +1016,7 @@ struct SubGroup {                    // one plan group in one precision mode and
 struct Mode {                        // one precision: one SubGroup per plan group, same order
     std::vector<SubGroup> groups;
     std::vector<Operand> ops;
-    std::map<OperandKey, int> index;
+    std::unordered_map<OperandKey, int, OperandHash> index;
     std::vector<std::vector<std::array<int, 2>>> use;   // operands (A, B) of each group's tensor-core problems
     std::vector<std::vector<char>> on_tc;               // which problems of each group run on the tensor cores
     size_t fixed_elems = 0, fixed_rows = 0, var_elems = 0, var_rows = 0;
@@ -1297,7 +1308,7 @@ static int finish_mode(Engine *e, Mode &M, int mode, const std::vector<const Gro
         for (size_t k = 0; k < plan[gi]->h.size(); ++k) {
             const TgemmDesc &t = plan[gi]->h[k];
             if (!M.on_tc[gi][k]) { sg.fp64.h.push_back(t); continue; }
-            const Operand &a = M.ops[M.use[gi][u][0]], &b = M.ops[M.use[gi][u][1]];
+            Operand &a = M.ops[M.use[gi][u][0]], &b = M.ops[M.use[gi][u][1]];
             ++u;
             TcDesc d;
             memset(&d, 0, sizeof(d));
@@ -1319,9 +1330,17 @@ static int finish_mode(Engine *e, Mode &M, int mode, const std::vector<const Gro
             sg.tiles += out_tiles * d.ksplit;
             d.expA = a.p.rexp;
             d.expB = b.p.rexp;
-            int rc = make_map(&d.mapA, a.p.dst, (long long)V.S * t.batch * t.M, t.K, a.p.Kp, BM, V.BK);
-            if (rc == HX_OK) rc = make_map(&d.mapB, b.p.dst, (long long)V.S * t.batch * t.N, t.K, b.p.Kp, V.BN, V.BK);
-            if (rc < 0) return rc;
+            for (int side = 0; side < 2; ++side) {
+                Operand &x = side ? b : a;
+                const int box = side ? V.BN : BM;
+                if (x.box[side] != box || x.bk[side] != V.BK) {
+                    const int rc = make_map(&x.map[side], x.p.dst, (long long)V.S * x.rows, t.K, x.p.Kp, box, V.BK);
+                    if (rc < 0) return rc;
+                    x.box[side] = box;
+                    x.bk[side] = V.BK;
+                }
+                (side ? d.mapB : d.mapA) = x.map[side];
+            }
             sg.tcd.push_back(d);
         }
         sg.fp64.tiles = hx_tgemm_f64_prepare(sg.fp64.h.data(), (int)sg.fp64.h.size());

@@ -11,7 +11,11 @@
 // (k_t_energy), over the triples i <= j <= k, each weighted by its number of
 // distinct permutations. E[4] + E[5] equals the spin-orbital (T) of the
 // connected and disconnected triples amplitudes. One block per occupied
-// triple, its threads over the v^3 virtual triples (32-bit index arithmetic).
+// triple, its threads over the virtual triples a >= b >= c: the FP64 pipe is
+// the bound, and the six permutations of (a, b, c) share D and the sums
+// P = W_abc + W_bca + W_cab, Q = W_acb + W_bac + W_cba (Y = 3W + P - 2Q on the
+// first three, 3W + Q - 2P on the others): 9 FP64 operations per element
+// instead of about 50 with two divisions each.
 #include <algorithm>
 
 #include "hx_common.cuh"
@@ -45,34 +49,55 @@ __global__ void k_t_pairs(const double *__restrict__ C, int N, int o, double *__
     }
 }
 
-// Per-block partials of E[4] and E[5] for one triple (i, j, k), i <= j <= k:
-// the block's W_ijk^abc (v^3, [a][b][c]) sits in the slab at pair `blockIdx.x`;
+// Per-block partials of 3 E[4] and 3 E[5] for one triple (i, j, k), i <= j <= k:
+// the block's W_ijk^abc (v^3, [a][b][c]) sits in the slab at triple `blockIdx.x`;
 // the triple counts w = 6, 3 or 1 times (its distinct permutations: the
 // energy of a triple is unchanged by a simultaneous permutation of (ia),
-// (jb), (kc)).
-__global__ void __launch_bounds__(TNT) k_t_energy(const double *__restrict__ W, const int2 *__restrict__ pairs, int i,
+// (jb), (kc)). abc: the nabc virtual triples a >= b >= c, packed 8 bits each.
+__global__ void __launch_bounds__(TNT) k_t_energy(const double *__restrict__ W, const int3 *__restrict__ triples,
+                                                  const unsigned *__restrict__ abc, int nabc,
                                                   const double *__restrict__ t1, const double *__restrict__ gov,
                                                   const double *__restrict__ Fmo, int N, int o, int v,
                                                   double *__restrict__ part)
 {
-    const int j = pairs[blockIdx.x].x, k = pairs[blockIdx.x].y;
-    const int v2 = v * v, v3 = v2 * v;
+    __shared__ double ev[256];
+    const int i = triples[blockIdx.x].x, j = triples[blockIdx.x].y, k = triples[blockIdx.x].z;
+    const int v2 = v * v;
     const long long ov = (long long)o * v;
-    const double *Wb = W + (long long)blockIdx.x * v3;
+    const double *Wb = W + (long long)blockIdx.x * v2 * v;
+    // (jb|kc), (ia|kc), (ia|jb) as v x v blocks of gov, and the rows of t1
+    const double *gjk = gov + (long long)j * v * ov + (long long)k * v, *gik = gov + (long long)i * v * ov + (long long)k * v,
+                 *gij = gov + (long long)i * v * ov + (long long)j * v;
+    const double *ti = t1 + (long long)i * v, *tj = t1 + (long long)j * v, *tk = t1 + (long long)k * v;
+    for (int a = threadIdx.x; a < v; a += TNT) ev[a] = Fmo[(long long)(o + a) * N + o + a];
+    __syncthreads();
     const double eijk = Fmo[(long long)i * N + i] + Fmo[(long long)j * N + j] + Fmo[(long long)k * N + k];
     const double wt = (i == j && j == k) ? 1.0 : ((i == j || j == k) ? 3.0 : 6.0);
     double e4 = 0.0, e5 = 0.0;
-    for (int abc = threadIdx.x; abc < v3; abc += TNT) {
-        const int c = abc % v, b = (abc / v) % v, a = abc / v2;
-        const double w = Wb[abc];
-        const double y = 4.0 * w + Wb[(c * v + a) * v + b] + Wb[(b * v + c) * v + a]
-                       - 2.0 * Wb[(a * v + c) * v + b] - 2.0 * Wb[(b * v + a) * v + c] - 2.0 * Wb[(c * v + b) * v + a];
-        const long long ia = (long long)i * v + a, jb = (long long)j * v + b, kc = (long long)k * v + c;
-        const double z = gov[jb * ov + kc] * t1[ia] + gov[ia * ov + kc] * t1[jb] + gov[ia * ov + jb] * t1[kc];
-        const double d = eijk - Fmo[(long long)(o + a) * N + o + a] - Fmo[(long long)(o + b) * N + o + b]
-                       - Fmo[(long long)(o + c) * N + o + c];
-        e4 += w * y / (3.0 * d);
-        e5 += z * y / (3.0 * d);
+    for (int e = threadIdx.x; e < nabc; e += TNT) {
+        const unsigned x = abc[e];
+        const int a = x >> 16, b = (x >> 8) & 255, c = x & 255;
+        // the six permutations (p, q, r) of (a, b, c): even ones first
+        const int p[6] = {a, b, c, a, b, c}, q[6] = {b, c, a, c, a, b}, r[6] = {c, a, b, b, c, a};
+        double w[6], s4 = 0.0, s5 = 0.0;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) w[m] = Wb[(p[m] * v + q[m]) * v + r[m]];
+        const double P = (w[0] + w[1]) + w[2], Q = (w[3] + w[4]) + w[5];
+        const double ye = fma(-2.0, Q, P), yo = fma(-2.0, P, Q);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const double y = fma(3.0, w[m], m < 3 ? ye : yo);
+            double z = gjk[q[m] * ov + r[m]] * ti[p[m]];
+            z = fma(gik[p[m] * ov + r[m]], tj[q[m]], z);
+            z = fma(gij[p[m] * ov + q[m]], tk[r[m]], z);
+            s4 = fma(w[m], y, s4);
+            s5 = fma(z, y, s5);
+        }
+        // equal indices: the six permutations repeat the distinct ones two or six times
+        const double rep = a == c ? 6.0 : (a == b || b == c) ? 2.0 : 1.0;
+        const double d = 1.0 / (rep * (eijk - ((ev[a] + ev[b]) + ev[c])));
+        e4 = fma(s4, d, e4);
+        e5 = fma(s5, d, e5);
     }
     __shared__ double sh[2][TNT / 32];
     e4 = t_warp_sum(e4);
@@ -92,6 +117,7 @@ __global__ void k_t_final(const double *__restrict__ part, long long nblk, doubl
 {
     __shared__ double sh[2][32];
     double s4 = 0.0, s5 = 0.0;
+#pragma unroll 8
     for (long long b = threadIdx.x; b < nblk; b += 32) { s4 += part[2 * b]; s5 += part[2 * b + 1]; }
     sh[0][threadIdx.x] = s4;
     sh[1][threadIdx.x] = s5;
@@ -99,8 +125,8 @@ __global__ void k_t_final(const double *__restrict__ part, long long nblk, doubl
     if (threadIdx.x == 0) {
         double a = 0.0, b = 0.0;
         for (int t = 0; t < 32; ++t) { a += sh[0][t]; b += sh[1][t]; }
-        out[0] = a;
-        out[1] = b;
+        out[0] = a / 3.0;
+        out[1] = b / 3.0;
     }
 }
 }  // namespace
@@ -114,15 +140,14 @@ cudaError_t hx_triples_pairs(const double *C, int N, int o, double *Bvv0, double
     return cudaGetLastError();
 }
 
-cudaError_t hx_triples_energy(const double *W, const int2 *pairs, int npairs, int i, const double *t1,
-                              const double *gov, const double *Fmo, int N, int o, double *part, double *out,
-                              cudaStream_t s)
+cudaError_t hx_triples_energy(const double *W, const int3 *triples, int ntriples, const unsigned *abc, int nabc,
+                              const double *t1, const double *gov, const double *Fmo, int N, int o, double *part,
+                              double *out, cudaStream_t s)
 {
-    const int v = N - o;
-    k_t_energy<<<(unsigned)npairs, TNT, 0, s>>>(W, pairs, i, t1, gov, Fmo, N, o, v, part);
+    k_t_energy<<<(unsigned)ntriples, TNT, 0, s>>>(W, triples, abc, nabc, t1, gov, Fmo, N, o, N - o, part);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_t_final<<<1, 32, 0, s>>>(part, npairs, out);
+    k_t_final<<<1, 32, 0, s>>>(part, ntriples, out);
     hx_count_launches(2);
     return cudaGetLastError();
 }
