@@ -23,11 +23,15 @@
 //  * a round is one pass: the rotated matrix is written to a second buffer, as
 //    2 x 2 blocks J_k^T A J_l of its upper triangle, so a round has one barrier
 //    and every CTA derives the next round's rotations from the finished matrix;
-//  * the rotation angle is taken in FP32 (a tangent within 1e-6 of the exact
-//    one leaves an off-diagonal 1e-6 of its size, which the quadratic
-//    convergence absorbs); its cosine is brought to FP64 by one third-order
-//    Newton step on 1/sqrt(1 + t^2), so the rotation is orthogonal to FP64;
-//  * pairs far below the convergence threshold are not rotated.
+//  * the SCF iterations take the rotation angle in FP32 (a tangent within 1e-6
+//    of the exact one leaves an off-diagonal 1e-6 of its size, which the
+//    quadratic convergence absorbs); its cosine is brought to FP64 by one
+//    third-order Newton step on 1/sqrt(1 + t^2), so the rotation is orthogonal
+//    to FP64;
+//  * they diagonalise to a millionth of the iteration's own accuracy, and pairs
+//    far below that are not rotated;
+//  * V's rows stay in shared memory, and a round's matrix elements are fetched
+//    while its angles are computed.
 // Measured on whole calls, one CTA (a cooperative grid for one molecule above
 // 64 sites) with three barriers a round before: a 38-site energy 88 -> 75 ms,
 // 63 sites 182 -> 143 ms, 160 sites 1672 -> 1591 ms, a batch of 128 molecules
@@ -163,13 +167,27 @@ __device__ __forceinline__ void circle_pair(int k, int r, int np, int &p, int &q
     if (p > q) { const int t = p; p = q; q = t; }
 }
 
-// Rotation (c, s) that annihilates apq to within FP32's precision of the
-// tangent; the identity when |apq| <= thr.
+// Rotation (c, s) that annihilates apq, the identity when |apq| <= thr. GUESS:
+// in FP64 throughout. The diagonalisation from scratch turns by large angles
+// whose choices between two nearly equal diagonal entries decide the orbitals'
+// signs; with FP32 tangents one molecule in ten of 90-112 sites came out with
+// other signs than the FP64 rotations give, and amplitudes follow those signs.
+// The SCF iterations start from the last basis, turn by small angles and keep
+// its signs: there the tangent is taken in FP32, and its cosine by one
+// third-order Newton step (no sign differed in 60 such molecules).
+template <bool GUESS>
 __device__ __forceinline__ void rotation(double app, double aqq, double apq, double thr, double &c, double &s)
 {
     c = 1.0;
     s = 0.0;
     if (!(fabs(apq) > thr)) return;
+    if (GUESS) {
+        const double theta = (aqq - app) / (2.0 * apq);
+        const double t = fabs(theta) > 1e150 ? 0.5 / theta : (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+        c = 1.0 / sqrt(t * t + 1.0);
+        s = t * c;
+        return;
+    }
     const float den = (float)(apq + apq);
     if (den == 0.0f) return;
     const float theta = (float)(aqq - app) / den;
@@ -182,18 +200,79 @@ __device__ __forceinline__ void rotation(double app, double aqq, double apq, dou
     s = t * c;
 }
 
+// Item e of a round: the 2 x 2 block (k, l), k <= l, of the upper triangle of
+// pairs (row k and row h - 1 - k folded into h + 1 items); false for the
+// repeated half of the middle row.
+__device__ __forceinline__ bool round_item(int e, int h, int &k, int &l)
+{
+    const int k0 = e / (h + 1), d = e - k0 * (h + 1);
+    if (d < h - k0) { k = k0; l = k0 + d; return true; }
+    k = h - 1 - k0;
+    l = k + d - (h - k0);
+    return k != k0;
+}
+
+// The elements of a block and where they sit (upper triangle) in round r.
+struct Block2 {
+    int i00, i01, i10, i11;
+    bool hq, hv;                                         // (a bye has no second player)
+    double a00, a01, a10, a11;
+    template <class Ctx>
+    __device__ __forceinline__ void load(const double *cur, int k, int l, int r, int np, int n)
+    {
+        int p, q, u, v;
+        circle_pair(k, r, np, p, q);
+        circle_pair(l, r, np, u, v);
+        hq = q < n;
+        hv = v < n;
+        i00 = p < u ? p * n + u : u * n + p;
+        i01 = p < v ? p * n + v : v * n + p;
+        i10 = q < u ? q * n + u : u * n + q;
+        i11 = q < v ? q * n + v : v * n + q;
+        a00 = Ctx::ld(cur + i00);
+        a01 = hv ? Ctx::ld(cur + i01) : 0.0;
+        a10 = hq ? Ctx::ld(cur + i10) : 0.0;
+        a11 = hq && hv ? Ctx::ld(cur + i11) : 0.0;
+    }
+    // J_k^T A J_l into nxt
+    __device__ __forceinline__ void rotate(double *nxt, double ck, double sk, double cl, double sl, bool diag) const
+    {
+        double x00 = a00, x01 = a01, x10 = a10, x11 = a11;
+        if (sl != 0.0) {
+            x00 = cl * a00 - sl * a01; x01 = sl * a00 + cl * a01;
+            x10 = cl * a10 - sl * a11; x11 = sl * a10 + cl * a11;
+        }
+        if (sk != 0.0) {
+            const double y00 = x00, y01 = x01;
+            x00 = ck * y00 - sk * x10; x01 = ck * y01 - sk * x11;
+            x10 = sk * y00 + ck * x10; x11 = sk * y01 + ck * x11;
+        }
+        nxt[i00] = x00;
+        if (hv) nxt[i01] = x01;
+        if (hq && !diag) nxt[i10] = x10;
+        if (hq && hv) nxt[i11] = x11;
+    }
+};
+
 // Jacobi eigen-decomposition of the symmetric n x n matrix in A (upper
-// triangle read; A and A2 are both overwritten); rotations accumulate into V.
-// W is n x n scratch. pc, ps, pd and rank_s are shared arrays of the CTA.
-template <class Ctx>
-__device__ void jacobi(Ctx &c, double *A, double *A2, double *V, double *E, double *W, int n, double *pc, double *ps,
-                       double *pd, int *rank_s)
+// triangle read; A and A2 are both overwritten) until its off-diagonal norm
+// is at most tol (and at least FP64's 1e-15 of the matrix); rotations
+// accumulate into V, this CTA's rows of it in the shared buffer vs. pc, ps,
+// pd and rank_s are shared arrays of the CTA. A round's chain is: the pairs'
+// entries from L2, their angles, the blocks, the barrier; the blocks' entries
+// are fetched with the pairs' by the warps that do not compute angles.
+template <bool GUESS, class Ctx>
+__device__ void jacobi(Ctx &c, double *A, double *A2, double *V, double *E, double *vs, int n, double tol, double *pc,
+                       double *ps, double *pd, int *rank_s)
 {
     const int np = n + (n & 1), h = np / 2;
-    // items of a round: 2 x 2 blocks (k, l), k <= l, of the upper triangle (row
-    // k and row h - 1 - k folded into h + 1 items), and row pieces of V
-    const int nblk = ((h + 1) / 2) * (h + 1);
+    const int nblk = ((h + 1) / 2) * (h + 1), step = c.size * NT;
     const int rows = (n + c.size - 1) / c.size, row0 = c.rank * rows, nrow = max(0, min(rows, n - row0));
+    for (int e = threadIdx.x; e < nrow * n; e += NT) vs[e] = V[row0 * n + e];
+    // items dealt out over the CTAs, within one to the last warps first
+    const int first = c.rank + c.size * (NT - 1 - (int)threadIdx.x);
+    int k1 = 0, l1 = 0;
+    const bool has = first < nblk && round_item(first, h, k1, l1);
     double *cur = A, *nxt = A2;
     for (int sweep = 0; sweep < 40; ++sweep) {
         double off = 0.0, tot = 0.0;
@@ -206,47 +285,28 @@ __device__ void jacobi(Ctx &c, double *A, double *A2, double *V, double *E, doub
         c.reduce2(off, tot, false);
         off += off;
         tot += off;
-        if (off <= 1e-30 * tot || off < 1e-300) break;
+        const double goal = fmax(1e-30 * tot, tol * tol);
+        if (off <= goal || off < 1e-300) break;
         // all pairs at thr would leave off at a quarter of its bound
-        const double thr = 0.5e-15 * sqrt(tot) / n;
+        const double thr = GUESS ? 1e-300 : 0.5 * sqrt(goal) / n;
         for (int r = 0; r < np - 1; ++r) {
+            Block2 b;
+            if (has) b.load<Ctx>(cur, k1, l1, r, np, n);
             for (int k = threadIdx.x; k < h; k += NT) {
                 int p, q;
                 double cc = 1.0, s = 0.0;
                 circle_pair(k, r, np, p, q);
-                if (q < n) rotation(c.ld(cur + p * n + p), c.ld(cur + q * n + q), c.ld(cur + p * n + q), thr, cc, s);
+                if (q < n) rotation<GUESS>(c.ld(cur + p * n + p), c.ld(cur + q * n + q), c.ld(cur + p * n + q), thr, cc, s);
                 pc[k] = cc;
                 ps[k] = s;
             }
             __syncthreads();
-            for (int e = c.tid; e < nblk; e += c.nt) {
-                const int k0 = e / (h + 1), d = e - k0 * (h + 1);
+            if (has) b.rotate(nxt, pc[k1], ps[k1], pc[l1], ps[l1], k1 == l1);
+            for (int e = first + step; e < nblk; e += step) {
                 int k, l;
-                if (d < h - k0) { k = k0; l = k0 + d; }
-                else { k = h - 1 - k0; l = k + d - (h - k0); if (k == k0) continue; }
-                int p, q, u, v;
-                circle_pair(k, r, np, p, q);
-                circle_pair(l, r, np, u, v);
-                const bool hq = q < n, hv = v < n;                     // (both p and u exist)
-                const int i00 = p < u ? p * n + u : u * n + p, i01 = p < v ? p * n + v : v * n + p;
-                const int i10 = q < u ? q * n + u : u * n + q, i11 = q < v ? q * n + v : v * n + q;
-                const double a00 = c.ld(cur + i00), a01 = hv ? c.ld(cur + i01) : 0.0;
-                const double a10 = hq ? c.ld(cur + i10) : 0.0, a11 = hq && hv ? c.ld(cur + i11) : 0.0;
-                const double ck = pc[k], sk = ps[k], cl = pc[l], sl = ps[l];
-                double x00 = a00, x01 = a01, x10 = a10, x11 = a11;
-                if (sl != 0.0) {
-                    x00 = cl * a00 - sl * a01; x01 = sl * a00 + cl * a01;
-                    x10 = cl * a10 - sl * a11; x11 = sl * a10 + cl * a11;
-                }
-                if (sk != 0.0) {
-                    const double y00 = x00, y01 = x01;
-                    x00 = ck * y00 - sk * x10; x01 = ck * y01 - sk * x11;
-                    x10 = sk * y00 + ck * x10; x11 = sk * y01 + ck * x11;
-                }
-                nxt[i00] = x00;
-                if (hv) nxt[i01] = x01;
-                if (hq && k != l) nxt[i10] = x10;
-                if (hq && hv) nxt[i11] = x11;
+                if (!round_item(e, h, k, l)) continue;
+                b.load<Ctx>(cur, k, l, r, np, n);
+                b.rotate(nxt, pc[k], ps[k], pc[l], ps[l], k == l);
             }
             // this CTA's rows of V: V <- V J
             for (int e = threadIdx.x; e < nrow * h; e += NT) {
@@ -256,7 +316,7 @@ __device__ void jacobi(Ctx &c, double *A, double *A2, double *V, double *E, doub
                 const double cs = pc[k];
                 int p, q;
                 circle_pair(k, r, np, p, q);
-                double *row = V + (row0 + i) * n;
+                double *row = vs + i * n;
                 const double x = row[p], y = row[q];
                 row[p] = cs * x - s * y;
                 row[q] = s * x + cs * y;
@@ -265,7 +325,7 @@ __device__ void jacobi(Ctx &c, double *A, double *A2, double *V, double *E, doub
             double *t = cur; cur = nxt; nxt = t;
         }
     }
-    // sort ascending: rank each eigenvalue, permute V's columns through W
+    // sort ascending: rank each eigenvalue, permute V's columns
     for (int p = threadIdx.x; p < n; p += NT) pd[p] = c.ld(cur + p * n + p);
     __syncthreads();
     for (int p = threadIdx.x; p < n; p += NT) {
@@ -277,16 +337,17 @@ __device__ void jacobi(Ctx &c, double *A, double *A2, double *V, double *E, doub
     }
     __syncthreads();
     for (int e = threadIdx.x; e < nrow * n; e += NT) {
-        const int row = row0 + e / n, p = e % n;
-        W[row * n + rank_s[p]] = V[row * n + p];
+        const int i = e / n, p = e - i * n;
+        V[(row0 + i) * n + rank_s[p]] = vs[e];
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nrow * n; e += NT) V[row0 * n + e] = W[row0 * n + e];
     c.sync();
 }
 
+// off-diagonal norm an iteration of accuracy acc diagonalises to
+__device__ __forceinline__ double current_tol(double acc, double eps) { return acc >= eps ? 1e-6 * acc : 0.0; }
+
 template <class Ctx>
-__device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, double *pc, double *ps, double *pd, int *rank_s)
+__device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, double *vs, double *pc, double *ps, double *pd, int *rank_s)
 {
     const int n = m.N, no = m.nocc, nn = n * n;
     double *F = m.F, *D = m.D, *V = m.V, *A = m.A, *W1 = m.W1, *W2 = m.W2;
@@ -302,7 +363,7 @@ __device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, double *
             V[e] = (e / n == e % n) ? 1.0 : 0.0;
         }
         c.sync();
-        jacobi(c, A, W2, V, m.E, W1, n, pc, ps, pd, rank_s);
+        jacobi<true>(c, A, W2, V, m.E, vs, n, 0.0, pc, ps, pd, rank_s);
         density(c, D, V, n, no);
     }
     fock(c, F, m.core, m.G, D, n);
@@ -325,10 +386,12 @@ __device__ void scf_body(Ctx &c, const ScfMol &m, const ScfParams &prm, double *
         for (int e = c.tid; e < nn; e += c.nt) D[e] -= prm.step * W1[e];
         c.sync();
         fock(c, F, m.core, m.G, D, n);
-        // diagonalise F in the current basis: A = V^T F V
+        // diagonalise F in the current basis: A = V^T F V, to a millionth of this
+        // iteration's accuracy (the density's own error stays that far below it;
+        // a converged iteration diagonalises to FP64)
         mm(c, W1, F, V, n, false, false, n);
         mm(c, A, V, W1, n, true, false, n);
-        jacobi(c, A, W2, V, m.E, W1, n, pc, ps, pd, rank_s);
+        jacobi<false>(c, A, W2, V, m.E, vs, n, current_tol(acc, prm.eps), pc, ps, pd, rank_s);
         density(c, D, V, n, no);
         fock(c, F, m.core, m.G, D, n);
 
@@ -369,19 +432,20 @@ __global__ void __launch_bounds__(NT) scf_kernel(const ScfMol *__restrict__ mols
     __shared__ double sh[2 * NT / 32];
     __shared__ double pc[HX_MAX_MOL_N / 2], ps[HX_MAX_MOL_N / 2], pd[HX_MAX_MOL_N];
     __shared__ int rank_s[HX_MAX_MOL_N];
-    __shared__ double mat[6][kBlockN * kBlockN];
+    extern __shared__ double dyn[];       // one CTA: seven matrices; a cluster: this CTA's rows of V
     const int cs = (int)cg::this_cluster().num_blocks(), mol = (int)blockIdx.x / cs;
     ScfMol m = mols[mol];
     if (m.N > kBlockN) {
         ClusterCtx c(sh, gpart + (long long)mol * 4 * cs);
-        scf_body(c, m, prm, pc, ps, pd, rank_s);
+        scf_body(c, m, prm, dyn, pc, ps, pd, rank_s);
         return;
     }
     if (cg::this_cluster().block_rank() != 0) return;
     BlockCtx c(sh);
     const ScfMol g = m;
-    m.F = mat[0]; m.D = mat[1]; m.V = mat[2]; m.A = mat[3]; m.W1 = mat[4]; m.W2 = mat[5];
-    scf_body(c, m, prm, pc, ps, pd, rank_s);
+    constexpr int NN = kBlockN * kBlockN;
+    m.F = dyn; m.D = dyn + NN; m.V = dyn + 2 * NN; m.A = dyn + 3 * NN; m.W1 = dyn + 4 * NN; m.W2 = dyn + 5 * NN;
+    scf_body(c, m, prm, dyn + 6 * NN, pc, ps, pd, rank_s);
     __syncthreads();
     for (int e = threadIdx.x; e < m.N * m.N; e += NT) { g.F[e] = m.F[e]; g.D[e] = m.D[e]; g.V[e] = m.V[e]; }
 }
@@ -403,8 +467,12 @@ cudaError_t hx_scf_launch(const ScfMol *d_mols, int nmol, int nmax, const ScfPar
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    const int kMaxSmem = sizeof(double) * (HX_MAX_MOL_N / 8) * HX_MAX_MOL_N;     // 8 CTAs at the largest N
+    cudaError_t ce = cudaFuncSetAttribute(scf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    if (ce != cudaSuccess) return ce;
     if (cs > 8) {
         int n = 0;
+        cfg.dynamicSmemBytes = kMaxSmem;
         at[0].val.clusterDim.x = cs;
         cfg.gridDim = dim3((unsigned)cs);
         if (cudaFuncSetAttribute(scf_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
@@ -413,6 +481,9 @@ cudaError_t hx_scf_launch(const ScfMol *d_mols, int nmol, int nmax, const ScfPar
             cs = 8;
         }
     }
+    // the smaller form's matrices, or the rows of V of the largest molecule
+    const size_t rows_v = (size_t)((nmax + cs - 1) / cs) * nmax;
+    cfg.dynamicSmemBytes = sizeof(double) * std::max<size_t>(7 * kBlockN * kBlockN, nmax > kBlockN ? rows_v : 0);
     at[0].val.clusterDim.x = cs;
     cfg.gridDim = dim3((unsigned)nmol * cs);
     hx_count_launches(1);
