@@ -227,4 +227,22 @@ __host__ __device__ __forceinline__ int class_count(float a, int q)
     return (u >> 31) ? -(int)n : (int)n;
 }
 
+// v 2^k as an FP64 value, rounded to nearest even, for a fixed-point v;
+// `ok` cleared where the result is not a normal number. Integer operations
+// only: the conversion, scaling and the sum it replaces take eight slots of
+// GB300's FP64 pipe per output.
+__host__ __device__ __forceinline__ double fixed_pow2(long long v, int k, bool &ok)
+{
+    if (v == 0) return 0.0;
+    const unsigned long long u = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+    const int lz = clz64(u);
+    const unsigned long long n = u << lz;                      // leading bit at 63
+    unsigned long long m = n >> 11;
+    const unsigned rem = (unsigned)n & 0x7FFu;
+    m += rem > 0x400u || (rem == 0x400u && (m & 1ull));        // (a carry out of m moves the exponent up)
+    const int e = 63 - lz + k + 1023;
+    if (e < 1 || e > 2046) { ok = false; return 0.0; }
+    return dfrom((v < 0 ? 0x8000000000000000ull : 0ull) + ((unsigned long long)(e - 1) << 52) + m);
+}
+
 }  // namespace tc

@@ -129,6 +129,8 @@ struct Cfg {
     // (units of 2^-8(NX-1)); the other modes use an FP32 (hi, lo) pair
     static constexpr bool INT_DRAIN = S_ >= 7;
     static constexpr float DRAIN_SCALE = (float)(1ull << (8 * (NX_ - 1)));
+    static constexpr int FIXED_K = 256;              // 7-slice products up to this K leave the tile in fixed point
+    static_assert(!INT_DRAIN || (NX_ == 5 && FIXED_K <= 32 * KC_ * BK_), "fixed-point headroom");
     static constexpr int PRODUCTS = [] { int n = 0; for (int i = 0; i < S_; ++i) for (int j = 0; j < S_; ++j) n += (i + j <= QMAX_); return n; }();
     // pairs in the largest exact class
     static constexpr int XPAIRS = [] { int m = 0; for (int q = 0; q < NX_; ++q) { int n = 0; for (int i = 0; i < S_; ++i) n += (q - i >= 0 && q - i < S_); m = n > m ? n : m; } return m; }();
@@ -637,7 +639,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr int LD = C::BN + 1;
     float2 *strip = (float2 *)(smem + C::STAGES * C::STAGE_BYTES);   // [STG_ROWS][BN + 1] (hi, lo) of the outputs
-    double *dstrip = (double *)strip;                                 // the same, 7-slice values
+    double *dstrip = (double *)strip;                                 // the same, 7-slice values: FP64
+    long long *istrip = (long long *)strip;                           // or fixed point (short K)
     long long *srow = (long long *)(strip + C::STG_ROWS * LD);       // [BM] row offsets into C
     int *sexp = (int *)(srow + BM);                                   // [BM] row exponents of A
     uint64_t *full = (uint64_t *)(sexp + BM);
@@ -857,14 +860,27 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
             }
             const bool load_c = d.ksplit == 1 && d.beta != 0.0;
             const uint32_t negmask = d.alpha_neg ? 0x80000000u : 0u;
+            // 7-slice products with K <= FIXED_K leave the tile as one fixed-point number, the
+            // exact classes' count with the merged class added at 2^-FBITS of a count: the sum
+            // stays below K 2^46.1 counts, so FBITS = 15 - ceil(log2 K) bits fit in int64 and
+            // the merged class is rounded (2^-40 at K = 256) below what truncating the operands to
+            // seven slices leaves (2^-37).
+            // Their epilogue is the bound (short K, FP64 pipe); longer products keep FP64.
+            int fbits = 0;
+            if constexpr (C::INT_DRAIN)
+                if (d.K <= C::FIXED_K) fbits = 15 - (32 - __clz(d.K - 1));
             for (int r0 = 0; r0 < mv; r0 += C::STG_ROWS) {
                 if (row >= r0 && row < r0 + C::STG_ROWS) {
 #pragma unroll
                     for (int e = 0; e < C::EPI_COLS; ++e) {
-                        if constexpr (C::INT_DRAIN)
-                            dstrip[(row - r0) * LD + col0 + e] =
-                                (dacc[e] + (double)iacc[e]) * (1.0 / (double)C::DRAIN_SCALE) + (double)macc[e];
-                        else
+                        if constexpr (C::INT_DRAIN) {
+                            if (fbits)
+                                istrip[(row - r0) * LD + col0 + e] =
+                                    (iacc[e] << fbits) + __float2int_rn(macc[e] * (C::DRAIN_SCALE * (float)(1 << fbits)));
+                            else
+                                dstrip[(row - r0) * LD + col0 + e] =
+                                    (dacc[e] + (double)iacc[e]) * (1.0 / (double)C::DRAIN_SCALE) + (double)macc[e];
+                        } else
                             strip[(row - r0) * LD + col0 + e] = make_float2(hi[e], lo[e]);
                     }
                 }
@@ -888,6 +904,12 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                                 const int k = ea + eb - 14 + d.alpha_e;
                                 bool fast = d.alpha_pow2 != 0 && k >= -896 && k <= 896;
                                 if constexpr (C::INT_DRAIN) {
+                                    if (fbits) {
+                                        const long long v = istrip[(mm - r0) * LD + nn];
+                                        if (fast) r = fixed_pow2(d.alpha_neg ? -v : v, k - 8 * (C::NX - 1) - fbits, fast);
+                                        if (!fast) r = d.alpha * scale_pow2((double)v / ((double)C::DRAIN_SCALE * (double)(1 << fbits)), ea, eb);
+                                        goto scaled;
+                                    }
                                     const double v = dstrip[(mm - r0) * LD + nn];
                                     if (fast) {
                                         r = pow2_int(v, k, fast);
@@ -900,6 +922,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                                     else r = d.alpha * scale_pow2((double)v.x + (double)v.y, ea, eb);
                                 }
                             }
+                        scaled:
                             double *p = Cn + srow[mm];
                             if (d.ksplit > 1) atomicAdd(p, r);
                             else *p = load_c ? (d.beta_one ? r + old[u] : fma(d.beta, old[u], r)) : r;
