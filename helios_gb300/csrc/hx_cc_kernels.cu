@@ -84,18 +84,25 @@ __global__ void k_dress_init(EW_ARGS)
 }
 
 // H2 = h - G o Pm + 2 diag(G diag Pm), Pm = Yo Xo^T (dressed half density)
-__global__ void k_dress_fock(EW_ARGS)
+__global__ void __launch_bounds__(NT) k_dress_fock(EW_ARGS)
 {
+    __shared__ double diag[HX_EW_CHUNK / 2 + 2];
     EW_PROLOGUE
     const int n = m.N;
+    // the diagonal elements of this block's stretch: rows r0 .. r1 - 1, a warp per sum
+    const long long end = min(base_ + HX_EW_CHUNK, (long long)n * n);
+    const int r0 = (int)((base_ + n) / (n + 1)), r1 = (int)((end + n) / (n + 1));
+    for (int i = r0 + (int)(threadIdx.x >> 5); i < r1; i += NT / 32) {
+        double s = 0.0;
+        for (int l = threadIdx.x & 31; l < n; l += 32) s += m.G[i * n + l] * m.Pm[l * n + l];
+        s = warp_sum(s);
+        if ((threadIdx.x & 31) == 0) diag[i - r0] = s;
+    }
+    __syncthreads();
     EW_LOOP(e, (long long)n * n) {
-        int i = (int)(e / n), j = (int)(e % n);
+        const int i = (int)(e / n), j = (int)(e % n);
         double f = m.h[e] - m.G[e] * m.Pm[e];
-        if (i == j) {
-            double s = 0.0;
-            for (int l = 0; l < n; ++l) s += m.G[i * n + l] * m.Pm[l * n + l];
-            f += 2.0 * s;
-        }
+        if (i == j) f += 2.0 * diag[i - r0];
         m.H2[e] = f;
     }
 }
@@ -224,8 +231,11 @@ __device__ __forceinline__ long long pair_off(int i, int a, int j, int b, int o,
 // tile, its lanes the columns b, so global reads and writes run along b (one
 // division per row, none per element); shared-memory index of (lb, a, b) is
 // (lb v + a)(v + 1) + b.
-#define ROW_LOOP(nrows) for (int row_ = threadIdx.x >> 5; row_ < (nrows); row_ += NT / 32)
-#define COL_LOOP(b, v) for (int b = threadIdx.x & 31; b < (v); b += 32)
+// With few virtual orbitals a warp walks several rows at once (lg: log2 of the
+// lanes per row), so that its FP64 slots are not spent on idle lanes.
+#define ROW_LANES(v) const int lg_ = (v) <= 4 ? 2 : (v) <= 8 ? 3 : (v) <= 16 ? 4 : 5;
+#define ROW_LOOP(nrows) for (int row_ = threadIdx.x >> lg_; row_ < (nrows); row_ += NT >> lg_)
+#define COL_LOOP(b, v) for (int b = threadIdx.x & ((1 << lg_) - 1); b < (v); b += 1 << lg_)
 
 // K sums over the block at once (two barriers); valid in thread 0
 template <int K>
@@ -295,6 +305,7 @@ __global__ void __launch_bounds__(NT) k_make_u(const CCMol *__restrict__ mols, c
     if ((active && !active[w.mol]) || w.u == 0) return;
     const CCMol &m = mols[w.mol];
     const int o = m.o, v = m.v, nrows = w.nb * v;
+    ROW_LANES(v)
     const double *__restrict__ t2 = m.t2;
     double *__restrict__ u = m.u;
 #pragma unroll 4
@@ -350,6 +361,7 @@ __global__ void __launch_bounds__(NT) k_step_push(const CCMol *__restrict__ mols
     double mx = 0.0;
     long long hoff;
     const int nrows = w.nb * v;
+    ROW_LANES(v)
     if (w.u == 0) {
         hoff = 0;
         for (int e = threadIdx.x; e < ov; e += NT) {
@@ -505,13 +517,10 @@ __global__ void __launch_bounds__(NT) k_diis_solve(const CCMol *__restrict__ mol
     }
     if (n == 1) return;                                // newCCVectors(1) returns early
     // the bordered system [B 1; 1 0] c = e by Gaussian elimination with partial
-    // pivoting in shared memory, the right-hand side as one more column: warp 0
-    // searches the pivot and divides the column by it, all threads update the
-    // rows (a serial elimination of 21 x 21 in one thread took 40 us of a
-    // 12-site iteration)
-    constexpr int MB = HX_MAX_DIIS + 1, LD = MB + 1;
-    __shared__ double A[MB * LD], f[MB];
-    __shared__ int piv_s;
+    // pivoting in shared memory, the right-hand side as one more column, by one
+    // warp (a lane per row, no block barriers): 21 pivots of a 21 x 21 system
+    constexpr int MB = HX_MAX_DIIS + 1, LD = MB + 1 + (MB & 1);
+    __shared__ double A[MB * LD];
     const int nb = n + 1;
     __syncthreads();
     for (int e = threadIdx.x; e < nb * (nb + 1); e += NT) {
@@ -524,41 +533,33 @@ __global__ void __launch_bounds__(NT) k_diis_solve(const CCMol *__restrict__ mol
         A[p * LD + q] = val;
     }
     __syncthreads();
+    if (warp != 0) return;
     for (int k = 0; k < nb; ++k) {
-        if (warp == 0) {
-            double best = -1.0;
-            int piv = k;
-            for (int r = k + lane; r < nb; r += 32)
-                if (fabs(A[r * LD + k]) > best) { best = fabs(A[r * LD + k]); piv = r; }
+        double best = -1.0;
+        int piv = k;
+        for (int r = k + lane; r < nb; r += 32)
+            if (fabs(A[r * LD + k]) > best) { best = fabs(A[r * LD + k]); piv = r; }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {         // the first row of the largest magnitude
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int op = __shfl_xor_sync(0xffffffffu, piv, o);
-                if (ob > best || (ob == best && op < piv)) { best = ob; piv = op; }
-            }
-            const double d = A[piv * LD + k];
-            for (int r = k + lane; r < nb; r += 32)    // row factors, in the order after the swap
-                if (r != k) f[r] = A[(r == piv ? k : r) * LD + k] / d;
-            if (lane == 0) piv_s = piv;
+        for (int o = 16; o > 0; o >>= 1) {             // the first row of the largest magnitude
+            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int op = __shfl_xor_sync(0xffffffffu, piv, o);
+            if (ob > best || (ob == best && op < piv)) { best = ob; piv = op; }
         }
-        __syncthreads();
-        const int piv = piv_s;
-        if (piv != k) {
-            for (int c = k + threadIdx.x; c <= nb; c += NT) {
+        if (piv != k)
+            for (int c = k + lane; c <= nb; c += 32) {
                 const double t = A[k * LD + c];
                 A[k * LD + c] = A[piv * LD + c];
                 A[piv * LD + c] = t;
             }
-            __syncthreads();
+        __syncwarp();
+        const double d = A[k * LD + k];
+        for (int r = k + 1 + lane; r < nb; r += 32) {
+            const double f = A[r * LD + k] / d;
+#pragma unroll 4
+            for (int c = k + 1; c <= nb; ++c) A[r * LD + c] -= f * A[k * LD + c];
         }
-        const int w = nb - k;                          // columns k + 1 .. nb
-        for (int e = threadIdx.x; e < (nb - 1 - k) * w; e += NT) {
-            const int r = k + 1 + e / w, c = k + 1 + e % w;
-            A[r * LD + c] -= f[r] * A[k * LD + c];
-        }
-        __syncthreads();
+        __syncwarp();
     }
-    if (warp != 0) return;
     // back substitution by columns: once x_k is known every row above takes its share
     for (int k = nb - 1; k >= 0; --k) {
         const double xk = A[k * LD + nb] / A[k * LD + k];
@@ -625,6 +626,7 @@ __global__ void __launch_bounds__(NT) k_amplitudes_energy(const CCMol *__restric
         }
         __syncthreads();
         const int nrows = w.nb * v;
+        ROW_LANES(v)
         const long long hoff = ov + (long long)w.k0 * v * v;
 #pragma unroll 2
         ROW_LOOP(nrows) {

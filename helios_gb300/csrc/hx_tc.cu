@@ -326,8 +326,16 @@ struct PrepDesc {
 // BAND_ELEMS doubles), so the row maxima come from the staged band and the
 // FP64 source is read once; wider operands take row_scale + split_gather.
 constexpr int BAND_KP = 1024, BAND_ELEMS = 4096;
-constexpr int BAND_SMEM = (BAND_ELEMS + 64) * 8 + BAND_KP * 8 + 32 * 8 + 32 * 4 + 16;
-__host__ __device__ constexpr int band_rows(int Kp) { return Kp <= 128 ? 32 : Kp <= 256 ? 16 : Kp <= 512 ? 8 : Kp <= BAND_KP ? 4 : 0; }
+constexpr int BAND_ROWS = 128;       // most rows of a band
+constexpr int BAND_SMEM = (BAND_ELEMS + 2 * BAND_ROWS) * 8 + BAND_KP * 8 + BAND_ROWS * 8 + BAND_ROWS * 4 + 16;
+// rows per band (a power of two) of about `elems` elements; 0: not banded
+static int band_rows(int Kp, int elems = BAND_ELEMS)
+{
+    if (Kp > BAND_KP) return 0;
+    int rb = 4;
+    while (rb < BAND_ROWS && 2 * rb * Kp <= elems) rb *= 2;
+    return rb;
+}
 
 __device__ __forceinline__ int find_desc(const PrepDesc *pd, int n, long long w)
 {
@@ -485,13 +493,23 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
 {
     extern __shared__ __align__(16) unsigned char band_raw[];
     double *x = (double *)band_raw;                                   // [rb][Kp + 2] (rows padded: fewer bank conflicts)
-    long long *koff = (long long *)(x + BAND_ELEMS + 64);             // [Kp]
+    long long *koff = (long long *)(x + BAND_ELEMS + 2 * BAND_ROWS);  // [Kp]
     long long *roff = koff + BAND_KP;                                 // [rb]
-    int *rexp_s = (int *)(roff + 32);                                 // [rb]
-    int *sdesc = rexp_s + 32;
+    int *rexp_s = (int *)(roff + BAND_ROWS);                          // [rb]
+    int *sdesc = rexp_s + BAND_ROWS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int di = -1;
     for (long long u = blockIdx.x; u < units; u += gridDim.x) {
-        if (threadIdx.x == 0) *sdesc = find_band(pd, n, u);
+        // the CTA's bands ascend: one binary search, then 32 operands per step
+        if (warp == 0) {
+            if (di < 0) di = find_band(pd, n, u);
+            for (int c = 32; c == 32;) {
+                const int k = di + 1 + lane;
+                c = __popc(__ballot_sync(0xffffffffu, k < n && pd[k].band_start <= u));
+                di += c;
+            }
+            if (lane == 0) *sdesc = di;
+        }
         __syncthreads();
         const PrepDesc &d = pd[*sdesc];
         if (d.rb == 0 || (active && !active[d.mol])) { __syncthreads(); continue; }
@@ -509,7 +527,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
         // e % Kp. Walked by the block size without divisions, the loads of
         // eight steps in flight before their values go to shared memory.
         {
-            const int lrb = rb == 32 ? 5 : rb == 16 ? 4 : rb == 8 ? 3 : 2;
+            const int lrb = __ffs(rb) - 1;
             int r = d.rfast ? (threadIdx.x & (rb - 1)) : threadIdx.x / Kp;
             int k = d.rfast ? (threadIdx.x >> lrb) : threadIdx.x % Kp;
             const int dr = d.rfast ? 0 : PT_THREADS / Kp, dk = d.rfast ? (PT_THREADS >> lrb) : PT_THREADS % Kp;
@@ -582,17 +600,31 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
 struct TileWork {
     int di, bt, tm, tn, kb0, nkb, nchunk;
 };
+// The problem of tile `tile`, at or after problem di, by a whole warp: 32
+// problems per step. A CTA's tiles ascend, so the next one's problem is
+// usually within a step of the last one's (a binary search from scratch was
+// a chain of ten loads per tile and role: 20 us per K = 32 tile of a 528-problem
+// launch).
+__device__ __forceinline__ int next_desc(const TcDesc *__restrict__ descs, int ndesc, long long tile, int di)
+{
+    for (;;) {
+        const int k = di + 1 + (int)(threadIdx.x & 31);
+        const int c = __popc(__ballot_sync(0xffffffffu, k < ndesc && descs[k].tile_start <= tile));
+        di += c;
+        if (c < 32) return di;
+    }
+}
+// Next tile of this CTA after the tiles of an inactive molecule's problem.
+__device__ __forceinline__ long long skip_desc(const TcDesc *__restrict__ descs, int ndesc, long long ntiles, long long tile, int di)
+{
+    const long long end = di + 1 < ndesc ? descs[di + 1].tile_start : ntiles, g = gridDim.x;
+    return tile + (end - tile + g - 1) / g * g;
+}
 template <class C>
-__device__ __forceinline__ TileWork tile_work(const TcDesc *__restrict__ descs, int ndesc, long long tile)
+__device__ __forceinline__ TileWork tile_work(const TcDesc &d, int di, long long tile)
 {
     TileWork w;
-    int lo = 0, hi = ndesc - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (descs[mid].tile_start <= tile) lo = mid; else hi = mid - 1;
-    }
-    w.di = lo;
-    const TcDesc &d = descs[lo];
+    w.di = di;
     // a problem's tiles number below 2^31: 32-bit divisions (64-bit ones are
     // emulated, and every epilogue thread does this for every tile)
     int local = (int)(tile - d.tile_start);
@@ -668,12 +700,14 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
     bool ok = true;
 
     if (warp == WP) {
-        if (lane == 0) {
-            long long g = 0;                                  // k-blocks loaded so far
-            for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-                const TileWork w = tile_work<C>(descs, ndesc, tile);
-                const TcDesc &d = descs[w.di];
-                if (active && !active[d.mol]) continue;
+        long long g = 0;                                  // k-blocks loaded so far
+        int di = 0;
+        for (long long tile = blockIdx.x; tile < ntiles && ok;) {
+            di = next_desc(descs, ndesc, tile, di);
+            const TcDesc &d = descs[di];
+            if (active && !active[d.mol]) { tile = skip_desc(descs, ndesc, ntiles, tile, di); continue; }
+            const TileWork w = tile_work<C>(d, di, tile);
+            if (lane == 0) {
                 const int arow0 = w.bt * d.M + w.tm * BM, brow0 = w.bt * d.N + w.tn * C::BN;
                 const int aplane = d.batch * d.M, bplane = d.batch * d.N;
                 for (int kb = 0; kb < w.nkb && ok; ++kb, ++g) {
@@ -690,13 +724,17 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     }
                 }
             }
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+            tile += gridDim.x;
         }
     } else if (warp == WM) {
-        if (lane == 0) {
-            long long g = 0, gc = 0;                          // k-blocks and chunks consumed so far
-            for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-                const TileWork w = tile_work<C>(descs, ndesc, tile);
-                if (active && !active[descs[w.di].mol]) continue;
+        long long g = 0, gc = 0;                          // k-blocks and chunks consumed so far
+        int di = 0;
+        for (long long tile = blockIdx.x; tile < ntiles && ok;) {
+            di = next_desc(descs, ndesc, tile, di);
+            if (active && !active[descs[di].mol]) { tile = skip_desc(descs, ndesc, ntiles, tile, di); continue; }
+            const TileWork w = tile_work<C>(descs[di], di, tile);
+            if (lane == 0) {
                 for (int c = 0; c < w.nchunk && ok; ++c, ++gc) {
                     const int buf = (int)(gc & 1);
                     const uint32_t use = (uint32_t)(gc >> 1);
@@ -750,6 +788,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     mma_commit(&acc_full[buf]);
                 }
             }
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+            tile += gridDim.x;
         }
     } else {
         // epilogue: warps 0 .. EPI_WARPS-1; warp w drains TMEM lanes 32*(w%4)..
@@ -765,10 +805,13 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
         constexpr int U = (C::STG_ROWS + RSTEP - 1) / RSTEP < 32 ? (C::STG_ROWS + RSTEP - 1) / RSTEP : 32;
         const int nn = threadIdx.x % C::BN, rr = threadIdx.x / C::BN;
         long long gc = 0;                                     // chunks drained so far
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const TileWork w = tile_work<C>(descs, ndesc, tile);
-            const TcDesc &d = descs[w.di];
-            if (active && !active[d.mol]) continue;
+        int di = 0;
+        for (long long tile = blockIdx.x; tile < ntiles;) {
+            di = next_desc(descs, ndesc, tile, di);
+            const TcDesc &d = descs[di];
+            if (active && !active[d.mol]) { tile = skip_desc(descs, ndesc, ntiles, tile, di); continue; }
+            const TileWork w = tile_work<C>(d, di, tile);
+            tile += gridDim.x;
             float hi[C::EPI_COLS], lo[C::EPI_COLS];
             // INT_DRAIN: each exact class of a chunk is an integer count of
             // 2^-8q below 2^24, so a[q] 2^8(NX-1) is an integer below 2^56 and
@@ -1242,7 +1285,6 @@ static int add_operand(Mode &M, int S, int gi, int mol, const double *src, int b
     plain_stride(K, p.Ki, p.s[2], p.s[3]);
     if (batch == 1) p.s[4] = 0;
     p.rfast = prep_rfast(p);
-    p.rb = band_rows(p.Kp);
     const OperandKey key{(long long)(size_t)src, batch, R, K, p.Ri, p.Ki, p.s[0], p.s[1], p.s[2], p.s[3], p.s[4],
                          fixed || keep ? -1 : gi};
     auto it = M.index.find(key);
@@ -1318,7 +1360,13 @@ static int finish_mode(Engine *e, Mode &M, int mode, const std::vector<const Gro
     }
     if (M.var_elems > e->scratch_elems) { hx_set_error("tensor-core scratch overflow"); return HX_ERR_STATE; }
     M.groups.resize(plan.size());
+    // bands of up to BAND_ELEMS elements, smaller where that would leave SMs without one
+    // (four bands per SM run at a time)
+    std::vector<double> elems(plan.size() + 1, 0.0);
+    for (const Operand &x : M.ops) elems[x.fixed ? plan.size() : x.first] += (double)x.rows * x.p.Kp;
     for (Operand &x : M.ops) {
+        const double per = elems[x.fixed ? plan.size() : x.first] / (4.0 * e->nsm);
+        x.p.rb = band_rows(x.p.Kp, (int)std::min<double>(std::max(per, 1024.0), BAND_ELEMS));
         x.p.dst = (x.fixed ? M.fixed_buf : e->scratch) + x.off;
         x.p.rexp = (x.fixed ? M.fixed_rexp : e->rexp) + x.roff;
         (x.fixed ? M.fixed : M.groups[x.first].var_ops).add(x.p);
