@@ -783,12 +783,12 @@ static int apply_learned_guess(hx_ccsd *h)
         hx_set_error("guess = 1 (learned) but no model was given (hx_ccsd_set_model)");
         return HX_ERR_STATE;
     }
+    std::vector<long long> npairs(h->nmol, 0);
     for (int mi = 0; mi < h->nmol; ++mi) {
-        if (h->scf_failed[mi]) continue;
         const long long ov = (long long)h->o[mi] * h->v[mi];
-        HX_CU(h->model->apply(h->d_cc, mi, ov * (ov + 1) / 2, h->st));
+        if (!h->scf_failed[mi]) npairs[mi] = ov * (ov + 1) / 2;
     }
-    HX_CU(cudaStreamSynchronize(h->st));
+    HX_CU(h->model->apply(h->d_cc, npairs.data(), h->nmol, h->st));
     if (int w = h->model->error_word()) {
         hx_set_error("learned guess: a tensor-core wait timed out (code %d)", w);
         return HX_ERR_KERNEL;

@@ -22,9 +22,12 @@ struct Model {
     CUtensorMap mapW2, mapW3;           // TMA maps of the bf16 weights (256 x 256, 128-byte swizzle)
     int load(const float *host_blob);   // HX_OK or an error code (message set)
     void release();
-    // t2 <- guess + prediction for every canonical pair (ia) <= (jb) of
-    // molecule mol (both t2 entries of the pair), after the reference guess.
-    cudaError_t apply(const CCMol *d_mols, int mol, long long npairs, cudaStream_t s) const;
+    int *tile_start = nullptr;          // apply: first tile of each molecule
+    int tiles_cap = 0;
+    // t2 <- guess + prediction for every canonical pair (ia) <= (jb) of the
+    // nmol molecules (both t2 entries of the pair), after the reference guess;
+    // npairs[k]: canonical pairs of molecule k (0: left out). Waits for the stream.
+    cudaError_t apply(const CCMol *d_mols, const long long *npairs, int nmol, cudaStream_t s);
     int error_word() const;
 };
 
