@@ -11,10 +11,12 @@
 // index arithmetic, shared memory) fits beside it even with one output per
 // thread. The time of a launch is therefore the FMAs of the busiest SM, and
 // the tile is as small as that allows: T x T outputs, T = 16 (256 threads) or,
-// when a launch would not give every SM two such tiles, T = 8 (64 threads).
+// when a launch would not give every SM two such tiles, T = 8, whose k-blocks
+// are then shared by four groups of 64 threads (a quarter of the chain of
+// dependent FMAs, one sum through shared memory at the end).
 // Warps whose outputs all lie outside M x N skip their FMAs. k runs in
-// ascending order for every output whatever the tile, 32 at a time, the next
-// 32 fetched into registers while the current ones are multiplied. Operand
+// ascending order for every output (of its group), 32 at a time, the next
+// k-block fetched into registers while the current one is multiplied. Operand
 // elements are gathered through the descriptor's split strides, so any index
 // permutation of a 4-index tensor is read in place; the loader walks the
 // operand's contiguous dimension first.
@@ -26,7 +28,7 @@
 #include "hx_kernels.h"
 
 namespace {
-constexpr int BK = 32;
+constexpr int BKG = 32;      // k per group and block
 
 __device__ __forceinline__ long long split_off(int x, int xi, long long s0, long long s1)
 {
@@ -34,11 +36,11 @@ __device__ __forceinline__ long long split_off(int x, int xi, long long s0, long
     return (long long)q * s0 + (long long)(x - q * xi) * s1;
 }
 
-template <int T>
-__global__ void __launch_bounds__(T * T) tgemm_f64_kernel(const TgemmDesc *__restrict__ descs, int ndesc,
+template <int T, int G>
+__global__ void __launch_bounds__(T * T * G) tgemm_f64_kernel(const TgemmDesc *__restrict__ descs, int ndesc,
                                                           const int *__restrict__ active)
 {
-    constexpr int NT = T * T, R = T * BK / NT;           // R elements of each operand per thread and k-block
+    constexpr int BK = BKG * G, NT = T * T * G, R = T * BK / NT;   // R elements of each operand per thread and k-block
     __shared__ double As[BK][T + 1];
     __shared__ double Bs[BK][T + 1];
     const long long tile = blockIdx.x;
@@ -91,9 +93,10 @@ __global__ void __launch_bounds__(T * T) tgemm_f64_kernel(const TgemmDesc *__res
             bv[r] = (boff[r] >= 0 && kb < kend) ? B[boff[r] + split_off(kb, Ki, b2, b3)] : 0.0;
         }
     };
-    // warp w computes T rows of 32 / T consecutive columns
-    const int mm = threadIdx.x % T, nn = threadIdx.x / T;
-    const bool live = n0 + (int)(threadIdx.x / 32) * (32 / T) < N;     // uniform over the warp
+    // a warp computes T rows of 32 / T consecutive columns, for its group's k
+    const int grp = threadIdx.x / (T * T), tid = threadIdx.x % (T * T);
+    const int mm = tid % T, nn = tid / T;
+    const bool live = n0 + (tid / 32) * (32 / T) < N;                  // uniform over the warp
     double acc = 0.0;
     fetch(kbeg);
     for (int k0 = kbeg; k0 < kend; k0 += BK) {
@@ -102,16 +105,24 @@ __global__ void __launch_bounds__(T * T) tgemm_f64_kernel(const TgemmDesc *__res
         __syncthreads();
         if (k0 + BK < kend) fetch(k0 + BK);
         if (live) {
-            const int kn = min(BK, kend - k0);
-            if (kn == BK) {
+            const int kb = grp * BKG, kn = min(BKG, kend - k0 - kb);
+            if (kn == BKG) {
 #pragma unroll
-                for (int kk = 0; kk < BK; ++kk) acc = fma(As[kk][mm], Bs[kk][nn], acc);
+                for (int kk = 0; kk < BKG; ++kk) acc = fma(As[kb + kk][mm], Bs[kb + kk][nn], acc);
             } else {
 #pragma unroll 4
-                for (int kk = 0; kk < kn; ++kk) acc = fma(As[kk][mm], Bs[kk][nn], acc);
+                for (int kk = 0; kk < kn; ++kk) acc = fma(As[kb + kk][mm], Bs[kb + kk][nn], acc);
             }
         }
         __syncthreads();
+    }
+    if (G > 1) {                                              // the groups' sums in order
+        double *red = &As[0][0];
+        if (grp > 0) red[(grp - 1) * T * T + tid] = acc;
+        __syncthreads();
+        if (grp > 0) return;
+#pragma unroll
+        for (int g = 1; g < G; ++g) acc += red[(g - 1) * T * T + tid];
     }
     const int m = m0 + mm, n = n0 + nn;
     if (m >= M || n >= N) return;
@@ -163,8 +174,8 @@ F64Tiles hx_tgemm_f64_prepare(TgemmDesc *descs, int n)
 cudaError_t hx_tgemm_f64_launch(const TgemmDesc *d_descs, int n, F64Tiles tiles, const int *d_active, cudaStream_t s)
 {
     if (tiles.count <= 0) return cudaSuccess;
-    if (tiles.size == 8) tgemm_f64_kernel<8><<<(unsigned)tiles.count, 64, 0, s>>>(d_descs, n, d_active);
-    else tgemm_f64_kernel<16><<<(unsigned)tiles.count, 256, 0, s>>>(d_descs, n, d_active);
+    if (tiles.size == 8) tgemm_f64_kernel<8, 4><<<(unsigned)tiles.count, 256, 0, s>>>(d_descs, n, d_active);
+    else tgemm_f64_kernel<16, 1><<<(unsigned)tiles.count, 256, 0, s>>>(d_descs, n, d_active);
     hx_count_launches(1);
     return cudaGetLastError();
 }
