@@ -535,16 +535,19 @@ __global__ void __launch_bounds__(NT) k_diis_solve(const CCMol *__restrict__ mol
     __syncthreads();
     if (warp != 0) return;
     for (int k = 0; k < nb; ++k) {
-        double best = -1.0;
-        int piv = k;
-        for (int r = k + lane; r < nb; r += 32)
-            if (fabs(A[r * LD + k]) > best) { best = fabs(A[r * LD + k]); piv = r; }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {             // the first row of the largest magnitude
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int op = __shfl_xor_sync(0xffffffffu, piv, o);
-            if (ob > best || (ob == best && op < piv)) { best = ob; piv = op; }
+        // the first row of the largest magnitude, compared as bit patterns word by word
+        // (two rows per lane at most; rows outside compare as zero)
+        unsigned long long bb = 0;
+        int br = k;
+        for (int r = k + lane; r < nb; r += 32) {
+            const unsigned long long x = (unsigned long long)__double_as_longlong(A[r * LD + k]) & 0x7FFFFFFFFFFFFFFFull;
+            if (x > bb) { bb = x; br = r; }
         }
+        const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(bb >> 32));
+        const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(bb >> 32) == hi ? (unsigned)bb : 0u);
+        const bool top = (unsigned)(bb >> 32) == hi && (unsigned)bb == lo;
+        const int piv = (int)__reduce_min_sync(0xffffffffu, top && (hi | lo) ? (unsigned)br : (unsigned)nb);
+        if (piv >= nb) return;                         // a zero column: singular, no mixing
         if (piv != k)
             for (int c = k + lane; c <= nb; c += 32) {
                 const double t = A[k * LD + c];

@@ -1447,15 +1447,15 @@ TgemmDesc triples_term(int t, const CCMol &m, const double *I1, const double *J,
     // P3 = X(jb, ia, kc): m = (b, a), n = (k, c)
     case 4: return tg(I1 + j * vvv, T2 + j * vov + i * v, Wj, 1, M, NK, v, v, v, v, {vv, v, 0, 1, 0}, {vov, ov, 0, 1, 0}, {v, vv, vvv, 1, 0}, 1.0, 1.0, 0);
     case 5: return tg(T2 + j * vov, J + j * voo + i * o, Wj, 1, M, NK, o, v, v, o, {ov, 1, 0, v, 0}, {voo, oo, 0, 1, 0}, {v, vv, vvv, 1, 0}, -1.0, 1.0, 0);
-    // P4 = X(kc, ia, jb): m = (c, a), n = b, batch k
-    case 6: return tg(I1 + j * vvv, T2 + j * vov + i * v, Wj, nk, M, v, v, v, v, v, {vv, v, 0, 1, vvv}, {0, ov, 0, 1, 0}, {1, vv, 0, v, vvv}, 1.0, 1.0, 0);
-    case 7: return tg(T2 + j * vov, J + j * voo + i * o, Wj, nk, M, v, o, v, v, o, {ov, 1, 0, v, vov}, {0, oo, 0, 1, 0}, {1, vv, 0, v, vvv}, -1.0, 1.0, 0);
+    // P4 = X(kc, ia, jb): m = (a, c), n = b, batch k (c inner: it is W's contiguous index)
+    case 6: return tg(I1 + j * vvv, T2 + j * vov + i * v, Wj, nk, M, v, v, v, v, v, {v, vv, 0, 1, vvv}, {0, ov, 0, 1, 0}, {vv, 1, 0, v, vvv}, 1.0, 1.0, 0);
+    case 7: return tg(T2 + j * vov, J + j * voo + i * o, Wj, nk, M, v, o, v, v, o, {1, ov, 0, v, vov}, {0, oo, 0, 1, 0}, {vv, 1, 0, v, vvv}, -1.0, 1.0, 0);
     // P5 = X(jb, kc, ia): m = (b, c), n = (k, a)
     case 8: return tg(I1 + j * vvv, T2 + i * vov + j * v, Wj, 1, M, NK, v, v, v, v, {vv, v, 0, 1, 0}, {v, ov, 0, 1, 0}, {v, 1, vvv, vv, 0}, 1.0, 1.0, 0);
     case 9: return tg(T2 + j * vov, J + i * voo + j * o, Wj, 1, M, NK, o, v, v, o, {ov, 1, 0, v, 0}, {o, oo, 0, 1, 0}, {v, 1, vvv, vv, 0}, -1.0, 1.0, 0);
-    // P6 = X(kc, jb, ia): m = (c, b), n = a, batch k
-    case 10: return tg(I1 + j * vvv, T2 + i * vov + j * v, Wj, nk, M, v, v, v, v, v, {vv, v, 0, 1, vvv}, {0, ov, 0, 1, 0}, {1, v, 0, vv, vvv}, 1.0, 1.0, 0);
-    default: return tg(T2 + j * vov, J + i * voo + j * o, Wj, nk, M, v, o, v, v, o, {ov, 1, 0, v, vov}, {0, oo, 0, 1, 0}, {1, v, 0, vv, vvv}, -1.0, 1.0, 0);
+    // P6 = X(kc, jb, ia): m = (b, c), n = a, batch k
+    case 10: return tg(I1 + j * vvv, T2 + i * vov + j * v, Wj, nk, M, v, v, v, v, v, {v, vv, 0, 1, vvv}, {0, ov, 0, 1, 0}, {v, 1, 0, vv, vvv}, 1.0, 1.0, 0);
+    default: return tg(T2 + j * vov, J + i * voo + j * o, Wj, nk, M, v, o, v, v, o, {1, ov, 0, v, vov}, {0, oo, 0, 1, 0}, {v, 1, 0, vv, vvv}, -1.0, 1.0, 0);
     }
 }
 }  // namespace
@@ -1545,7 +1545,7 @@ int hx_ccsd_triples(hx_ccsd *h, int32_t mol, double e[4])
             for (int k = j; k < o; ++k) triples.push_back(make_int3(i, j, k));
         }
         tc::Engine *te = nullptr;
-        rc = tc::create(&te, plan, h->st, 2, 0, 3);      // the 7-slice (emulated FP64) mode only
+        rc = tc::create(&te, plan, h->st, 2, 2, 3);      // the 7-slice (emulated FP64) mode only, its short-K tile
         for (int t = 0; t < 12 && rc == HX_OK && ce == cudaSuccess; ++t)
             ce = tc::run_group(te, plan[t].h.data(), (int)plan[t].h.size(), nullptr, h->st, 3);
         if (rc == HX_OK && ce == cudaSuccess)

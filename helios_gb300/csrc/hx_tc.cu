@@ -142,6 +142,7 @@ struct Cfg {
     static_assert(STG_ROWS * (BN_ + 1) * 8 <= 232448 - 1280 - 128 * 12 - RING_BYTES, "staging strip");
     static_assert(EPIW_ % 4 == 0 && EPI_COLS % 8 == 0, "epilogue split");
     static_assert(EPIW_ * 32 >= 128 && EPIW_ * 32 >= BN_, "epilogue threads cover the tile's rows and columns");
+    static_assert(EPIW_ * 32 % STG_ROWS == 0, "epilogue threads walk whole columns of the strip");
     // int64 drain: a chunk adds below 2^(24 + 8(NX-1) + 1); 32 chunks stay below 2^63
     static_assert(!INT_DRAIN || 24 + 8 * (NX_ - 1) + 1 + 5 < 63, "int64 drain headroom");
 };
@@ -160,6 +161,7 @@ struct TcDesc {
     double alpha, beta;
     int alpha_e, alpha_neg;          // alpha = (-1)^alpha_neg 2^alpha_e when alpha_pow2
     int alpha_pow2, beta_one;        // beta_one: beta == 1 (C += r without a multiply)
+    int mfast;                       // consecutive m (not n) are the closer ones in C
     double *C;
     int tiles_m, tiles_n;
     long long tile_start;
@@ -614,11 +616,23 @@ __device__ __forceinline__ int next_desc(const TcDesc *__restrict__ descs, int n
         if (c < 32) return di;
     }
 }
-// Next tile of this CTA after the tiles of an inactive molecule's problem.
-__device__ __forceinline__ long long skip_desc(const TcDesc *__restrict__ descs, int ndesc, long long ntiles, long long tile, int di)
+// The same from scratch, for the producer's and the MMA's single thread: their
+// search runs ahead of the epilogue, and the MMA loop is sensitive to its
+// surroundings (with the search carried on from tile to tile, or the loop run
+// by the whole warp, 4800^3 products took 4 % longer).
+__device__ __forceinline__ int find_problem(const TcDesc *__restrict__ descs, int ndesc, long long tile)
 {
-    const long long end = di + 1 < ndesc ? descs[di + 1].tile_start : ntiles, g = gridDim.x;
-    return tile + (end - tile + g - 1) / g * g;
+    int lo = 0, hi = ndesc - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (descs[mid].tile_start <= tile) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+// First tile after problem di.
+__device__ __forceinline__ long long problem_end(const TcDesc *__restrict__ descs, int ndesc, long long ntiles, int di)
+{
+    return di + 1 < ndesc ? descs[di + 1].tile_start : ntiles;
 }
 template <class C>
 __device__ __forceinline__ TileWork tile_work(const TcDesc &d, int di, long long tile)
@@ -700,14 +714,15 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
     bool ok = true;
 
     if (warp == WP) {
-        long long g = 0;                                  // k-blocks loaded so far
-        int di = 0;
-        for (long long tile = blockIdx.x; tile < ntiles && ok;) {
-            di = next_desc(descs, ndesc, tile, di);
-            const TcDesc &d = descs[di];
-            if (active && !active[d.mol]) { tile = skip_desc(descs, ndesc, ntiles, tile, di); continue; }
-            const TileWork w = tile_work<C>(d, di, tile);
-            if (lane == 0) {
+        if (lane == 0) {
+            long long g = 0;                                  // k-blocks loaded so far
+            long long skip = 0;                               // tiles below: an inactive molecule's problem
+            for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+                if (tile < skip) continue;
+                const int di = find_problem(descs, ndesc, tile);
+                const TcDesc &d = descs[di];
+                if (active && !active[d.mol]) { skip = problem_end(descs, ndesc, ntiles, di); continue; }
+                const TileWork w = tile_work<C>(d, di, tile);
                 const int arow0 = w.bt * d.M + w.tm * BM, brow0 = w.bt * d.N + w.tn * C::BN;
                 const int aplane = d.batch * d.M, bplane = d.batch * d.N;
                 for (int kb = 0; kb < w.nkb && ok; ++kb, ++g) {
@@ -724,17 +739,16 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     }
                 }
             }
-            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-            tile += gridDim.x;
         }
     } else if (warp == WM) {
-        long long g = 0, gc = 0;                          // k-blocks and chunks consumed so far
-        int di = 0;
-        for (long long tile = blockIdx.x; tile < ntiles && ok;) {
-            di = next_desc(descs, ndesc, tile, di);
-            if (active && !active[descs[di].mol]) { tile = skip_desc(descs, ndesc, ntiles, tile, di); continue; }
-            const TileWork w = tile_work<C>(descs[di], di, tile);
-            if (lane == 0) {
+        if (lane == 0) {
+            long long g = 0, gc = 0;                          // k-blocks and chunks consumed so far
+            long long skip = 0;
+            for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+                if (tile < skip) continue;
+                const int di = find_problem(descs, ndesc, tile);
+                if (active && !active[descs[di].mol]) { skip = problem_end(descs, ndesc, ntiles, di); continue; }
+                const TileWork w = tile_work<C>(descs[di], di, tile);
                 for (int c = 0; c < w.nchunk && ok; ++c, ++gc) {
                     const int buf = (int)(gc & 1);
                     const uint32_t use = (uint32_t)(gc >> 1);
@@ -788,8 +802,6 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     mma_commit(&acc_full[buf]);
                 }
             }
-            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-            tile += gridDim.x;
         }
     } else {
         // epilogue: warps 0 .. EPI_WARPS-1; warp w drains TMEM lanes 32*(w%4)..
@@ -806,12 +818,13 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
         const int nn = threadIdx.x % C::BN, rr = threadIdx.x / C::BN;
         long long gc = 0;                                     // chunks drained so far
         int di = 0;
-        for (long long tile = blockIdx.x; tile < ntiles;) {
+        long long skip = 0;
+        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            if (tile < skip) continue;
             di = next_desc(descs, ndesc, tile, di);
             const TcDesc &d = descs[di];
-            if (active && !active[d.mol]) { tile = skip_desc(descs, ndesc, ntiles, tile, di); continue; }
+            if (active && !active[d.mol]) { skip = problem_end(descs, ndesc, ntiles, di); continue; }
             const TileWork w = tile_work<C>(d, di, tile);
-            tile += gridDim.x;
             float hi[C::EPI_COLS], lo[C::EPI_COLS];
             // INT_DRAIN: each exact class of a chunk is an integer count of
             // 2^-8q below 2^24, so a[q] 2^8(NX-1) is an integer below 2^56 and
@@ -889,17 +902,21 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
             // C = alpha 2^(e_m + f_n - 14) x + beta C with the power of two and
             // a power-of-two alpha applied by exponent arithmetic
             const int mv = min(BM, d.M - w.tm * BM), nv = min(C::BN, d.N - w.tn * C::BN);
-            if (threadIdx.x < mv) {
-                const int m = w.tm * BM + threadIdx.x;
-                srow[threadIdx.x] = split_off(m, d.Mi, d.c[0], d.c[1]);
-                sexp[threadIdx.x] = d.expA[(long long)w.bt * d.M + m];
+            // mfast: the roles of rows and columns change below -- srow and sexp are
+            // the columns', a thread keeps one row and walks the columns
+            const bool mfast = d.mfast != 0;
+            double *const Cb = d.C + (long long)w.bt * d.c[4];
+            if (threadIdx.x < (mfast ? nv : mv)) {
+                const int x = (mfast ? w.tn * C::BN : w.tm * BM) + threadIdx.x;
+                srow[threadIdx.x] = mfast ? split_off(x, d.Ni, d.c[2], d.c[3]) : split_off(x, d.Mi, d.c[0], d.c[1]);
+                sexp[threadIdx.x] = mfast ? d.expB[(long long)w.bt * d.N + x] : d.expA[(long long)w.bt * d.M + x];
             }
             int eb = INT_MIN;
             double *Cn = nullptr;
-            if (rr < RSTEP && nn < nv) {
+            if (!mfast && rr < RSTEP && nn < nv) {
                 const int n = w.tn * C::BN + nn;
                 eb = d.expB[(long long)w.bt * d.N + n];
-                Cn = d.C + (long long)w.bt * d.c[4] + split_off(n, d.Ni, d.c[2], d.c[3]);
+                Cn = Cb + split_off(n, d.Ni, d.c[2], d.c[3]);
             }
             const bool load_c = d.ksplit == 1 && d.beta != 0.0;
             const uint32_t negmask = d.alpha_neg ? 0x80000000u : 0u;
@@ -929,46 +946,74 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                 }
                 asm volatile("bar.sync 1, %0;" ::"r"(C::EPI_THREADS) : "memory");
                 const int rend = min(r0 + C::STG_ROWS, mv);
-                if (ok && Cn) {
-                    for (int m0 = r0 + rr; m0 < rend; m0 += RSTEP * U) {
-                        double old[U];
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            const int mm = m0 + u * RSTEP;
-                            old[u] = (load_c && mm < rend) ? Cn[srow[mm]] : 0.0;
-                        }
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            const int mm = m0 + u * RSTEP;
-                            if (mm >= rend) break;
-                            const int ea = sexp[mm];
+                // value of strip element at (row index in the strip x LD + column), exponents ea and eb
+                auto value = [&](int at, int ea, int eb) -> double {
+                    if (ea == INT_MIN || eb == INT_MIN) return 0.0;
+                    const int k = ea + eb - 14 + d.alpha_e;
+                    bool fast = d.alpha_pow2 != 0 && k >= -896 && k <= 896;
+                    if constexpr (C::INT_DRAIN) {
+                        if (fbits) {
+                            const long long v = istrip[at];
                             double r = 0.0;
-                            if (ea != INT_MIN && eb != INT_MIN) {
-                                const int k = ea + eb - 14 + d.alpha_e;
-                                bool fast = d.alpha_pow2 != 0 && k >= -896 && k <= 896;
-                                if constexpr (C::INT_DRAIN) {
-                                    if (fbits) {
-                                        const long long v = istrip[(mm - r0) * LD + nn];
-                                        if (fast) r = fixed_pow2(d.alpha_neg ? -v : v, k - 8 * (C::NX - 1) - fbits, fast);
-                                        if (!fast) r = d.alpha * scale_pow2((double)v / ((double)C::DRAIN_SCALE * (double)(1 << fbits)), ea, eb);
-                                        goto scaled;
-                                    }
-                                    const double v = dstrip[(mm - r0) * LD + nn];
-                                    if (fast) {
-                                        r = pow2_int(v, k, fast);
-                                        if (d.alpha_neg) r = -r;
-                                    }
-                                    if (!fast) r = d.alpha * scale_pow2(v, ea, eb);
-                                } else {
-                                    const float2 v = strip[(mm - r0) * LD + nn];
-                                    if (fast) r = f2d_pow2(v.x, k, negmask) + f2d_pow2(v.y, k, negmask);
-                                    else r = d.alpha * scale_pow2((double)v.x + (double)v.y, ea, eb);
-                                }
+                            if (fast) r = fixed_pow2(d.alpha_neg ? -v : v, k - 8 * (C::NX - 1) - fbits, fast);
+                            if (!fast) r = d.alpha * scale_pow2((double)v / ((double)C::DRAIN_SCALE * (double)(1 << fbits)), ea, eb);
+                            return r;
+                        }
+                        const double v = dstrip[at];
+                        double r = 0.0;
+                        if (fast) {
+                            r = pow2_int(v, k, fast);
+                            if (d.alpha_neg) r = -r;
+                        }
+                        if (!fast) r = d.alpha * scale_pow2(v, ea, eb);
+                        return r;
+                    } else {
+                        const float2 v = strip[at];
+                        return fast ? f2d_pow2(v.x, k, negmask) + f2d_pow2(v.y, k, negmask)
+                                    : d.alpha * scale_pow2((double)v.x + (double)v.y, ea, eb);
+                    }
+                };
+                auto store = [&](double *p, double r, double old) {
+                    if (d.ksplit > 1) atomicAdd(p, r);
+                    else *p = load_c ? (d.beta_one ? r + old : fma(d.beta, old, r)) : r;
+                };
+                if (!mfast) {
+                    if (ok && Cn) {
+                        for (int m0 = r0 + rr; m0 < rend; m0 += RSTEP * U) {
+                            double old[U];
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                const int mm = m0 + u * RSTEP;
+                                old[u] = (load_c && mm < rend) ? Cn[srow[mm]] : 0.0;
                             }
-                        scaled:
-                            double *p = Cn + srow[mm];
-                            if (d.ksplit > 1) atomicAdd(p, r);
-                            else *p = load_c ? (d.beta_one ? r + old[u] : fma(d.beta, old[u], r)) : r;
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                const int mm = m0 + u * RSTEP;
+                                if (mm >= rend) break;
+                                store(Cn + srow[mm], value((mm - r0) * LD + nn, sexp[mm], eb), old[u]);
+                            }
+                        }
+                    }
+                } else if (ok) {
+                    // consecutive threads on consecutive rows of the strip, CSTEP columns apart
+                    constexpr int CSTEP = C::EPI_THREADS / C::STG_ROWS;
+                    const int mr = threadIdx.x % C::STG_ROWS, m = r0 + mr;
+                    if (m < rend && CSTEP > 0) {
+                        const int x = w.tm * BM + m, ea = d.expA[(long long)w.bt * d.M + x];
+                        double *Cm = Cb + split_off(x, d.Mi, d.c[0], d.c[1]);
+                        for (int n0 = threadIdx.x / C::STG_ROWS; n0 < nv; n0 += 4 * CSTEP) {
+                            double old[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const int nx = n0 + u * CSTEP;
+                                old[u] = (load_c && nx < nv) ? Cm[srow[nx]] : 0.0;
+                            }
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const int nx = n0 + u * CSTEP;
+                                if (nx >= nv) break;
+                                store(Cm + srow[nx], value(mr * LD + nx, ea, sexp[nx]), old[u]);
+                            }
                         }
                     }
                 }
@@ -999,6 +1044,7 @@ using Mid48 = Cfg<4, 3, 2, 48, 2, 6, 12, 64>;
 using Mid32 = Cfg<4, 3, 2, 32, 2, 6, 8, 64>;
 using High32 = Cfg<5, 4, 3, 32, 3, 8, 8, 32>;
 using Exact16 = Cfg<7, 6, 5, 16, 3, 6, 8, 32>;
+using ExactS2 = Cfg<7, 6, 5, 32, 2, 6, 16, 32>;    // two stages: the strip takes the whole tile (short K)
 struct Variant {
     int S, BN, BK, products, smem;
     cudaError_t (*attr)();
@@ -1020,13 +1066,13 @@ static Variant variant()
     return Variant{C::S, C::BN, C::BK, C::PRODUCTS, C::SMEM_BYTES, &attr_tc<C>, &launch_tc<C>};
 }
 constexpr int MAX_VARIANTS = 3;
-static const int kNumVariants[4] = {3, 3, 2, 2};
+static const int kNumVariants[4] = {3, 3, 2, 3};
 static const Variant &variant_of(int mode, int k)
 {
     static const Variant table[4][MAX_VARIANTS] = {{variant<Low>(), variant<Low32>(), variant<LowS3>()},
                                                    {variant<Mid>(), variant<Mid48>(), variant<Mid32>()},
                                                    {variant<High>(), variant<High32>(), variant<High32>()},
-                                                   {variant<Exact>(), variant<Exact16>(), variant<Exact16>()}};
+                                                   {variant<Exact>(), variant<Exact16>(), variant<ExactS2>()}};
     return table[mode][k];
 }
 
@@ -1388,6 +1434,10 @@ static int finish_mode(Engine *e, Mode &M, int mode, const std::vector<const Gro
             for (int c = 0; c < 5; ++c) d.c[c] = t.c[c];
             set_scalars(d, t.alpha, t.beta);
             d.C = t.C; d.mol = t.mol;
+            // the epilogue's threads run along the dimension of C whose consecutive elements
+            // are closer (a column-strided store moves a 32-byte sector per 8-byte output)
+            const long long ms = t.Mi > 1 ? t.c[1] : t.c[0], ns = t.Ni > 1 ? t.c[3] : t.c[2];
+            d.mfast = t.N == 1 || (t.M > 1 && std::llabs(ms) < std::llabs(ns));
             d.tiles_m = (t.M + BM - 1) / BM; d.tiles_n = (t.N + V.BN - 1) / V.BN;
             // long K over few output tiles: cut K into slices that fill the GPU
             const int nkb = (t.K + V.BK - 1) / V.BK, n64 = (t.K + 63) / 64;
