@@ -76,13 +76,6 @@ __device__ __forceinline__ int sched_mol(const int *__restrict__ start, int nmol
 #define EW_ARGS const CCMol *__restrict__ mols, const int *__restrict__ active, const int *__restrict__ start, int nmol
 
 // ---------------------------------------------------------------- dressing
-// X = [Co | Cv], Y = [Co | Cv]; the t1 corrections are added by GEMMs.
-__global__ void k_dress_init(EW_ARGS)
-{
-    EW_PROLOGUE
-    EW_LOOP(e, (long long)m.N * m.N) { m.X[e] = m.Cmo[e]; m.Y[e] = m.Cmo[e]; }
-}
-
 // H2 = h - G o Pm + 2 diag(G diag Pm), Pm = Yo Xo^T (dressed half density)
 __global__ void __launch_bounds__(NT) k_dress_fock(EW_ARGS)
 {
@@ -143,41 +136,6 @@ __global__ void k_gamma_scale(EW_ARGS)
     }
 }
 
-// r1[i][a] = Fd[o+a][i];  Fvv2 = Fd_vv;  Foo2 = Fd_oo
-__global__ void k_fock_blocks(EW_ARGS)
-{
-    EW_PROLOGUE
-    const int n = m.N, o = m.o, v = m.v;
-    EW_LOOP(e, (long long)o * v + v * v + o * o) {
-        if (e < o * v) {
-            int i = (int)(e / v), a = (int)(e % v);
-            m.r1[e] = m.Fd[(o + a) * n + i];
-        } else if (e < o * v + v * v) {
-            int f = (int)(e - o * v), b = f / v, c = f % v;
-            m.Fvv2[f] = m.Fd[(o + b) * n + o + c];
-        } else {
-            int f = (int)(e - o * v - v * v), k = f / o, j = f % o;
-            m.Foo2[f] = m.Fd[k * n + j];
-        }
-    }
-}
-
-// X2[i][a][j][b] += Cint[i][a][j][b] + 0.5 Cp[i][a][j][b] + Cp[j][a][i][b]  (consecutive b read
-// consecutively; X2 and Cint hold the two E products)
-__global__ void k_c_combine(EW_ARGS)
-{
-    EW_PROLOGUE
-    const unsigned o = (unsigned)m.o, v = (unsigned)m.v;
-    const double *__restrict__ Cp = m.Cp;
-    const double *__restrict__ E2 = m.Cint;
-    double *__restrict__ X2 = m.X2;
-    EW_LOOP(e, (long long)o * v * o * v) {
-        const unsigned x = (unsigned)e;                  // o^2 v^2 < 2^32
-        const unsigned b = x % v, r = x / v, j = r % o, r2 = r / o, a = r2 % v, i = r2 / v;
-        X2[e] = (X2[e] + E2[e]) + (0.5 * Cp[e] + Cp[((j * v + a) * o + i) * v + b]);
-    }
-}
-
 // ---------------------------------------------------------------- pair units
 // Units of one molecule: unit 0 is the singles; unit u >= 1 holds the v x v
 // blocks [(u-1) g, min(u g, nb)) of the occupied pairs (i, j), in row-major
@@ -231,9 +189,19 @@ __device__ __forceinline__ long long pair_off(int i, int a, int j, int b, int o,
 // tile, its lanes the columns b, so global reads and writes run along b (one
 // division per row, none per element); shared-memory index of (lb, a, b) is
 // (lb v + a)(v + 1) + b.
-// With few virtual orbitals a warp walks several rows at once (lg: log2 of the
-// lanes per row), so that its FP64 slots are not spent on idle lanes.
-#define ROW_LANES(v) const int lg_ = (v) <= 4 ? 2 : (v) <= 8 ? 3 : (v) <= 16 ? 4 : 5;
+// A warp walks several rows at once with as many lanes per row (32, 16, 8 or 4;
+// lg_: the log2) as leave the fewest idle, so that its FP64 slots are not spent
+// on idle lanes (v = 80: 16 lanes x 5 instead of 32 x 3; v = 18: 8 x 3).
+__device__ __forceinline__ int row_lanes(int v)
+{
+    int lg = 5, width = (v + 31) & ~31;
+    for (int l = 4; l >= 2; --l) {
+        const int w = (v + (1 << l) - 1) >> l << l;
+        if (w < width && (l > 2 || v <= 4)) { width = w; lg = l; }
+    }
+    return lg;
+}
+#define ROW_LANES(v) const int lg_ = row_lanes(v);
 #define ROW_LOOP(nrows) for (int row_ = threadIdx.x >> lg_; row_ < (nrows); row_ += NT >> lg_)
 #define COL_LOOP(b, v) for (int b = threadIdx.x & ((1 << lg_) - 1); b < (v); b += 1 << lg_)
 
@@ -295,15 +263,21 @@ __device__ __forceinline__ double max_abs(double mx, double x)
     return b > m && b <= 0x7FF0000000000000ull ? __longlong_as_double((long long)b) : mx;
 }
 
-// u[i][a][j][b] = 2 t[i][a][j][b] - t[i][b][j][a]  (SK_FULL units)
+// u[i][a][j][b] = 2 t[i][a][j][b] - t[i][b][j][a]  (SK_FULL units); a molecule's
+// unit 0 starts its dressed factors, X = Y = [Co | Cv] (the t1 corrections are
+// added by GEMMs).
 __global__ void __launch_bounds__(NT) k_make_u(const CCMol *__restrict__ mols, const int *__restrict__ active,
                                                const int *__restrict__ start, int nmol)
 {
     extern __shared__ double sm[];
     __shared__ int bi[64], bj[64];
     const Unit w = unit_of(mols, start, nmol, false, bi, bj);
-    if ((active && !active[w.mol]) || w.u == 0) return;
+    if (active && !active[w.mol]) return;
     const CCMol &m = mols[w.mol];
+    if (w.u == 0) {
+        for (int e = threadIdx.x; e < m.N * m.N; e += NT) { const double c = m.Cmo[e]; m.X[e] = c; m.Y[e] = c; }
+        return;
+    }
     const int o = m.o, v = m.v, nrows = w.nb * v;
     ROW_LANES(v)
     const double *__restrict__ t2 = m.t2;
@@ -326,9 +300,10 @@ __global__ void __launch_bounds__(NT) k_make_u(const CCMol *__restrict__ mols, c
 }
 
 // Residual, Jacobi step and DIIS push of one unit (SK_UP units).
-//   singles: d1 = r1; t1 += s1 d1 / D1.
+//   singles: d1 = r1 + r1b; t1 += s1 d1 / D1.
 //   doubles of a block (i, j), i <= j: w = Omega2(ia, jb) assembled as
-//     r2 + X2 + X2 pair-transposed (the E and C/D terms), d2 = 2 w(ab) - w(ba)
+//     r2 + P + P pair-transposed, P_iajb = D_iajb + (E1 + E2)_iajb +
+//     1/2 C_iajb + C_jaib (X2, Et and Cint, Cp), d2 = 2 w(ab) - w(ba)
 //     (= w on a diagonal block, whose canonical element is the same for both);
 //     g = 3 w ("2-1") or d2 ("1"); t2 += s2 g / D2, the quotient as
 //     q = s2 g R2 and one correction q + (s2 g - q D2) R2 with the stored
@@ -365,7 +340,7 @@ __global__ void __launch_bounds__(NT) k_step_push(const CCMol *__restrict__ mols
     if (w.u == 0) {
         hoff = 0;
         for (int e = threadIdx.x; e < ov; e += NT) {
-            const double d = m.r1[e];
+            const double d = m.r1[e] + m.r1b[e];
             mx = fmax(mx, fabs(d));
             const double t = m.t1[e] + s1 * d / m.D1[e];
             if (push) { h.Ht[(long long)slot * h.L + e] = t; h.He[(long long)slot * h.L + e] = d; }
@@ -373,21 +348,23 @@ __global__ void __launch_bounds__(NT) k_step_push(const CCMol *__restrict__ mols
         }
     } else {
         hoff = ov + (long long)w.k0 * v * v;
-        // S = r2 + (X2 + X2[q][p]): element (a, b) of block (i, j) takes X2[j][b][i][a],
+        // S = r2 + (P + P[q][p]): element (a, b) of block (i, j) takes P[j][b][i][a],
         // read along a (coalesced) and added at the transposed tile position
+        const double *__restrict__ Cp = m.Cp, *__restrict__ Et = m.Et, *__restrict__ E2 = m.Cint;
 #pragma unroll 4
         ROW_LOOP(nrows) {
             const int lb = row_ / v, a = row_ - lb * v;
-            const double *src = X2 + pair_off(bi[lb], a, bj[lb], 0, o, v);
+            const long long f = pair_off(bi[lb], a, bj[lb], 0, o, v), g = pair_off(bj[lb], a, bi[lb], 0, o, v);
             double *srow = S + (lb * v + a) * (v + 1);
-            COL_LOOP(b, v) srow[b] = src[b];
+            COL_LOOP(b, v) srow[b] = (X2[f + b] + (Et[f + b] + E2[f + b])) + fma(0.5, Cp[f + b], Cp[g + b]);
         }
         __syncthreads();
 #pragma unroll 4
         ROW_LOOP(nrows) {
-            const int lb = row_ / v, x = row_ - lb * v;              // x plays b
-            const double *src = X2 + pair_off(bj[lb], x, bi[lb], 0, o, v);
-            COL_LOOP(y, v) S[(lb * v + y) * (v + 1) + x] += src[y];  // y plays a
+            const int lb = row_ / v, x = row_ - lb * v;              // x plays b, y plays a
+            const long long f = pair_off(bj[lb], x, bi[lb], 0, o, v), g = pair_off(bi[lb], x, bj[lb], 0, o, v);
+            COL_LOOP(y, v)
+                S[(lb * v + y) * (v + 1) + x] += (X2[f + y] + (Et[f + y] + E2[f + y])) + fma(0.5, Cp[f + y], Cp[g + y]);
         }
         __syncthreads();
 #pragma unroll 4
@@ -665,24 +642,27 @@ __global__ void __launch_bounds__(NT) k_amplitudes_energy(const CCMol *__restric
         }
     }
     const double r = block_red(acc, false);
-    if (threadIdx.x == 0) { P[0] = w.u == 0 ? r : 0.0; P[1] = w.u == 0 ? 0.0 : r; }
-}
-
-// E = 2 sum F_ia t_ia + sum_(ia),(jb) L(ia,jb) (t2 + t1 t1)   (energyCC r-ccsd):
-// the units' partials summed in a fixed order (strided per thread, fixed tree)
-__global__ void __launch_bounds__(NT) k_energy_finish(const CCMol *__restrict__ mols, const int *__restrict__ active,
-                                                      const int *__restrict__ start, const double *__restrict__ part)
-{
-    const int mol = blockIdx.x;
-    if (active && !active[mol]) return;
+    // E = 2 sum F_ia t_ia + sum_(ia),(jb) L(ia,jb) (t2 + t1 t1)   (energyCC r-ccsd):
+    // the molecule's last block sums the units' partials in a fixed order
+    // (strided per thread, fixed tree); the counter wraps to zero for the next launch
+    __shared__ bool last;
+    const int u0 = start[w.mol], u1 = start[w.mol + 1];
+    if (threadIdx.x == 0) {
+        P[0] = w.u == 0 ? r : 0.0;
+        P[1] = w.u == 0 ? 0.0 : r;
+        __threadfence();
+        last = atomicInc(h.done, (unsigned)(u1 - u0 - 1)) == (unsigned)(u1 - u0 - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
     double x[2] = {0.0, 0.0};
-    for (int u = start[mol] + threadIdx.x; u < start[mol + 1]; u += NT) {
-        x[0] += part[(long long)u * HX_PART_STRIDE + 0];
-        x[1] += part[(long long)u * HX_PART_STRIDE + 1];
+    for (int u = u0 + threadIdx.x; u < u1; u += NT) {
+        x[0] += __ldcg(part + (long long)u * HX_PART_STRIDE + 0);
+        x[1] += __ldcg(part + (long long)u * HX_PART_STRIDE + 1);
     }
     block_sum_n<2>(x);
     if (threadIdx.x != 0) return;
-    const CCMol &m = mols[mol];
     m.res[2] = 2.0 * x[0] + x[1] + m.eref;
     m.res[3] = m.eref;
     m.res[4] = 2.0 * x[0];
@@ -806,18 +786,12 @@ __global__ void k_setup2(EW_ARGS, int guess)
         if (e_ != cudaSuccess) return e_;                                                           \
     } while (0)
 
-cudaError_t hx_ew_dress_init(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s)
-{ LAUNCH_EW(k_dress_init, SK_NN); return cudaSuccess; }
 cudaError_t hx_ew_dress_fock(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s)
 { LAUNCH_EW(k_dress_fock, SK_NN); return cudaSuccess; }
 cudaError_t hx_ew_zdo_products(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s)
 { LAUNCH_EW(k_zdo_products, SK_ZDO); return cudaSuccess; }
 cudaError_t hx_ew_gamma_scale(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s)
 { LAUNCH_EW(k_gamma_scale, SK_ONON); return cudaSuccess; }
-cudaError_t hx_ew_fock_blocks(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s)
-{ LAUNCH_EW(k_fock_blocks, SK_FOCK); return cudaSuccess; }
-cudaError_t hx_ew_c_combine(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s)
-{ LAUNCH_EW(k_c_combine, SK_PAIR); return cudaSuccess; }
 cudaError_t hx_ew_setup(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s)
 { LAUNCH_EW(k_setup, SK_SETUP); return cudaSuccess; }
 cudaError_t hx_ew_setup2(const CCMol *m, const int *act, const HxSched &S, int guess, cudaStream_t s)
@@ -883,9 +857,7 @@ cudaError_t hx_tail(const CCMol *m, const DiisMol *h, const int *act, const HxSc
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_amplitudes_energy<<<(unsigned)S.blocks[SK_UP], NT, smem[1], s>>>(m, h, act, S.start[SK_UP], S.nmol, use_diis,
                                                                        part);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_energy_finish<<<S.nmol, NT, 0, s>>>(m, act, S.start[SK_UP], part);
-    hx_count_launches(4);
+    hx_count_launches(3);
     return cudaGetLastError();
 }
 
@@ -894,9 +866,6 @@ cudaError_t hx_energy(const CCMol *m, const DiisMol *h, const int *act, const Hx
                       cudaStream_t s)
 {
     k_amplitudes_energy<<<(unsigned)S.blocks[SK_UP], NT, smem, s>>>(m, h, act, S.start[SK_UP], S.nmol, 0, part);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_energy_finish<<<S.nmol, NT, 0, s>>>(m, act, S.start[SK_UP], part);
-    hx_count_launches(2);
+    hx_count_launches(1);
     return cudaGetLastError();
 }

@@ -419,7 +419,7 @@ static bool mo_ladder(const hx_ccsd *h, int mi)
 // (and the element-wise kernels between them, iteration_body) wrote, and no
 // two of them write the same tensor, so a level is one launch. An iteration
 // of a small molecule is a chain of launches, so its length is what counts:
-// seven levels instead of one launch per contraction (35), and what several
+// six levels instead of one launch per contraction (35), and what several
 // contractions of a level read is sliced once.
 // Index conventions are spelled out in hx_plan.h; each block cites the term
 // of the T1-dressed closed-shell CCSD equations it evaluates.
@@ -429,10 +429,9 @@ static void build_plan(hx_ccsd *h)
     enum { G_DRESS_XY = 0, G_LAD_A = 0, G_S_U = 0, G_W_MO = 0,
            G_DRESS_P = 1, G_GB = 1, G_LAD_B = 1, G_S_UG = 1,
            G_FD1 = 2, G_LEAD = 2, G_CINT1 = 2, G_DINT1 = 2, G_V_MO = 2, G_LAD_D = 2, G_S_V = 2,
-           G_FD2 = 3, G_CINT2 = 3, G_DINT2 = 3, G_LAD_E = 3, G_W_E = 3, G_W_INT_MO = 3,
-           G_FVOO = 4, G_S1 = 4, G_DINT3 = 4, G_CTERM = 4, G_W_INT = 4, G_HH_MO = 4,
-           G_E1 = 5, G_E2 = 5, G_HH = 5, G_S_R1 = 5,
-           G_DTERM = 6, G_S_R1B = 6, G_COUNT = 7 };
+           G_FD2 = 3, G_CINT2 = 3, G_DINT2 = 3, G_LAD_E = 3, G_W_E = 3, G_W_INT_MO = 3, G_S_R1 = 3,
+           G_FVOO = 4, G_S1 = 4, G_DINT3 = 4, G_CTERM = 4, G_W_INT = 4, G_HH_MO = 4, G_S_R1B = 4,
+           G_E1 = 5, G_E2 = 5, G_HH = 5, G_DTERM = 5, G_COUNT = 6 };
     h->plan.assign(G_COUNT, Group());
     auto &P = h->plan;
     for (int mi = 0; mi < h->nmol; ++mi) {
@@ -446,7 +445,11 @@ static void build_plan(hx_ccsd *h)
         P[G_DRESS_P].h.push_back(tg(m.Y, m.X, m.Pm, 1, N, N, o, N, N, o, {0, N, 0, 1, 0}, {0, N, 0, 1, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
         // Fd = X^T H2 Y
         P[G_FD1].h.push_back(tg(m.H2, m.Y, m.W1, 1, N, N, N, N, N, N, {0, N, 0, 1, 0}, {0, 1, 0, N, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
-        P[G_FD2].h.push_back(tg(m.X, m.W1, m.Fd, 1, N, N, N, N, N, N, {0, 1, 0, N, 0}, {0, 1, 0, N, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
+        // (the blocks where they are used: Fd_ia for the singles, Fd_ai^T starts r1, Fd_vv and Fd_oo start F')
+        P[G_FD2].h.push_back(tg(m.X, m.W1 + o, m.Fd + o, 1, o, v, N, o, v, N, {0, 1, 0, N, 0}, {0, 1, 0, N, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
+        P[G_FD2].h.push_back(tg(m.W1, m.X + o, m.r1, 1, o, v, N, o, v, N, {0, 1, 0, N, 0}, {0, 1, 0, N, 0}, {0, v, 0, 1, 0}, 1.0, 0.0, mi));
+        P[G_FD2].h.push_back(tg(m.X + o, m.W1 + o, m.Fvv2, 1, v, v, N, v, v, N, {0, 1, 0, N, 0}, {0, 1, 0, N, 0}, {0, v, 0, 1, 0}, 1.0, 0.0, mi));
+        P[G_FD2].h.push_back(tg(m.X, m.W1, m.Foo2, 1, o, o, N, o, o, N, {0, 1, 0, N, 0}, {0, 1, 0, N, 0}, {0, o, 0, 1, 0}, 1.0, 0.0, mi));
         // G . B for the dressed ZDO products
         P[G_GB].h.push_back(tg(G, m.Bia, m.GBia, 1, N, ov, N, N, ov, N, {0, N, 0, 1, 0}, {0, 1, 0, ov, 0}, {0, ov, 0, 1, 0}, 1.0, 0.0, mi));
         P[G_GB].h.push_back(tg(G, m.Boo, m.GBoo, 1, N, o * o, N, N, o * o, N, {0, N, 0, 1, 0}, {0, 1, 0, o * o, 0}, {0, o * o, 0, 1, 0}, 1.0, 0.0, mi));
@@ -483,22 +486,23 @@ static void build_plan(hx_ccsd *h)
         P[G_DINT1].h.push_back(tg(m.Bia, m.GBov0, m.Dint, 1, ov, ov, N, ov, ov, N, {0, 1, 0, ov, 0}, {0, 1, 0, ov, 0}, {0, ov, 0, 1, 0}, 2.0, 0.0, mi));
         P[G_DINT2].h.push_back(tg(m.Bvv, m.GBoo, m.Dint, 1, v * v, o * o, N, v, o, N, {v, 1, 0, v * v, 0}, {o, 1, 0, o * o, 0}, {ov, 1, v, (long long)v * ov, 0}, -1.0, 1.0, mi));
         P[G_DINT3].h.push_back(tg(m.u, m.Lov, m.Dint, 1, ov, ov, ov, ov, ov, ov, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, 0.5, 1.0, mi));
-        P[G_DTERM].h.push_back(tg(m.Dint, m.u, m.X2, 1, ov, ov, ov, ov, ov, ov, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, 0.5, 1.0, mi));
+        P[G_DTERM].h.push_back(tg(m.Dint, m.u, m.X2, 1, ov, ov, ov, ov, ov, ov, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, 0.5, 0.0, mi));
         // E: F'_bc = F~_bc - sum_kld u_kl^bd (ld|kc);  F'_kj = F~_kj + sum_lcd u_lj^cd (kd|lc)
         P[G_FVOO].h.push_back(tg(m.u, m.gov, m.Fvv2, 1, v, v, o * ov, v, v, ov, {0, ov, (long long)v * ov, 1, 0}, {0, ov, (long long)v * ov, 1, 0}, {0, v, 0, 1, 0}, -1.0, 1.0, mi));
         P[G_FVOO].h.push_back(tg(m.gov, m.u, m.Foo2, 1, o, o, v * ov, o, o, ov, {0, (long long)v * ov, ov, 1, 0}, {0, (long long)v * ov, ov, 1, 0}, {0, o, 0, 1, 0}, 1.0, 1.0, mi));
         //    E_ij^ab = sum_c t_ij^ac F'_bc - sum_k t_ik^ab F'_kj
-        P[G_E1].h.push_back(tg(m.t2, m.Fvv2, m.X2, 1, o * v * o, v, v, o * v * o, v, v, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, 1.0, 0.0, mi));
+        P[G_E1].h.push_back(tg(m.t2, m.Fvv2, m.Et, 1, o * v * o, v, v, o * v * o, v, v, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, {0, v, 0, 1, 0}, 1.0, 0.0, mi));
         //    (one GEMM per molecule: N runs over (ia, b), so C rows are contiguous in b; into Cint,
-        //    which CTERM was the last to read, so that both E products share a level: c_combine adds it)
+        //    which CTERM was the last to read: each product of the level has its own tensor, the
+        //    step adds them)
         P[G_E2].h.push_back(tg(m.Foo2, m.t2, m.Cint, 1, o, ov * v, o, o, v, o, {0, 1, 0, o, 0}, {ov, 1, 0, v, 0}, {0, v, ov, 1, 0}, -1.0, 0.0, mi));
         // singles: r1 = F~_ai + sum_kc u_ik^ac F~_kc + sum_kcd u_ki^cd (ad|kc)~ - sum_klc u_kl^ac (ki|lc)~
         P[G_S1].h.push_back(tg(m.u, m.Fd + o, m.r1, 1, ov, 1, ov, ov, 1, v, {0, ov, v, 1, 0}, {0, 0, N, 1, 0}, {0, 1, 0, 0, 0}, 1.0, 1.0, mi));
         P[G_S_U].h.push_back(tg(m.u, m.Bov0, m.U, 1, ov, N, ov, ov, N, ov, {0, ov, 0, 1, 0}, {0, ov, 0, 1, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
         P[G_S_UG].h.push_back(tg(m.U, G, m.UG, 1, ov, N, N, ov, N, N, {0, N, 0, 1, 0}, {0, N, 0, 1, 0}, {0, N, 0, 1, 0}, 1.0, 0.0, mi));
         P[G_S_V].h.push_back(tg(m.UG, m.Y + o, m.Vs, N, o, 1, v, o, 1, v, {0, (long long)v * N, 0, N, 1}, {0, 0, 0, 1, N}, {0, N, 0, 0, 1}, 1.0, 0.0, mi));
-        P[G_S_R1].h.push_back(tg(m.Vs, m.X + o, m.r1, 1, o, v, N, o, v, N, {0, N, 0, 1, 0}, {0, 1, 0, N, 0}, {0, v, 0, 1, 0}, 1.0, 1.0, mi));
-        P[G_S_R1B].h.push_back(tg(m.Boo, m.UG, m.r1, 1, o, v, o * N, o, v, N, {0, 1, o, (long long)o * o, 0}, {0, N, (long long)v * N, 1, 0}, {0, v, 0, 1, 0}, -1.0, 1.0, mi));
+        P[G_S_R1].h.push_back(tg(m.Vs, m.X + o, m.r1b, 1, o, v, N, o, v, N, {0, N, 0, 1, 0}, {0, 1, 0, N, 0}, {0, v, 0, 1, 0}, 1.0, 0.0, mi));
+        P[G_S_R1B].h.push_back(tg(m.Boo, m.UG, m.r1b, 1, o, v, o * N, o, v, N, {0, 1, o, (long long)o * o, 0}, {0, N, (long long)v * N, 1, 0}, {0, v, 0, 1, 0}, -1.0, 1.0, mi));
     }
     // longest products first: the tiles of a launch are dealt out in order, so
     // the short ones fill its last wave
@@ -533,7 +537,7 @@ static int allocate(hx_ccsd *h)
             m.gov = A.take<double>(pr); m.Lov = A.take<double>(pr);
             m.D1 = A.take<double>(ov); m.D2 = A.take<double>(pr); m.R2 = A.take<double>(pr);
             m.t1 = A.take<double>(ov); m.t2 = A.take<double>(pr);
-            m.r1 = A.take<double>(ov); m.r2 = A.take<double>(pr); m.u = A.take<double>(pr);
+            m.r1 = A.take<double>(ov); m.r1b = A.take<double>(ov); m.r2 = A.take<double>(pr); m.u = A.take<double>(pr);
             m.X = A.take<double>(nn); m.Y = A.take<double>(nn); m.Pm = A.take<double>(nn);
             m.H2 = A.take<double>(nn); m.W1 = A.take<double>(nn); m.Fd = A.take<double>(nn);
             m.Bia = A.take<double>(N * ov); m.GBia = A.take<double>(N * ov);
@@ -546,7 +550,7 @@ static int allocate(hx_ccsd *h)
             }
             m.Woo = A.take<double>((size_t)o * o * o * o);
             m.Vvv = mo_ladder(h, mi) ? A.take<double>((size_t)v * v * v * v) : nullptr;
-            m.Cint = A.take<double>(pr); m.Cp = A.take<double>(pr); m.Dint = A.take<double>(pr); m.X2 = A.take<double>(pr);
+            m.Cint = A.take<double>(pr); m.Cp = A.take<double>(pr); m.Dint = A.take<double>(pr); m.X2 = A.take<double>(pr); m.Et = A.take<double>(pr);
             m.Fvv2 = A.take<double>((size_t)v * v); m.Foo2 = A.take<double>((size_t)o * o);
             m.U = A.take<double>(ov * N); m.UG = A.take<double>(ov * N); m.Vs = A.take<double>((size_t)o * N);
             DiisMol &d = h->diis[mi];
@@ -557,6 +561,7 @@ static int allocate(hx_ccsd *h)
             d.gram = A.take<double>((size_t)HX_MAX_DIIS * HX_MAX_DIIS);
             d.coef = A.take<double>(HX_MAX_DIIS + 2);
             d.count = A.take<int>(1);
+            d.done = A.take<unsigned>(1);
             h->maxw_oNoN = std::max<long long>(h->maxw_oNoN, (long long)(ov + pr + N * ov));
         }
         double *resblock = A.take<double>((size_t)8 * h->nmol);
@@ -592,7 +597,6 @@ static int allocate(hx_ccsd *h)
                 case SK_ZDO: work = N * (ov + o * o + v * v); break;
                 case SK_PAIR: work = ov * ov; break;
                 case SK_ONON: work = mo_ladder(h, mi) ? 0 : o * N * o * N; break;
-                case SK_FOCK: work = ov + v * v + o * o; break;
                 case SK_SETUP: work = ov + ov * ov + N * ov; break;
                 }
                 st[(size_t)k * (n + 1) + mi] = (int)acc;
@@ -861,21 +865,17 @@ int hx_ccsd_init(hx_ccsd *h)
 static int iteration_body(hx_ccsd *h, int ph, const int *act, cudaStream_t s)
 {
     auto &P = h->plan;
-    HX_CU(hx_ew_dress_init(h->d_cc, act, h->sched, s));
-    HX_CU(hx_ew_make_u(h->d_cc, act, h->sched, h->unit_smem[0], s));
+    HX_CU(hx_ew_make_u(h->d_cc, act, h->sched, h->unit_smem[0], s));      // (and X = Y = C)
     HX_TRY(run_group(h, P[0], ph, act, s));               // X, Y; T1s = t2 Cv; U = u Bov0; (kc|ld) t2
     HX_CU(hx_ew_zdo_products(h->d_cc, act, h->sched, s));
     HX_TRY(run_group(h, P[1], ph, act, s));               // Pm; G B; Ts = Cv T1s; UG
     HX_CU(hx_ew_dress_fock(h->d_cc, act, h->sched, s));
     HX_CU(hx_ew_gamma_scale(h->d_cc, act, h->sched, s));
     HX_TRY(run_group(h, P[2], ph, act, s));               // H2 Y; leading term; Cint, Dint, (ac|bd)~; Z; Vs
-    HX_TRY(run_group(h, P[3], ph, act, s));               // Fd; Cint; Dint; ladder; W_klij
-    HX_CU(hx_ew_fock_blocks(h->d_cc, act, h->sched, s));
-    HX_TRY(run_group(h, P[4], ph, act, s));               // F'vv, F'oo; u F; Dint; C ring; W_klij or hole-hole ladder
-    HX_TRY(run_group(h, P[5], ph, act, s));               // E terms; hole-hole ladder; r1 += Vs Xv
-    HX_CU(hx_ew_c_combine(h->d_cc, act, h->sched, s));
-    HX_TRY(run_group(h, P[6], ph, act, s));               // D ring; r1 -= Boo UG
-    // (r2 += X2 + X2 pair-transposed is part of the step below)
+    HX_TRY(run_group(h, P[3], ph, act, s));               // dressed Fock blocks; Cint; Dint; ladder; W_klij; Vs Xv
+    HX_TRY(run_group(h, P[4], ph, act, s));               // F'vv, F'oo; u F; Dint; C ring; W_klij or hole-hole ladder; Boo UG
+    HX_TRY(run_group(h, P[5], ph, act, s));               // D ring; E terms; hole-hole ladder
+    // (the C, D and E terms and their pair-transposes are added in the step)
     const int use_diis = h->p.diis_enabled ? 1 : 0;
     HX_CU(hx_tail(h->d_cc, h->d_diis, act, h->sched, h->unit_smem + 1, h->p.t1_step, h->p.t2_step,
                   h->p.projection_type, use_diis, h->d_gate, h->d_part, s));

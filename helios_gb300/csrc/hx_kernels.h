@@ -8,12 +8,9 @@ cudaError_t hx_tgemm_f64_launch(const TgemmDesc *d_descs, int n, F64Tiles tiles,
 cudaError_t hx_scf_launch(const ScfMol *d_mols, int nmol, int nmax, const ScfParams &p, double *d_gpart,
                           cudaStream_t s);
 
-cudaError_t hx_ew_dress_init(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s);
 cudaError_t hx_ew_dress_fock(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s);
 cudaError_t hx_ew_zdo_products(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s);
 cudaError_t hx_ew_gamma_scale(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s);
-cudaError_t hx_ew_fock_blocks(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s);
-cudaError_t hx_ew_c_combine(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s);
 cudaError_t hx_ew_setup(const CCMol *m, const int *act, const HxSched &S, cudaStream_t s);
 cudaError_t hx_ew_setup2(const CCMol *m, const int *act, const HxSched &S, int guess, cudaStream_t s);
 // pair-unit kernels: dynamic shared memory for kernel 0 (make_u), 1 (step and

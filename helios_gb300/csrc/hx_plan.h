@@ -36,6 +36,7 @@ struct CCMol {
     double *D1, *D2, *R2;                 // denominators F_ii-F_aa, F_ii+F_jj-F_aa-F_bb, and 1/D2
     // amplitudes and residuals
     double *t1, *t2, *r1, *r2, *u;
+    double *r1b;                          // r1's products of the dressed half densities (added by the step)
     // T1-dressed factors
     double *X, *Y, *Pm, *H2, *W1, *Fd;    // N x N
     double *Bia, *GBia;                   // [N][o*v]  X_mu,a Y_mu,i (index i*v+a)
@@ -45,7 +46,7 @@ struct CCMol {
     double *T1s, *Ts, *Z, *Woo;           // ladder: o*v*o*N, o*N*o*N, Ts X: o*N*o*N, o^4
     double *Vvv;                          // MO-basis ladder integrals (ac|bd)~ [(a c)][(b d)], v^4
                                           // (small molecules in mixed precision; else null)
-    double *Cint, *Cp, *Dint, *X2;        // o^2 v^2 each
+    double *Cint, *Cp, *Dint, *X2, *Et;   // o^2 v^2 each (Et: the virtual half of the E term; Cint takes the other)
     double *Fvv2, *Foo2;                  // v*v, o*o
     double *U, *UG, *Vs;                  // [o*v][N], [o*v][N], [o][N]
     // results of the iteration (device): [0] max|d1| [1] max|d2| [2] E_total
@@ -66,6 +67,7 @@ struct CCMol {
 struct DiisMol {
     double *Ht, *He, *gram, *coef;
     int *count;
+    unsigned *done;                 // blocks of k_amplitudes_energy that have finished (wraps to 0)
     int nd;
     long long L;
 };
@@ -93,7 +95,7 @@ struct Group {
 #define HX_UNIT_ELEMS 1024
 #define HX_PART_STRIDE (2 + HX_MAX_DIIS)   // partials per unit: two maxima or sums, then DIIS dots
 
-enum { SK_NN, SK_ZDO, SK_PAIR, SK_ONON, SK_FOCK, SK_SETUP, SK_UP, SK_FULL, SK_COUNT };
+enum { SK_NN, SK_ZDO, SK_PAIR, SK_ONON, SK_SETUP, SK_UP, SK_FULL, SK_COUNT };
 
 struct HxSched {
     const int *start[SK_COUNT];    // device: first block of each molecule, then the total

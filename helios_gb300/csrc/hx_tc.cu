@@ -1154,6 +1154,8 @@ struct Engine {
     double tot[4] = {0, 0, 0, 0};
     int nsm = 152;                       // SMs of the device: CTAs of a persistent launch
     double tune_ms = 0.0;                // time spent timing candidates at creation
+    cudaStream_t side = nullptr;         // a group's FP64 problems run beside its slicing and tensor-core launches
+    cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 static cudaEvent_t take_event(Engine *e)
@@ -1512,8 +1514,15 @@ static cudaError_t slice_fixed(Engine *e, Mode &M, int mode, cudaStream_t s)
 static cudaError_t run_sub(Engine *e, Mode &M, SubGroup &sg, int mode, const int *d_active, cudaStream_t s)
 {
     const Variant &V = variant_of(mode, sg.var);
-    cudaError_t r = hx_tgemm_f64_launch(sg.fp64.d, (int)sg.fp64.h.size(), sg.fp64.tiles, d_active, s);
+    const bool beside = sg.tiles > 0 && sg.fp64.tiles.count > 0;
+    cudaError_t r = cudaSuccess;
+    if (beside) {                                        // (in a captured iteration: a parallel branch)
+        if ((r = cudaEventRecord(e->fork, s)) != cudaSuccess) return r;
+        if ((r = cudaStreamWaitEvent(e->side, e->fork, 0)) != cudaSuccess) return r;
+    }
+    r = hx_tgemm_f64_launch(sg.fp64.d, (int)sg.fp64.h.size(), sg.fp64.tiles, d_active, beside ? e->side : s);
     if (r != cudaSuccess || sg.tiles == 0) return r;
+    if (beside && (r = cudaEventRecord(e->join, e->side)) != cudaSuccess) return r;
     if ((r = slice_fixed(e, M, mode, s)) != cudaSuccess) return r;
     if ((r = prep_launch(sg.var_ops.d, (int)sg.var_ops.h.size(), sg.var_ops.work, sg.var_ops.rows, sg.var_ops.bands,
                          V.S, d_active, s, e->nsm)) != cudaSuccess)
@@ -1537,6 +1546,7 @@ static cudaError_t run_sub(Engine *e, Mode &M, SubGroup &sg, int mode, const int
         cudaEventRecord(pend.b, s);
         e->pending.push_back(pend);
     }
+    if (r == cudaSuccess && beside) r = cudaStreamWaitEvent(s, e->join, 0);
     return r;
 }
 
@@ -1652,6 +1662,13 @@ int create(Engine **out, const std::vector<Group> &plan, cudaStream_t s, int tun
         destroy(e);
         return HX_ERR_NOMEM;
     }
+    if (cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&e->join, cudaEventDisableTiming) != cudaSuccess) {
+        hx_set_error("cannot create the tensor-core backend's stream");
+        destroy(e);
+        return HX_ERR_CUDA;
+    }
     e->scratch_elems = need;
     cudaMemsetAsync(e->d_err, 0, sizeof(int), s);
     for (int md = 0; md < 4; ++md)
@@ -1727,6 +1744,9 @@ void destroy(Engine *e)
     for (Mode &md : e->mode) free_mode(md);
     for (auto &p : e->pending) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (auto x : e->pool) cudaEventDestroy(x);
+    if (e->side) { cudaStreamSynchronize(e->side); cudaStreamDestroy(e->side); }
+    if (e->fork) cudaEventDestroy(e->fork);
+    if (e->join) cudaEventDestroy(e->join);
     cudaFree(e->scratch);
     cudaFree(e->rexp);
     cudaFree(e->d_err);
