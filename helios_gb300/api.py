@@ -77,7 +77,7 @@ def library():
                      "hx_ccsd_iterate", "hx_ccsd_energy", "hx_ccsd_solve", "hx_ccsd_solve_batch",
                      "hx_ccsd_get_amplitudes", "hx_ccsd_get_scf", "hx_ccsd_dims", "hx_ccsd_trace",
                      "hx_gemm", "hx_gemm_tile", "hx_ccsd_timing", "hx_last_error", "hx_ccsd_set_model", "hx_ccsd_training_rows",
-                     "hx_mlp_nparam", "hx_mlp_predict", "hx_mlp_grad", "hx_mlp_train", "hx_ccsd_triples",
+                     "hx_mlp_nparam", "hx_mlp_predict", "hx_mlp_grad", "hx_mlp_train", "hx_ccsd_triples", "hx_ccsd_jacobian",
                      "hx_tile_table", "hx_tile_table_load", "hx_tile_variants", "hx_ccsd_tile_choices"):
             getattr(lib, name).restype = ctypes.c_int
         _lib = lib
@@ -361,6 +361,29 @@ class CoupledCluster:
         t2 = np.empty((o, o, v, v), order="F")
         _check(library().hx_ccsd_get_amplitudes(self._h, int(mol), t1.ctypes.data_as(_c_d), t2.ctypes.data_as(_c_d)))
         return t1, t2
+
+    def jacobian(self, t1, t2, vecs, step: float):
+        """J r of the residual's Jacobian at (t1, t2) for the vectors (r1, r2), through four copies of the
+        molecule each (hx_ccsd_jacobian); row-major arrays."""
+        def order(x1, x2):
+            x1, x2 = (np.asarray(x, dtype=np.float64) for x in (x1, x2))
+            if x1.flags.f_contiguous and x2.flags.f_contiguous:
+                return 0, x1, x2
+            return 1, np.ascontiguousarray(x1), np.ascontiguousarray(x2)
+
+        N, o, v, _ = self.dims[0]
+        n = len(vecs)
+        ins = [order(t1, t2)] + [order(*r) for r in vecs]
+        for _, x1, x2 in ins:
+            if x1.shape != (o, v) or x2.shape != (o, o, v, v):
+                raise ValueError(f"expected amplitudes of shapes {(o, v)} and {(o, o, v, v)}, got {x1.shape} and {x2.shape}")
+        outs = [(np.empty((o, v)), np.empty((o, o, v, v))) for _ in range(n)]      # every element is written
+        ptrs = lambda xs: (_c_d * n)(*[x.ctypes.data_as(_c_d) for x in xs])  # noqa: E731
+        _check(library().hx_ccsd_jacobian(
+            self._h, n, ins[0][1].ctypes.data_as(_c_d), ins[0][2].ctypes.data_as(_c_d), ins[0][0], ptrs([x[1] for x in ins[1:]]),
+            ptrs([x[2] for x in ins[1:]]), (ctypes.c_int32 * n)(*[x[0] for x in ins[1:]]), ctypes.c_double(step),
+            ptrs([x[0] for x in outs]), ptrs([x[1] for x in outs])))
+        return outs
 
     def scf(self, mol: int = 0):
         N = self.dims[mol][0]

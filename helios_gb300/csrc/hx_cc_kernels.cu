@@ -717,6 +717,109 @@ __global__ void __launch_bounds__(256) k_layout(double *__restrict__ t1, double 
         }
 }
 
+// ---------------------------------------------------------------- Jacobian products
+// The four points t +- h r, t +- 2 h r of each vector's stencil, into the
+// amplitudes of molecules 4q .. 4q + 3 (blockIdx.z = q). t and r come as
+// staging copies on the device, column-major (o, o, v, v) (order 0) or
+// row-major [i][j][a][b] (order 1); tiles as k_layout's.
+__device__ __forceinline__ double stage_at(const double *__restrict__ f, int order, int i, int j, int a, int b, int o, int v)
+{
+    return order ? f[(((long long)i * o + j) * v + a) * v + b]
+                 : f[i + (long long)o * j + (long long)o * o * a + (long long)o * o * v * b];
+}
+__device__ __forceinline__ void stencil_points(double t, double r, double h, double (&x)[4])
+{
+    const double hr = h * r, h2 = hr + hr;
+    x[0] = t + hr;
+    x[1] = t - hr;
+    x[2] = t + h2;
+    x[3] = t - h2;
+}
+__global__ void __launch_bounds__(256) k_jacobian_points(const CCMol *__restrict__ mols, const double *__restrict__ t1s,
+                                                         const double *__restrict__ t2s, int t_order,
+                                                         const int *__restrict__ r_order, double h, int o, int v)
+{
+    __shared__ double st[LT][LT + 1], sr[LT][LT + 1];
+    const int q = blockIdx.z, ti = (o + LT - 1) / LT, tb = (v + LT - 1) / LT, ro = r_order[q];
+    unsigned x = blockIdx.x;
+    const int b0 = (int)(x % tb) * LT;
+    x /= tb;
+    const int i0 = (int)(x % ti) * LT;
+    x /= ti;
+    const int j = (int)(x % o), a = (int)(x / o);
+    const CCMol *m = mols + 4 * q;
+    const double *r1s = m[0].U, *r2s = m[0].Cp;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    // both into [i][b]: a column-major array is read along i, a row-major one along b
+    for (int w = 0; w < 2; ++w) {
+        const double *f = w ? r2s : t2s;
+        const int order = w ? ro : t_order;
+        double (*s)[LT + 1] = w ? sr : st;
+        for (int y = ty; y < LT; y += 8) {
+            const int i = order ? i0 + y : i0 + tx, b = order ? b0 + tx : b0 + y;
+            if (i < o && b < v) s[i - i0][b - b0] = stage_at(f, order, i, j, a, b, o, v);
+        }
+    }
+    __syncthreads();
+    for (int y = ty; y < LT; y += 8) {
+        const int i = i0 + y, b = b0 + tx;
+        if (i >= o || b >= v) continue;
+        double p[4];
+        stencil_points(st[y][tx], sr[y][tx], h, p);
+        const long long e = pair_off(i, a, j, b, o, v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) m[k].t2[e] = p[k];
+    }
+    if (blockIdx.x == 0)
+        for (int e = threadIdx.x; e < o * v; e += 256) {
+            const int f = e / v + o * (e % v);
+            double p[4];
+            stencil_points(t1s[t_order ? e : f], r1s[ro ? e : f], h, p);
+            for (int k = 0; k < 4; ++k) m[k].t1[e] = p[k];
+        }
+}
+// J r = [8 (W(+h) - W(-h)) - (W(+2h) - W(-2h))] / 12 h of the residuals W that
+// the step left in the DIIS error slots (d1, and g = 3 W2 of the canonical
+// blocks i <= j), row-major into U and X2 of molecule 4q. Block = one pair
+// (i, j), i <= j, of vector blockIdx.y; both (i, j, a, b) and its mirror
+// (j, i, b, a) are written, the transpose through shared memory.
+__global__ void __launch_bounds__(256) k_jacobian_sum(const CCMol *__restrict__ mols, const DiisMol *__restrict__ diis, double h,
+                                                      int o, int v)
+{
+    __shared__ double s[LT][LT + 1];
+    const int q = blockIdx.y, ov = o * v;
+    const CCMol &m = mols[4 * q];
+    const double *E[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) E[k] = diis[4 * q + k].He;
+    auto sum = [&](long long e) { return 8.0 * (E[0][e] - E[1][e]) - (E[2][e] - E[3][e]); };
+    int i, j;
+    up_block(blockIdx.x, o, i, j);
+    const long long base = ov + (long long)blockIdx.x * v * v;
+    double *__restrict__ J2 = m.X2;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int a0 = 0; a0 < v; a0 += LT)
+        for (int b0 = 0; b0 < v; b0 += LT) {
+            __syncthreads();
+            for (int y = ty; y < LT; y += 8) {
+                const int a = a0 + y, b = b0 + tx;
+                if (a >= v || b >= v) continue;
+                const long long e = (i == j && a > b) ? base + (long long)b * v + a : base + (long long)a * v + b;
+                const double d = sum(e) / (36.0 * h);
+                s[y][tx] = d;
+                J2[(((long long)i * o + j) * v + a) * v + b] = d;
+            }
+            __syncthreads();
+            if (i < j)
+                for (int y = ty; y < LT; y += 8) {
+                    const int b = b0 + y, a = a0 + tx;
+                    if (a < v && b < v) J2[(((long long)j * o + i) * v + b) * v + a] = s[tx][y];
+                }
+        }
+    if (blockIdx.x == 0)
+        for (int e = threadIdx.x; e < ov; e += 256) m.U[e] = sum(e) / (12.0 * h);
+}
+
 // ---------------------------------------------------------------- set-up
 // Constants after SCF: denominators, ZDO vectors of the undressed ov space,
 // and the reference guess (guessCC r-ccsd, mod_cc.f90:634-650) when asked.
@@ -802,6 +905,21 @@ cudaError_t hx_layout(double *t1, double *t2, double *f1, double *f2, int o, int
     const unsigned g = (unsigned)o * v * ((o + LT - 1) / LT) * ((v + LT - 1) / LT);
     if (to_engine) k_layout<true><<<g, 256, 0, s>>>(t1, t2, f1, f2, o, v);
     else k_layout<false><<<g, 256, 0, s>>>(t1, t2, f1, f2, o, v);
+    hx_count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t hx_jacobian_points(const CCMol *m, int nvec, const double *t1, const double *t2, int t_order, const int *r_order,
+                               double h, int o, int v, cudaStream_t s)
+{
+    const dim3 g((unsigned)o * v * ((o + LT - 1) / LT) * ((v + LT - 1) / LT), 1, (unsigned)nvec);
+    k_jacobian_points<<<g, 256, 0, s>>>(m, t1, t2, t_order, r_order, h, o, v);
+    hx_count_launches(1);
+    return cudaGetLastError();
+}
+cudaError_t hx_jacobian_sum(const CCMol *m, const DiisMol *d, int nvec, double h, int o, int v, cudaStream_t s)
+{
+    k_jacobian_sum<<<dim3((unsigned)(o * (o + 1) / 2), (unsigned)nvec), 256, 0, s>>>(m, d, h, o, v);
     hx_count_launches(1);
     return cudaGetLastError();
 }

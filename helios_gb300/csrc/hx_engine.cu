@@ -1297,6 +1297,69 @@ int hx_ccsd_set_guess(hx_ccsd *h, int32_t mol, const double *t1, const double *t
     return HX_OK;
 }
 
+// J r of the residual's Jacobian at (t1, t2) for nvec vectors, each through
+// four copies of one molecule (the five-point stencil is exact: the residual
+// is a quartic in the amplitudes). Per call t and r go to the device once and
+// J r comes back; the points, the residuals of all copies and the stencil's
+// sum stay there. Staging: t in Et of molecule 0 and U of molecule 1, r in Cp
+// and U of molecule 4q, the orders in the reductions' scratch; an iteration
+// writes all of these before it reads them.
+int hx_ccsd_jacobian(hx_ccsd *h, int32_t nvec, const double *t1, const double *t2, int32_t t_order, const double *const *r1,
+                     const double *const *r2, const int32_t *r_order, double step, double *const *s1, double *const *s2)
+{
+    if (!h || !h->initialized) { hx_set_error("hx_ccsd_jacobian before hx_ccsd_init"); return HX_ERR_STATE; }
+    if (nvec <= 0 || 4LL * nvec > h->nmol || !t1 || !t2 || !r1 || !r2 || !r_order || !s1 || !s2 || !(step > 0.0) || t_order < 0 ||
+        t_order > 1) {
+        hx_set_error("hx_ccsd_jacobian: bad arguments (%d vectors need %d copies, the handle has %d)", nvec, 4 * nvec, h->nmol);
+        return HX_ERR_ARG;
+    }
+    const int o = h->o[0], v = h->v[0], used = 4 * nvec;
+    for (int q = 0; q < nvec; ++q)
+        if (!r1[q] || !r2[q] || !s1[q] || !s2[q] || r_order[q] < 0 || r_order[q] > 1) { hx_set_error("hx_ccsd_jacobian: bad vector %d", q); return HX_ERR_ARG; }
+    for (int k = 0; k < used; ++k)
+        if (h->o[k] != o || h->v[k] != v || h->scf_failed[k]) { hx_set_error("hx_ccsd_jacobian: molecule %d is not a copy of molecule 0", k); return HX_ERR_ARG; }
+    if (!h->p.diis_enabled || h->p.projection_type != 2) {
+        hx_set_error("hx_ccsd_jacobian needs diis-enabled and projection-type 2-1 (the residuals are read from the DIIS slots)");
+        return HX_ERR_STATE;
+    }
+    const size_t ov = (size_t)o * v, b1 = sizeof(double) * ov, b2 = b1 * ov;
+    const CCMol &m0 = h->cc[0], &m1 = h->cc[1];
+    HX_CU(cudaMemcpyAsync(m1.U, t1, b1, cudaMemcpyHostToDevice, h->st));
+    HX_CU(cudaMemcpyAsync(m0.Et, t2, b2, cudaMemcpyHostToDevice, h->st));
+    for (int q = 0; q < nvec; ++q) {
+        HX_CU(cudaMemcpyAsync(h->cc[4 * q].U, r1[q], b1, cudaMemcpyHostToDevice, h->st));
+        HX_CU(cudaMemcpyAsync(h->cc[4 * q].Cp, r2[q], b2, cudaMemcpyHostToDevice, h->st));
+    }
+    int *d_order = reinterpret_cast<int *>(h->d_part);
+    HX_CU(cudaMemcpyAsync(d_order, r_order, sizeof(int) * nvec, cudaMemcpyHostToDevice, h->st));
+    HX_CU(hx_jacobian_points(h->d_cc, nvec, m1.U, m0.Et, t_order, d_order, step, o, v, h->st));
+    for (int k = 0; k < used; ++k) {
+        HX_CU(cudaMemsetAsync(h->diis[k].count, 0, sizeof(int), h->st));    // slot 0 takes the residual
+        diis_mirror_reset(h, k);
+        h->rules[k] = Rules();
+    }
+    const bool idle = used < h->nmol;                    // the other molecules keep their state
+    std::vector<int> keep = h->active;
+    if (idle) {
+        for (int k = used; k < h->nmol; ++k) h->active[k] = 0;
+        HX_TRY(upload_masks(h));
+    }
+    int rc = iterate_phases(h);
+    if (idle) {
+        h->active = keep;
+        const int rc2 = upload_masks(h);
+        if (rc == HX_OK) rc = rc2;
+    }
+    HX_TRY(rc);
+    HX_CU(hx_jacobian_sum(h->d_cc, h->d_diis, nvec, step, o, v, h->st));
+    for (int q = 0; q < nvec; ++q) {
+        HX_CU(cudaMemcpyAsync(s1[q], h->cc[4 * q].U, b1, cudaMemcpyDeviceToHost, h->st));
+        HX_CU(cudaMemcpyAsync(s2[q], h->cc[4 * q].X2, b2, cudaMemcpyDeviceToHost, h->st));
+    }
+    HX_CU(cudaStreamSynchronize(h->st));
+    return HX_OK;
+}
+
 int hx_ccsd_get_scf(hx_ccsd *h, int32_t mol, double *C, double *eps, double *fmo, double scf[4], int32_t scf_status[2])
 {
     if (!h || mol < 0 || mol >= h->nmol) { hx_set_error("bad handle or molecule index"); return HX_ERR_ARG; }

@@ -27,6 +27,13 @@ cudaError_t hx_energy(const CCMol *m, const DiisMol *h, const int *act, const Hx
 // arrays on the device (f1: o*v, f2: (o*v)^2 doubles)
 cudaError_t hx_layout(double *t1, double *t2, double *f1, double *f2, int o, int v, bool to_engine, cudaStream_t s);
 
+// Jacobian products of the residual (hx_ccsd_jacobian): the stencil's points
+// from staged t (t1, t2) and r (U, Cp of molecule 4q) into molecules 4q .. 4q + 3,
+// and the stencil's sum of their residuals into U and X2 of molecule 4q
+cudaError_t hx_jacobian_points(const CCMol *m, int nvec, const double *t1, const double *t2, int t_order, const int *r_order,
+                               double h, int o, int v, cudaStream_t s);
+cudaError_t hx_jacobian_sum(const CCMol *m, const DiisMol *d, int nvec, double h, int o, int v, cudaStream_t s);
+
 // (T) triples (hx_triples.cu): ZDO pair products of the occupied and virtual
 // orbitals; the energy partials of a slab of triples i <= j <= k, and their
 // ordered sum (out[0] = E[4], out[1] = E[5] of the slab, each triple weighted

@@ -244,6 +244,10 @@ class DeviceSigma:
             self.DS1.append(np.asfortranarray(DS1))
             self.DS2.append(np.asfortranarray(DS2))
 
+        # (a stand-in engine has no jacobian(); without DIIS the residuals come back through the steps)
+        self.on_device = (hasattr(self.cc, "jacobian") and kw.diis_enabled
+                          and all(self._sign_tensors[key] is None for key in self.signs))
+
     def _basis_of(self, key, x1, x2):
         """Amplitudes between the ground state's orbital signs and a copy's (a product with +-1)."""
         S = self._sign_tensors[key]
@@ -255,6 +259,10 @@ class DeviceSigma:
         formed in place (the signs are exact: (a - x s) s d = (a s - x) d bit for bit)."""
         if len(vecs) > self.nvec:
             raise ValueError(f"{len(vecs)} vectors for an evaluator of {self.nvec}")
+        # every copy in the ground state's orbital signs: points, residuals and stencil on the device
+        if len(vecs) and self.on_device:
+            self.calls += 1
+            return self.cc.jacobian(self.t1, self.t2, vecs, self.h)
         guesses = []
         for q, (r1, r2) in enumerate(vecs):
             hr1 = np.multiply(self.h, r1, dtype=np.float64, order="F")

@@ -60,7 +60,7 @@ module helios_cc
     public :: hx_cc_params_default, hx_ccsd_create, hx_ccsd_create_batch, hx_ccsd_init, hx_ccsd_set_guess
     public :: hx_mlp_nparam, hx_ccsd_set_model, hx_ccsd_training_rows, hx_mlp_predict, hx_mlp_grad, hx_mlp_train
     public :: hx_ccsd_iterate, hx_ccsd_energy, hx_ccsd_solve, hx_ccsd_solve_batch, hx_ccsd_get_amplitudes
-    public :: hx_ccsd_get_scf, hx_ccsd_trace, hx_ccsd_triples, hx_ccsd_timing, hx_ccsd_dims, hx_ccsd_cancel
+    public :: hx_ccsd_get_scf, hx_ccsd_trace, hx_ccsd_triples, hx_ccsd_jacobian, hx_ccsd_timing, hx_ccsd_dims, hx_ccsd_cancel
     public :: hx_ccsd_destroy, hx_gemm, hx_gemm_tile, hx_gemm_noalloc, hx_tile_table, hx_tile_table_load, hx_tile_variants
     public :: hx_ccsd_tile_choices, hx_last_error
 
@@ -197,6 +197,18 @@ module helios_cc
             type(c_ptr), value :: h
             integer(c_int32_t), value :: mol
             real(c_double), intent(out) :: e(4)
+        end function
+
+        ! r1, r2, s1, s2: nvec addresses (c_loc) each; orders 0 column-major, 1 row-major
+        integer(c_int) function hx_ccsd_jacobian(h, nvec, t1, t2, t_order, r1, r2, r_order, step, s1, s2) &
+                bind(c, name='hx_ccsd_jacobian')
+            import :: c_ptr, c_int, c_int32_t, c_double
+            type(c_ptr), value :: h
+            integer(c_int32_t), value :: nvec, t_order
+            real(c_double), intent(in) :: t1(*), t2(*)
+            type(c_ptr), intent(in) :: r1(*), r2(*), s1(*), s2(*)
+            integer(c_int32_t), intent(in) :: r_order(*)
+            real(c_double), value :: step
         end function
 
         integer(c_int) function hx_ccsd_timing(h, out, profile) bind(c, name='hx_ccsd_timing')

@@ -204,6 +204,19 @@ int hx_ccsd_solve_batch(hx_ccsd *h, int32_t *status, int32_t *iters, double *e);
 /* Amplitudes of molecule mol in the reference layout (t1: o*v, t2: o*o*v*v). */
 int hx_ccsd_get_amplitudes(hx_ccsd *h, int32_t mol, double *t1, double *t2);
 
+/* Products of the residual's Jacobian, the sigma vectors of LR-CCSD on singlets
+ * (no counterpart in the reference, whose sigma equations are spin-orbital):
+ * for nvec vectors (r1, r2) the derivative J r of (d1, Omega2) at the amplitudes
+ * (t1, t2), by the stencil [8(W(t+hr) - W(t-hr)) - (W(t+2hr) - W(t-2hr))]/12h
+ * with h = step, exact for the residual's degree of four. The handle is a
+ * batch whose first 4 nvec molecules are copies of one; the contractions run
+ * as hx_ccsd_iterate's, the copies' amplitudes and DIIS histories are
+ * replaced, the other molecules keep theirs. t_order and r_order[q]: 0 for the
+ * reference layout (column-major), 1 for row-major [i][a], [i][j][a][b]; the
+ * results s1[q], s2[q] are row-major. r2 is taken as pair-symmetric. */
+int hx_ccsd_jacobian(hx_ccsd *h, int32_t nvec, const double *t1, const double *t2, int32_t t_order, const double *const *r1,
+                     const double *const *r2, const int32_t *r_order, double step, double *const *s1, double *const *s2);
+
 /* SCF results of molecule mol: C (N x N, column p = MO p, row-major [site][MO]),
  * orbital energies (N), MO Fock (N x N row-major); scf[0..3] = E_total, E_el,
  * E_nuc, last accuracy; scf_status[0..1] = status, iterations. Any pointer may
