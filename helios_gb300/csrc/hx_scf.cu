@@ -452,13 +452,16 @@ __global__ void __launch_bounds__(NT) scf_kernel(const ScfMol *__restrict__ mols
 }  // namespace
 
 // Cluster size: 16 CTAs (the non-portable size, where the device takes it)
-// while every molecule's cluster has its SMs to itself, else 8. Molecules of
-// at most kBlockN sites use one CTA of their cluster, so a launch of only
-// such molecules takes clusters of one.
+// while every molecule's cluster has its SMs to itself; 8 while at most four
+// CTAs share an SM; 4 for more molecules than that, whose reductions and
+// cluster barriers then span half the CTAs (initialisation of 128 molecules of
+// 8 to 64 sites: 65 ms with 8, 55 with 4). Molecules of at most kBlockN sites
+// use one CTA of their cluster, so a launch of only such molecules takes
+// clusters of one.
 cudaError_t hx_scf_launch(const ScfMol *d_mols, int nmol, int nmax, const ScfParams &p, double *d_gpart,
                           cudaStream_t s)
 {
-    int cs = nmax <= kBlockN ? 1 : (nmol * 16 <= HX_SCF_GRID_MAX ? 16 : 8);
+    int cs = nmax <= kBlockN ? 1 : nmol * 16 <= HX_SCF_GRID_MAX ? 16 : nmol * 8 <= 4 * HX_SCF_GRID_MAX ? 8 : 4;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     cfg.blockDim = dim3(NT);
@@ -467,7 +470,7 @@ cudaError_t hx_scf_launch(const ScfMol *d_mols, int nmol, int nmax, const ScfPar
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    const int kMaxSmem = sizeof(double) * (HX_MAX_MOL_N / 8) * HX_MAX_MOL_N;     // 8 CTAs at the largest N
+    const int kMaxSmem = sizeof(double) * (HX_MAX_MOL_N / 4) * HX_MAX_MOL_N;     // 4 CTAs at the largest N
     cudaError_t ce = cudaFuncSetAttribute(scf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (ce != cudaSuccess) return ce;
     if (cs > 8) {
