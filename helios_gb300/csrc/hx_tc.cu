@@ -132,6 +132,9 @@ struct Cfg {
     static constexpr int FIXED_K = 256;              // 7-slice products up to this K leave the tile in fixed point
     static_assert(!INT_DRAIN || (NX_ == 5 && FIXED_K <= 32 * KC_ * BK_), "fixed-point headroom");
     static constexpr int PRODUCTS = [] { int n = 0; for (int i = 0; i < S_; ++i) for (int j = 0; j < S_; ++j) n += (i + j <= QMAX_); return n; }();
+    // some A slice reaches a block that no earlier one did (LOW's i = 1: q = 3): its MMA
+    // is two where those blocks are overwritten
+    static constexpr bool SPLIT_FIRST = QMAX_ > S_ - 1;
     // pairs in the largest exact class
     static constexpr int XPAIRS = [] { int m = 0; for (int q = 0; q < NX_; ++q) { int n = 0; for (int i = 0; i < S_; ++i) n += (q - i >= 0 && q - i < S_); m = n > m ? n : m; } return m; }();
     // exactness of a chunk: (pairs per exact class) * KC*64 * 2^14 < 2^24
@@ -775,9 +778,22 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                         // Blocks 0..covered were written earlier in this k-step (the
                         // ranges issued so far cover a prefix of the blocks) and
                         // accumulate; the MMA of the new blocks overwrites them at
-                        // the chunk's first k-step.
+                        // the chunk's first k-step. Every later k-step accumulates
+                        // into all of them, one MMA per A slice (in LOW three instead
+                        // of four: the kernel is bound by shared memory, and an MMA
+                        // reads its A slice of 4 KB whatever its width).
 #pragma unroll
                         for (int kk = 0; kk < C::BK / 16; ++kk) {
+                            if (C::SPLIT_FIRST && !(chunk_start && kk == 0)) {
+#pragma unroll
+                                for (int i = 0; i < C::S; ++i) {
+                                    const int jmax = min(C::S - 1, C::QMAX - i);
+                                    if (jmax >= 0)
+                                        mma_bf16(dbase + i * C::BN, a0 + (uint64_t)((i * C::ATILE + kk * 32) >> 4),
+                                                 b0 + (uint64_t)((kk * 32) >> 4), idesc_bf16(BM, (jmax + 1) * C::BN), 1u);
+                                }
+                                continue;
+                            }
                             int covered = -1;
 #pragma unroll
                             for (int i = 0; i < C::S; ++i) {
