@@ -35,7 +35,8 @@
 //      do not depend on the tile or on the side it is used on, and one that
 //      several products read is sliced once (per iteration, where it is marked
 //      so). Integer arithmetic only.
-//   3. tc_gemm: one CTA per 128 x BN output tile (or per K slice of it).
+//   3. tc_gemm: one CTA per 128 x BN output tile (or per K slice of it), or a
+//      pair of CTAs per 256 x BN tile (cta_group::2) where that is faster.
 //      A producer warp streams 64-deep k-blocks of all slices with TMA
 //      (cp.async.bulk.tensor, 128-byte swizzle) through a ring of stages; one
 //      thread of the MMA warp issues tcgen05.mma (kind::f16, BF16 x BF16 ->
@@ -78,7 +79,7 @@ namespace tc {
 // times 2^-8q below 2^24 per chunk); the classes q >= NX are accumulated in
 // FP32 (error about K * 2^-32 relative for a chunk of depth K) and summed
 // in the epilogue, their rounding scaled down by 2^-8NX.
-//   LOW:  3 slices, pairs i + j <= 3 (8 products, 4 MMAs per k-step), NX = 1:
+//   LOW:  3 slices, pairs i + j <= 3 (8 products, 3 MMAs per k-step), NX = 1:
 //         about 2^-24 of the row maxima; 128 x 64 tiles.
 //   MID:  4 slices, pairs i + j <= 3 (10 products, 4 MMAs), NX = 2: about
 //         2^-32; 128 x 64.
@@ -96,7 +97,7 @@ namespace tc {
 //         blocks fit in TMEM.
 // These errors set the residual level a phase can reach (the GEMM outputs
 // are ~1e3-1e4 times the residual they cancel down to).
-template <int S_, int QMAX_, int NX_, int BN_, int STAGES_, int KC_, int EPIW_, int BK_>
+template <int S_, int QMAX_, int NX_, int BN_, int STAGES_, int KC_, int EPIW_, int BK_, int CTAS_ = 1>
 struct Cfg {
     static constexpr int S = S_;                     // integer slices per FP64 operand
     static constexpr int QMAX = QMAX_;               // slice pairs with i + j <= QMAX are multiplied
@@ -112,12 +113,29 @@ struct Cfg {
     static constexpr int EPI_THREADS = EPIW_ * 32;
     static constexpr int ATILE = BM * BK * 2;        // bytes per A slice tile
     static constexpr int BTILE = BN * BK * 2;        // bytes per B slice tile
-    static constexpr int STAGE_BYTES = S * (ATILE + BTILE);
+    // A pair of CTAs (cta_group::2) computes 256 x BN: each holds its 128 rows
+    // of A and half of B, and one MMA reads both halves of B for both CTAs, so
+    // a CTA reads and stores half of B per output and BN can be twice as wide
+    // (one accumulator buffer instead of two). D's columns are the even CTA's
+    // B rows, then the odd one's. Of B slices 2t and 2t+1 the even CTA holds the
+    // first and the odd CTA the second whole: one MMA of N = 2 BN, and
+    // its columns are the blocks of two consecutive classes. A slice that is the last
+    // one of some i and has no partner (even j) is held as half of its rows
+    // in each CTA: an MMA of N = BN.
+    static constexpr int CTAS = CTAS_, NBUF = CTAS_ == 1 ? 2 : 1, TM = BM * CTAS_;
+    __host__ __device__ static constexpr int jmax(int i) { return S_ - 1 < QMAX_ - i ? S_ - 1 : QMAX_ - i; }
+    __host__ __device__ static constexpr int covered(int i) { int c = -1; for (int k = 0; k < i; ++k) c = c > k + jmax(k) ? c : k + jmax(k); return c; }   // blocks written by A slices below i
+    static constexpr int PAIRS = CTAS_ == 2 ? S_ / 2 : 0;
+    __host__ __device__ static constexpr int single(bool last) { int f = 1 << 20, l = -1; for (int i = 0; i < S_; ++i) if (jmax(i) >= 0 && jmax(i) % 2 == 0) { f = f < jmax(i) ? f : jmax(i); l = l > jmax(i) ? l : jmax(i); } return last ? l : f; }
+    static constexpr int SINGLE0 = single(false), SINGLES = CTAS_ == 2 ? (single(true) - single(false)) / 2 + 1 : 0;
+    static constexpr int BROWS = CTAS_ == 2 ? BN / 2 : BN;     // rows of B per TMA box
+    static constexpr int BBYTES = CTAS_ == 2 ? PAIRS * BTILE + SINGLES * (BTILE / 2) : S * BTILE;
+    static constexpr int STAGE_BYTES = S * ATILE + BBYTES;
     // output staging strip: (hi, lo) pairs of STG_ROWS rows (all 128 where the
     // ring leaves room), row offsets and exponents of C
-    static constexpr int RING_BYTES = STAGES * S * (128 * BK * 2 + BN * BK * 2);
+    static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
     static constexpr int STG_ROWS = [] {
-        const int avail = 232448 - 1280 - 128 * 12 - STAGES_ * S_ * (128 * BK_ * 2 + BN_ * BK_ * 2);
+        const int avail = 232448 - 1280 - 128 * 12 - RING_BYTES;
         int r = 128;
         while (r > 8 && r * (BN_ + 1) * 8 > avail) r >>= 1;
         return r;
@@ -140,7 +158,9 @@ struct Cfg {
     // exactness of a chunk: (pairs per exact class) * KC*64 * 2^14 < 2^24
     static_assert((long long)XPAIRS * KC_ * BK_ * 16384LL < (1LL << 24), "chunk too deep for exact sums");
     static_assert(BK_ == 64 || BK_ == 32, "k-block depth");
-    static_assert(2 * NQ * BN_ <= 512, "two TMEM buffers must fit in 512 columns");
+    static_assert(NBUF * NQ * BN_ <= 512, "the accumulators must fit in 512 columns");
+    static_assert(CTAS_ == 1 || (BN_ % 32 == 0 && 2 * BN_ <= 256 && !(S_ >= 7)), "pair: N in steps of 32 up to 256");
+    static_assert(STAGE_BYTES % (16 * BK_) == 0 && ATILE % (16 * BK_) == 0 && (CTAS_ == 1 || (BTILE / 2) % (16 * BK_) == 0), "swizzle atoms");
     static_assert(RING_BYTES + STG_BYTES + 1280 <= 232448, "shared memory");
     static_assert(STG_ROWS * (BN_ + 1) * 8 <= 232448 - 1280 - 128 * 12 - RING_BYTES, "staging strip");
     static_assert(EPIW_ % 4 == 0 && EPI_COLS % 8 == 0, "epilogue split");
@@ -190,16 +210,27 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// CLUSTER: arrivals come from the other CTA too (acquire at cluster scope)
+template <bool CLUSTER>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
+    if constexpr (CLUSTER)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
     return ok != 0;
 }
 // Bounded wait: false (and an error record) if the phase never completes.
@@ -209,12 +240,18 @@ __device__ __forceinline__ unsigned long long globaltimer()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err, int code)
 {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     const unsigned long long t0 = globaltimer();
     for (;;) {
-        if (mbar_try_wait(bar, parity)) return true;
+        // pair: 16 tries between reads of the timer (the wait for a drain is on the critical
+        // path there, and reads at every try made it 0.3 us longer)
+#pragma unroll 1
+        for (int k = 1; CLUSTER && k < 16; ++k)
+            if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
+        if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         if (globaltimer() - t0 > WAIT_NS) break;
     }
     if (err) atomicCAS(err, 0, code);
@@ -227,6 +264,36 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, u
             smem_u32(dst)),
         "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
+}
+// Pair of CTAs: addresses in the even CTA's shared memory, loads that complete
+// on its barrier, arrivals at it, and the cluster barrier.
+__device__ __forceinline__ uint32_t cta_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t leader_addr(const void *p)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(p)));
+    return r;
+}
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t leader_bar, int x, int y)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(leader_bar), "r"(x), "r"(y)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // Shared-memory matrix descriptor of a configuration's k-block depth: K-major,
 // 128-byte rows (BK = 64, SWIZZLE_128B) or 64-byte rows (BK = 32,
@@ -250,24 +317,46 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
+__device__ __forceinline__ void mma_bf16_pair(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+// PAIR: arrives at the barrier of both CTAs
+template <bool PAIR>
 __device__ __forceinline__ void mma_commit(uint64_t *bar)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                         smem_u32(bar)), "h"((uint16_t)3)
+                     : "memory");
+    else asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
-// TMEM loads of eight columns without a wait: several loads in flight, then
-// tmem_wait_ld and tmem_tie8 on their registers (the tie names them after the
+// TMEM loads of four or eight columns without a wait: several loads in flight, then
+// tmem_wait_ld and tmem_tie on their registers (the tie names them after the
 // wait, so no use moves above it).
-__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t *r)
+template <int W>
+__device__ __forceinline__ void tmem_ld_issue(uint32_t taddr, uint32_t *r)
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    static_assert(W == 4 || W == 8, "columns per load");
+    if constexpr (W == 4)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(taddr));
+    else asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_tie8(uint32_t *r)
+template <int W>
+__device__ __forceinline__ void tmem_tie(uint32_t *r)
 {
-    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
+#pragma unroll
+    for (int k = 0; k < W; k += 4) asm volatile("" : "+r"(r[k]), "+r"(r[k + 1]), "+r"(r[k + 2]), "+r"(r[k + 3]));
 }
 
 __device__ __forceinline__ long long split_off(int x, int xi, long long s0, long long s1)
@@ -650,7 +739,7 @@ __device__ __forceinline__ TileWork tile_work(const TcDesc &d, int di, long long
     const int per_batch = d.tiles_m * d.tiles_n;
     w.bt = local / per_batch;
     local -= w.bt * per_batch;
-    const int GM = 16;
+    const int GM = 16 / C::CTAS;
     const int group = local / (GM * d.tiles_n);
     const int first_m = group * GM;
     const int gsz = min(d.tiles_m - first_m, GM);
@@ -699,19 +788,29 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
     uint32_t *tmem_slot = (uint32_t *)(acc_empty + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr bool PAIR = C::CTAS == 2;
+    const int rank = PAIR ? (int)cta_rank() : 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], C::EPI_THREADS); }
+        // pair: one arrival per epilogue warp of both CTAs, at the even CTA's barrier
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], PAIR ? 2 * C::EPI_WARPS : C::EPI_THREADS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     constexpr int WP = C::EPI_WARPS, WM = C::EPI_WARPS + 1;   // producer and MMA warps
     if (warp == WM) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                         "r"(TMEM_COLS));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                         "r"(TMEM_COLS));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();       // both CTAs' barriers are set up, both hold their TMEM
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
@@ -720,13 +819,13 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
         if (lane == 0) {
             long long g = 0;                                  // k-blocks loaded so far
             long long skip = 0;                               // tiles below: an inactive molecule's problem
-            for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+            for (long long tile = blockIdx.x / C::CTAS; tile < ntiles && ok; tile += gridDim.x / C::CTAS) {
                 if (tile < skip) continue;
                 const int di = find_problem(descs, ndesc, tile);
                 const TcDesc &d = descs[di];
                 if (active && !active[d.mol]) { skip = problem_end(descs, ndesc, ntiles, di); continue; }
                 const TileWork w = tile_work<C>(d, di, tile);
-                const int arow0 = w.bt * d.M + w.tm * BM, brow0 = w.bt * d.N + w.tn * C::BN;
+                const int arow0 = w.bt * d.M + w.tm * C::TM + rank * BM, brow0 = w.bt * d.N + w.tn * C::BN;
                 const int aplane = d.batch * d.M, bplane = d.batch * d.N;
                 for (int kb = 0; kb < w.nkb && ok; ++kb, ++g) {
                     const int st = (int)(g % C::STAGES);
@@ -735,6 +834,20 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     if (!ok) break;
                     uint8_t *sa = smem + st * C::STAGE_BYTES;
                     uint8_t *sb = sa + C::S * C::ATILE;
+                    if constexpr (PAIR) {
+                        const int x = (w.kb0 + kb) * C::BK;
+                        // both CTAs' bytes complete on the even CTA's barrier: its MMAs read both
+                        if (rank == 0) mbar_expect_tx(&full[st], 2 * C::STAGE_BYTES);
+                        const uint32_t bar = leader_addr(&full[st]);
+                        for (int p = 0; p < C::S; ++p) tma_load_2d_pair(sa + p * C::ATILE, &d.mapA, bar, x, p * aplane + arow0);
+                        for (int h = 0; h < 2 * C::PAIRS; ++h)
+                            tma_load_2d_pair(sb + h * (C::BTILE / 2), &d.mapB, bar, x,
+                                             ((h & ~1) + rank) * bplane + brow0 + (h & 1) * C::BROWS);
+                        for (int k = 0; k < C::SINGLES; ++k)
+                            tma_load_2d_pair(sb + C::PAIRS * C::BTILE + k * (C::BTILE / 2), &d.mapB, bar, x,
+                                             (C::SINGLE0 + 2 * k) * bplane + brow0 + rank * C::BROWS);
+                        continue;
+                    }
                     mbar_expect_tx(&full[st], C::STAGE_BYTES);
                     for (int p = 0; p < C::S; ++p) {
                         tma_load_2d(sa + p * C::ATILE, &d.mapA, &full[st], (w.kb0 + kb) * C::BK, p * aplane + arow0);
@@ -744,18 +857,18 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
             }
         }
     } else if (warp == WM) {
-        if (lane == 0) {
+        if (lane == 0 && rank == 0) {
             long long g = 0, gc = 0;                          // k-blocks and chunks consumed so far
             long long skip = 0;
-            for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+            for (long long tile = blockIdx.x / C::CTAS; tile < ntiles && ok; tile += gridDim.x / C::CTAS) {
                 if (tile < skip) continue;
                 const int di = find_problem(descs, ndesc, tile);
                 if (active && !active[descs[di].mol]) { skip = problem_end(descs, ndesc, ntiles, di); continue; }
                 const TileWork w = tile_work<C>(descs[di], di, tile);
                 for (int c = 0; c < w.nchunk && ok; ++c, ++gc) {
-                    const int buf = (int)(gc & 1);
-                    const uint32_t use = (uint32_t)(gc >> 1);
-                    ok = mbar_wait(&acc_empty[buf], (use & 1) ^ 1, err, 4);
+                    const int buf = C::NBUF == 2 ? (int)(gc & 1) : 0;
+                    const uint32_t use = (uint32_t)(gc >> (C::NBUF - 1));
+                    ok = mbar_wait<PAIR>(&acc_empty[buf], (use & 1) ^ 1, err, 4);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t dbase = tmem + (uint32_t)(buf * C::NQ * C::BN);
@@ -784,6 +897,21 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                         // reads its A slice of 4 KB whatever its width).
 #pragma unroll
                         for (int kk = 0; kk < C::BK / 16; ++kk) {
+                            if constexpr (PAIR) {
+#pragma unroll
+                                for (int i = 0; i < C::S; ++i) {
+                                    const uint64_t ad = a0 + (uint64_t)((i * C::ATILE + kk * 32) >> 4);
+#pragma unroll
+                                    for (int j = 0; j <= C::jmax(i); j += 2) {
+                                        const uint32_t acc = (chunk_start && kk == 0 && i + j > C::covered(i)) ? 0u : 1u;
+                                        const bool two = j < C::jmax(i);
+                                        const int at = two ? j / 2 * C::BTILE : C::PAIRS * C::BTILE + (j - C::SINGLE0) / 2 * (C::BTILE / 2);
+                                        mma_bf16_pair(dbase + (i + j) * C::BN, ad, b0 + (uint64_t)((at + kk * 32) >> 4),
+                                                      idesc_bf16(C::TM, two ? 2 * C::BN : C::BN), acc);
+                                    }
+                                }
+                                continue;
+                            }
                             if (C::SPLIT_FIRST && !(chunk_start && kk == 0)) {
 #pragma unroll
                                 for (int i = 0; i < C::S; ++i) {
@@ -813,9 +941,9 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                                 covered = max(covered, i + jmax);
                             }
                         }
-                        mma_commit(&empty[st]);
+                        mma_commit<PAIR>(&empty[st]);
                     }
-                    mma_commit(&acc_full[buf]);
+                    mma_commit<PAIR>(&acc_full[buf]);
                 }
             }
         }
@@ -830,12 +958,17 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
         // pass (up to 32) read from C before any is stored, so the reads of
         // C cost one round trip per pass (the drain's registers are free then)
         constexpr int RSTEP = C::EPI_THREADS / C::BN;
-        constexpr int U = (C::STG_ROWS + RSTEP - 1) / RSTEP < 32 ? (C::STG_ROWS + RSTEP - 1) / RSTEP : 32;
+        constexpr int ULIM = PAIR ? 4 : 32;                   // (pair: the sums of the strip's other passes stay in registers)
+        constexpr int U = (C::STG_ROWS + RSTEP - 1) / RSTEP < ULIM ? (C::STG_ROWS + RSTEP - 1) / RSTEP : ULIM;
         const int nn = threadIdx.x % C::BN, rr = threadIdx.x / C::BN;
+        // columns per TMEM load: the pair's accumulators (32 columns per thread) leave
+        // registers for four (with eight, the sums spilled to memory behind an L1 that
+        // shared memory has all but taken: 4 us per drain)
+        constexpr int LDW = PAIR ? 4 : 8;
         long long gc = 0;                                     // chunks drained so far
         int di = 0;
         long long skip = 0;
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        for (long long tile = blockIdx.x / C::CTAS; tile < ntiles; tile += gridDim.x / C::CTAS) {
             if (tile < skip) continue;
             di = next_desc(descs, ndesc, tile, di);
             const TcDesc &d = descs[di];
@@ -853,30 +986,31 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
 #pragma unroll
             for (int e = 0; e < C::EPI_COLS; ++e) { hi[e] = 0.f; lo[e] = 0.f; iacc[e] = 0; dacc[e] = 0.0; macc[e] = 0.f; }
             for (int c = 0; c < w.nchunk; ++c, ++gc) {
-                const int buf = (int)(gc & 1);
-                const uint32_t use = (uint32_t)(gc >> 1);
-                if (ok) ok = mbar_wait(&acc_full[buf], use & 1, err, 3);
+                const int buf = C::NBUF == 2 ? (int)(gc & 1) : 0;
+                const uint32_t use = (uint32_t)(gc >> (C::NBUF - 1));
+                if (ok) ok = mbar_wait<PAIR>(&acc_full[buf], use & 1, err, 3);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                for (int c0 = 0; c0 < C::EPI_COLS; c0 += 8) {
-                    // chunk value of 8 columns: the classes (exact ones first) summed
-                    // by TwoSum, then added into (hi, lo); rounding errors go to lo
-                    // all classes of the 8 columns in flight, one wait
-                    uint32_t ra[C::NQ][8];
+                for (int c0 = 0; c0 < C::EPI_COLS; c0 += LDW) {
+                    // chunk value of LDW columns: the exact classes summed by TwoSum and
+                    // added into (hi, lo); the rounding errors and the classes from NX
+                    // on (2^-8NX of the value, rounded already) go to lo
+                    // all classes of the columns in flight, one wait
+                    uint32_t ra[C::NQ][LDW];
 #pragma unroll
                     for (int q = 0; q < C::NQ; ++q)
-                        tmem_ld8_issue(tmem + lane_base + (uint32_t)(buf * C::NQ * C::BN + q * C::BN + col0 + c0), ra[q]);
+                        tmem_ld_issue<LDW>(tmem + lane_base + (uint32_t)(buf * C::NQ * C::BN + q * C::BN + col0 + c0), ra[q]);
                     tmem_wait_ld();
-                    float a[C::NQ][8];
+                    float a[C::NQ][LDW];
 #pragma unroll
                     for (int q = 0; q < C::NQ; ++q) {
-                        tmem_tie8(ra[q]);
+                        tmem_tie<LDW>(ra[q]);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) a[q][e] = __uint_as_float(ra[q][e]);
+                        for (int e = 0; e < LDW; ++e) a[q][e] = __uint_as_float(ra[q][e]);
                     }
                     if constexpr (C::INT_DRAIN) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) {
+                        for (int e = 0; e < LDW; ++e) {
                             // sum of n_q 2^8(NX-1-q) (Horner), integer arithmetic only
                             long long v = class_count(a[0][e], 0);
 #pragma unroll
@@ -887,10 +1021,12 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                         }
                     } else {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            float x = a[0][e], err = 0.f;
+                        for (int e = 0; e < LDW; ++e) {
+                            float x = a[0][e], err = a[C::NX][e];
 #pragma unroll
-                            for (int q = 1; q < C::NQ; ++q) {
+                            for (int q = C::NX + 1; q < C::NQ; ++q) err += a[q][e];
+#pragma unroll
+                            for (int q = 1; q < C::NX; ++q) {
                                 const float sq = x + a[q][e];
                                 const float bq = sq - x;
                                 err += (x - (sq - bq)) + (a[q][e] - bq);
@@ -904,7 +1040,10 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(&acc_empty[buf]);
+                if constexpr (PAIR) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(leader_addr(&acc_empty[buf]));
+                } else mbar_arrive(&acc_empty[buf]);
                 if constexpr (C::INT_DRAIN) {
                     if ((c & 31) == 31) {
 #pragma unroll
@@ -917,13 +1056,14 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
             // so that consecutive threads store consecutive columns of C;
             // C = alpha 2^(e_m + f_n - 14) x + beta C with the power of two and
             // a power-of-two alpha applied by exponent arithmetic
-            const int mv = min(BM, d.M - w.tm * BM), nv = min(C::BN, d.N - w.tn * C::BN);
+            const int row0 = w.tm * C::TM + rank * BM;
+            const int mv = max(0, min(BM, d.M - row0)), nv = min(C::BN, d.N - w.tn * C::BN);
             // mfast: the roles of rows and columns change below -- srow and sexp are
             // the columns', a thread keeps one row and walks the columns
             const bool mfast = d.mfast != 0;
             double *const Cb = d.C + (long long)w.bt * d.c[4];
             if (threadIdx.x < (mfast ? nv : mv)) {
-                const int x = (mfast ? w.tn * C::BN : w.tm * BM) + threadIdx.x;
+                const int x = (mfast ? w.tn * C::BN : row0) + threadIdx.x;
                 srow[threadIdx.x] = mfast ? split_off(x, d.Ni, d.c[2], d.c[3]) : split_off(x, d.Mi, d.c[0], d.c[1]);
                 sexp[threadIdx.x] = mfast ? d.expB[(long long)w.bt * d.N + x] : d.expA[(long long)w.bt * d.M + x];
             }
@@ -1015,7 +1155,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     constexpr int CSTEP = C::EPI_THREADS / C::STG_ROWS;
                     const int mr = threadIdx.x % C::STG_ROWS, m = r0 + mr;
                     if (m < rend && CSTEP > 0) {
-                        const int x = w.tm * BM + m, ea = d.expA[(long long)w.bt * d.M + x];
+                        const int x = row0 + m, ea = d.expA[(long long)w.bt * d.M + x];
                         double *Cm = Cb + split_off(x, d.Mi, d.c[0], d.c[1]);
                         for (int n0 = threadIdx.x / C::STG_ROWS; n0 < nv; n0 += 4 * CSTEP) {
                             double old[4];
@@ -1041,30 +1181,52 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();       // neither CTA leaves while the other one's MMAs or arrivals may reach it
     if (warp == WM) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
     }
 }
 
 // ------------------------------------------------------------------ tile-shape candidates
-// Every precision mode has a few configurations that differ only in the
-// output tile width BN (with the pipeline depth and epilogue
-// warps that fit it); slices, slice pairs, exact classes, k-block depth and
-// chunk length are the mode's own, so every candidate forms the same sums.
-// Narrow tiles waste less on the thin operands of small molecules; wide ones
-// reuse each A tile over more columns. The autotuner (choose_variant) picks one
-// per plan group, precision mode and size class.
+// Every precision mode has a few configurations that differ in the output
+// tile (with the pipeline depth and epilogue warps that fit it); slices, slice
+// pairs and exact classes are the mode's own, so every candidate forms the
+// same sums (the pairs' chunks are longer: the classes from NX on, kept in
+// FP32, are summed over 480 to 960 k instead of 256 to 512). Narrow tiles waste less
+// on the thin operands of small molecules; wide ones reuse each A tile over
+// more columns. Four stages of 32 k hide the loads better than two of 64 where
+// K is long and cost more barriers where it is short (LOW 4800^3 1.51 -> 1.43
+// ms, 600^3 0.033 -> 0.036; MID 1.77 -> 1.69, 0.039 -> 0.043).
+// A pair of CTAs reads and stages half of B per output, and its tile is twice as wide:
+// per k-step and column 0.6 of a single CTA's shared-memory traffic, which bounds
+// those. Its accumulators fill TMEM, so that a drain (a chunk's end) stops the
+// MMAs: about 2.6 to 3 us, 1.2 of it the barriers between the two CTAs and the
+// rest the 256 KB read back. LOW 6400^3 3.35 (S4: 3.13) -> 2.77 ms, HIGH 6.12 -> 5.51;
+// at 1500^3 there are too few of its tiles and it loses (0.093 -> 0.099, 0.146 -> 0.183).
+// MID drains every 480 k and gains no more than S4 does (3.97, S4 3.77, pair
+// 3.85), EXACT's chunks end every 192: no pair there. Other forms that were no faster:
+// the classes from NX on in one accumulator, which leaves room for two buffers (LOW 2.83,
+// and less exact); 16-deep k-blocks (HIGH 4800^3 2.60 -> 3.86: rows of 32 bytes).
+// The autotuner (choose_variant) picks one candidate per plan group, precision mode
+// and size class.
 using Low32 = Cfg<3, 3, 1, 32, 3, 8, 8, 64>;
-using LowS3 = Cfg<3, 3, 1, 64, 3, 8, 16, 64>;      // three stages
+using LowS4 = Cfg<3, 3, 1, 64, 4, 16, 16, 32>;     // four stages of half the depth
 using Mid48 = Cfg<4, 3, 2, 48, 2, 6, 12, 64>;
 using Mid32 = Cfg<4, 3, 2, 32, 2, 6, 8, 64>;
+using MidS4 = Cfg<4, 3, 2, 64, 4, 12, 16, 32>;
 using High32 = Cfg<5, 4, 3, 32, 3, 8, 8, 32>;
 using Exact16 = Cfg<7, 6, 5, 16, 3, 6, 8, 32>;
 using ExactS2 = Cfg<7, 6, 5, 32, 2, 6, 16, 32>;    // two stages: the strip takes the whole tile (short K)
+using LowPair = Cfg<3, 3, 1, 128, 4, 30, 16, 32, 2>;          // two CTAs, 256 x 128
+using HighPair = Cfg<5, 4, 3, 96, 3, 10, 16, 32, 2>;
 struct Variant {
     int S, BN, BK, products, smem;
+    int TM, BROWS;                   // rows of a tile; rows of B per TMA box
+    int ctas;                        // CTAs per tile
     cudaError_t (*attr)();
     void (*launch)(unsigned grid, cudaStream_t s, const TcDesc *d, int nd, long long tiles, const int *act, int *err);
+    int (*clusters)(int nsm);
 };
 template <class C>
 static cudaError_t attr_tc()
@@ -1072,23 +1234,54 @@ static cudaError_t attr_tc()
     return cudaFuncSetAttribute(tc_gemm<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
 }
 template <class C>
+static void pair_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, unsigned grid, cudaStream_t s)
+{
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(C::NTHREADS);
+    cfg.dynamicSmemBytes = C::SMEM_BYTES;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+}
+template <class C>
 static void launch_tc(unsigned grid, cudaStream_t s, const TcDesc *d, int nd, long long tiles, const int *act, int *err)
 {
-    tc_gemm<C><<<grid, C::NTHREADS, C::SMEM_BYTES, s>>>(d, nd, tiles, act, err);
+    if constexpr (C::CTAS == 1) {
+        tc_gemm<C><<<grid, C::NTHREADS, C::SMEM_BYTES, s>>>(d, nd, tiles, act, err);
+    } else {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        pair_config<C>(cfg, at, grid, s);
+        cudaLaunchKernelEx(&cfg, tc_gemm<C>, d, nd, tiles, act, err);
+    }
+}
+// clusters of the configuration that the device holds at once
+template <class C>
+static int clusters_tc(int nsm)
+{
+    if constexpr (C::CTAS == 1) return nsm;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    pair_config<C>(cfg, at, (unsigned)(nsm / 2 * 2), nullptr);
+    int n = 0;
+    return cudaOccupancyMaxActiveClusters(&n, tc_gemm<C>, &cfg) == cudaSuccess ? n : 0;
 }
 template <class C>
 static Variant variant()
 {
-    return Variant{C::S, C::BN, C::BK, C::PRODUCTS, C::SMEM_BYTES, &attr_tc<C>, &launch_tc<C>};
+    return Variant{C::S, C::BN, C::BK, C::PRODUCTS, C::SMEM_BYTES, C::TM, C::BROWS, C::CTAS, &attr_tc<C>, &launch_tc<C>, &clusters_tc<C>};
 }
-constexpr int MAX_VARIANTS = 3;
-static const int kNumVariants[4] = {3, 3, 2, 3};
+constexpr int MAX_VARIANTS = 4;
+static const int kNumVariants[4] = {4, 4, 3, 3};
 static const Variant &variant_of(int mode, int k)
 {
-    static const Variant table[4][MAX_VARIANTS] = {{variant<Low>(), variant<Low32>(), variant<LowS3>()},
-                                                   {variant<Mid>(), variant<Mid48>(), variant<Mid32>()},
-                                                   {variant<High>(), variant<High32>(), variant<High32>()},
-                                                   {variant<Exact>(), variant<Exact16>(), variant<ExactS2>()}};
+    static const Variant table[4][MAX_VARIANTS] = {{variant<Low>(), variant<Low32>(), variant<LowS4>(), variant<LowPair>()},
+                                                   {variant<Mid>(), variant<Mid48>(), variant<Mid32>(), variant<MidS4>()},
+                                                   {variant<High>(), variant<High32>(), variant<HighPair>(), variant<HighPair>()},
+                                                   {variant<Exact>(), variant<Exact16>(), variant<ExactS2>(), variant<ExactS2>()}};
     return table[mode][k];
 }
 
@@ -1169,6 +1362,7 @@ struct Engine {
     std::vector<cudaEvent_t> pool;
     double tot[4] = {0, 0, 0, 0};
     int nsm = 152;                       // SMs of the device: CTAs of a persistent launch
+    int nclusters = 76;                  // pairs of CTAs that it holds at once
     double tune_ms = 0.0;                // time spent timing candidates at creation
     cudaStream_t side = nullptr;         // a group's FP64 problems run beside its slicing and tensor-core launches
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -1456,13 +1650,14 @@ static int finish_mode(Engine *e, Mode &M, int mode, const std::vector<const Gro
             // are closer (a column-strided store moves a 32-byte sector per 8-byte output)
             const long long ms = t.Mi > 1 ? t.c[1] : t.c[0], ns = t.Ni > 1 ? t.c[3] : t.c[2];
             d.mfast = t.N == 1 || (t.M > 1 && std::llabs(ms) < std::llabs(ns));
-            d.tiles_m = (t.M + BM - 1) / BM; d.tiles_n = (t.N + V.BN - 1) / V.BN;
+            d.tiles_m = (t.M + V.TM - 1) / V.TM; d.tiles_n = (t.N + V.BN - 1) / V.BN;
             // long K over few output tiles: cut K into slices that fill the GPU
             const int nkb = (t.K + V.BK - 1) / V.BK, n64 = (t.K + 63) / 64;
             const long long out_tiles = (long long)d.batch * d.tiles_m * d.tiles_n;
             int ks = 1;
-            if (t.beta == 1.0 && out_tiles < e->nsm && n64 >= 16)
-                ks = (int)std::min<long long>((e->nsm + out_tiles - 1) / out_tiles, n64 / 8);
+            const int workers = V.ctas == 1 ? e->nsm : e->nclusters;
+            if (t.beta == 1.0 && out_tiles < workers && n64 >= 16)
+                ks = (int)std::min<long long>((workers + out_tiles - 1) / out_tiles, n64 / 8);
             d.kb_per = (nkb + ks - 1) / ks;
             d.ksplit = (nkb + d.kb_per - 1) / d.kb_per;
             d.tile_start = sg.tiles;
@@ -1471,7 +1666,7 @@ static int finish_mode(Engine *e, Mode &M, int mode, const std::vector<const Gro
             d.expB = b.p.rexp;
             for (int side = 0; side < 2; ++side) {
                 Operand &x = side ? b : a;
-                const int box = side ? V.BN : BM;
+                const int box = side ? V.BROWS : BM;
                 if (x.box[side] != box || x.bk[side] != V.BK) {
                     const int rc = make_map(&x.map[side], x.p.dst, (long long)V.S * x.rows, t.K, x.p.Kp, box, V.BK);
                     if (rc < 0) return rc;
@@ -1550,12 +1745,12 @@ static cudaError_t run_sub(Engine *e, Mode &M, SubGroup &sg, int mode, const int
         pend.b = take_event(e);
         for (const TcDesc &d : sg.tcd) {
             pend.flops += 2.0 * d.batch * (double)d.M * d.N * d.K;
-            pend.hwflops += 2.0 * d.batch * (double)d.tiles_m * BM * d.tiles_n * V.BN * rup(d.K, V.BK) * V.products;
+            pend.hwflops += 2.0 * d.batch * (double)d.tiles_m * V.TM * d.tiles_n * V.BN * rup(d.K, V.BK) * V.products;
         }
         cudaEventRecord(pend.a, s);
     }
-    // persistent: one CTA per SM (shared memory allows one), each looping over tiles
-    const unsigned grid = (unsigned)std::min<long long>(sg.tiles, e->nsm);
+    // persistent: one CTA (or pair) per SM (or two), each looping over tiles; shared memory allows one per SM
+    const unsigned grid = (unsigned)(std::min<long long>(sg.tiles, V.ctas == 1 ? e->nsm : e->nclusters) * V.ctas);
     V.launch(grid, s, sg.d_tcd, (int)sg.tcd.size(), sg.tiles, d_active, e->d_err);
     r = cudaGetLastError();
     if (e->profile) {
@@ -1641,6 +1836,9 @@ static int choose_variant(Engine *e, int mode, int gi, const Group &g, double fp
         auto it = g_tile_table.find(key);
         if (it != g_tile_table.end()) return std::min(it->second, kNumVariants[mode] - 1);
     }
+    // not in the table: the wide tiles where they were faster in every product timed from this
+    // size on (4800^3: LOW 1.51 -> 1.31 ms, MID 1.77 -> 1.70, HIGH 2.61 -> 2.48)
+    if (tuning == 0) return key[2] >= 12 && key[3] >= 36 && mode < 3 ? kNumVariants[mode] - 1 : 0;
     if (tuning != 1) return 0;
     int best = 0;
     const int rc = tune_group(e, mode, g, fp64_work, s, &best, &e->tune_ms);
@@ -1694,6 +1892,15 @@ int create(Engine **out, const std::vector<Group> &plan, cudaStream_t s, int tun
                 hx_set_error("cannot reserve shared memory for tc_gemm");
                 return HX_ERR_CUDA;
             }
+    e->nclusters = e->nsm / 2;
+    for (int md = 0; md < 4; ++md)
+        for (int v = 0; v < kNumVariants[md]; ++v)
+            if (variant_of(md, v).ctas > 1) e->nclusters = std::min(e->nclusters, variant_of(md, v).clusters(e->nsm));
+    if (e->nclusters < 1) {
+        destroy(e);
+        hx_set_error("the device holds no pair of tc_gemm's CTAs");
+        return HX_ERR_CUDA;
+    }
     if (band_attrs() != cudaSuccess) {
         destroy(e);
         hx_set_error("cannot reserve shared memory for slice_band");
