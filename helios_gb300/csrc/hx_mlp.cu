@@ -19,8 +19,11 @@
 // and the result goes straight into t2. What bounds a tile is the activation
 // arithmetic (98k SiLUs) and the FP64 features; the weights' TMA loads run
 // behind them (W2 from the tile's start, W3 from the moment the layer-2
-// products are done), one thread per row computes the features. Measured:
-// the initialisation of 128 molecules of 8-64 sites 77 -> 66 ms, of 160 sites 119 -> 109 ms.
+// products are done). Sixteen warps share the columns of a tile (eight left each
+// scheduler two warps, and most of a tile was their latency), and four more
+// compute the next tile's inputs meanwhile, one thread per row. Measured
+// (16 warps and the inputs ahead, from eight and none): 128 molecules of 8 to
+// 64 sites 23.5 -> 14.9 ms, the initialisation of 160 sites 109 -> 99 ms.
 //
 // Training (hx_mlp_grad / hx_mlp_train): the six 256-wide products of a step
 // (layers 2 and 3 forward, their weight gradients and the gradients of their
@@ -145,8 +148,10 @@ constexpr int A_KB = TILE * 128;               // one K-block of activations: 12
 constexpr int B_KB = H * 128;                  // one K-block of weights: 256 rows x 64 bf16
 constexpr int A_BYTES = 4 * A_KB;              // 64 KB
 constexpr int B_BYTES = 4 * B_KB;              // 128 KB
-constexpr int MLP_THREADS = 256;
-constexpr int MLP_SMEM = 1024 + A_BYTES + B_BYTES + (H * F + 4 * H + TILE + TILE * F) * 4;
+constexpr int MLP_PARTS = 4;                   // column parts of a tile: 4 warps each
+constexpr int MLP_COMPUTE = MLP_PARTS * TILE;  // threads of the layers; 128 more work out the next tile's inputs
+constexpr int MLP_THREADS = MLP_COMPUTE + TILE;
+constexpr int MLP_SMEM = 1024 + A_BYTES + B_BYTES + (H * F + 4 * H + MLP_PARTS * TILE + 2 * TILE * F) * 4 + 2 * TILE * 24;
 
 struct InferArgs {
     const float *X;          // [n x F] features (hx_mlp_predict) or NULL (engine)
@@ -193,14 +198,20 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_infer(InferArgs a, const _
     float *sb2 = sb1 + H;
     float *sb3 = sb2 + H;
     float *sw4 = sb3 + H;                       // [H] output weights
-    float *sred = sw4 + H;                      // [TILE] half-row dot products
-    float *sx = sred + TILE;                    // [F][TILE] normalised inputs
+    float *sred = sw4 + H;                      // [MLP_PARTS][TILE] dot products of the column parts
+    float *sx = sred + MLP_PARTS * TILE;        // [2][F][TILE] normalised inputs, of this tile and the next
+    double *sguess = (double *)(sx + 2 * TILE * F);               // [2][TILE] reference guesses
+    long long *spq = (long long *)(sguess + 2 * TILE);            // [2][TILE] pairs' positions in t2 (-1: no row)
+    long long *sqp = spq + 2 * TILE;
+    __shared__ const CCMol *smol[2];
     __shared__ __align__(8) uint64_t bar_full, bar_done;
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row = (warp & 3) * 32 + lane;     // TMEM lane = tile row of this thread
-    const int half = warp >> 2;                 // column half [128*half, +128) of this thread
+    const int part = warp >> 2;                 // column part [PC*part, +PC) of this thread; MLP_PARTS: the inputs' warps
+    constexpr int PC = H / MLP_PARTS;
+    auto compute_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(MLP_COMPUTE) : "memory"); };
     for (int k = tid; k < H * F; k += MLP_THREADS) sW1[k] = a.P[O_W1 + k];
     for (int k = tid; k < H; k += MLP_THREADS) {
         sb1[k] = a.P[O_B1 + k];
@@ -242,8 +253,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_infer(InferArgs a, const _
                 "l"(map), "r"(smem_u32(&bar_full)), "r"(kb * 64), "r"(0)
                 : "memory");
     };
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        if (tid == 0) load_weights(&mapW2);
+    // inputs of a tile into buffer b, one thread per row
+    auto load_tile = [&](long long tile, int b) {
         const CCMol *m = nullptr;
         long long gr = tile * TILE + row, n = a.n;
         if (a.mols) {
@@ -260,17 +271,29 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_infer(InferArgs a, const _
         float x[F];
         long long pq = -1, qp = -1;
         double guess = 0.0;
-        if (half == 0) {
-            load_row(a, m, gr, n, x, pq, qp, guess);
+        load_row(a, m, gr, n, x, pq, qp, guess);
 #pragma unroll
-            for (int f = 0; f < F; ++f) sx[f * TILE + row] = x[f] = (x[f] - xs[f]) * xc[f];
+        for (int f = 0; f < F; ++f) sx[(b * F + f) * TILE + row] = (x[f] - xs[f]) * xc[f];
+        spq[b * TILE + row] = m ? pq : gr < n ? gr : -1;
+        sqp[b * TILE + row] = qp;
+        sguess[b * TILE + row] = guess;
+        if (row == 0) smol[b] = m;
+    };
+    int buf = 0;
+    if (part == MLP_PARTS && blockIdx.x < ntiles) load_tile(blockIdx.x, 0);
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
+        __syncthreads();                                // this tile's inputs are there; the other buffer is free
+        if (s_abort) break;
+        if (part == MLP_PARTS) {
+            if (tile + gridDim.x < ntiles) load_tile(tile + gridDim.x, buf ^ 1);
+            continue;
         }
-        __syncthreads();
-        if (half == 1)
+        if (tid == 0) load_weights(&mapW2);
+        float x[F];
 #pragma unroll
-            for (int f = 0; f < F; ++f) x[f] = sx[f * TILE + row];
-        // layer 1: hidden units [128*half, +128) of this row, 8 per 16-byte store
-        for (int c = half * 16; c < half * 16 + 16; ++c) {
+        for (int f = 0; f < F; ++f) x[f] = sx[(buf * F + f) * TILE + row];
+        // layer 1: hidden units [PC*part, +PC) of this row, 8 per 16-byte store
+        for (int c = part * (PC / 8); c < (part + 1) * (PC / 8); ++c) {
             __align__(16) __nv_bfloat16 h8[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
@@ -287,7 +310,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_infer(InferArgs a, const _
         for (int layer = 0; layer < 2; ++layer) {
             const float *sb = layer == 0 ? sb2 : sb3;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic smem writes -> tensor core
-            __syncthreads();
+            compute_sync();
             if (tid == 0) {
                 if (!wait_bar(&bar_full, ph_full, a.err, 11)) {
                     s_abort = 1;
@@ -313,11 +336,11 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_infer(InferArgs a, const _
             if (!wait_bar(&bar_done, ph_done, a.err, 12)) s_abort = 1;
             ph_done ^= 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            __syncthreads();
+            compute_sync();
             if (s_abort) break;
             if (layer == 0 && tid == 0) load_weights(&mapW3);
-            // epilogue: this row, columns [128*half, +128)
-            for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 16) {
+            // epilogue: this row, columns [PC*part, +PC)
+            for (int c0 = part * PC; c0 < (part + 1) * PC; c0 += 16) {
                 uint32_t r[16];
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -340,17 +363,19 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_infer(InferArgs a, const _
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         }
-        if (half == 1) sred[row] = dot;
-        __syncthreads();
-        if (s_abort) break;
-        if (half == 0 && gr < n) {
-            const float y = (dot + sred[row] + b4) * ys;
+        if (part) sred[part * TILE + row] = dot;
+        compute_sync();
+        const long long pq = spq[buf * TILE + row];
+        if (part == 0 && pq >= 0 && !s_abort) {
+            for (int k = 1; k < MLP_PARTS; ++k) dot += sred[k * TILE + row];
+            const float y = (dot + b4) * ys;
+            const CCMol *m = smol[buf];
             if (!m) {
-                a.Y[gr] = y;
+                a.Y[pq] = y;
             } else {
-                const double t = guess + (double)y;
+                const double t = sguess[buf * TILE + row] + (double)y;
                 m->t2[pq] = t;
-                m->t2[qp] = t;
+                m->t2[sqp[buf * TILE + row]] = t;
             }
         }
     }
