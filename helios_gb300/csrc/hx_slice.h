@@ -84,10 +84,11 @@ __host__ __device__ __forceinline__ void slice_digits_fast(double x, int e, int 
         // are enough, (mant + 2^(n-1)) >> n = ((mant >> (n-1)) + 1) >> 1 with n = -sh
         const unsigned m = 0x80000000u | (unsigned)(bits >> 21);
         const unsigned w = shr_clamped(m, (unsigned)(-sh - 22));
-        unsigned A = (w >> 1) + (w & 1u);
+        unsigned A = S <= 3 ? (w + 1u) >> 1 : (w >> 1) + (w & 1u);     // (S <= 3: w < 2^25)
         if (ex == 0) {                                                 // zero or subnormal
             const unsigned long long mant = bits & 0xFFFFFFFFFFFFFull;
-            A = mant == 0 || sh < -62 ? 0u : (unsigned)(sh >= 0 ? mant << sh : (mant + (1ull << (-sh - 1))) >> (-sh));
+            A = 0;
+            if (mant != 0 && sh >= -62) A = (unsigned)(sh >= 0 ? mant << sh : (mant + (1ull << (-sh - 1))) >> (-sh));
         }
         const bool neg = (bits >> 63) != 0;
         if (neg) A = 0u - A;

@@ -441,6 +441,9 @@ __device__ __forceinline__ int find_desc(const PrepDesc *pd, int n, long long w)
     return lo;
 }
 
+// high word of a staged FP64 value without its sign
+__device__ __forceinline__ unsigned high_word(const double *x) { return reinterpret_cast<const unsigned *>(x)[1] & 0x7FFFFFFFu; }
+
 struct PrepTile {
     double x[PT_R][PT_K + 1];
     long long roff[PT_R], koff[PT_K];
@@ -515,17 +518,19 @@ __global__ void __launch_bounds__(PT_THREADS) row_scale(const PrepDesc *__restri
         int b, r0, k0;
         if (load_tile(pd, n, u, active, t, b, r0, k0)) {
             const PrepDesc &d = pd[t.desc];
-            // magnitudes compare as their bit patterns with the sign cleared
-            unsigned long long mb = 0;
+            // magnitudes compare as their bit patterns with the sign cleared; the high words
+            // decide the exponent unless every entry is zero or subnormal
+            const unsigned group = 0xFFu << (threadIdx.x & 24);
+            unsigned mh = 0;
 #pragma unroll
-            for (int kk = part; kk < PT_K; kk += 8) {
-                const unsigned long long v = dbits(t.x[rr][kk]) & 0x7FFFFFFFFFFFFFFFull;
-                mb = v > mb ? v : mb;
-            }
+            for (int kk = part; kk < PT_K; kk += 8) mh = max(mh, high_word(&t.x[rr][kk]));
+            mh = __reduce_max_sync(group, mh);
+            unsigned long long mb = (unsigned long long)mh << 32;
+            if (mh < 0x00100000u) {
+                mb = 0;
+                for (int kk = part; kk < PT_K; kk += 8) mb = max(mb, dbits(t.x[rr][kk]) & 0x7FFFFFFFFFFFFFFFull);
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                const unsigned long long v = __shfl_xor_sync(0xffffffffu, mb, o);
-                mb = v > mb ? v : mb;
+                for (int o = 1; o < 8; o <<= 1) mb = max(mb, __shfl_xor_sync(group, mb, o));
             }
             if (part == 0 && mb != 0 && r0 + rr < d.R)
                 atomicMax(&d.rexp[(long long)b * d.R + r0 + rr], exp_of_bits(mb));
@@ -644,15 +649,16 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
         }
         __syncthreads();
         for (int r = warp; r < rb; r += PT_THREADS / 32) {
-            unsigned long long mb = 0;
-            for (int k = lane; k < Kp; k += 32) {
-                const unsigned long long v = dbits(x[r * ld + k]) & 0x7FFFFFFFFFFFFFFFull;
-                mb = v > mb ? v : mb;
-            }
+            // high words decide the exponent unless every entry is zero or subnormal
+            unsigned mh = 0;
+            for (int k = lane; k < Kp; k += 32) mh = max(mh, high_word(x + r * ld + k));
+            mh = __reduce_max_sync(0xffffffffu, mh);
+            unsigned long long mb = (unsigned long long)mh << 32;
+            if (mh < 0x00100000u) {
+                mb = 0;
+                for (int k = lane; k < Kp; k += 32) mb = max(mb, dbits(x[r * ld + k]) & 0x7FFFFFFFFFFFFFFFull);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const unsigned long long v = __shfl_xor_sync(0xffffffffu, mb, o);
-                mb = v > mb ? v : mb;
+                for (int o = 16; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
             }
             if (lane == 0) {
                 rexp_s[r] = mb ? exp_of_bits(mb) : 0;
