@@ -62,6 +62,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -625,26 +626,38 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
         // k e / rb (consecutive threads on consecutive rows); else row e / Kp, k
         // e % Kp. Walked by the block size without divisions, the loads of
         // eight steps in flight before their values go to shared memory.
+        auto load = [&](auto rf, auto full, int e0, int &r, int &k, int dr, int dk) {
+            constexpr bool RF = decltype(rf)::value, FULL = decltype(full)::value;   // FULL: every row and element is there
+            double buf[8];
+            int at[8];
+            const double *const base = src + (RF ? roff[r] : 0);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const bool in = FULL || e0 + j * PT_THREADS + (int)threadIdx.x < total;
+                at[j] = in ? r * ld + k : -1;
+                buf[j] = (in && (FULL || r < rlim) && k < K) ? __ldg(base + ((RF ? 0 : roff[r]) + koff[k])) : 0.0;
+                if (!RF) r += dr;
+                k += dk;
+                if (!RF && k >= Kp) { k -= Kp; ++r; }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (FULL || at[j] >= 0) x[at[j]] = buf[j];
+        };
         {
+            using T = std::true_type;
+            using N = std::false_type;
             const int lrb = __ffs(rb) - 1;
-            int r = d.rfast ? (threadIdx.x & (rb - 1)) : threadIdx.x / Kp;
-            int k = d.rfast ? (threadIdx.x >> lrb) : threadIdx.x % Kp;
-            const int dr = d.rfast ? 0 : PT_THREADS / Kp, dk = d.rfast ? (PT_THREADS >> lrb) : PT_THREADS % Kp;
+            const bool rf = d.rfast != 0;
+            int r = rf ? (threadIdx.x & (rb - 1)) : threadIdx.x / Kp;
+            int k = rf ? (threadIdx.x >> lrb) : threadIdx.x % Kp;
+            const int dr = rf ? 0 : PT_THREADS / Kp, dk = rf ? (PT_THREADS >> lrb) : PT_THREADS % Kp;
             for (int e0 = 0; e0 < total; e0 += 8 * PT_THREADS) {
-                double buf[8];
-                int at[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const bool in = e0 + j * PT_THREADS + (int)threadIdx.x < total;
-                    at[j] = in ? r * ld + k : -1;
-                    buf[j] = (in && r < rlim && k < K) ? __ldg(src + roff[r] + koff[k]) : 0.0;
-                    r += dr;
-                    k += dk;
-                    if (!d.rfast && k >= Kp) { k -= Kp; ++r; }
+                if (rlim == rb && e0 + 8 * PT_THREADS <= total) {
+                    if (rf) load(T{}, T{}, e0, r, k, dr, dk); else load(N{}, T{}, e0, r, k, dr, dk);
+                } else {
+                    if (rf) load(T{}, N{}, e0, r, k, dr, dk); else load(N{}, N{}, e0, r, k, dr, dk);
                 }
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (at[j] >= 0) x[at[j]] = buf[j];
             }
         }
         __syncthreads();
