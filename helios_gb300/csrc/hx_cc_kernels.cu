@@ -12,12 +12,12 @@
 // 2133-2193, 1916-1952) works on "pair units": v x v blocks [a][b] of the
 // pair matrix for occupied pairs (i, j), staged in shared memory so that the
 // (a, b) transposes the equations need are read and written coalesced.
-//   k_step_push   residual assembly (r2 + X2 + X2 pair-transposed), the
-//                 Jacobi step, the push into the DIIS ring and the dots of
-//                 the new error vector with every stored one, per unit;
-//   k_diis_solve  per molecule: maxima, Gram row, bordered solve;
-//   k_extrapolate t = sum c_k t_k written to both halves of t2, and the
-//                 energy partials of the result.
+//   k_step_push   residual assembly (r2, the C, D and E terms and their pair
+//                 transposes), the Jacobi step, the push into the DIIS ring and
+//                 the dots of the new error vector with every stored one, per unit;
+//   k_diis_solve  per molecule: maxima, Gram row, bordered solve by one warp;
+//   k_amplitudes_energy  t = sum c_k t_k written to both halves of t2 and the
+//                 energy of the result (the last block sums the partials).
 // Only the canonical blocks i <= j are stepped and stored, as the reference
 // stores only the pairs (ia) <= (jb).
 #include <mutex>

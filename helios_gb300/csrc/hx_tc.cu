@@ -34,7 +34,9 @@
 //      products only reach outputs that are not stored. So an operand's slices
 //      do not depend on the tile or on the side it is used on, and one that
 //      several products read is sliced once (per iteration, where it is marked
-//      so). Integer arithmetic only.
+//      so). Integer arithmetic only. Operands of at most BAND_KP columns
+//      (slice_band) and large ones with contiguous rows (slice_rows) take both
+//      steps in one pass.
 //   3. tc_gemm: one CTA per 128 x BN output tile (or per K slice of it), or a
 //      pair of CTAs per 256 x BN tile (cta_group::2) where that is faster.
 //      A producer warp streams 64-deep k-blocks of all slices with TMA
@@ -422,7 +424,8 @@ struct PrepDesc {
 // Operands whose padded K is at most BAND_KP are sliced in one pass by
 // slice_band: rb rows x the whole K staged in shared memory (at most
 // BAND_ELEMS doubles), so the row maxima come from the staged band and the
-// FP64 source is read once; wider operands take row_scale + split_gather.
+// FP64 source is read once; wider operands take slice_rows (large, contiguous
+// rows) or row_scale + split_gather.
 constexpr int BAND_KP = 1024, BAND_ELEMS = 4096;
 constexpr int BAND_ROWS = 128;       // most rows of a band
 constexpr int BAND_SMEM = (BAND_ELEMS + 2 * BAND_ROWS) * 8 + BAND_KP * 8 + BAND_ROWS * 8 + BAND_ROWS * 4 + 16;
@@ -463,7 +466,7 @@ __device__ __forceinline__ bool load_tile(const PrepDesc *__restrict__ pd, int n
     __syncthreads();
     const PrepDesc &d = pd[t.desc];
     if (active && !active[d.mol]) return false;
-    if (d.rb) return false;                              // sliced by slice_band (holds no tiles)
+    if (d.rb) return false;                              // sliced by slice_band or slice_rows (holds no tiles)
     long long local = u - d.work_start;
     const int tk = (d.Kp + PT_K - 1) / PT_K, tr = (d.R + PT_R - 1) / PT_R;
     k0 = (int)(local % tk) * PT_K;
@@ -505,7 +508,7 @@ __global__ void rexp_init(const PrepDesc *__restrict__ pd, int n, long long rows
             if (pd[mid].row_start <= w) lo = mid; else hi = mid - 1;
         }
         const PrepDesc &d = pd[lo];
-        if ((active && !active[d.mol]) || d.rb) continue;   // slice_band writes its own exponents
+        if ((active && !active[d.mol]) || d.rb) continue;   // slice_band and slice_rows write their own exponents
         d.rexp[w - d.row_start] = INT_MIN;
     }
 }

@@ -21,7 +21,8 @@ advance in the same launches. The engine hands a residual back through one
 stepCC: after ``set_guess(x)`` (which also clears the DIIS history, so the
 iteration mixes nothing) and one ``iterationCC`` with unit steps,
 t1' = x1 + d1 / (F_ii - F_aa) and t2' = x2 + 3 Omega2 / (F_ii + F_jj - F_aa - F_bb)
-(mod_cc.f90:987-1017).
+(mod_cc.f90:987-1017). Where the engine has ``jacobian`` (hx_ccsd_jacobian),
+the points, the residuals and their sum stay on the device.
 
 The host part restates the reference's iteration on those coordinates:
 

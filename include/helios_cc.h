@@ -101,7 +101,8 @@ typedef struct hx_cc_params {
     double mixed_switch;          /* mixed precision: residual at which a molecule moves from
                                      3-slice to 4-slice tensor-core iterations (1e-3); 4-slice
                                      run to 1e-3 mixed_switch, then 5-slice; any of them hands
-                                     over to the check iterations below 0.1 eps */
+                                     over to the check iterations below 0.1 eps (5-slice
+                                     ones at 1e-10 where that is tighter) */
     int32_t mixed_patience;       /* mixed precision: iterations without a new lowest residual
                                      after which a molecule moves on to the next phase (3) */
     int32_t mixed_check;          /* mixed precision: the iterations that may declare
