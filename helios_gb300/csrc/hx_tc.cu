@@ -421,7 +421,8 @@ struct PrepDesc {
     long long line_start;            // prefix of slice_rows' blocks of rows over the launch
 };
 
-// Operands whose padded K is at most BAND_KP are sliced in one pass by
+// Operands whose padded K is at most BAND_KP (but for large ones whose rows are
+// contiguous, slice_rows) are sliced in one pass by
 // slice_band: rb rows x the whole K staged in shared memory (at most
 // BAND_ELEMS doubles), so the row maxima come from the staged band and the
 // FP64 source is read once; wider operands take slice_rows (large, contiguous
@@ -712,12 +713,15 @@ __global__ void __launch_bounds__(PT_THREADS, 4) slice_band(const PrepDesc *__re
     }
 }
 
-// One pass for operands of more than BAND_KP and at most ROW_KP columns that
-// are contiguous in eights: a row is held in registers by tpr threads, four
-// 8-wide chunks each (32 loads in flight, 16-byte ones where the chunks are
-// aligned), so the source is read once and nothing is staged. row_scale and
-// split_gather read it twice (an iteration of 160 sites with six such operands of
-// 41M elements: 26.5 -> 26.15 ms with 3 slices, 44.5 -> 44.0 with 5).
+// One pass for large operands of at most ROW_KP columns that are contiguous in
+// eights: a row is held in registers by tpr threads, four 8-wide chunks each
+// (32 loads in flight, 16-byte ones where the chunks are aligned), so the
+// source is read once and nothing is staged. row_scale and split_gather, which
+// slice the other operands of more than BAND_KP columns, read it twice (an
+// iteration of 160 sites with six such operands of 41M elements: 26.5 -> 26.15
+// ms with 3 slices, 44.5 -> 44.0 with 5); slice_band stages it, some 17 more
+// instructions per element (two operands of 41M and 164M elements, K = 80 and
+// 160: 26.05 -> 25.65 and 43.8 -> 43.45 ms).
 constexpr int ROW_CHUNKS = 4, ROW_KP = PT_THREADS * ROW_CHUNKS * 8;
 constexpr long long ROW_MIN = 1 << 21;      // elements
 
@@ -772,22 +776,25 @@ __global__ void __launch_bounds__(PT_THREADS, 2) slice_rows(const PrepDesc *__re
         for (int c = 0; c < ROW_CHUNKS; ++c)
 #pragma unroll
             for (int e = 0; e < 8; ++e) mh = max(mh, (unsigned)(dbits(v[c][e]) >> 32) & 0x7FFFFFFFu);
-        mh = __reduce_max_sync(0xffffffffu, mh);
+        const int lpr = min(tpr, 32);                   // lanes of the warp that share a row
+        for (int o = lpr >> 1; o > 0; o >>= 1) mh = max(mh, __shfl_xor_sync(0xffffffffu, mh, o));
         unsigned long long mb = (unsigned long long)mh << 32;
-        if (mh < 0x00100000u) {                         // the warp holds only zeros and subnormals
-            mb = 0;
+        if (__any_sync(0xffffffffu, mh < 0x00100000u)) {   // some row's lanes hold only zeros and subnormals
+            unsigned long long ms = 0;
 #pragma unroll
             for (int c = 0; c < ROW_CHUNKS; ++c)
 #pragma unroll
-                for (int e = 0; e < 8; ++e) mb = max(mb, dbits(v[c][e]) & 0x7FFFFFFFFFFFFFFFull);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+                for (int e = 0; e < 8; ++e) ms = max(ms, dbits(v[c][e]) & 0x7FFFFFFFFFFFFFFFull);
+            for (int o = lpr >> 1; o > 0; o >>= 1) ms = max(ms, __shfl_xor_sync(0xffffffffu, ms, o));
+            mb = ms;
         }
         if (lane == 0) wmax[warp] = mb;
         __syncthreads();
-        const int w0 = threadIdx.x / tpr * (tpr / 32);
-        mb = 0;
-        for (int w = w0; w < w0 + tpr / 32; ++w) mb = max(mb, wmax[w]);
+        if (tpr > 32) {
+            const int w0 = threadIdx.x / tpr * (tpr / 32);
+            mb = 0;
+            for (int w = w0; w < w0 + tpr / 32; ++w) mb = max(mb, wmax[w]);
+        }
         const int e0 = mb ? exp_of_bits(mb) : 0;
         if (valid) {
             if (t == 0) d.rexp[(long long)b * d.R + row] = mb ? e0 : INT_MIN;
@@ -813,8 +820,8 @@ static int row_threads(const PrepDesc &p)
 {
     if ((long long)p.batch * p.R * p.Kp < ROW_MIN) return 0;
     const bool contiguous = p.s[3] == 1 && (p.Ki >= p.K || p.Ki % 8 == 0 || p.s[2] == p.Ki);
-    if (p.Kp <= BAND_KP || p.Kp > ROW_KP || !contiguous) return 0;
-    int t = 32;
+    if (p.Kp > ROW_KP || !contiguous || (p.Kp <= BAND_KP && p.rfast)) return 0;
+    int t = 1;
     while (t * ROW_CHUNKS * 8 < p.Kp) t *= 2;
     return t;
 }
