@@ -912,6 +912,16 @@ static int fetch_results(hx_ccsd *h)
     return HX_OK;
 }
 
+// An error if a tensor-core wait of this handle has run out: the CTA that gave
+// up left its outputs as they were, so what was computed from them is void.
+static int check_waits(hx_ccsd *h, const char *call)
+{
+    const int w = h->tce ? tc::error_word(h->tce) : 0;
+    if (!w) return HX_OK;
+    hx_set_error("%s: a tensor-core kernel timed out waiting (code %d)", call, w);
+    return HX_ERR_KERNEL;
+}
+
 int hx_ccsd_iterate(hx_ccsd *h, int32_t iteration, double eps, double acc[5])
 {
     if (!h || !h->initialized) { hx_set_error("hx_ccsd_iterate before hx_ccsd_init"); return HX_ERR_STATE; }
@@ -919,6 +929,7 @@ int hx_ccsd_iterate(hx_ccsd *h, int32_t iteration, double eps, double acc[5])
     if (eps != h->gate_eps) { h->gate_eps = eps; HX_TRY(upload_masks(h)); }
     HX_TRY(iterate_phases(h));
     HX_TRY(fetch_results(h));
+    HX_TRY(check_waits(h, "hx_ccsd_iterate"));
     if (acc) {
         acc[0] = h->res[0]; acc[1] = h->res[1];
         acc[2] = acc[3] = acc[4] = -1.0;
@@ -1357,6 +1368,15 @@ int hx_ccsd_jacobian(hx_ccsd *h, int32_t nvec, const double *t1, const double *t
         HX_CU(cudaMemcpyAsync(s2[q], h->cc[4 * q].X2, b2, cudaMemcpyDeviceToHost, h->st));
     }
     HX_CU(cudaStreamSynchronize(h->st));
+    return check_waits(h, "hx_ccsd_jacobian");
+}
+
+// For tests of the status paths only (in no header): leaves `code` in the
+// handle's error word, as a tensor-core wait that runs out does; 0 clears it.
+int hx_ccsd_test_wait_code(hx_ccsd *h, int32_t code)
+{
+    if (!h || !h->tce) { hx_set_error("hx_ccsd_test_wait_code: a handle with a tensor-core backend is needed"); return HX_ERR_ARG; }
+    HX_CU(tc::set_error_word(h->tce, code));
     return HX_OK;
 }
 

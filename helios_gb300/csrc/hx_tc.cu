@@ -2111,6 +2111,8 @@ int error_word(Engine *e)
     return v;
 }
 
+cudaError_t set_error_word(Engine *e, int code) { return cudaMemcpy(e->d_err, &code, sizeof(int), cudaMemcpyHostToDevice); }
+
 int choices(Engine *e, int *var, int cap)
 {
     const int ng = e ? (int)e->keys.size() : 0;

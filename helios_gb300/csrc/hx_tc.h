@@ -27,6 +27,7 @@ void destroy(Engine *e);
 cudaError_t prepare_fixed(Engine *e, cudaStream_t s);
 // Device error word of the tensor-core kernels (0 = no wait timed out).
 int error_word(Engine *e);
+cudaError_t set_error_word(Engine *e, int code);
 // Live timing of the tcgen05 GEMM launches (CUDA events on the launching
 // stream): enable/disable, then collect after the stream has synchronised.
 void set_profile(Engine *e, bool on);
