@@ -1363,6 +1363,8 @@ int hx_ccsd_jacobian(hx_ccsd *h, int32_t nvec, const double *t1, const double *t
     }
     HX_TRY(rc);
     HX_CU(hx_jacobian_sum(h->d_cc, h->d_diis, nvec, step, o, v, h->st));
+    // the step counted the points as history; the copies are left without any, as the host's mirror has it
+    for (int k = 0; k < used; ++k) HX_CU(cudaMemsetAsync(h->diis[k].count, 0, sizeof(int), h->st));
     for (int q = 0; q < nvec; ++q) {
         HX_CU(cudaMemcpyAsync(s1[q], h->cc[4 * q].U, b1, cudaMemcpyDeviceToHost, h->st));
         HX_CU(cudaMemcpyAsync(s2[q], h->cc[4 * q].X2, b2, cudaMemcpyDeviceToHost, h->st));

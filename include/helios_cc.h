@@ -212,8 +212,8 @@ int hx_ccsd_get_amplitudes(hx_ccsd *h, int32_t mol, double *t1, double *t2);
  * (t1, t2), by the stencil [8(W(t+hr) - W(t-hr)) - (W(t+2hr) - W(t-2hr))]/12h
  * with h = step, exact for the residual's degree of four. The handle is a
  * batch whose first 4 nvec molecules are copies of one; the contractions run
- * as hx_ccsd_iterate's, the copies' amplitudes and DIIS histories are
- * replaced, the other molecules keep theirs. t_order and r_order[q]: 0 for the
+ * as hx_ccsd_iterate's, the copies' amplitudes are replaced and their
+ * DIIS histories emptied, the other molecules keep theirs. t_order and r_order[q]: 0 for the
  * reference layout (column-major), 1 for row-major [i][a], [i][j][a][b]; the
  * results s1[q], s2[q] are row-major. r2 is taken as pair-symmetric. */
 int hx_ccsd_jacobian(hx_ccsd *h, int32_t nvec, const double *t1, const double *t2, int32_t t_order, const double *const *r1,
