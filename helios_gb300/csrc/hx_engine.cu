@@ -56,6 +56,12 @@ struct HostModel {
     std::vector<double> coords, G, core, huckel;
 };
 
+// the same PPP problem, so the same orbitals and integrals
+static bool same_model(const HostModel &a, const HostModel &b)
+{
+    return a.N == b.N && a.nel == b.nel && a.G == b.G && a.core == b.core && a.huckel == b.huckel;
+}
+
 // readMoleculeInformation.f90:20-159 + gamma :216-264 + perturbate
 // (mod_helios.f90:577-601) with the diagonal field of setCore/applyField.
 static int build_model(const hx_ppp_model *m, const hx_cc_params *p, HostModel &out)
@@ -1328,7 +1334,10 @@ int hx_ccsd_jacobian(hx_ccsd *h, int32_t nvec, const double *t1, const double *t
     for (int q = 0; q < nvec; ++q)
         if (!r1[q] || !r2[q] || !s1[q] || !s2[q] || r_order[q] < 0 || r_order[q] > 1) { hx_set_error("hx_ccsd_jacobian: bad vector %d", q); return HX_ERR_ARG; }
     for (int k = 0; k < used; ++k)
-        if (h->o[k] != o || h->v[k] != v || h->scf_failed[k]) { hx_set_error("hx_ccsd_jacobian: molecule %d is not a copy of molecule 0", k); return HX_ERR_ARG; }
+        if (h->o[k] != o || h->v[k] != v || h->scf_failed[k] || !same_model(h->models[0], h->models[k])) {
+            hx_set_error("hx_ccsd_jacobian: molecule %d is not a copy of molecule 0", k);
+            return HX_ERR_ARG;
+        }
     if (!h->p.diis_enabled || h->p.projection_type != 2) {
         hx_set_error("hx_ccsd_jacobian needs diis-enabled and projection-type 2-1 (the residuals are read from the DIIS slots)");
         return HX_ERR_STATE;
