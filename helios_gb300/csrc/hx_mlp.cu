@@ -23,7 +23,10 @@
 // scheduler two warps, and most of a tile was their latency), and four more
 // compute the next tile's inputs meanwhile, one thread per row. Measured
 // (16 warps and the inputs ahead, from eight and none): 128 molecules of 8 to
-// 64 sites 23.5 -> 14.9 ms, the initialisation of 160 sites 109 -> 99 ms.
+// 64 sites 23.5 -> 14.9 ms, the initialisation of 160 sites 109 -> 99 ms, both
+// with an approximate division in the SiLU. With the correctly rounded one the
+// guess takes 14.8 ms of those 128 molecules' initialisation (12.2 before) and
+// 21.0 ms at 160 sites (18.6).
 //
 // Training (hx_mlp_grad / hx_mlp_train): the six 256-wide products of a step
 // (layers 2 and 3 forward, their weight gradients and the gradients of their
@@ -50,9 +53,7 @@
 
 namespace mlp {
 
-// (__fdividef: two ulps, against the bf16 rounding or the FP32 sum that follows; exp(-z) stays
-// below its 2^126 limit for z > -87, where z / (1 + exp(-z)) is zero to FP32)
-__device__ __forceinline__ float silu(float z) { return z < -87.f ? 0.f : __fdividef(z, 1.f + __expf(-z)); }
+__device__ __forceinline__ float silu(float z) { return z / (1.f + __expf(-z)); }
 __device__ __forceinline__ float dsilu(float z)
 {
     const float s = 1.f / (1.f + __expf(-z));
