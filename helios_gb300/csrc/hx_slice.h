@@ -1,6 +1,7 @@
 // Exact splitting of FP64 values into signed base-256 digits for the
 // tensor-core GEMM (integer arithmetic; host and device).
 #pragma once
+#include <cmath>
 #include <cstring>
 
 #ifndef __CUDACC__
@@ -244,6 +245,30 @@ __host__ __device__ __forceinline__ double fixed_pow2(long long v, int k, bool &
     const int e = 63 - lz + k + 1023;
     if (e < 1 || e > 2046) { ok = false; return 0.0; }
     return dfrom((v < 0 ? 0x8000000000000000ull : 0ull) + ((unsigned long long)(e - 1) << 52) + m);
+}
+
+// n 2^-BITS + m in fixed point, for a count n of the exact classes and the FP32
+// sum m of the lower ones: (n 2^fb + m 2^(BITS + fb)), m rounded to an integer
+// of that. A group of counts whose bits (signs removed) are ORed in u shares
+// fb = sum_bits(u, cap): as many bits as the largest leaves below 2^62, at most
+// cap, which keeps m's part below 2^31.
+__host__ __device__ __forceinline__ int sum_bits(unsigned long long u, int cap)
+{
+    const int fb = clz64(u | 1ull) - 2;
+    return fb < cap ? fb : cap;
+}
+template <int BITS>
+__host__ __device__ __forceinline__ long long sum_fixed(long long n, float m, int fb)
+{
+    const unsigned sb = (unsigned)(127 + BITS + fb) << 23;              // 2^(BITS + fb)
+#ifdef __CUDA_ARCH__
+    const int w = __float2int_rn(m * __uint_as_float(sb));
+#else
+    float scale;
+    memcpy(&scale, &sb, sizeof scale);
+    const int w = (int)nearbyintf(m * scale);
+#endif
+    return (long long)((unsigned long long)n << fb) + w;
 }
 
 }  // namespace tc

@@ -151,7 +151,7 @@ struct Cfg {
     static constexpr bool INT_DRAIN = S_ >= 7;
     static constexpr float DRAIN_SCALE = (float)(1ull << (8 * (NX_ - 1)));
     static constexpr int FIXED_K = 256;              // 7-slice products up to this K leave the tile in fixed point
-    static_assert(!INT_DRAIN || (NX_ == 5 && FIXED_K <= 32 * KC_ * BK_), "fixed-point headroom");
+    static_assert(!INT_DRAIN || (NX_ == 5 && FIXED_K < 32 * KC_ * BK_ && EPIW_ <= 16), "fixed-point headroom");
     static constexpr int PRODUCTS = [] { int n = 0; for (int i = 0; i < S_; ++i) for (int j = 0; j < S_; ++j) n += (i + j <= QMAX_); return n; }();
     // some A slice reaches a block that no earlier one did (LOW's i = 1: q = 3): its MMA
     // is two where those blocks are overwritten
@@ -927,6 +927,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
     float2 *strip = (float2 *)(smem + C::STAGES * C::STAGE_BYTES);   // [STG_ROWS][BN + 1] (hi, lo) of the outputs
     double *dstrip = (double *)strip;                                 // the same, 7-slice values: FP64
     long long *istrip = (long long *)strip;                           // or fixed point (short K)
+    auto spare = [&](int r) { return (short *)(strip + r * LD + C::BN); };   // [column groups] bits of the fixed point
     long long *srow = (long long *)(strip + C::STG_ROWS * LD);       // [BM] row offsets into C
     int *sexp = (int *)(srow + BM);                                   // [BM] row exponents of A
     uint64_t *full = (uint64_t *)(sexp + BM);
@@ -1224,23 +1225,33 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
             }
             const bool load_c = d.ksplit == 1 && d.beta != 0.0;
             const uint32_t negmask = d.alpha_neg ? 0x80000000u : 0u;
-            // 7-slice products with K <= FIXED_K leave the tile as one fixed-point number, the
-            // exact classes' count with the merged class added at 2^-FBITS of a count: the sum
-            // stays below K 2^46.1 counts, so FBITS = 15 - ceil(log2 K) bits fit in int64 and
-            // the merged class is rounded (2^-40 at K = 256) below what truncating the operands to
-            // seven slices leaves (2^-37).
-            // Their epilogue is the bound (short K, FP64 pipe); longer products keep FP64.
-            int fbits = 0;
-            if constexpr (C::INT_DRAIN)
-                if (d.K <= C::FIXED_K) fbits = 15 - (32 - __clz(d.K - 1));
+            // 7-slice products with K <= FIXED_K leave the tile as fixed-point numbers (their epilogue
+            // is the bound: short K, FP64 pipe; longer products keep FP64): the exact classes' count
+            // with the merged class added at 2^-fb of a count. A thread's columns of a row share fb,
+            // kept in the row's spare element of the strip: what their largest count leaves of 62 bits,
+            // 7 at least (a count stays below K 2^46.1), so that the merged class is rounded below
+            // 2^-62 of the largest of them. With the same fb for every output, 15 - ceil(log2 K), the
+            // error of K = 129 to 256 was 2 to 4 % larger; rounding each one to FP64 here took half
+            // as long again ((T) at 64 sites 41 -> 59 ms).
+            const bool fixed = C::INT_DRAIN && d.K <= C::FIXED_K;
+            const int fcap = 22 - (32 - __clz(d.K - 1));      // (the merged class is below 6 K 2^-26)
             for (int r0 = 0; r0 < mv; r0 += C::STG_ROWS) {
                 if (row >= r0 && row < r0 + C::STG_ROWS) {
+                    int fb = 0;
+                    if constexpr (C::INT_DRAIN) {
+                        if (fixed) {
+                            unsigned long long u = 0;
+#pragma unroll
+                            for (int e = 0; e < C::EPI_COLS; ++e) u |= (unsigned long long)(iacc[e] ^ (iacc[e] >> 63));
+                            fb = sum_bits(u, fcap);
+                            spare(row - r0)[warp >> 2] = (short)fb;
+                        }
+                    }
 #pragma unroll
                     for (int e = 0; e < C::EPI_COLS; ++e) {
                         if constexpr (C::INT_DRAIN) {
-                            if (fbits)
-                                istrip[(row - r0) * LD + col0 + e] =
-                                    (iacc[e] << fbits) + __float2int_rn(macc[e] * (C::DRAIN_SCALE * (float)(1 << fbits)));
+                            if (fixed)
+                                istrip[(row - r0) * LD + col0 + e] = sum_fixed<8 * (C::NX - 1)>(iacc[e], macc[e], fb);
                             else
                                 dstrip[(row - r0) * LD + col0 + e] =
                                     (dacc[e] + (double)iacc[e]) * (1.0 / (double)C::DRAIN_SCALE) + (double)macc[e];
@@ -1250,21 +1261,22 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                 }
                 asm volatile("bar.sync 1, %0;" ::"r"(C::EPI_THREADS) : "memory");
                 const int rend = min(r0 + C::STG_ROWS, mv);
-                // value of strip element at (row index in the strip x LD + column), exponents ea and eb
-                auto value = [&](int at, int ea, int eb) -> double {
+                // value of the strip's row rw, column cl, for exponents ea and eb
+                auto value = [&](int rw, int cl, int ea, int eb) -> double {
                     if (ea == INT_MIN || eb == INT_MIN) return 0.0;
                     const int k = ea + eb - 14 + d.alpha_e;
                     bool fast = d.alpha_pow2 != 0 && k >= -896 && k <= 896;
+                    const int at = rw * LD + cl;
                     if constexpr (C::INT_DRAIN) {
-                        if (fbits) {
+                        double r = 0.0;
+                        if (fixed) {
                             const long long v = istrip[at];
-                            double r = 0.0;
-                            if (fast) r = fixed_pow2(d.alpha_neg ? -v : v, k - 8 * (C::NX - 1) - fbits, fast);
-                            if (!fast) r = d.alpha * scale_pow2((double)v / ((double)C::DRAIN_SCALE * (double)(1 << fbits)), ea, eb);
+                            const int fb = spare(rw)[cl / C::EPI_COLS];
+                            if (fast) r = fixed_pow2(d.alpha_neg ? -v : v, k - 8 * (C::NX - 1) - fb, fast);
+                            if (!fast) r = d.alpha * scale_pow2((double)v / ((double)C::DRAIN_SCALE * (double)(1 << fb)), ea, eb);
                             return r;
                         }
                         const double v = dstrip[at];
-                        double r = 0.0;
                         if (fast) {
                             r = pow2_int(v, k, fast);
                             if (d.alpha_neg) r = -r;
@@ -1294,7 +1306,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                             for (int u = 0; u < U; ++u) {
                                 const int mm = m0 + u * RSTEP;
                                 if (mm >= rend) break;
-                                store(Cn + srow[mm], value((mm - r0) * LD + nn, sexp[mm], eb), old[u]);
+                                store(Cn + srow[mm], value(mm - r0, nn, sexp[mm], eb), old[u]);
                             }
                         }
                     }
@@ -1316,7 +1328,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                             for (int u = 0; u < 4; ++u) {
                                 const int nx = n0 + u * CSTEP;
                                 if (nx >= nv) break;
-                                store(Cm + srow[nx], value(mr * LD + nx, ea, sexp[nx]), old[u]);
+                                store(Cm + srow[nx], value(mr, nx, ea, sexp[nx]), old[u]);
                             }
                         }
                     }
