@@ -25,6 +25,7 @@
 #include "hx_common.cuh"
 #include "hx_plan.h"
 #include "hx_kernels.h"
+#include "hx_quotient.h"
 
 namespace {
 constexpr int NT = 256;
@@ -305,10 +306,8 @@ __global__ void __launch_bounds__(NT) k_make_u(const CCMol *__restrict__ mols, c
 //     r2 + P + P pair-transposed, P_iajb = D_iajb + (E1 + E2)_iajb +
 //     1/2 C_iajb + C_jaib (X2, Et and Cint, Cp), d2 = 2 w(ab) - w(ba)
 //     (= w on a diagonal block, whose canonical element is the same for both);
-//     g = 3 w ("2-1") or d2 ("1"); t2 += s2 g / D2, the quotient as
-//     q = s2 g R2 and one correction q + (s2 g - q D2) R2 with the stored
-//     reciprocal R2 = 1/D2 (Markstein's division: three FP64 operations
-//     instead of a division's dozen).
+//     g = 3 w ("2-1") or d2 ("1"); t2 += s2 g / D2 with the stored
+//     reciprocal R2 = 1/D2 (stored_quotient).
 // push = 1: (t, g) go into the ring slot count % nd and part gets the dots of
 // g with every stored error vector. The error vector keeps the pair (ia, ib)
 // of a diagonal block once (a <= b; the mirror element is stored as 0), so a
@@ -389,7 +388,7 @@ __global__ void __launch_bounds__(NT) k_step_push(const CCMol *__restrict__ mols
                 else { wv = a <= b ? sab : sba; d2 = wv; }
                 mx = max_abs(mx, d2);
                 const double g = proj == 1 ? d2 : 3.0 * wv, sg = s2 * g, R = Rrow[b];
-                const double q = sg * R, t = trow[b] + fma(fma(-q, Drow[b], sg), R, q);
+                const double t = trow[b] + stored_quotient(sg, Drow[b], R);
                 if (push) {
                     h.Ht[(long long)slot * h.L + hrow + b] = t;
                     // a diagonal block holds (ia, ib) and (ib, ia), the same pair: the
