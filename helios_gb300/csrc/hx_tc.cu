@@ -72,6 +72,7 @@
 #include "hx_kernels.h"
 #include "hx_slice.h"
 #include "hx_tc.h"
+#include "hx_tiles.h"
 
 namespace tc {
 
@@ -1959,6 +1960,19 @@ static TileKey tile_key(int mode, int gi, const Group &g, const std::vector<char
     return TileKey{mode, gi, nb, work > 0.0 ? (int)std::floor(std::log2(work)) : 0};
 }
 
+// Multiply-adds per output of a group's tensor-core problems.
+static double k_per_output(const Group &g, const std::vector<char> &on_tc)
+{
+    double outputs = 0.0, work = 0.0;
+    for (size_t k = 0; k < g.h.size(); ++k) {
+        const TgemmDesc &t = g.h[k];
+        if (!on_tc[k]) continue;
+        outputs += (double)t.batch * t.M * t.N;
+        work += (double)t.batch * t.M * t.N * t.K;
+    }
+    return outputs > 0.0 ? work / outputs : 0.0;
+}
+
 // Time every candidate of one group (one warm-up run that also slices the
 // constant operands, then the mean of three runs, CUDA events on s) and
 // return the fastest; *ms gets the time spent.
@@ -2009,9 +2023,7 @@ static int choose_variant(Engine *e, int mode, int gi, const Group &g, double fp
         auto it = g_tile_table.find(key);
         if (it != g_tile_table.end()) return std::min(it->second, kNumVariants[mode] - 1);
     }
-    // not in the table: the wide tiles where they were faster in every product timed from this
-    // size on (4800^3: LOW 1.51 -> 1.31 ms, MID 1.77 -> 1.70, HIGH 2.61 -> 2.48)
-    if (tuning == 0) return key[2] >= 12 && key[3] >= 36 && mode < 3 ? kNumVariants[mode] - 1 : 0;
+    if (tuning == 0) return fallback_candidate(mode, kNumVariants[mode], {key[2], key[3], k_per_output(g, e->mode[mode].on_tc[gi])});
     if (tuning != 1) return 0;
     int best = 0;
     const int rc = tune_group(e, mode, g, fp64_work, s, &best, &e->tune_ms);
