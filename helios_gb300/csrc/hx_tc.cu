@@ -1428,7 +1428,9 @@ static int clusters_tc(int nsm)
     cudaLaunchAttribute at[1];
     pair_config<C>(cfg, at, (unsigned)(nsm / 2 * 2), nullptr);
     int n = 0;
-    return cudaOccupancyMaxActiveClusters(&n, tc_gemm<C>, &cfg) == cudaSuccess ? n : 0;
+    if (cudaOccupancyMaxActiveClusters(&n, tc_gemm<C>, &cfg) == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
 }
 template <class C>
 static Variant variant()
@@ -1525,7 +1527,7 @@ struct Engine {
     std::vector<cudaEvent_t> pool;
     double tot[4] = {0, 0, 0, 0};
     int nsm = 152;                       // SMs of the device: CTAs of a persistent launch
-    int nclusters = 76;                  // pairs of CTAs that it holds at once
+    int nclusters = 76;                  // pairs of CTAs that it holds at once (0: pair candidates are left out)
     double tune_ms = 0.0;                // time spent timing candidates at creation
     cudaStream_t side = nullptr;         // a group's FP64 problems run beside its slicing and tensor-core launches
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -1988,6 +1990,7 @@ static int tune_group(Engine *e, int mode, const Group &g, double fp64_work, cud
     const auto t0 = std::chrono::steady_clock::now();
     int rc = HX_OK;
     for (int v = 0; v < kNumVariants[mode] && rc == HX_OK; ++v) {
+        if (held_candidate(v, variant_of(mode, v).ctas, e->nclusters, true) < 0) continue;
         Mode M;
         const std::vector<const Group *> one{&g};
         lay_out(M, mode, one, fp64_work);
@@ -2016,14 +2019,19 @@ static int tune_group(Engine *e, int mode, const Group &g, double fp64_work, cud
 
 static int choose_variant(Engine *e, int mode, int gi, const Group &g, double fp64_work, cudaStream_t s, int tuning, int force)
 {
-    if (force >= 0) return std::min(force, kNumVariants[mode] - 1);
+    if (force >= 0) {
+        const int c = std::min(force, kNumVariants[mode] - 1), held = held_candidate(c, variant_of(mode, c).ctas, e->nclusters, true);
+        if (held < 0) hx_set_error("tile candidate %d of mode %d: the device holds no pair of tc_gemm's CTAs", c, mode);
+        return held < 0 ? HX_ERR_CUDA : held;
+    }
+    auto held = [&](int c) { return held_candidate(c, variant_of(mode, c).ctas, e->nclusters, false); };
     const TileKey key = tile_key(mode, gi, g, e->mode[mode].on_tc[gi]);
     if (tuning != 2) {
         std::lock_guard<std::mutex> lock(g_tile_mu);
         auto it = g_tile_table.find(key);
-        if (it != g_tile_table.end()) return std::min(it->second, kNumVariants[mode] - 1);
+        if (it != g_tile_table.end()) return held(std::min(it->second, kNumVariants[mode] - 1));
     }
-    if (tuning == 0) return fallback_candidate(mode, kNumVariants[mode], {key[2], key[3], k_per_output(g, e->mode[mode].on_tc[gi])});
+    if (tuning == 0) return held(fallback_candidate(mode, kNumVariants[mode], {key[2], key[3], k_per_output(g, e->mode[mode].on_tc[gi])}));
     if (tuning != 1) return 0;
     int best = 0;
     const int rc = tune_group(e, mode, g, fp64_work, s, &best, &e->tune_ms);
@@ -2081,11 +2089,6 @@ int create(Engine **out, const std::vector<Group> &plan, cudaStream_t s, int tun
     for (int md = 0; md < 4; ++md)
         for (int v = 0; v < kNumVariants[md]; ++v)
             if (variant_of(md, v).ctas > 1) e->nclusters = std::min(e->nclusters, variant_of(md, v).clusters(e->nsm));
-    if (e->nclusters < 1) {
-        destroy(e);
-        hx_set_error("the device holds no pair of tc_gemm's CTAs");
-        return HX_ERR_CUDA;
-    }
     if (band_attrs() != cudaSuccess) {
         destroy(e);
         hx_set_error("cannot reserve shared memory for slice_band");

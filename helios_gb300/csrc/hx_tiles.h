@@ -28,4 +28,13 @@ inline int fallback_candidate(int mode, int candidates, const LevelShape &s)
     return s.k_per_output >= (mode == 1 ? kDeepK : kPairK) ? candidates - 1 : 0;
 }
 
+// A candidate of a mode (its tiles take `ctas` CTAs each) on a device that
+// holds `clusters` pairs of them at once: the default one instead of a pair
+// that does not fit, -1 (an error) where the caller asked for it by number.
+inline int held_candidate(int candidate, int ctas, int clusters, bool forced)
+{
+    if (ctas == 1 || clusters > 0) return candidate;
+    return forced ? -1 : 0;
+}
+
 }  // namespace tc

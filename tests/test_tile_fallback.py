@@ -41,3 +41,12 @@ def test_no_choice_is_slower_than_the_default(tmp_path):
         assert (last if c else first) <= 1.01 * first, row
         if w >= 36 and last < 0.96 * first:
             assert c, row
+
+
+def test_a_pair_that_does_not_fit_is_left_out(tmp_path):
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text('#include <cstdio>\n#include "hx_tiles.h"\nint main() { printf("%d %d %d %d %d\\n", tc::held_candidate(3, 2, 76, false), '
+                   'tc::held_candidate(3, 2, 0, false), tc::held_candidate(3, 2, 0, true), tc::held_candidate(2, 1, 0, false), '
+                   'tc::held_candidate(2, 1, 0, true)); }')
+    subprocess.run(["g++", "-O2", "-std=c++17", "-I", os.path.join(ROOT, "helios_gb300", "csrc"), str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split() == ["3", "0", "-1", "2", "2"]
