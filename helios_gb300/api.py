@@ -88,6 +88,7 @@ def library():
 
 # ---------------------------------------------------------------- tile autotuner
 TILE_TABLE_PATH = os.path.join(_HERE, "data", "tile_table.json")
+PLAN_LEVELS = 6      # contraction levels of an iteration: the plan groups of a table's entries
 TILE_TUNING = {"table": 0, "tune": 1, "default": 2}
 
 
@@ -114,9 +115,19 @@ def load_tile_table(entries):
 
 
 def read_tile_table(path):
+    """Entries of a table file; none (with a warning) if it was measured for an iteration of other
+    levels, whose entries would pick tiles for contractions that they were not timed on. A file
+    without a level count has as many as its entries name."""
     import json
+    import warnings
     with open(path) as f:
         d = json.load(f)
+    levels = d.get("levels")
+    if levels is None:
+        levels = PLAN_LEVELS if all(e[1] < PLAN_LEVELS for e in d["entries"]) else 1 + max(e[1] for e in d["entries"])
+    if levels != PLAN_LEVELS:
+        warnings.warn(f"{path}: a tile table for {levels} contraction levels, an iteration has {PLAN_LEVELS}: not used")
+        return []
     return [tuple(int(x) for x in e) for e in d["entries"]]
 
 
@@ -124,7 +135,7 @@ def write_tile_table(path, entries, note=""):
     import json
     entries = sorted(tuple(int(x) for x in e) for e in entries)
     head = json.dumps({"format": "mode, plan group, ceil log2 of the widest N, floor log2 of the multiply-adds, variant",
-                       "note": note})
+                       "levels": PLAN_LEVELS, "note": note})
     with open(path, "w") as f:       # one entry per line
         f.write(head[:-1] + ', "entries": [\n' + ",\n".join(json.dumps(list(e)) for e in entries) + "\n]}\n")
 
