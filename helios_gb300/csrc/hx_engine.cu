@@ -13,6 +13,7 @@
 #include "../../include/helios_cc.h"
 #include "hx_kernels.h"
 #include "hx_mlp.h"
+#include "hx_slabs.h"
 #include "hx_tc.h"
 
 cudaError_t hx_mlp_sample(const CCMol *d_mols, int mol, const long long *d_rows, int n, float *dX, float *dT,
@@ -1564,28 +1565,21 @@ int hx_ccsd_triples(hx_ccsd *h, int32_t mol, double e[4])
     const long long ov = (long long)o * v, vvv = (long long)v * v * v;
     const size_t nI1 = (size_t)ov * v * v, nJ = (size_t)ov * o * o;
     const size_t nBvv = (size_t)N * v * v, nBoo = (size_t)N * o * o;
-    // slab budget: W (v^3 doubles per triple) plus the 7-slice bf16 copies of the
-    // operands a k-batched term (P4, P6) slices per triple (14 B per element of a
-    // v^2 x K tile, K padded to 64)
-    // (its own operands are sliced once per slab: 14 B per element of (bd|ai), (ck|jl) and t2)
-    const double per_pair = 8.0 * vvv + 14.0 * (double)(v * v) * ((v + 7) / 8 * 8);
     size_t fre = 0, tot = 0;
     HX_CU(cudaMemGetInfo(&fre, &tot));
-    const double fixed_bytes = 8.0 * (nI1 + nJ + nBvv + 2 * nBoo) + 28.0 * (2.0 * nI1 + 4.0 * nJ + 6.0 * (double)ov * ov);
-    const double budget = std::min(24e9, 0.5 * ((double)fre - fixed_bytes));
-    const long long max_pairs = (long long)(budget / per_pair);
-    if (max_pairs < o) {
+    SlabPlan sp = plan_slabs(N, o, v, (double)fre);
+    if (sp.triples < o) {
         hx_set_error("hx_ccsd_triples: N = %d needs about %.1f GB of device memory for one slab of triples, "
-                     "%.1f GB are free", N, (fixed_bytes + o * per_pair) / 1e9, fre / 1e9);
+                     "%.1f GB are free", N, sp.bytes / 1e9, fre / 1e9);
         return HX_ERR_NOMEM;
     }
-    // slabs of rows (i, j) with sum (o - j) <= max_pairs triples
+    // slabs of rows (i, j) with sum (o - j) <= sp.triples
     struct Slab { std::vector<std::array<int, 2>> rows; long long pairs = 0; };
     std::vector<Slab> slabs(1);
     long long maxp = 0;
     for (int i = 0; i < o; ++i)
         for (int j = i; j < o; ++j) {
-            if (slabs.back().pairs + (o - j) > max_pairs) slabs.emplace_back();
+            if (slabs.back().pairs + (o - j) > sp.triples) slabs.emplace_back();
             slabs.back().rows.push_back({i, j});
             slabs.back().pairs += o - j;
             maxp = std::max(maxp, slabs.back().pairs);
@@ -1633,13 +1627,20 @@ int hx_ccsd_triples(hx_ccsd *h, int32_t mol, double e[4])
             double *Wj = W + (long long)triples.size() * vvv;
             for (int t = 0; t < 12; ++t) {
                 TgemmDesc d = triples_term(t, m, I1, J, Wj, i, j);
-                d.a_keep = d.b_keep = 1;                 // t2 and the integrals stay: sliced once for all terms
+                d.a_keep = d.b_keep = sp.keep;           // t2 and the integrals stay: sliced once for all terms
                 plan[t].h.push_back(d);
             }
             for (int k = j; k < o; ++k) triples.push_back(make_int3(i, j, k));
         }
         tc::Engine *te = nullptr;
         rc = tc::create(&te, plan, h->st, 2, 2, 3);      // the 7-slice (emulated FP64) mode only, its short-K tile
+        if (rc == HX_ERR_NOMEM && sp.keep) {             // less memory than was free: from here on term by term
+            cudaGetLastError();
+            sp.keep = false;
+            for (auto &g : plan)
+                for (auto &d : g.h) d.a_keep = d.b_keep = 0;
+            rc = tc::create(&te, plan, h->st, 2, 2, 3);
+        }
         for (int t = 0; t < 12 && rc == HX_OK && ce == cudaSuccess; ++t)
             ce = tc::run_group(te, plan[t].h.data(), (int)plan[t].h.size(), nullptr, h->st, 3);
         if (rc == HX_OK && ce == cudaSuccess)
