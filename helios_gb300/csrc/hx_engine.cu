@@ -557,7 +557,10 @@ static int allocate(hx_ccsd *h)
             }
             m.Woo = A.take<double>((size_t)o * o * o * o);
             m.Vvv = mo_ladder(h, mi) ? A.take<double>((size_t)v * v * v * v) : nullptr;
-            m.Cint = A.take<double>(pr); m.Cp = A.take<double>(pr); m.Dint = A.take<double>(pr); m.X2 = A.take<double>(pr); m.Et = A.take<double>(pr);
+            m.Cint = A.take<double>(pr); m.Cp = A.take<double>(pr); m.Dint = A.take<double>(pr);
+            // (the last level's products: the ladder's intermediates are done with by then)
+            m.X2 = mo_ladder(h, mi) ? A.take<double>(pr) : m.Ts;
+            m.Et = mo_ladder(h, mi) ? A.take<double>(pr) : m.Z;
             m.Fvv2 = A.take<double>((size_t)v * v); m.Foo2 = A.take<double>((size_t)o * o);
             m.U = A.take<double>(ov * N); m.UG = A.take<double>(ov * N); m.Vs = A.take<double>((size_t)o * N);
             DiisMol &d = h->diis[mi];
@@ -751,6 +754,12 @@ int hx_ccsd_create_batch(const hx_ppp_model *ms, int32_t n, const hx_cc_params *
     }
     if (p->precision != HX_PRECISION_FP64) {
         rc = tc::create(&h->tce, h->plan, h->st, p->tile_tuning, p->tile_force, -1, kFp64Work);
+        if (rc == HX_ERR_NOMEM) {                // without slices kept over an iteration: each level makes its own
+            cudaGetLastError();
+            for (auto &g : h->plan)
+                for (auto &d : g.h) d.a_keep = d.b_keep = 0;
+            rc = tc::create(&h->tce, h->plan, h->st, p->tile_tuning, p->tile_force, -1, kFp64Work);
+        }
         if (rc < 0) { hx_ccsd_destroy(h); return rc; }
     }
     if (cudaStreamSynchronize(h->st) != cudaSuccess) { hx_set_error("set-up failed"); hx_ccsd_destroy(h); return HX_ERR_CUDA; }
