@@ -1005,6 +1005,11 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
                     }
                 }
             }
+            // no copy is in flight when the CTA leaves, after a wait that ran out either (pair: the even
+            // CTA's barriers count both CTAs' bytes, and the cluster barrier below holds the odd one)
+            if (rank == 0)
+                for (long long j = g > C::STAGES ? g - C::STAGES : 0; j < g; ++j)
+                    mbar_wait(&full[(int)(j % C::STAGES)], (uint32_t)((j / C::STAGES) & 1), nullptr, 0);
         }
     } else if (warp == WM) {
         if (lane == 0 && rank == 0) {
