@@ -17,8 +17,9 @@
 // MMA multiplies slice i of A by slices j = 0..J of B stacked along N into the
 // blocks q = i..i+J: one MMA per A slice instead of one per slice pair, which
 // divides the shared-memory operand reads (the kernel's bound) by about the
-// number of pairs per A slice. Every chunk of KC k-blocks the accumulators are
-// summed by TwoSum and added into an FP32 (hi, lo) pair per output, so the
+// number of pairs per A slice. Every chunk of KC k-blocks the exact accumulators are
+// summed by TwoSum and added into an FP32 (hi, lo) pair per output, the
+// others (rounded sums already, 2^-8NX of the value) into its low part, so the
 // result carries the accuracy of the splitting relative to the operands' row
 // maxima without the tensor core's accumulation error. (A drain in FP64 would
 // be exact too, but at GB300's FP64 rate it costs more than the MMAs.)
@@ -1359,7 +1360,9 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) tc_gemm(const TcDesc *__restri
 // tile (with the pipeline depth and epilogue warps that fit it); slices, slice
 // pairs and exact classes are the mode's own, so every candidate forms the
 // same sums (the pairs' chunks are longer: the classes from NX on, kept in
-// FP32, are summed over 480 to 960 k instead of 256 to 512). Narrow tiles waste less
+// FP32, are summed over 960 k in LOW and 320 in HIGH instead of 512 and 256; the
+// error against extended precision is the same to 1 % of its rms, K = 512 to
+// 51200, entries of both signs and of one). Narrow tiles waste less
 // on the thin operands of small molecules; wide ones reuse each A tile over
 // more columns. Four stages of 32 k hide the loads better than two of 64 where
 // K is long and cost more barriers where it is short (LOW 4800^3 1.51 -> 1.43

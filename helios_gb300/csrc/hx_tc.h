@@ -1,4 +1,4 @@
-// Tensor-core (tcgen05, BF16x3 split precision) backend of the grouped tensor-GEMM.
+// Tensor-core (tcgen05, exact BF16 slices) backend of the grouped tensor-GEMM.
 #pragma once
 #include <vector>
 #include "hx_plan.h"
@@ -8,7 +8,7 @@ struct Engine;
 // Build the backend for the GEMM groups of a plan (scratch sized to the largest
 // operand). Tile variants: force >= 0 takes candidate `force` of every mode;
 // otherwise tuning 0 looks each (mode, group, size class) up in the tile
-// table and takes the default on a miss, 1 times every candidate on a miss
+// table and goes by the level's size and depth on a miss (hx_tiles.h), 1 times every candidate on a miss
 // (and records the winner), 2 takes the defaults. only_mode >= 0 builds that
 // precision mode alone (the others have no groups to run). fp64_work: the
 // smallest problems of a group stay on the FP64 CUDA-core kernel while they

@@ -1,7 +1,8 @@
 """Measure the tensor-core tile table on this GPU: ``python -m helios_gb300.tune``.
 
-The exact-slice GEMM of every precision mode has a few candidate output tile
-widths (``api.tile_variants``) that form the same sums and differ in speed.
+The exact-slice GEMM of every precision mode has a few candidate output tiles
+(``api.tile_variants``) that form the same sums (the pairs of CTAs in longer chunks)
+and differ in speed.
 Which one is fastest depends on the contraction shapes: narrow tiles waste
 less on the thin operands of small molecules, wide ones reuse each operand
 tile over more columns. This script creates mixed-precision handles for the

@@ -110,9 +110,9 @@ typedef struct hx_cc_params {
                                      emulate FP64 (default), 1 = FP64 on the CUDA cores */
     int32_t tile_tuning;          /* mixed precision, tensor-core tile shapes per (precision
                                      mode, contraction group, size class): 0 = from the tile
-                                     table (hx_tile_table_load); where it has no entry, the
-                                     widest shape for the largest groups and the default
-                                     shape otherwise (default); 1 = the same, but a missing entry
+                                     table (hx_tile_table_load); where it has no entry, a wide
+                                     or deep shape for the largest groups of long K and the
+                                     default shape otherwise (default); 1 = the same, but a missing entry
                                      is found by timing every candidate on this handle's own
                                      contractions when it is created, and added to the table;
                                      2 = the default shapes */
